@@ -25,6 +25,8 @@ UNITS = [
     ("t3_noalloc.cu", "t3_noalloc", []),
     ("t3_table.cu", "t3_table", []),
     ("t3_prefill.cu", "t3_prefill", []),
+    ("t3_gemm.cu", "t3_gemm_cb0", ["-DT3_CB=0"]),
+    ("t3_gemm.cu", "t3_gemm_cb1", ["-DT3_CB=1"]),
     ("t3_api.cu", "t3_api", []),
     ("t3_dequant.cu", "t3_dequant", []),
     ("t3_decode_rows.cu", "t3_decode_rows_cb0", ["-DT3_CB=0"]),

@@ -1,0 +1,630 @@
+// The decode GEMM of the prefill rows: z = f16(xp W_hat) and the output rotation, with the trellis decoded into TENSOR MEMORY.
+//
+// The product is taken transposed: D [128 outputs x rows] = W_hat^T x xp^T. The weight tile is the MMA's A operand, read from
+// tensor memory, and the prepared rows are its B operand, K-major in shared memory as they lie in global memory. A lane's
+// decoded words of a 16x16 tile are the A fragment of the transposed tile (the pack's tensor-core order), which is the register
+// layout of tcgen05.st.16x128b: a tile goes to tensor memory in one instruction, with no swizzled shared-memory stores and no
+// proxy fence, and shared memory carries only the rows. The accumulator's columns are rows, so a tile is any multiple of 16
+// rows up to 256 and an expert of 80 rows costs five sixteenths of the MMA time of a 256-row one: nothing is padded to 128.
+//
+// What bounds it: a decoded 16x16 tile costs about 50 issued warp instructions whatever its rows, an MMA of 64 inputs x 128
+// outputs x R rows takes 2 R cycles, so up to about 200 rows a tile the decode's issue slots bound the kernel and past that the
+// tensor cores do. (An MMA that reads its A operand from tensor memory ran at the full rate from 128 columns on: 64 cycles at
+// 128, 128 at 256; with both operands in shared memory a 256-column one took 171.)
+//
+// One persistent CTA a multiprocessor, 27 warps by role (the rings run on across tiles, so nothing is set up per tile):
+//   warps 0-7    epilogue     warps 8-23  decode     24  codes: TMA into the code ring
+//   25  rows: TMA into the row ring     26  tcgen05.mma
+// A ring stage is 64 weight tiles (64 tensor-memory columns), one of two shapes chosen per tile of rows:
+//   wide   two 128-output blocks x 64 inputs, up to 128 rows: both blocks read one copy of the rows
+//   deep   one block x 128 inputs, up to 256 rows
+// A decode warp takes four tiles along K of a stage: waits, fences and arrivals are paid once a stage.
+//
+// Epilogue: the 128-point output rotation is a tensor-core product as well, D2 = H128 x z^T with H128 (+-1, f16) resident in
+// tensor memory: accumulators -> f16 z, transposed to shared memory by stmatrix -> MMA over the same columns -> scaled by svh,
+// rounded, transposed again and stored in 256-byte runs. (On the warps' mma.sync with butterflies a row cost four times the
+// instructions, and issue slots are what the decode needs.)
+//
+// Every wait is bounded: one that runs out sets a bit of the device error word and a flag that ends every other role's waits,
+// and the CTA walks to its exit, freeing its tensor memory on the way.
+#include <atomic>
+
+#include "t3_common.cuh"
+#include "t3_gemm.h"
+#include "t3_internal.h"
+#include "t3_tcgen05.cuh"
+
+#ifndef T3_CB
+#error "T3_CB: the codebook this unit is compiled for"
+#endif
+
+namespace t3 {
+namespace {
+
+constexpr uint32_t kEpiWarps = 8, kDecWarps = 16;
+constexpr uint32_t kCodeWarp = kEpiWarps + kDecWarps, kRowWarp = kCodeWarp + 1, kMmaWarp = kCodeWarp + 2;
+constexpr uint32_t kThreads = 32u * (kMmaWarp + 1u);
+constexpr uint32_t kStages = 3;            // operand stages in tensor memory
+constexpr uint32_t kCodeStages = 4;        // stages of the code ring
+constexpr uint32_t kStageTiles = 64;       // weight tiles a stage
+constexpr uint32_t kStageCols = 64;        // tensor-memory columns a stage (32 a 64 x 128 block)
+// tensor memory: accumulators in columns 0-255, operand stages in 256-447, H128 (128 x 128 f16) in 448-511
+constexpr uint32_t kTmemCols = 512, kTmemA = 256, kTmemH = 448;
+constexpr uint32_t kRowBytes = kGemmTileRows * 128u;   // a row slot: 64 inputs of up to 256 rows
+constexpr uint32_t kKeptBytes = 128u * 128u;           // 64 inputs of a kept weight's 128 outputs, behind the slot's rows
+constexpr uint32_t kZBytes = 2u * 128u * 128u;         // 128 rows x 128 outputs, f16, as two K-major halves; two of them
+
+constexpr uint32_t row_slots(uint32_t n) { return n != 0u && n <= 64u ? 4u : 3u; }  // what fits beside the code ring
+constexpr uint32_t smem_bytes(uint32_t n, uint32_t slots) {
+    return slots * kRowBytes + 2u * kZBytes + kCodeStages * kStageTiles * 2u * n + 512u + 1024u;
+}
+static_assert(smem_bytes(128, 3) <= 227u * 1024u && smem_bytes(64, 4) <= 227u * 1024u, "shared memory of a CTA");
+
+// one accumulator's worth of work: `blocks` 128-output blocks (2 in wide form) from block `blk` on, of one tile of rows
+struct Sub {
+    uint32_t e, first, rows, cols, op, blk, blocks;
+    uint32_t k0, k1;  // its range of 64-input steps
+    bool wide;
+};
+
+// the CTA's units in order; f(sub) returns false to stop
+template <typename F>
+__device__ __forceinline__ void for_each_sub(const DecodeGemmArgs& a, F&& f) {
+    const uint32_t ncol = a.N / 128u, per_op = (ncol + a.pair - 1u) / a.pair, per_tile = per_op * a.ops;
+    const uint32_t tiles = a.tiles ? *a.n_tiles : a.dense_tiles;
+    const uint32_t total = tiles * per_tile;
+    const bool sliced = a.ksplit > 1u;
+    for (uint32_t u = sliced ? blockIdx.y : blockIdx.x; u < total; u += sliced ? total : gridDim.x) {
+        const uint32_t t = u / per_tile, r = u - t * per_tile;
+        Sub s;
+        s.op = r / per_op;
+        const uint32_t b0 = (r - s.op * per_op) * a.pair, nb = min(a.pair, ncol - b0);
+        if (a.tiles) {
+            const int4 d = a.tiles[t];
+            s.e = (uint32_t)d.x, s.first = (uint32_t)d.y, s.rows = (uint32_t)d.z;
+        } else {
+            s.e = 0, s.first = t * a.tile_rows, s.rows = min(a.tile_rows, a.dense_rows - s.first);
+        }
+        s.cols = (s.rows + 15u) & ~15u;
+        s.wide = a.pair == 2u && s.cols <= 128u;
+        s.blocks = s.wide ? nb : 1u;
+        s.k0 = 0, s.k1 = a.K / 64u;
+        if (sliced) s.k0 = 2u * (a.K / 128u * blockIdx.x / a.ksplit), s.k1 = 2u * (a.K / 128u * (blockIdx.x + 1u) / a.ksplit);
+        for (uint32_t b = 0; b < nb; b += s.blocks) {
+            s.blk = b0 + b;
+            if (!f(s)) return;
+        }
+    }
+}
+
+// Waits for a barrier phase; false when the wait ran out, or once any wait of the CTA has (`dead` says so to all of them: from
+// then on no wait takes time, so every role still walks to the end of its work, on values nobody will use). NAP: nanoseconds
+// a warp sleeps between polls, for the roles whose waits are long and not urgent.
+constexpr uint32_t kTries = 1u << 22;
+template <uint32_t NAP = 0>
+__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, volatile uint32_t* dead, uint32_t* err, uint32_t bit) {
+    if (mbar_try(bar, parity)) return true;
+#pragma unroll 1
+    for (uint32_t i = 0; i < kTries; ++i) {
+        if (NAP) __nanosleep(NAP);
+        if (mbar_try(bar, parity)) return true;
+        if (*dead) return false;
+    }
+    *dead = 1u;
+    if (err) atomicOr(err, bit);
+    return false;
+}
+
+// a ring position and the parity of its round
+template <uint32_t SLOTS>
+struct Ring {
+    uint32_t slot = 0, parity = 0;
+    bool first_round = true;
+    __device__ __forceinline__ void next() {
+        if (++slot == SLOTS) slot = 0, parity ^= 1u, first_round = false;
+    }
+};
+
+// The decode warps' pass over one sub-tile's stages: a warp's four tiles lie a row of 8 tiles apart in the code stage.
+template <int NN, int CB>
+__device__ __forceinline__ void decode_stages(uint32_t stages, Ring<kCodeStages>& cring, Ring<kStages>& ring, uint32_t codes,
+                                              uint32_t stage_bytes, uint32_t n, uint32_t first_tile,
+                                              const LanePlan<(NN > 0 ? NN : 16)>& plan, uint32_t mask, uint32_t lane,
+                                              uint32_t tmem_dst, uint32_t full_c, uint32_t empty_c, uint32_t full_a,
+                                              uint32_t empty_a, volatile uint32_t* dead, uint32_t* err) {
+    constexpr int NP = NN > 0 ? NN : 16;
+    constexpr uint32_t kRaw = raw_words(NP);
+    const uint32_t tile_bytes = 2u * (NN > 0 ? (uint32_t)NN : n);
+    uint32_t at[kRaw];
+#pragma unroll
+    for (uint32_t j = 0; j < kRaw; ++j) at[j] = codes + first_tile * tile_bytes + plan.idx[j] * 4u;
+#pragma unroll 1
+    for (uint32_t k = 0; k < stages; ++k) {
+        const uint32_t s = ring.slot, cs = cring.slot;
+        wait_phase<20>(full_c + 8u * cs, cring.parity, dead, err, kErrFullWait);
+        uint32_t raw[4][kRaw];
+        if (NN > 0) {
+#pragma unroll
+            for (uint32_t j = 0; j < kRaw; ++j)
+#pragma unroll
+                for (uint32_t i = 0; i < 4u; ++i)
+                    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(raw[i][j]) : "r"(at[j] + cs * stage_bytes + i * 16u * (uint32_t)NP));
+        }
+        if (!ring.first_round) wait_phase<20>(empty_a + 8u * s, ring.parity ^ 1u, dead, err, kErrEmptyWait);
+        tc_fence_after();
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; ++i) {
+            uint32_t w[4];
+            if (NN > 0)
+                decode_raw<NP, CB>(raw[i], plan, mask, w);
+            else
+                decode_lane_any<CB>(static_cast<const uint32_t*>(__cvta_shared_to_generic(
+                                        codes + cs * stage_bytes + (first_tile + i * 8u) * tile_bytes)), n, lane, mask, w);
+            tmem_st_tile(tmem_dst + s * kStageCols + 8u * i, w);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        if (lane == 0) mbar_arrive_addr(full_a + 8u * s), mbar_arrive_addr(empty_c + 8u * cs);
+        ring.next(), cring.next();
+    }
+}
+
+// the stages of a sub-tile that a decode warp has no tiles in (the second block's warps when a wide unit has one block)
+__device__ __forceinline__ void skip_stages(uint32_t stages, Ring<kCodeStages>& cring, Ring<kStages>& ring, uint32_t lane, uint32_t empty_c,
+                                            uint32_t full_a, uint32_t empty_a, volatile uint32_t* dead, uint32_t* err) {
+    for (uint32_t k = 0; k < stages; ++k, ring.next(), cring.next()) {
+        if (!ring.first_round) wait_phase<20>(empty_a + 8u * ring.slot, ring.parity ^ 1u, dead, err, kErrEmptyWait);
+        __syncwarp();
+        if (lane == 0) mbar_arrive_addr(full_a + 8u * ring.slot), mbar_arrive_addr(empty_c + 8u * cring.slot);
+    }
+}
+
+// One 128-column part of a finished accumulator, warp (q, h)'s 16 outputs of it: rotated sums x scale, rounded to f16, then in
+// the output's dtype (PLAIN: rounded once). 16-bit results are transposed into the part's buffer (st_at: where this lane's
+// stmatrix row goes), f32 ones go to y, rows below `live`, at once (y at the part's first row and this lane's output g).
+template <bool PLAIN>
+__device__ __forceinline__ void finish_part(uint32_t taddr, uint32_t cols, float s0, float s1, int dt, uint32_t st_at, float* y,
+                                            size_t N, uint32_t live, uint32_t t) {
+#pragma unroll
+    for (uint32_t r = 0; r < 128u; r += 64u) {
+        if (r >= cols) break;
+        uint32_t v[32];
+        tmem_ld_16x64(taddr + r, v);
+#pragma unroll
+        for (uint32_t p = 0; p < 4u; ++p) {
+            float f[8];
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; ++j) {
+                f[j] = __uint_as_float(v[8u * p + j]);
+                if (!PLAIN) f[j] *= (j & 2u) ? s1 : s0;
+            }
+            if (dt == (int)kF32) {
+#pragma unroll
+                for (uint32_t j = 0; j < 8u; ++j) {
+                    const uint32_t row = r + 16u * p + (j >> 2) * 8u + 2u * t + (j & 1u);
+                    if (row < live) y[row * N + ((j & 2u) ? 8u : 0u)] = round_half(f[j]);
+                }
+            } else if (r + 16u * p < cols) {
+                uint32_t w[4];
+#pragma unroll
+                for (uint32_t j = 0; j < 4u; ++j) {
+                    float2 u = make_float2(f[2u * j], f[2u * j + 1u]);
+                    w[j] = pack_half2(u.x, u.y);
+                    if (dt == (int)kBf16) {
+                        if (!PLAIN) u = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+                        const __nv_bfloat162 o = __floats2bfloat162_rn(u.x, u.y);
+                        w[j] = *reinterpret_cast<const uint32_t*>(&o);
+                    }
+                }
+                stmatrix4_trans(st_at + (r + 16u * p) * 128u, w[0], w[1], w[2], w[3]);
+            }
+        }
+    }
+}
+
+// A part's 16-bit rows from its buffer to y, 256 bytes a row (`warp` of the epilogue's eight)
+__device__ __forceinline__ void store_part(uint32_t buffer, uint16_t* y, size_t N, uint32_t rows, uint32_t warp, uint32_t lane) {
+    const uint32_t j = lane & 15u;
+#pragma unroll 4
+    for (uint32_t r = 2u * warp + (lane >> 4); r < rows; r += 2u * kEpiWarps) {
+        uint4 w;
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
+                     : "r"(buffer + (j >> 3) * 16384u + r * 128u + (((j & 7u) ^ (r & 7u)) << 4)));
+        *reinterpret_cast<uint4*>(y + r * N + 8u * j) = w;
+    }
+}
+
+// The output rotation of a part on the tensor cores (one thread): D2 = H128 x z^T over the part's accumulator columns
+__device__ __forceinline__ void rotate_part(uint32_t tmem, uint32_t z_s, uint32_t c, uint32_t idesc, uint32_t rot_full) {
+    const uint32_t hi = (uint32_t)(umma_desc(0) >> 32), lo = (uint32_t)umma_desc(z_s + c * kZBytes);
+#pragma unroll
+    for (uint32_t kk = 0; kk < 8u; ++kk)
+        umma_f16_ts(tmem + 128u * c, tmem + kTmemH + 8u * kk, lo + (((kk >> 2) * 16384u + (kk & 3u) * 32u) >> 4), hi, kk != 0u, idesc);
+    umma_commit(rot_full + 8u * c);
+}
+
+// KEPT: the weight is a kept W_hat (or W_std), [N, K] 16-bit, loaded by TMA beside the rows as a shared-memory operand: the
+// same products in the same order, nothing decoded.
+template <int NN, int CB, bool KEPT = false>
+__global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_constant__ GemmMaps maps, const DecodeGemmArgs a) {
+    constexpr uint32_t kSlots = KEPT ? 3u : row_slots(NN), kSlotBytes = KEPT ? kRowBytes + kKeptBytes : kRowBytes;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem = (smem_addr(smem_raw) + 1023u) & ~1023u;
+    const uint32_t n = NN > 0 ? (uint32_t)NN : (KEPT ? 0u : a.n), tile_bytes = 2u * n, stage_bytes = kStageTiles * tile_bytes;
+    const uint32_t z_s = smem + kSlots * kSlotBytes, codes = z_s + 2u * kZBytes;
+    const uint32_t bars = codes + kCodeStages * stage_bytes;
+    const uint32_t full_c = bars, empty_c = full_c + 8u * kCodeStages, full_a = empty_c + 8u * kCodeStages;
+    const uint32_t empty_a = full_a + 8u * kStages, full_b = empty_a + 8u * kStages, empty_b = full_b + 8u * 4u;
+    const uint32_t acc_full = empty_b + 8u * 4u, acc_free = acc_full + 8u;
+    // z_full, rot_full: a pair each, one barrier a 128-column part (the epilogue and the MMA warp run both parts ahead)
+    const uint32_t z_full = acc_full + 16u, rot_full = acc_full + 32u;
+    uint8_t* generic = smem_raw + (smem - smem_addr(smem_raw));
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(generic + (acc_full + 48u - smem));
+    volatile uint32_t* dead = tmem_slot + 1;
+
+    const uint32_t tid = threadIdx.x, lane = tid & 31u;
+    // the warp's number as a value the compiler knows to be the same in every lane: the roles' loops then run on uniform registers
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
+    if (tid == 0) {
+        auto init = [&](uint32_t bar, uint32_t count) { mbar_init(reinterpret_cast<uint64_t*>(generic + (bar - smem)), count); };
+        for (uint32_t s = 0; s < kCodeStages; ++s) init(full_c + 8u * s, 1u), init(empty_c + 8u * s, kDecWarps);
+        for (uint32_t s = 0; s < kStages; ++s) init(full_a + 8u * s, kDecWarps), init(empty_a + 8u * s, 1u);
+        for (uint32_t s = 0; s < kSlots; ++s) init(full_b + 8u * s, 1u), init(empty_b + 8u * s, 1u);
+        init(acc_full, 1u), init(acc_free, kEpiWarps);
+        for (uint32_t c = 0; c < 2u; ++c) init(z_full + 8u * c, kEpiWarps), init(rot_full + 8u * c, 1u);
+        *dead = 0u;
+        mbar_init_fence();
+    }
+    if (warp == kMmaWarp) tmem_alloc(tmem_slot, kTmemCols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
+    const bool sliced = a.ksplit > 1u;
+    // H128 as an A operand in tensor memory: element (i, j) has the sign of popcount(i & j)
+    if (warp >= kEpiWarps && warp < kEpiWarps + 8u) {
+        const uint32_t i = 32u * (warp & 3u) + 16u * ((warp >> 2) & 1u) + (lane >> 2), j0 = 2u * (lane & 3u);
+        auto pair = [](uint32_t r, uint32_t c) {
+            return ((__popc(r & c) & 1) ? 0xBC00u : 0x3C00u) | ((__popc(r & (c + 1u)) & 1) ? 0xBC000000u : 0x3C000000u);
+        };
+        for (uint32_t kk = 0; kk < 8u; ++kk) {
+            const uint32_t j = 16u * kk + j0;
+            const uint32_t w[4] = {pair(i, j), pair(i, j + 8u), pair(i + 8u, j), pair(i + 8u, j + 8u)};
+            tmem_st_tile(tmem + kTmemH + 8u * kk + ((i & ~7u) << 16), w);
+        }
+        tmem_st_wait();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+
+    if (warp >= kEpiWarps && warp < kCodeWarp) {
+        // ---- decode: quarter q of the lanes (32 outputs a block), tile column 2q + half of a block; part: the block (wide) or
+        // the 64-input half of the stage (deep)
+        const uint32_t q = warp & 3u, half = ((warp - kEpiWarps) >> 2) & 1u, part = (warp - kEpiWarps) >> 3;
+        LanePlan<(NN > 0 ? NN : 16)> plan;
+        plan.init(lane);
+        const uint32_t dst = tmem + kTmemA + part * 32u + ((32u * q + 16u * half) << 16);
+        const uint32_t col = 2u * q + half;
+        Ring<kCodeStages> cring;
+        Ring<kStages> ring;
+        if (!KEPT) for_each_sub(a, [&](const Sub& s) {
+            const uint32_t k64 = s.k1 - s.k0;
+            if (s.wide && s.blocks == 1u && part == 1u)
+                skip_stages(k64, cring, ring, lane, empty_c, full_a, empty_a, dead, a.err);
+            else
+                decode_stages<NN, CB>(s.wide ? k64 : k64 / 2u, cring, ring, codes, stage_bytes, n, part * 32u + col, plan, a.mask, lane,
+                                      dst, full_c, empty_c, full_a, empty_a, dead, a.err);
+            return true;
+        });
+    } else if (warp == kCodeWarp) {
+        // ---- code ring: a stage is two boxes of 4 tile rows x 8 tiles, the unit's two blocks (wide) or two runs of 64 inputs
+        // (deep). A slot is free again when every decode warp has decoded it.
+        Ring<kCodeStages> ring;
+        if (!KEPT) for_each_sub(a, [&](const Sub& s) {
+            const CUtensorMap* map = &maps.codes[s.op];
+            const uint32_t words = n * 2u, box = 4u * 8u * tile_bytes;  // 64-bit words of a row of 8 tiles
+            const bool two = !s.wide || s.blocks == 2u;
+            const int x0 = (int)(s.blk * words), x1 = x0 + (s.wide ? (int)words : 0), e = (int)s.e, dy = s.wide ? 0 : 4;
+            for (uint32_t k = 4u * s.k0; k < 4u * s.k1; k += s.wide ? 4u : 8u, ring.next()) {
+                const uint32_t bar = full_c + 8u * ring.slot, dst = codes + ring.slot * stage_bytes;
+                if (!ring.first_round && !wait_phase<150>(empty_c + 8u * ring.slot, ring.parity ^ 1u, dead, a.err, kErrEmptyWait)) return false;
+                __syncwarp();
+                if (elect_one()) {
+                    mbar_arrive_expect_tx_addr(bar, two ? 2u * box : box);
+                    tma_load_3d(dst, map, x0, (int)k, e, bar);
+                    if (two) tma_load_3d(dst + box, map, x1, (int)k + dy, e, bar);
+                }
+            }
+            return true;
+        });
+    } else if (warp == kRowWarp) {
+        // ---- row ring: 64 inputs of the tile's rows a slot
+        Ring<kSlots> ring;
+        for_each_sub(a, [&](const Sub& s) {
+            const int row0 = (int)(s.op * a.op_rows + s.first);
+            // one box, or one and a half-sized one
+            const uint32_t load = tiled_rows(s.cols), big = load == 192u ? 128u : load == 96u ? 64u : load;
+            const CUtensorMap* map = &maps.rows[big == 256u ? 0 : big == 128u ? 1 : big == 64u ? 2 : 3];
+            for (uint32_t k = s.k0; k < s.k1; ++k, ring.next()) {
+                const uint32_t bar = full_b + 8u * ring.slot, dst = smem + ring.slot * kSlotBytes;
+                if (!ring.first_round && !wait_phase<32>(empty_b + 8u * ring.slot, ring.parity ^ 1u, dead, a.err, kErrEmptyWait)) return false;
+                __syncwarp();
+                if (elect_one()) {
+                    mbar_arrive_expect_tx_addr(bar, load * 128u + (KEPT ? kKeptBytes : 0u));
+                    if (KEPT) tma_load_2d(dst + kRowBytes, &maps.codes[0], (int)(k * 64u), (int)(s.blk * 128u), bar);
+                    tma_load_2d(dst, map, (int)(k * 64u), row0, bar);
+                    if (load != big) tma_load_2d(dst + big * 128u, map + 1, (int)(k * 64u), row0 + (int)big, bar);
+                }
+            }
+            return true;
+        });
+    } else if (warp == kMmaWarp) {
+        // ---- MMA: the whole warp walks the rings, one elected lane issues (see elect_one)
+        uint32_t subs = 0, rots[2] = {0, 0};
+        Ring<kStages> ring_a;
+        Ring<kSlots> ring_b;
+        auto wait = [&](uint32_t bar, uint32_t parity, uint32_t bit) {
+            wait_phase(bar, parity, dead, a.err, bit);
+            tc_fence_after();
+            __syncwarp();
+        };
+        const uint32_t desc_hi = (uint32_t)(umma_desc(0) >> 32), desc0 = (uint32_t)umma_desc(smem);
+        for_each_sub(a, [&](const Sub& s) {
+            if (subs > 0u) wait(acc_free, (subs - 1u) & 1u, kErrMmaWait);
+            ++subs;
+            const uint32_t idesc = idesc_m128(s.cols) | (KEPT && a.bf16 ? kIdescBf16 : 0u), k64 = s.k1 - s.k0;
+            uint32_t acc = 0;
+            // four steps of 16 inputs on one row slot against one 64-input operand block (a second block's into its accumulator)
+            auto steps = [&](uint32_t a_col, bool both) {
+                const uint32_t lo = desc0 + ring_b.slot * (kSlotBytes >> 4);
+#pragma unroll
+                for (uint32_t kk = 0; kk < 4u; ++kk) {
+                    if (KEPT) {
+                        const uint64_t hi = (uint64_t)desc_hi << 32;
+                        umma_f16(tmem, hi | (lo + (kRowBytes >> 4) + kk * 2u), hi | (lo + kk * 2u), kk ? 1u : acc, idesc);
+                        continue;
+                    }
+                    umma_f16_ts(tmem, a_col + kk * 8u, lo + kk * 2u, desc_hi, kk ? 1u : acc, idesc);
+                    if (both) umma_f16_ts(tmem + 128u, a_col + 32u + kk * 8u, lo + kk * 2u, desc_hi, kk ? 1u : acc, idesc);
+                }
+                umma_commit(empty_b + 8u * ring_b.slot);
+            };
+            const uint32_t stages = s.wide ? k64 : k64 / 2u;
+#pragma unroll 1
+            for (uint32_t k = 0; k < stages; ++k, ring_a.next()) {
+                const uint32_t a_col = tmem + kTmemA + ring_a.slot * kStageCols;
+                wait(full_b + 8u * ring_b.slot, ring_b.parity, kErrFullWait);
+                if (!KEPT) wait(full_a + 8u * ring_a.slot, ring_a.parity, kErrFullWait);
+                if (s.wide) {
+                    if (elect_one()) {
+                        if (s.blocks == 2u) steps(a_col, true);
+                        else steps(a_col, false);
+                        umma_commit(empty_a + 8u * ring_a.slot);
+                    }
+                } else {
+                    if (elect_one()) steps(a_col, false);
+                    acc = 1u;
+                    ring_b.next();
+                    wait(full_b + 8u * ring_b.slot, ring_b.parity, kErrFullWait);
+                    if (elect_one()) {
+                        steps(a_col + 32u, false);
+                        if (!KEPT) umma_commit(empty_a + 8u * ring_a.slot);
+                    }
+                }
+                acc = 1u;
+                ring_b.next();
+            }
+            if (elect_one()) umma_commit(acc_full);
+            if (sliced || a.svh[0] == nullptr) return true;
+            // the output rotation, 128 accumulator columns at a time
+            const uint32_t parts = s.wide ? s.blocks : (s.cols > 128u ? 2u : 1u);
+#pragma unroll
+            for (uint32_t c = 0; c < 2u; ++c) {
+                if (c >= parts) break;
+                wait(z_full + 8u * c, rots[c]++ & 1u, kErrMmaWait);
+                const uint32_t rdesc = idesc_m128(s.wide ? s.cols : min(128u, s.cols - 128u * c));
+                if (elect_one()) rotate_part(tmem, z_s, c, rdesc, rot_full);
+            }
+            return true;
+        });
+    } else {
+        // ---- epilogue, warp (q, h): tensor-memory lanes (outputs) 32 q + 16 h .. + 15
+        const uint32_t q = warp & 3u, h = warp >> 2, g = lane >> 2, t = lane & 3u;
+        // where this lane's stmatrix row goes: row 8 (m >> 1) + i of 16, outputs 32 q + 16 h + 8 (m & 1) ..
+        const uint32_t m = lane >> 3, i8 = lane & 7u;
+        const uint32_t st_at = z_s + (q >> 1) * 16384u + ((m >> 1) * 8u + i8) * 128u + ((((q & 1u) * 4u + h * 2u + (m & 1u)) ^ i8) << 4);
+        const uint32_t my_lanes = tmem + ((32u * q + 16u * h) << 16);
+        const int dt = a.y ? a.y_dt : (int)kF16;
+        const bool plain = KEPT && a.svh[0] == nullptr;
+        uint16_t* const y16 = a.y ? static_cast<uint16_t*>(a.y) : reinterpret_cast<uint16_t*>(a.z);
+        uint32_t subs = 0, rots[2] = {0, 0};
+        auto arrive = [&](uint32_t bar) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive_addr(bar);
+        };
+        // one warp polls, the others wait at the named barrier, where they issue nothing (every wait ends, so all eight get there)
+        auto meet = [&]() { named_sync(1, 32u * kEpiWarps); };
+        auto await = [&](uint32_t bar, uint32_t parity) {
+            if (warp == 0) wait_phase<32>(bar, parity, dead, a.err, kErrMmaWait);
+            meet();
+            tc_fence_after();
+        };
+        for_each_sub(a, [&](const Sub& s) {
+            float sc[2][2] = {};  // the scales of outputs g and g + 8 of this warp's 16, per block
+            if (!plain) {
+                const __half* svh = (s.op ? a.svh[1] : a.svh[0]) + (size_t)s.e * a.svh_stride + s.blk * 128u + 32u * q + 16u * h + g;
+#pragma unroll
+                for (uint32_t b = 0; b < 2u; ++b)
+#pragma unroll
+                    for (uint32_t j = 0; j < 2u; ++j)
+                        if (b < s.blocks) sc[b][j] = kHadScale * __half2float(svh[b * 128u + 8u * j]);
+            }
+            await(acc_full, subs++ & 1u);
+            const uint32_t parts = s.wide ? s.blocks : (s.cols > 128u ? 2u : 1u);
+            auto part_cols = [&](uint32_t c) { return s.wide ? s.cols : min(128u, s.cols - 128u * c); };
+            if (sliced) {  // this slice's sums to its place in the slab
+                float* slab = a.part + (((size_t)s.blk * a.ksplit + blockIdx.x) * a.dense_rows + s.first) * 128u + 32u * q + 16u * h + g;
+                for (uint32_t r = 0; r < s.cols; r += 64u) {
+                    uint32_t v[32];
+                    tmem_ld_16x64(my_lanes + r, v);
+#pragma unroll
+                    for (uint32_t j = 0; j < 32u; ++j) {
+                        const uint32_t row = r + (j >> 2) * 8u + 2u * t + (j & 1u);
+                        if (row < s.rows) __stcg(slab + (size_t)row * 128u + ((j & 2u) ? 8u : 0u), __uint_as_float(v[j]));
+                    }
+                }
+                return true;
+            }
+            for (uint32_t c = 0; c < parts && !plain; ++c) {
+                const uint32_t cols = part_cols(c);
+#pragma unroll
+                for (uint32_t r = 0; r < 128u; r += 64u) {
+                    if (r >= cols) break;
+                    uint32_t v[32];
+                    tmem_ld_16x64(my_lanes + 128u * c + r, v);
+#pragma unroll
+                    for (uint32_t p = 0; p < 4u; ++p) {
+                        auto pk = [&](uint32_t j) { return pack_half2(__uint_as_float(v[8u * p + j]), __uint_as_float(v[8u * p + j + 1u])); };
+                        if (r + 16u * p < cols) stmatrix4_trans(st_at + c * kZBytes + (r + 16u * p) * 128u, pk(0), pk(2), pk(4), pk(6));
+                    }
+                }
+                proxy_fence();
+                tc_fence_before();
+                arrive(z_full + 8u * c);
+            }
+#pragma unroll
+            for (uint32_t c = 0; c < 2u; ++c) {
+                if (c >= parts) break;
+                if (!plain) await(rot_full + 8u * c, rots[c]++ & 1u);
+                const uint32_t blk = s.blk + (s.wide ? c : 0u), row0 = s.wide ? 0u : 128u * c;
+                const bool second = s.wide && c == 1u;
+                const float s0 = second ? sc[1][0] : sc[0][0], s1 = second ? sc[1][1] : sc[0][1];
+                float* y32 = static_cast<float*>(a.y) + (size_t)(s.first + row0) * a.N + blk * 128u + 32u * q + 16u * h + g;
+                if (plain)
+                    finish_part<true>(my_lanes + 128u * c, part_cols(c), s0, s1, dt, st_at + c * kZBytes, y32, a.N, s.rows - row0, t);
+                else
+                    finish_part<false>(my_lanes + 128u * c, part_cols(c), s0, s1, dt, st_at + c * kZBytes, y32, a.N, s.rows - row0, t);
+            }
+            // the accumulators are read: the next tile may start
+            tc_fence_before();
+            arrive(acc_free);
+            if (dt == (int)kF32) return true;
+            meet();
+            for (uint32_t c = 0; c < parts; ++c) {
+                const uint32_t row0 = s.wide ? 0u : 128u * c;
+                store_part(z_s + c * kZBytes, y16 + s.op * a.z_op_stride + (size_t)(s.first + row0) * a.N + (s.blk + (s.wide ? c : 0u)) * 128u,
+                           a.N, min(part_cols(c), s.rows - row0), warp, lane);
+            }
+            meet();  // the buffers are read: the next tile's values may overwrite them
+            return true;
+        });
+    }
+    if (sliced) {
+        // The slices of a unit meet: every CTA of the cluster has left its sums in the slab once the cluster's barrier is passed;
+        // CTA z then adds the slices, in slice order, of its share of the rows and finishes those.
+        tc_fence_before();
+        __threadfence();
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        __syncthreads();
+        tc_fence_after();
+        Sub s = {};
+        for_each_sub(a, [&](const Sub& mine) { s = mine; return true; });
+        const uint32_t per = (s.rows + a.ksplit - 1u) / a.ksplit, lo = min(per * blockIdx.x, s.rows), live = min(per, s.rows - lo);
+        const float4* slab = reinterpret_cast<const float4*>(a.part) + ((size_t)s.blk * a.ksplit * a.dense_rows + s.first + lo) * 32u;
+        const size_t next = (size_t)a.dense_rows * 32u;
+        for (uint32_t i = tid; i < live * 32u; i += kThreads) {
+            float4 p[8];
+#pragma unroll
+            for (uint32_t z = 0; z < 8u; ++z)
+                if (z < a.ksplit) p[z] = __ldcg(slab + z * next + i);
+            float4 sum = p[0];
+#pragma unroll
+            for (uint32_t z = 1; z < 8u; ++z)
+                if (z < a.ksplit) sum.x += p[z].x, sum.y += p[z].y, sum.z += p[z].z, sum.w += p[z].w;
+            const uint32_t r = i >> 5, o = 4u * (i & 31u);
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(z_s + (o >> 6) * 16384u + r * 128u + ((((o & 63u) >> 3) ^ (r & 7u)) << 4) +
+                                                                   (o & 7u) * 2u),
+                         "r"(pack_half2(sum.x, sum.y)), "r"(pack_half2(sum.z, sum.w))
+                         : "memory");
+        }
+        proxy_fence();
+        __syncthreads();
+        const uint32_t cols = (live + 15u) & ~15u;
+        if (live > 0u) {
+            if (warp == kMmaWarp) {
+                if (elect_one()) rotate_part(tmem, z_s, 0, idesc_m128(cols), rot_full);
+            } else if (warp < kEpiWarps) {
+                const uint32_t q = warp & 3u, h = warp >> 2, g = lane >> 2, t = lane & 3u, m = lane >> 3, i8 = lane & 7u;
+                const uint32_t st_at = z_s + (q >> 1) * 16384u + ((m >> 1) * 8u + i8) * 128u + ((((q & 1u) * 4u + h * 2u + (m & 1u)) ^ i8) << 4);
+                const uint32_t o = 32u * q + 16u * h + g;
+                const size_t out0 = (size_t)(s.first + lo) * a.N + s.blk * 128u;
+                const __half* svh = a.svh[0] + s.blk * 128u + o;
+                const float s0 = kHadScale * __half2float(svh[0]), s1 = kHadScale * __half2float(svh[8]);
+                wait_phase(rot_full, 0u, dead, a.err, kErrMmaWait);
+                __syncwarp();
+                tc_fence_after();
+                finish_part<false>(tmem + ((32u * q + 16u * h) << 16), cols, s0, s1, a.y_dt, st_at, static_cast<float*>(a.y) + out0 + o, a.N,
+                                   live, t);
+                if (a.y_dt != (int)kF32) {
+                    named_sync(1, 32u * kEpiWarps);
+                    store_part(z_s, static_cast<uint16_t*>(a.y) + out0, a.N, live, warp, lane);
+                }
+            }
+        }
+    }
+    // a CTA that gave up lets the copies in flight land before its shared memory goes away
+    if (*dead)
+        for (uint32_t i = 0; i < 1000u; ++i) __nanosleep(1000);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        tc_fence_after();
+        tmem_dealloc(tmem, kTmemCols);
+    }
+}
+
+template <int NN, int CB, bool KEPT = false>
+cudaError_t launch_one(const GemmMaps& maps, const DecodeGemmArgs& a, uint32_t units, uint32_t sms, cudaStream_t stream) {
+    void (*const fn)(const GemmMaps, const DecodeGemmArgs) = decode_gemm_kernel<NN, CB, KEPT>;
+    auto bytes = [](uint32_t n) { return KEPT ? smem_bytes(0, 3) + 3u * kKeptBytes : smem_bytes(n, row_slots(NN)); };
+    static std::atomic<uint64_t> ready{0};  // devices (by ordinal) on which the kernel may use its shared memory
+    const cudaError_t rc = allow_smem_once(ready, reinterpret_cast<const void*>(fn), bytes(NN > 0 ? NN : 128));
+    if (rc != cudaSuccess) return rc;
+    if (a.ksplit <= 1u) {
+        fn<<<units < sms ? units : sms, kThreads, bytes(a.n), stream>>>(maps, a);
+        return cudaGetLastError();
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.ksplit, units, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = bytes(a.n);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = a.ksplit;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, maps, a);
+}
+
+}  // namespace
+
+#define T3_GEMM_NAME2(cb) launch_decode_gemm_cb##cb
+#define T3_GEMM_NAME(cb) T3_GEMM_NAME2(cb)
+cudaError_t T3_GEMM_NAME(T3_CB)(const GemmMaps& maps, const DecodeGemmArgs& a, uint32_t units, uint32_t sms, cudaStream_t stream) {
+#if T3_CB == 0
+    if (a.kept) return launch_one<0, 0, true>(maps, a, units, sms, stream);
+#endif
+    switch (a.n) {
+#define T3_CASE(NN) \
+    case NN: return launch_one<NN, T3_CB>(maps, a, units, sms, stream);
+        T3_CASE(16) T3_CASE(32) T3_CASE(48) T3_CASE(64) T3_CASE(80) T3_CASE(96) T3_CASE(112) T3_CASE(128)
+#undef T3_CASE
+        default: return launch_one<0, T3_CB>(maps, a, units, sms, stream);
+    }
+}
+
+}  // namespace t3

@@ -1,6 +1,8 @@
 // Host-side declarations shared by the library's translation units (not part of the public C ABI).
 #pragma once
 
+#include <atomic>
+
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -70,6 +72,19 @@ struct MoeArgs {
     int overlap;
     uint32_t* err;
 };
+
+// Raises a kernel's dynamic shared-memory limit on the current device, once a device (`ready`: a bit an ordinal, one word a
+// kernel): the driver call costs more than the check.
+inline cudaError_t allow_smem_once(std::atomic<uint64_t>& ready, const void* kernel, uint32_t bytes) {
+    int dev = 0;
+    cudaError_t rc = cudaGetDevice(&dev);
+    if (rc != cudaSuccess) return rc;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;
+    if (ready.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (rc == cudaSuccess) ready.fetch_or(bit, std::memory_order_release);
+    return rc;
+}
 
 // remembers, per host thread, the kernel a decode-row launch is about to run (t3_last_kernel_symbol names it)
 void note_symbol(const void* kernel);
