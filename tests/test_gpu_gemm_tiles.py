@@ -1,0 +1,48 @@
+"""The decode GEMM of the prefill rows at the sizes where its tiles can go wrong: tiles of every loaded height (32, 64, 96, 128,
+192, 256 rows) with one row more and one less, both stage shapes (two blocks up to 128 rows, one block past that), an odd number
+of 128-output blocks, the smallest K, and the two operand rings at the extreme rates."""
+import numpy as np
+import pytest
+import torch
+
+import turboexl3_b200 as t3
+from oracle import binding as ob
+from turboexl3_b200 import synth
+
+from gpu_util import TORCH_DT, check, dev, host_f32, x_as
+from test_gpu_moe import check_moe, make_bank
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("case", [(128, 128, 16, t3.MUL1, "f16"), (256, 384, 128, t3.MCG, "f32"), (384, 256, 36, t3.MUL1, "bf16")])
+def test_dense_tile_edges(case):
+    in_dim, out_dim, n, cb, dt = case
+    trellis, suh, svh = synth.linear(2100 + n, in_dim, out_dim, n, scaled=True)
+    what = ob.reconstruct_inner(trellis, in_dim, out_dim, n, cb, 16)
+    t, a, b = dev(trellis), dev(suh), dev(svh)
+    for rows in (33, 48, 63, 65, 97, 127, 129, 191, 193, 255, 256, 513, 1100):
+        x = x_as(synth.activations(2101 + rows, rows, in_dim), dt)
+        y = t3.linear(x, t, a, b, t3.Decode(cb, 16))
+        sample = sorted({0, 1, 15, 16, 31, 32, rows // 2, rows - 17, rows - 1})
+        ref = ob.linear_rows_what(host_f32(x)[sample], what, suh, svh, in_dim, out_dim)
+        check(host_f32(y)[sample], ref, dt, ("tile edges", case, rows))
+    assert t3.device_error() == 0
+
+
+@pytest.mark.parametrize("case", [(384, 128, 48, t3.MUL1, "f16"), (256, 384, 128, t3.MCG, "f32"), (128, 256, 20, t3.MUL1, "bf16")])
+def test_routed_tile_edges(case):
+    """One expert for each height around the edges; every row goes to one expert at weight 1."""
+    hidden, inter, n, cb, dt = case
+    heights = [1, 15, 16, 17, 32, 33, 64, 65, 96, 97, 128, 129, 192, 193, 256, 257, 513]
+    bank, obank = make_bank(2200 + n, len(heights) + 1, hidden, inter, n)  # the last expert gets no row
+    inds = np.repeat(np.arange(len(heights)), heights).astype(np.int32)
+    np.random.default_rng(7).shuffle(inds)
+    rows = inds.size
+    x = x_as(synth.activations(2201 + n, rows, hidden), dt)
+    y = t3.moe(x.view(1, rows, hidden), bank, dev(inds).view(1, rows, 1), torch.ones((1, rows, 1), device="cuda"), t3.Decode(cb, 16))
+    assert y.dtype == TORCH_DT[dt]
+    sample = sorted(int(r) for e in range(len(heights)) for r in np.flatnonzero(inds == e)[[0, -1]])
+    ref = ob.moe_rows(obank, host_f32(x)[sample], inds[sample].reshape(-1, 1), np.ones((len(sample), 1), np.float32), cb, 16, 0.0, 0)
+    check_moe(host_f32(y).reshape(rows, hidden)[sample], ref, dt, ("routed tile edges", case))
+    assert t3.device_error() == 0
