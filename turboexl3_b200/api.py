@@ -124,6 +124,22 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_call = None
+
+
+def native():
+    """The binding of the hot calls (_call.so over libt3.so), loaded once. Raises when it has not been built."""
+    global _call
+    if _call is None:
+        lib()
+        try:
+            from . import _call as built
+        except ImportError as exc:
+            raise RuntimeError(f"{_HERE}/_call.so cannot be loaded ({exc}): build it with `python -m turboexl3_b200.build`") from exc
+        _call = built
+    return _call
+
+
 def status_name(status: int) -> str:
     return lib().t3_status_name(status).decode()
 
@@ -273,25 +289,22 @@ def dequantize(trellis: torch.Tensor, dec: Decode = Decode.mul1) -> torch.Tensor
 def linear(x: torch.Tensor, trellis: torch.Tensor, suh: torch.Tensor, svh: torch.Tensor,
            dec: Decode = Decode.mul1) -> torch.Tensor:
     """root.linear (src/root.zig:309-351): y [..., out] in x's dtype for x [..., in]."""
+    y = (_call or native()).linear(x, trellis, suh, svh, dec)
+    return y if y.__class__ is torch.Tensor else _refuse_linear(y, x, trellis, suh, svh)
+
+
+def _refuse_linear(status, x, trellis, suh, svh):
+    """Names why a linear did not run: a status of the engine, or the argument the binding would not take."""
+    if status is not None:
+        _check(status)
     _need_cuda(x, trellis, suh, svh)
     if x.dim() < 1 or trellis.dim() != 3:
         raise Exl3Error(1, "BadExl3Shape")
-    in_dim, out_dim, n = trellis.shape[0] * 16, trellis.shape[1] * 16, trellis.shape[2]
-    if x.shape[-1] != in_dim or suh.numel() != in_dim or svh.numel() != out_dim:
+    if x.shape[-1] != trellis.shape[0] * 16 or suh.numel() != trellis.shape[0] * 16 or svh.numel() != trellis.shape[1] * 16:
         raise Exl3Error(1, "BadExl3Shape")
     if x.dtype not in _DTYPES or not _trellis_ok(trellis) or suh.dtype != torch.float16 or svh.dtype != torch.float16:
         raise Exl3Error(2, "BadExl3Dtype")
-    rows = x.numel() // in_dim
-    if rows < 1:
-        raise Exl3Error(1, "BadExl3Shape")
-    y = torch.empty(x.shape[:-1] + (out_dim,), dtype=x.dtype, device=x.device)
-    L = lib()
-    ws_bytes = L.t3_linear_workspace_bytes(rows, in_dim, out_dim, n)
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device) if ws_bytes else None
-    _check(L.t3_linear(x.data_ptr(), _DTYPES[x.dtype], rows, trellis.data_ptr(), suh.data_ptr(), svh.data_ptr(),
-                       in_dim, out_dim, n, dec._c(), y.data_ptr(), ws.data_ptr() if ws is not None else None,
-                       ws_bytes, _stream_ptr(x)))
-    return y
+    raise Exl3Error(1, "BadExl3Shape")
 
 
 def resident_build(trellis: torch.Tensor, dec: Decode = Decode.mul1) -> torch.Tensor:
@@ -352,7 +365,17 @@ def _bank_c(bank: Bank, hidden: int) -> _Bank:
                  d.trellis.shape[3])
 
 
-def _moe(x, bank, inds, scores, dec, limit, clamp_at, shared, entry: str, shared_ready=None):
+def _moe(x, bank, inds, scores, dec, limit, clamp_at, shared, clamped: bool = False, shared_ready=None):
+    y = None
+    if not clamped or 0 < limit <= 128:
+        y = (_call or native()).moe(x, bank, inds, scores, dec, limit, clamp_at, shared, shared_ready.cuda_event if shared_ready else 0)
+    return y if y.__class__ is torch.Tensor else _refuse_moe(y, x, bank, inds, scores, shared, clamped)
+
+
+def _refuse_moe(status, x, bank, inds, scores, shared, clamped):
+    """Names why a routed call did not run."""
+    if status is not None:
+        _check(status)
     _need_cuda(x, inds, scores)
     if x.dim() != 3 or inds.dim() != 3 or x.shape[:2] != inds.shape[:2] or inds.shape != scores.shape:
         raise Exl3Error(1, "BadExl3Shape")  # root.validateCall, src/root.zig:128-141
@@ -361,37 +384,20 @@ def _moe(x, bank, inds, scores, dec, limit, clamp_at, shared, entry: str, shared
         raise Exl3Error(1, "BadExl3Shape")
     if x.dtype not in _DTYPES or inds.dtype not in (torch.int32, torch.uint32) or scores.dtype not in _DTYPES:
         raise Exl3Error(2, "BadExl3Dtype")
-    hidden = x.shape[2]
-    cb = _bank_c(bank, hidden)
-    rows = x.shape[0] * x.shape[1]
+    _bank_c(bank, x.shape[2])
     if shared is not None:
         _need_cuda(shared)
         if shared.dtype != x.dtype or shared.numel() != x.numel():
             raise Exl3Error(1, "BadExl3Shape")
-    L = lib()
-    ws_bytes = L.t3_moe_workspace_bytes(rows, topk, C.byref(cb))
-    ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=x.device)
-    y = torch.empty_like(x)
-    common = (x.data_ptr(), _DTYPES[x.dtype], rows, C.byref(cb), inds.data_ptr(), scores.data_ptr(),
-              _DTYPES[scores.dtype], topk, dec._c())
-    tail = (y.data_ptr(), ws.data_ptr(), ws_bytes, _stream_ptr(x))
-    if entry == "moe":
-        _check(L.t3_moe(*common, *tail))
-    elif entry == "swiglu":
-        _check(L.t3_moe_swiglu(*common, limit, clamp_at, *tail))
-    elif entry == "clamped":
-        _check(L.t3_moe_clamped(*common, limit, *tail))
-    elif shared_ready is not None:
-        _check(L.t3_moe_with_shared_after(*common, shared.data_ptr(), shared_ready.cuda_event, *tail))
-    else:
-        _check(L.t3_moe_with_shared(*common, shared.data_ptr(), *tail))
-    return y
+    if clamped:
+        raise Exl3Error(6, "InvalidExl3Clamp")
+    raise Exl3Error(1, "BadExl3Shape")
 
 
 def moe(x, bank: Bank, inds, scores, dec: Decode = Decode.mul1, verify_rows: bool = False) -> torch.Tensor:
     """root.moe (src/root.zig:822-825): x [B, S, D], inds/scores [B, S, K]; y in x's shape and dtype."""
     del verify_rows  # accepted and ignored, as the reference does
-    return _moe(x, bank, inds, scores, dec, 0, CLAMP_GATE_IN, None, "moe")
+    return _moe(x, bank, inds, scores, dec, 0, CLAMP_GATE_IN, None)
 
 
 def moe_swiglu_rows(x: torch.Tensor, rows: torch.Tensor, bank: Bank, inds: torch.Tensor, scores: torch.Tensor,
@@ -518,12 +524,12 @@ def ep_plan(inds: torch.Tensor, experts: int, world: int):
 
 def moe_swiglu(x, bank: Bank, inds, scores, dec: Decode, limit: int, clamp_at: int = CLAMP_GATE_IN) -> torch.Tensor:
     """root.moeSwiglu (src/root.zig:831-833)."""
-    return _moe(x, bank, inds, scores, dec, limit, clamp_at, None, "swiglu")
+    return _moe(x, bank, inds, scores, dec, limit, clamp_at, None)
 
 
 def moe_clamped(x, bank: Bank, inds, scores, dec: Decode, limit: int) -> torch.Tensor:
     """root.moeClamped (src/root.zig:1001-1004): limit in 1..128, else InvalidExl3Clamp."""
-    return _moe(x, bank, inds, scores, dec, limit, CLAMP_GATE_IN, None, "clamped")
+    return _moe(x, bank, inds, scores, dec, limit, CLAMP_GATE_IN, None, clamped=True)
 
 
 def moe_with_shared(x, bank: Bank, inds, scores, dec: Decode, shared: torch.Tensor,
@@ -531,4 +537,4 @@ def moe_with_shared(x, bank: Bank, inds, scores, dec: Decode, shared: torch.Tens
     """root.moeWithShared (src/root.zig:976-984). shared_ready: an event recorded on the stream that computes `shared`;
     only the call's last launch waits for it (t3_moe_with_shared_after)."""
     del verify_rows
-    return _moe(x, bank, inds, scores, dec, 0, CLAMP_GATE_IN, shared, "shared", shared_ready)
+    return _moe(x, bank, inds, scores, dec, 0, CLAMP_GATE_IN, shared, shared_ready=shared_ready)

@@ -1,5 +1,5 @@
-"""Builds libt3.so (the C-ABI library) in-tree with nvcc for sm_100a. No torch, no JIT cache: the .so sits next to the
-sources so it travels with the tree.
+"""Builds libt3.so (the C-ABI library) in-tree with nvcc for sm_100a, and the Python binding of the hot calls (_call.so, g++
+against torch's headers) beside it. No JIT cache: the libraries sit next to the sources so they travel with the tree.
 
     python -m turboexl3_b200.build [--force] [--verbose]
 """
@@ -16,6 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "libt3.so")
+BINDING = os.path.join(HERE, "_call.so")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
               "--expt-relaxed-constexpr"]
@@ -47,7 +48,7 @@ def _nvcc() -> str:
 def _digest() -> str:
     h = hashlib.sha256()
     for name in sorted(os.listdir(CSRC)):
-        if name.endswith((".cu", ".cuh", ".h")):
+        if name.endswith((".cu", ".cuh", ".h", ".cpp")):
             with open(os.path.join(CSRC, name), "rb") as f:
                 h.update(name.encode() + b"\0" + f.read())
     for header in ("t3.h", "t3_table.h"):
@@ -84,18 +85,48 @@ def _compile(unit, verbose: bool) -> str:
     return obj
 
 
+def _compile_binding() -> str:
+    """t3_binding.cpp to an object (the host compiler only: it launches nothing itself)."""
+    import sysconfig
+
+    import torch
+    root = os.path.join(os.path.dirname(torch.__file__), "include")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    obj = os.path.join(OBJ, "t3_binding.o")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-isystem", root,
+           "-isystem", os.path.join(root, "torch", "csrc", "api", "include"), "-isystem", os.path.join(cuda, "include"),
+           "-isystem", sysconfig.get_paths()["include"], "-c", os.path.join(CSRC, "t3_binding.cpp"), "-o", obj]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed on t3_binding.cpp:\n{res.stdout}\n{res.stderr}")
+    return obj
+
+
+def _link_binding(obj: str) -> None:
+    import torch
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["g++", "-shared", "-o", BINDING, obj, "-L" + HERE, "-lt3", "-L" + libs, "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+           "-ltorch_python", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"link of _call.so failed:\n{res.stdout}\n{res.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every translation unit for sm_100a and link libt3.so; returns its path. Skips when up to date."""
+    """Compile every translation unit for sm_100a, link libt3.so and the binding; returns the library's path. Skips when up to
+    date."""
     os.makedirs(OBJ, exist_ok=True)
     stamp = os.path.join(OBJ, "digest.txt")
     digest = _digest()
-    if not force and os.path.exists(LIB) and os.path.exists(stamp) and open(stamp).read() == digest:
+    if not force and os.path.exists(LIB) and os.path.exists(BINDING) and os.path.exists(stamp) and open(stamp).read() == digest:
         return LIB
     with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as pool:
+        binding = pool.submit(_compile_binding)
         objs = list(pool.map(lambda u: _compile(u, verbose), UNITS))
     res = subprocess.run([_nvcc(), "-shared", "-o", LIB, *objs], capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _link_binding(binding.result())
     with open(stamp, "w") as f:
         f.write(digest)
     return LIB

@@ -136,7 +136,10 @@ class Block:
 def matmul(w: Weight, x: np.ndarray, stream: int = 0, dtype: int | None = None):
     """`matmul` on host arrays: returns (verdict, y) with y a new numpy array of x's dtype."""
     y = np.empty(x.shape[:-1] + (w.out_dim,), x.dtype)
-    out = host_array(y, dtype)
+    native = api._call or api.native()
+    if x.flags.c_contiguous and native.table_matmul(w, x, y, stream, _NP_DTYPE[x.dtype] if dtype is None else dtype):
+        return Verdict(), y
+    out = host_array(y, dtype)  # what the binding does not take, and the refusals: the table's verdict says why
     v = table().matmul(C.byref(w), C.byref(host_array(x, dtype)), stream, C.byref(out))
     return v, y
 
