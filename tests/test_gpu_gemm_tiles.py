@@ -15,7 +15,8 @@ from test_gpu_moe import check_moe, make_bank
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("case", [(128, 128, 16, t3.MUL1, "f16"), (256, 384, 128, t3.MCG, "f32"), (384, 256, 36, t3.MUL1, "bf16")])
+@pytest.mark.parametrize("case", [(128, 128, 16, t3.MUL1, "f16"), (256, 384, 128, t3.MCG, "f32"), (384, 256, 36, t3.MUL1, "bf16"),
+                                  (256, 128, 32, t3.MCG, "f16"), (128, 256, 64, t3.MUL1, "f32")])
 def test_dense_tile_edges(case):
     in_dim, out_dim, n, cb, dt = case
     trellis, suh, svh = synth.linear(2100 + n, in_dim, out_dim, n, scaled=True)

@@ -28,6 +28,7 @@
 // Every wait is bounded: one that runs out sets a bit of the device error word and a flag that ends every other role's waits,
 // and the CTA walks to its exit, freeing its tensor memory on the way.
 #include <atomic>
+#include <type_traits>
 
 #include "t3_common.cuh"
 #include "t3_gemm.h"
@@ -44,8 +45,13 @@ namespace {
 constexpr uint32_t kEpiWarps = 8, kDecWarps = 16;
 constexpr uint32_t kCodeWarp = kEpiWarps + kDecWarps, kRowWarp = kCodeWarp + 1, kMmaWarp = kCodeWarp + 2;
 constexpr uint32_t kThreads = 32u * (kMmaWarp + 1u);
+constexpr uint32_t kCodeStages = 4;        // stages of the code ring: even, so that a slot is always the same decode group's
 constexpr uint32_t kStages = 3;            // operand stages in tensor memory
-constexpr uint32_t kCodeStages = 4;        // stages of the code ring
+static_assert(kCodeStages % 2u == 0u, "see decode_stages");
+// The decode warps work as two groups of eight on alternate stages, a warp on both of a stage's 64 x 128 blocks: eight tiles a
+// visit, so that a visit's waits, arrivals and ring arithmetic are paid half as often as with sixteen warps on every stage
+// (59 -> 54 issued instructions a tile), and sixteen warps to issue from (eight alone left a third of the issue slots empty).
+constexpr uint32_t kGroupWarps = 8;
 constexpr uint32_t kStageTiles = 64;       // weight tiles a stage
 constexpr uint32_t kStageCols = 64;        // tensor-memory columns a stage (32 a 64 x 128 block)
 // tensor memory: accumulators in columns 0-255, operand stages in 256-447, H128 (128 x 128 f16) in 448-511
@@ -115,23 +121,30 @@ __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, volati
     return false;
 }
 
-// a ring position and the parity of its round
+// a ring position and the parity of its round (a wait for the parity before a fresh barrier's first phase returns at once, so a
+// first round needs no case of its own)
 template <uint32_t SLOTS>
 struct Ring {
     uint32_t slot = 0, parity = 0;
-    bool first_round = true;
-    __device__ __forceinline__ void next() {
-        if (++slot == SLOTS) slot = 0, parity ^= 1u, first_round = false;
+    __device__ __forceinline__ void next(uint32_t by = 1) {
+        slot += by;
+        if (slot >= SLOTS) slot -= SLOTS, parity ^= 1u;
     }
 };
 
-// The decode warps' pass over one sub-tile's stages: a warp's four tiles lie a row of 8 tiles apart in the code stage.
-template <int NN, int CB>
-__device__ __forceinline__ void decode_stages(uint32_t stages, Ring<kCodeStages>& cring, Ring<kStages>& ring, uint32_t codes,
-                                              uint32_t stage_bytes, uint32_t n, uint32_t first_tile,
-                                              const LanePlan<(NN > 0 ? NN : 16)>& plan, uint32_t mask, uint32_t lane,
-                                              uint32_t tmem_dst, uint32_t full_c, uint32_t empty_c, uint32_t full_a,
-                                              uint32_t empty_a, volatile uint32_t* dead, uint32_t* err) {
+// A decode group's pass over its stages of one sub-tile (every other one, `visits` of them from the ring's position on). A warp's
+// tiles lie a row of 8 tiles apart in the code stage: four along K of the stage's first block, four of its second (PARTS 2).
+// FULL: the codeword is the whole 16-bit window (no mask).
+//
+// A wait by parity can only tell a barrier's current phase from the one before, so whoever waits for a phase must know that the
+// phase before it is over. A group that came back to a code slot which the OTHER group used last would not (its codes may not
+// even have landed: the wait would return at once, on the round before); with an even ring a slot stays with one group. On the
+// operand ring of three stages the group has always seen a later stage's MMAs complete than the ones before those it waits for.
+template <int NN, int CB, bool FULL, uint32_t PARTS>
+__device__ __forceinline__ void decode_stages(uint32_t visits, Ring<kCodeStages>& cring, Ring<kStages>& ring, uint32_t codes, uint32_t stage_bytes, uint32_t n,
+                                              uint32_t first_tile, const LanePlan<(NN > 0 ? NN : 16)>& plan, uint32_t mask,
+                                              uint32_t lane, uint32_t tmem_dst, uint32_t full_c, uint32_t full_a, volatile uint32_t* dead,
+                                              uint32_t* err) {
     constexpr int NP = NN > 0 ? NN : 16;
     constexpr uint32_t kRaw = raw_words(NP);
     const uint32_t tile_bytes = 2u * (NN > 0 ? (uint32_t)NN : n);
@@ -139,43 +152,47 @@ __device__ __forceinline__ void decode_stages(uint32_t stages, Ring<kCodeStages>
 #pragma unroll
     for (uint32_t j = 0; j < kRaw; ++j) at[j] = codes + first_tile * tile_bytes + plan.idx[j] * 4u;
 #pragma unroll 1
-    for (uint32_t k = 0; k < stages; ++k) {
-        const uint32_t s = ring.slot, cs = cring.slot;
-        wait_phase<20>(full_c + 8u * cs, cring.parity, dead, err, kErrFullWait);
-        uint32_t raw[4][kRaw];
-        if (NN > 0) {
+    for (uint32_t k = 0; k < visits; ++k) {
+        const uint32_t cbar = full_c + 16u * cring.slot, abar = full_a + 16u * ring.slot, off = cring.slot * stage_bytes;
+        const uint32_t col = tmem_dst + ring.slot * kStageCols;
+        wait_phase<20>(cbar, cring.parity, dead, err, kErrFullWait);
 #pragma unroll
-            for (uint32_t j = 0; j < kRaw; ++j)
+        for (uint32_t p = 0; p < PARTS; ++p) {
+            uint32_t raw[4][kRaw];
+            if (NN > 0) {
 #pragma unroll
                 for (uint32_t i = 0; i < 4u; ++i)
-                    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(raw[i][j]) : "r"(at[j] + cs * stage_bytes + i * 16u * (uint32_t)NP));
-        }
-        if (!ring.first_round) wait_phase<20>(empty_a + 8u * s, ring.parity ^ 1u, dead, err, kErrEmptyWait);
-        tc_fence_after();
 #pragma unroll
-        for (uint32_t i = 0; i < 4u; ++i) {
-            uint32_t w[4];
-            if (NN > 0)
-                decode_raw<NP, CB>(raw[i], plan, mask, w);
-            else
-                decode_lane_any<CB>(static_cast<const uint32_t*>(__cvta_shared_to_generic(
-                                        codes + cs * stage_bytes + (first_tile + i * 8u) * tile_bytes)), n, lane, mask, w);
-            tmem_st_tile(tmem_dst + s * kStageCols + 8u * i, w);
+                    for (uint32_t j = 0; j < kRaw; ++j)
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(raw[i][j]) : "r"(at[j] + off + (p * 4u + i) * 16u * (uint32_t)NP));
+            }
+            if (p == 0) {
+                wait_phase<20>(abar + 8u, ring.parity ^ 1u, dead, err, kErrEmptyWait);
+                tc_fence_after();
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i) {
+                uint32_t w[4];
+                if (NN > 0)
+                    decode_raw<NP, CB, FULL>(raw[i], plan, mask, w);
+                else
+                    decode_lane_any<CB>(static_cast<const uint32_t*>(__cvta_shared_to_generic(
+                                            codes + off + (first_tile + (p * 4u + i) * 8u) * tile_bytes)), n, lane, mask, w);
+                tmem_st_tile(col + 32u * p + 8u * i, w);
+                // the last tile's words are in registers by now: the code slot may be refilled while this stage is finished
+                if (p + 1u == PARTS && i == 2u && NN > 0) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_addr(cbar + 8u);
+                }
+            }
         }
         tmem_st_wait();
         tc_fence_before();
-        if (lane == 0) mbar_arrive_addr(full_a + 8u * s), mbar_arrive_addr(empty_c + 8u * cs);
-        ring.next(), cring.next();
-    }
-}
-
-// the stages of a sub-tile that a decode warp has no tiles in (the second block's warps when a wide unit has one block)
-__device__ __forceinline__ void skip_stages(uint32_t stages, Ring<kCodeStages>& cring, Ring<kStages>& ring, uint32_t lane, uint32_t empty_c,
-                                            uint32_t full_a, uint32_t empty_a, volatile uint32_t* dead, uint32_t* err) {
-    for (uint32_t k = 0; k < stages; ++k, ring.next(), cring.next()) {
-        if (!ring.first_round) wait_phase<20>(empty_a + 8u * ring.slot, ring.parity ^ 1u, dead, err, kErrEmptyWait);
-        __syncwarp();
-        if (lane == 0) mbar_arrive_addr(full_a + 8u * ring.slot), mbar_arrive_addr(empty_c + 8u * cring.slot);
+        if (lane == 0) {
+            if (NN == 0) mbar_arrive_addr(cbar + 8u);
+            mbar_arrive_addr(abar);
+        }
+        cring.next(2), ring.next(2);
     }
 }
 
@@ -253,9 +270,9 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
     const uint32_t smem = (smem_addr(smem_raw) + 1023u) & ~1023u;
     const uint32_t n = NN > 0 ? (uint32_t)NN : (KEPT ? 0u : a.n), tile_bytes = 2u * n, stage_bytes = kStageTiles * tile_bytes;
     const uint32_t z_s = smem + kSlots * kSlotBytes, codes = z_s + 2u * kZBytes;
-    const uint32_t bars = codes + kCodeStages * stage_bytes;
-    const uint32_t full_c = bars, empty_c = full_c + 8u * kCodeStages, full_a = empty_c + 8u * kCodeStages;
-    const uint32_t empty_a = full_a + 8u * kStages, full_b = empty_a + 8u * kStages, empty_b = full_b + 8u * 4u;
+    // barriers, a full / empty pair a ring slot: codes, operands in tensor memory, rows
+    const uint32_t full_c = codes + kCodeStages * stage_bytes, full_a = full_c + 16u * kCodeStages;
+    const uint32_t full_b = full_a + 16u * kStages, empty_b = full_b + 8u * 4u;
     const uint32_t acc_full = empty_b + 8u * 4u, acc_free = acc_full + 8u;
     // z_full, rot_full: a pair each, one barrier a 128-column part (the epilogue and the MMA warp run both parts ahead)
     const uint32_t z_full = acc_full + 16u, rot_full = acc_full + 32u;
@@ -268,8 +285,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
     const uint32_t warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);
     if (tid == 0) {
         auto init = [&](uint32_t bar, uint32_t count) { mbar_init(reinterpret_cast<uint64_t*>(generic + (bar - smem)), count); };
-        for (uint32_t s = 0; s < kCodeStages; ++s) init(full_c + 8u * s, 1u), init(empty_c + 8u * s, kDecWarps);
-        for (uint32_t s = 0; s < kStages; ++s) init(full_a + 8u * s, kDecWarps), init(empty_a + 8u * s, 1u);
+        for (uint32_t s = 0; s < kCodeStages; ++s) init(full_c + 16u * s, 1u), init(full_c + 16u * s + 8u, kGroupWarps);
+        for (uint32_t s = 0; s < kStages; ++s) init(full_a + 16u * s, kGroupWarps), init(full_a + 16u * s + 8u, 1u);
         for (uint32_t s = 0; s < kSlots; ++s) init(full_b + 8u * s, 1u), init(empty_b + 8u * s, 1u);
         init(acc_full, 1u), init(acc_free, kEpiWarps);
         for (uint32_t c = 0; c < 2u; ++c) init(z_full + 8u * c, kEpiWarps), init(rot_full + 8u * c, 1u);
@@ -283,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, *tmem_slot, 0);
     const bool sliced = a.ksplit > 1u;
     // H128 as an A operand in tensor memory: element (i, j) has the sign of popcount(i & j)
-    if (warp >= kEpiWarps && warp < kEpiWarps + 8u) {
+    if (warp < 8u) {
         const uint32_t i = 32u * (warp & 3u) + 16u * ((warp >> 2) & 1u) + (lane >> 2), j0 = 2u * (lane & 3u);
         auto pair = [](uint32_t r, uint32_t c) {
             return ((__popc(r & c) & 1) ? 0xBC00u : 0x3C00u) | ((__popc(r & (c + 1u)) & 1) ? 0xBC000000u : 0x3C000000u);
@@ -300,27 +317,32 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
     tc_fence_after();
 
     if (warp >= kEpiWarps && warp < kCodeWarp) {
-        // ---- decode: quarter q of the lanes (32 outputs a block), tile column 2q + half of a block; part: the block (wide) or
-        // the 64-input half of the stage (deep)
-        const uint32_t q = warp & 3u, half = ((warp - kEpiWarps) >> 2) & 1u, part = (warp - kEpiWarps) >> 3;
+        // ---- decode: quarter q of the lanes (32 outputs a block), tile column 2q + half of a block, stages of the group's parity
+        const uint32_t q = warp & 3u, half = ((warp - kEpiWarps) >> 2) & 1u, group = (warp - kEpiWarps) / kGroupWarps;
         LanePlan<(NN > 0 ? NN : 16)> plan;
         plan.init(lane);
-        const uint32_t dst = tmem + kTmemA + part * 32u + ((32u * q + 16u * half) << 16);
-        const uint32_t col = 2u * q + half;
+        const uint32_t dst = tmem + kTmemA + ((32u * q + 16u * half) << 16), col = 2u * q + half;
         Ring<kCodeStages> cring;
         Ring<kStages> ring;
+        if (group) cring.next(), ring.next();
+        uint32_t ahead = group;  // stages from a sub-tile's first to the group's next one: 0 or 1
+        const bool full = a.mask == 0xFFFFu;
         if (!KEPT) for_each_sub(a, [&](const Sub& s) {
-            const uint32_t k64 = s.k1 - s.k0;
-            if (s.wide && s.blocks == 1u && part == 1u)
-                skip_stages(k64, cring, ring, lane, empty_c, full_a, empty_a, dead, a.err);
-            else
-                decode_stages<NN, CB>(s.wide ? k64 : k64 / 2u, cring, ring, codes, stage_bytes, n, part * 32u + col, plan, a.mask, lane,
-                                      dst, full_c, empty_c, full_a, empty_a, dead, a.err);
+            const uint32_t stages = s.wide ? s.k1 - s.k0 : (s.k1 - s.k0) / 2u, visits = (stages + 1u - ahead) / 2u;
+            auto run = [&](auto fullw, auto parts) {
+                decode_stages<NN, CB, decltype(fullw)::value, decltype(parts)::value>(visits, cring, ring, codes, stage_bytes, n, col, plan,
+                                                                                      a.mask, lane, dst, full_c, full_a, dead, a.err);
+            };
+            using One = std::integral_constant<uint32_t, 1>;
+            using Two = std::integral_constant<uint32_t, 2>;
+            if (s.wide && s.blocks == 1u) full ? run(std::true_type(), One()) : run(std::false_type(), One());  // no second block
+            else full ? run(std::true_type(), Two()) : run(std::false_type(), Two());
+            ahead = (ahead + stages) & 1u;  // an odd number of stages hands the next sub-tile's first one to the other group
             return true;
         });
     } else if (warp == kCodeWarp) {
         // ---- code ring: a stage is two boxes of 4 tile rows x 8 tiles, the unit's two blocks (wide) or two runs of 64 inputs
-        // (deep). A slot is free again when every decode warp has decoded it.
+        // (deep). A slot is free again when every decode warp has its words in registers.
         Ring<kCodeStages> ring;
         if (!KEPT) for_each_sub(a, [&](const Sub& s) {
             const CUtensorMap* map = &maps.codes[s.op];
@@ -328,8 +350,8 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
             const bool two = !s.wide || s.blocks == 2u;
             const int x0 = (int)(s.blk * words), x1 = x0 + (s.wide ? (int)words : 0), e = (int)s.e, dy = s.wide ? 0 : 4;
             for (uint32_t k = 4u * s.k0; k < 4u * s.k1; k += s.wide ? 4u : 8u, ring.next()) {
-                const uint32_t bar = full_c + 8u * ring.slot, dst = codes + ring.slot * stage_bytes;
-                if (!ring.first_round && !wait_phase<150>(empty_c + 8u * ring.slot, ring.parity ^ 1u, dead, a.err, kErrEmptyWait)) return false;
+                const uint32_t bar = full_c + 16u * ring.slot, dst = codes + ring.slot * stage_bytes;
+                if (!wait_phase<64>(bar + 8u, ring.parity ^ 1u, dead, a.err, kErrEmptyWait)) return false;
                 __syncwarp();
                 if (elect_one()) {
                     mbar_arrive_expect_tx_addr(bar, two ? 2u * box : box);
@@ -349,7 +371,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
             const CUtensorMap* map = &maps.rows[big == 256u ? 0 : big == 128u ? 1 : big == 64u ? 2 : 3];
             for (uint32_t k = s.k0; k < s.k1; ++k, ring.next()) {
                 const uint32_t bar = full_b + 8u * ring.slot, dst = smem + ring.slot * kSlotBytes;
-                if (!ring.first_round && !wait_phase<32>(empty_b + 8u * ring.slot, ring.parity ^ 1u, dead, a.err, kErrEmptyWait)) return false;
+                if (!wait_phase<32>(empty_b + 8u * ring.slot, ring.parity ^ 1u, dead, a.err, kErrEmptyWait)) return false;
                 __syncwarp();
                 if (elect_one()) {
                     mbar_arrive_expect_tx_addr(bar, load * 128u + (KEPT ? kKeptBytes : 0u));
@@ -396,12 +418,12 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
             for (uint32_t k = 0; k < stages; ++k, ring_a.next()) {
                 const uint32_t a_col = tmem + kTmemA + ring_a.slot * kStageCols;
                 wait(full_b + 8u * ring_b.slot, ring_b.parity, kErrFullWait);
-                if (!KEPT) wait(full_a + 8u * ring_a.slot, ring_a.parity, kErrFullWait);
+                if (!KEPT) wait(full_a + 16u * ring_a.slot, ring_a.parity, kErrFullWait);
                 if (s.wide) {
                     if (elect_one()) {
                         if (s.blocks == 2u) steps(a_col, true);
                         else steps(a_col, false);
-                        umma_commit(empty_a + 8u * ring_a.slot);
+                        umma_commit(full_a + 16u * ring_a.slot + 8u);
                     }
                 } else {
                     if (elect_one()) steps(a_col, false);
@@ -410,7 +432,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
                     wait(full_b + 8u * ring_b.slot, ring_b.parity, kErrFullWait);
                     if (elect_one()) {
                         steps(a_col + 32u, false);
-                        if (!KEPT) umma_commit(empty_a + 8u * ring_a.slot);
+                        if (!KEPT) umma_commit(full_a + 16u * ring_a.slot + 8u);
                     }
                 }
                 acc = 1u;

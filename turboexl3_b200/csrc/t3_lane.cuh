@@ -208,6 +208,46 @@ T3_HD uint32_t window_at(const uint32_t (&w)[NW], uint32_t pos, uint32_t mask) {
     return shr_pair(w[q], w[q + 1 < NW ? q + 1 : q], 48u - b) & mask;
 }
 
+// The 16-bit window `pos` bits into w as one byte permutation, where its bytes lie in a word whole: with the windows of a lane
+// at multiples of n / 16 bits, K = 8 has all eight there, K = 4 and K = 2 have them in a few common realignments of the span.
+// One instruction a window instead of a shift and a mask.
+#if defined(__CUDA_ARCH__)
+#define T3_BYTES(w, hi, lo) __byte_perm((w), 0u, 0x4400u | ((hi) << 4) | (lo))
+#else
+#define T3_BYTES(w, hi, lo) (((((w) >> (8u * (hi))) & 0xFFu) << 8) | (((w) >> (8u * (lo))) & 0xFFu))
+#endif
+// the byte-aligned window `at` bits (0, 8 or 16) below w's top bit
+T3_HD uint32_t byte_window(uint32_t w, uint32_t at) {
+    return at == 0u ? w >> 16 : (at == 8u ? T3_BYTES(w, 2u, 1u) : w & 0xFFFFu);
+}
+
+// The eight full-width windows of a lane whose span starts `o` bits into w, windows K = N / 16 bits apart (K 2, 4 or 8): the
+// words starting at o + s for every s that is a distinct window offset modulo 8, then byte windows of those.
+template <uint32_t K, uint32_t NW>
+T3_HD void even_windows(const uint32_t (&w)[NW], uint32_t o, uint32_t (&cw)[8]) {
+    // word starting at bit p of the span (p a constant wherever this is called from)
+    auto from = [&](uint32_t p) {
+        const uint32_t q = (o + p) >> 5, b = (o + p) & 31u;
+        return b == 0u ? w[q] : shl_pair(w[q], w[q + 1 < NW ? q + 1 : q], b);
+    };
+    if (K == 8u) {
+#pragma unroll
+        for (uint32_t m = 0; m < 8u; ++m) {
+            const uint32_t q = (o + 8u * m) >> 5, b = (o + 8u * m) & 31u;
+            cw[m] = b <= 16u ? byte_window(w[q], b) : byte_window(from(8u * m), 0u);
+        }
+    } else if (K == 4u) {
+        const uint32_t a = from(0), b = from(4), c = from(8), d = from(12);
+        cw[0] = byte_window(a, 0), cw[2] = byte_window(a, 8), cw[4] = byte_window(a, 16);
+        cw[1] = byte_window(b, 0), cw[3] = byte_window(b, 8), cw[5] = byte_window(b, 16);
+        cw[6] = byte_window(c, 16), cw[7] = byte_window(d, 16);
+    } else {
+        const uint32_t a = from(0), b = from(2), c = from(4), d = from(6);
+        cw[0] = byte_window(a, 0), cw[4] = byte_window(a, 8), cw[1] = byte_window(b, 0), cw[5] = byte_window(b, 8);
+        cw[2] = byte_window(c, 0), cw[6] = byte_window(c, 8), cw[3] = byte_window(d, 0), cw[7] = byte_window(d, 8);
+    }
+}
+
 // The lane's raw words of one tile (`tile` points at the tile's first word, shared or global memory).
 template <int N>
 T3_HD void load_lane(const uint32_t* tile, const LanePlan<N>& plan, uint32_t (&raw)[raw_words(N)]) {
@@ -218,7 +258,8 @@ T3_HD void load_lane(const uint32_t* tile, const LanePlan<N>& plan, uint32_t (&r
 // The lane's eight weights from its raw words as four half2 words: {w0,w1}, {w2,w3}, {w4,w5}, {w6,w7}; b[0], b[1] are
 // the mma.m16n8k16 B fragment of tile columns 0-7, b[2], b[3] of columns 8-15. `mask` is the pack's codeword-width mask
 // (format.zig:60-62).
-template <int N, int CB>
+// FULL: the pack's codewords are the whole 16-bit windows, `mask` is not read.
+template <int N, int CB, bool FULL = false>
 T3_HD void decode_raw(const uint32_t (&raw)[raw_words(N)], const LanePlan<N>& plan, uint32_t mask, uint32_t (&b)[4]) {
     constexpr uint32_t kRaw = raw_words(N);
     if (CB >= kProbeNoFunnel) {
@@ -227,7 +268,19 @@ T3_HD void decode_raw(const uint32_t (&raw)[raw_words(N)], const LanePlan<N>& pl
         return;
     }
     uint32_t cw[8];
-    if (uniform_shift(N)) {
+    if (FULL) mask = 0xFFFFu;
+    if (FULL && (N == 32 || N == 64 || N == 128)) {
+        if (uniform_shift(N)) {
+            constexpr uint32_t o = (win_end(N, 0) + 16u * N - 16u) & 31u;
+            even_windows<N / 16u>(raw, o, cw);
+        } else {
+            constexpr uint32_t kAl = aligned_words(N);
+            uint32_t al[kAl];
+#pragma unroll
+            for (uint32_t i = 0; i < kAl; ++i) al[i] = shl_pair(raw[i], raw[i + 1 < kRaw ? i + 1 : i], plan.shift);
+            even_windows<N / 16u>(al, 0u, cw);
+        }
+    } else if (uniform_shift(N)) {
         constexpr uint32_t o = (win_end(N, 0) + 16u * N - 16u) & 31u;
 #pragma unroll
         for (uint32_t m = 0; m < 8u; ++m) cw[m] = window_at<kRaw>(raw, o + win_end(N, m) - win_end(N, 0), mask);
