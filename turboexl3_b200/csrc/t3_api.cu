@@ -766,7 +766,7 @@ int moe_call(const void* x, int x_dtype, size_t rows, const t3_bank* bank, const
     note_engine(rows > T3_DECODE_ROWS_MAX ? 2 : 0, ((uint64_t)a.hidden << 32) | a.inter, a.experts, a.n, a.topk);
     if (rows > T3_DECODE_ROWS_MAX) {
         int launches = 0;
-        const cudaError_t rc = launch_prefill_moe(a, workspace, dec.codebook, static_cast<cudaStream_t>(stream), &launches);
+        const cudaError_t rc = launch_prefill_moe(a, nullptr, workspace, dec.codebook, static_cast<cudaStream_t>(stream), &launches);
         g_launches.fetch_add((uint64_t)launches, std::memory_order_relaxed);
         return cuda_status(rc);
     }
@@ -1025,7 +1025,7 @@ int t3_moe_swiglu_rows(const void* x, int x_dtype, size_t x_rows, const void* ro
     a.err = dev_error_ptr();
     note_engine(2, ((uint64_t)a.hidden << 32) | a.inter, a.experts, a.n, 1);
     int launches = 0;
-    const cudaError_t rc = launch_prefill_moe(a, workspace, dec.codebook, static_cast<cudaStream_t>(stream), &launches);
+    const cudaError_t rc = launch_prefill_moe(a, nullptr, workspace, dec.codebook, static_cast<cudaStream_t>(stream), &launches);
     g_launches.fetch_add((uint64_t)launches, std::memory_order_relaxed);
     return cuda_status(rc);
 }

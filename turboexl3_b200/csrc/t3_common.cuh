@@ -123,45 +123,72 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// ---- the 128-point Hadamard on tensor cores (the prefill-row prepares and finishes) ---------------------------------
+// ---- the 128-point Hadamard on tensor cores (the prefill-row prepares) -----------------------------------------------
 //
-// The 128-point Hadamards of these kernels run on the tensor cores. The sign of entry (i, j) of H128 is the parity of
-// popcount(i & j), which splits over the bit fields of i = 16 i8 + i16, so H128 = H8 (x) H16 and a block viewed as an
-// 8 x 16 matrix X becomes H8 . X . H16: X . H16 is m16n8k16 steps against a constant +-1 fragment, H8 a three-level
-// butterfly over values one thread already holds. A warp works on EIGHT positions at a time, one 128-block each: quad g
-// (lanes 4g .. 4g + 3) owns position g, and lane q of the quad holds, for every i8, the four elements 16 i8 + 4q .. + 3:
-// one 8-byte (f16) or 16-byte (f32) access per i8 on the way in and on the way out. The butterfly on a warp costs twenty
-// shuffles per block, and the shuffle unit (one warp instruction per SM per cycle) bounded these kernels; this form has none.
-// f32 accumulation of +-1 products is exact per term, so the result differs from the butterfly (and from the oracle's
-// dense sum) only in summation order, as before.
+// The sign of entry (i, j) of H128 is the parity of popcount(i & j), which splits over the bit fields of i = 8 i16 + i8, so
+// H128 = H16 (x) H8 and a block viewed as a 16 x 8 matrix X becomes H16 . X . H8: the H16 side is m16n8k16 steps against a
+// constant +-1 fragment, the H8 side a three-level butterfly over values one thread already holds. A warp works on EIGHT
+// positions at a time, one 128-block each: quad g (lanes 4g .. 4g + 3) owns position g, and lane q of the quad holds the
+// elements 8 (4 s + q) .. + 7, s = 0 .. 3: sixteen bytes of f16 a load, sixty-four contiguous bytes a quad. (With the fields the
+// other way round a lane's runs were eight bytes and L1 bounded the prepare: 121 us at 40960 slots of 2048 x 2.) The butterfly
+// on a warp costs twenty shuffles per block, and the shuffle unit (one warp instruction per SM per cycle) bounded these kernels;
+// this form has none. f32 accumulation of +-1 products is exact per term, so the result differs from the butterfly (and from
+// the oracle's dense sum) only in summation order.
 
 struct HadB {
     uint32_t b[2][2];  // the +-1 H16 fragment of each 8-column half (t): {k 0-7 part, k 8-15 part}
 };
 
-// Matrix index <-> element maps (both free to choose): A/B index k of thread q covers elements 4q, 4q+1 (k = 2q, 2q+1) and
-// 4q+2, 4q+3 (k = 2q+8, 2q+9); output column n = 2q+b of half t is element 4q + 2t + b. So a thread's inputs and outputs
-// are the same four consecutive elements.
+// Matrix index <-> i16 maps (both free to choose): A/B index k of thread q covers i16 = q, 4 + q (k = 2q, 2q+1) and 8 + q, 12 + q
+// (k = 2q+8, 2q+9); output column n = 2q+b of half t is i16 = 4 (2t + b) + q. So a thread's inputs and outputs are the same four
+// i16, s = 0 .. 3 at 4 s + q.
 __device__ __forceinline__ HadB had_b(uint32_t lane) {
     const uint32_t g = lane >> 2, q = lane & 3u;
     HadB h;
 #pragma unroll
     for (uint32_t t = 0; t < 2u; ++t) {
-        const uint32_t en = 4u * (g >> 1) + 2u * t + (g & 1u);
+        const uint32_t en = 4u * (2u * t + (g & 1u)) + (g >> 1);
         uint32_t s[4];
 #pragma unroll
-        for (uint32_t b = 0; b < 4u; ++b) s[b] = (__popc((4u * q + b) & en) & 1) ? 0xBC00u : 0x3C00u;
+        for (uint32_t b = 0; b < 4u; ++b) s[b] = (__popc((4u * b + q) & en) & 1) ? 0xBC00u : 0x3C00u;
         h.b[t][0] = s[0] | (s[1] << 16);
         h.b[t][1] = s[2] | (s[3] << 16);
     }
     return h;
 }
 
-// out[i8][e] = sum over the block of sign * value, for the position this quad owns. a[i8] = the four f16 values
-// {16 i8 + 4q .. + 3} as two packed pairs; a second set (the f16 remainders of values that are not f16 themselves) is
-// accumulated into the same sums when `use_lo` is set.
-__device__ __forceinline__ void h128_mma(const uint32_t (&a)[8][2], const uint32_t (&lo)[8][2], bool use_lo,
-                                         const HadB& hb, float (&out)[8][4]) {
+// two f32 adds / subtractions / products in one instruction
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&b)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {  // a + (-1) b: one rounding, as a subtraction
+    float2 m = make_float2(-1.0f, -1.0f);
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<uint64_t*>(&b)), "l"(*reinterpret_cast<uint64_t*>(&m)), "l"(*reinterpret_cast<uint64_t*>(&a)));
+    return *reinterpret_cast<float2*>(&d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float c) {
+    float2 m = make_float2(c, c);
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(*reinterpret_cast<uint64_t*>(&a)), "l"(*reinterpret_cast<uint64_t*>(&m)));
+    return *reinterpret_cast<float2*>(&d);
+}
+
+__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ float2 unpack_half2(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+
+// Unscaled sums of the position this quad owns. a[i8] = this thread's values at i8: {s = 0, 1}, {s = 2, 3} as f16 pairs; `lo` (the
+// f16 remainders of values that are not f16 themselves) is accumulated into the same sums when `use_lo` is set. out[i8][t]: s =
+// 2t, 2t + 1.
+__device__ __forceinline__ void h128_mma(const uint32_t (&a)[8][2], const uint32_t (&lo)[8][2], bool use_lo, const HadB& hb,
+                                         float2 (&out)[8][2]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -169,8 +196,8 @@ __device__ __forceinline__ void h128_mma(const uint32_t (&a)[8][2], const uint32
             float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             mma16816(c, a[2 * j][0], a[2 * j + 1][0], a[2 * j][1], a[2 * j + 1][1], hb.b[t][0], hb.b[t][1]);
             if (use_lo) mma16816(c, lo[2 * j][0], lo[2 * j + 1][0], lo[2 * j][1], lo[2 * j + 1][1], hb.b[t][0], hb.b[t][1]);
-            out[2 * j][2 * t] = c[0], out[2 * j][2 * t + 1] = c[1];
-            out[2 * j + 1][2 * t] = c[2], out[2 * j + 1][2 * t + 1] = c[3];
+            out[2 * j][t] = make_float2(c[0], c[1]);
+            out[2 * j + 1][t] = make_float2(c[2], c[3]);
         }
 #pragma unroll
     for (int bit = 1; bit < 8; bit <<= 1)
@@ -178,47 +205,85 @@ __device__ __forceinline__ void h128_mma(const uint32_t (&a)[8][2], const uint32
         for (int i = 0; i < 8; ++i)
             if (!(i & bit))
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float lo_v = out[i][e], hi_v = out[i | bit][e];
-                    out[i][e] = lo_v + hi_v;
-                    out[i | bit][e] = lo_v - hi_v;
+                for (int t = 0; t < 2; ++t) {
+                    const float2 lo_v = out[i][t], hi_v = out[i | bit][t];
+                    out[i][t] = add2(lo_v, hi_v);
+                    out[i | bit][t] = sub2(lo_v, hi_v);
                 }
 }
 
-__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
-    const __half2 h = __floats2half2_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// v (f32 values, not necessarily f16) as an f16 part and the f16 of what is left; returns nonzero when any remainder is
-__device__ __forceinline__ uint32_t split4(const float (&v)[4], uint32_t (&hi)[2], uint32_t (&lo)[2]) {
-    float r[4];
+// format.prepareInput's rotation of a block: w (f16 pairs, w[s][p] = elements 8 (4 s + q) + 2 p, + 1 of this quad's position) times
+// the scales sc (f16, the same elements), H128, / sqrt(128), rounded to f16; in place. Sign scales (the usual suh) are a sign
+// flip of the f16 values; with any other a product is taken in f32 and split into an f16 part and the f16 of what is left, so
+// that the sums see the f32 products.
+__device__ __forceinline__ void rotate_block(uint32_t (&w)[4][4], const uint32_t (&sc)[4][4], const HadB& hb) {
+    uint32_t a[8][2], lo[8][2], odd = 0, rest = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) r[j] = v[j] - round_half(v[j]);
-    hi[0] = pack_half2(v[0], v[1]), hi[1] = pack_half2(v[2], v[3]);
-    lo[0] = pack_half2(r[0], r[1]), lo[1] = pack_half2(r[2], r[3]);
-    return (lo[0] | lo[1]) & 0x7FFF7FFFu;
-}
-
-// H128 of the block whose values are `v` (v[i8] = elements 16 i8 + 4q .. + 3), any f32 values. `unit_scales`: the caller
-// knows (for the whole warp) that every v is an f16 value times +-1 — sign vectors, the usual suh — so v is an f16 value
-// itself and there are no remainders to compute.
-__device__ __forceinline__ void h128_split(const float (&v)[8][4], bool unit_scales, const HadB& hb, float (&out)[8][4]) {
-    uint32_t hi[8][2], lo[8][2], rest = 0;
-    if (unit_scales) {
+    for (int s = 0; s < 4; ++s)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) hi[i][0] = pack_half2(v[i][0], v[i][1]), hi[i][1] = pack_half2(v[i][2], v[i][3]);
-        h128_mma(hi, hi, false, hb, out);
-        return;
+        for (int p = 0; p < 4; ++p) odd |= (sc[s][p] & 0x7FFF7FFFu) ^ 0x3C003C00u;
+    float2 out[8][2];
+    if (__any_sync(0xFFFFFFFFu, odd != 0u) == 0) {
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t u = w[2 * h][p] ^ (sc[2 * h][p] & 0x80008000u), v = w[2 * h + 1][p] ^ (sc[2 * h + 1][p] & 0x80008000u);
+                a[2 * p][h] = pack_lo(u, v);
+                a[2 * p + 1][h] = pack_hi(u, v);
+            }
+        h128_mma(a, a, false, hb, out);
+    } else {
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 x0 = unpack_half2(w[2 * h][p]), x1 = unpack_half2(w[2 * h + 1][p]);
+                const float2 c0 = unpack_half2(sc[2 * h][p]), c1 = unpack_half2(sc[2 * h + 1][p]);
+                const float v[2][2] = {{x0.x * c0.x, x1.x * c1.x}, {x0.y * c0.y, x1.y * c1.y}};
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    a[2 * p + i][h] = pack_half2(v[i][0], v[i][1]);
+                    lo[2 * p + i][h] = pack_half2(v[i][0] - round_half(v[i][0]), v[i][1] - round_half(v[i][1]));
+                    rest |= lo[2 * p + i][h] & 0x7FFF7FFFu;
+                }
+            }
+        h128_mma(a, lo, __any_sync(0xFFFFFFFFu, rest != 0u) != 0, hb, out);
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) rest |= split4(v[i], hi[i], lo[i]);
-    h128_mma(hi, lo, __any_sync(0xFFFFFFFFu, rest != 0u) != 0, hb, out);
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const float2 e = mul2(out[2 * p][t], kHadScale), f = mul2(out[2 * p + 1][t], kHadScale);
+            w[2 * t][p] = pack_half2(e.x, f.x);
+            w[2 * t + 1][p] = pack_half2(e.y, f.y);
+        }
 }
 
-// whether four scales are all +1 or -1 (as f32 values converted from f16)
-__device__ __forceinline__ bool all_unit(const float (&sc)[4]) {
-    return fabsf(sc[0]) == 1.0f && fabsf(sc[1]) == 1.0f && fabsf(sc[2]) == 1.0f && fabsf(sc[3]) == 1.0f;
+// sixteen bytes as four words; `wide`: p is 16-byte aligned, else it is to 8 bytes
+__device__ __forceinline__ void load_16b(const void* p, bool wide, uint32_t (&w)[4]) {
+    if (wide) {
+        const uint4 u = *static_cast<const uint4*>(p);
+        w[0] = u.x, w[1] = u.y, w[2] = u.z, w[3] = u.w;
+    } else {
+        const uint2 u = *static_cast<const uint2*>(p), v = static_cast<const uint2*>(p)[1];
+        w[0] = u.x, w[1] = u.y, w[2] = v.x, w[3] = v.y;
+    }
+}
+__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
+
+// eight consecutive elements i .. i + 7 (i a multiple of 8) of an activation array, each rounded to f16
+__device__ __forceinline__ void load_half8(const void* p, int dt, bool wide, size_t i, uint32_t (&w)[4]) {
+    if (dt == kF32) {
+        const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(p) + i);
+        const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(p) + i + 4);
+        w[0] = pack_half2(a.x, a.y), w[1] = pack_half2(a.z, a.w), w[2] = pack_half2(b.x, b.y), w[3] = pack_half2(b.z, b.w);
+        return;
+    }
+    load_16b(static_cast<const uint16_t*>(p) + i, wide, w);
+    if (dt == kBf16)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = pack_half2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xFFFF0000u));
 }
 
 // ---- shared-memory barriers and bulk copies ------------------------------------------------------------------------

@@ -77,7 +77,7 @@ struct Sub {
 template <typename F>
 __device__ __forceinline__ void for_each_sub(const DecodeGemmArgs& a, F&& f) {
     const uint32_t ncol = a.N / 128u, per_op = (ncol + a.pair - 1u) / a.pair, per_tile = per_op * a.ops;
-    const uint32_t tiles = a.tiles ? *a.n_tiles : a.dense_tiles;
+    const uint32_t tile0 = a.tiles ? a.range[0] : 0u, tiles = a.tiles ? a.range[1] - tile0 : a.dense_tiles;
     const uint32_t total = tiles * per_tile;
     const bool sliced = a.ksplit > 1u;
     for (uint32_t u = sliced ? blockIdx.y : blockIdx.x; u < total; u += sliced ? total : gridDim.x) {
@@ -86,7 +86,7 @@ __device__ __forceinline__ void for_each_sub(const DecodeGemmArgs& a, F&& f) {
         s.op = r / per_op;
         const uint32_t b0 = (r - s.op * per_op) * a.pair, nb = min(a.pair, ncol - b0);
         if (a.tiles) {
-            const int4 d = a.tiles[t];
+            const int4 d = a.tiles[tile0 + t];
             s.e = (uint32_t)d.x, s.first = (uint32_t)d.y, s.rows = (uint32_t)d.z;
         } else {
             s.e = 0, s.first = t * a.tile_rows, s.rows = min(a.tile_rows, a.dense_rows - s.first);

@@ -28,9 +28,9 @@ struct DecodeGemmArgs {
     uint32_t K, N;              // one op's inner and outer widths
     uint32_t n, mask, ops;
     uint32_t op_rows;           // rows between op 0's and op 1's activations
-    // Tiles of rows: (expert, first row, rows, 0), *n_tiles of them (routed); null: one matrix cut every `tile_rows` rows
+    // Tiles of rows: (expert, first row, rows, 0), entries range[0] .. range[1] (routed); null: one matrix cut every `tile_rows` rows
     const int4* tiles;
-    const uint32_t* n_tiles;
+    const uint32_t* range;
     uint32_t dense_rows, tile_rows, dense_tiles;
     uint32_t pair;              // 128-output blocks a unit of work takes: 1 or 2
     // The output rotation in the epilogue: svh[op] + expert * svh_stride is the op's scale vector; the finished values go to y

@@ -124,9 +124,19 @@ struct PrefillLinearArgs {
 };
 size_t prefill_linear_workspace(size_t rows, uint32_t in, uint32_t out);
 cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cudaStream_t stream, int* launches);
+// Several banks of one geometry, each at a rate of its own (a layer whose experts were quantised at different bit widths): the
+// router's expert g is expert local_of[g] of bank bank_of[g] (device arrays of `ids` entries).
+constexpr uint32_t kMixedBanksMax = 8;
+struct MixedBanks {
+    uint32_t count, ids;
+    const int64_t *bank_of, *local_of;
+    BankTab bank[kMixedBanksMax];
+    uint32_t n[kMixedBanksMax];
+};
 // The routed chain at prefill rows: route -> prepare -> GEMM(gate|up) -> mid -> GEMM(down) -> finish
 size_t prefill_moe_workspace(size_t rows, uint32_t topk, uint32_t experts, uint32_t hidden, uint32_t inter);
-cudaError_t launch_prefill_moe(const MoeArgs& a, void* workspace, int codebook, cudaStream_t stream, int* launches);
+// mixed: the banks in the place of a's own (whose geometry, rows and clamp count; a.experts is the sum of the banks'), or null
+cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* workspace, int codebook, cudaStream_t stream, int* launches);
 
 // W_hat f16 from the trellis: [in, out], or transposed [out, in]
 cudaError_t launch_dequant(const uint8_t* trellis, uint32_t in, uint32_t out, uint32_t n, uint32_t mask, int codebook,

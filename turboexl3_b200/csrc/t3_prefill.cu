@@ -17,12 +17,8 @@
 namespace t3 {
 namespace {
 
-// ---- route ---------------------------------------------------------------------------------------------------------
 
-__global__ void route_count_kernel(const uint32_t* inds, uint32_t slots, uint32_t experts, uint32_t* counts) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < slots) atomicAdd(&counts[min(inds[s], experts - 1u)], 1u);
-}
+// ---- route ---------------------------------------------------------------------------------------------------------
 
 // How an expert's c rows are cut into tiles: as few as hold them (a tile decodes its expert's weights once whatever its rows,
 // and the decode is most of what a routed GEMM costs), of equal height in multiples of 16.
@@ -37,48 +33,116 @@ size_t routed_tiles_max(size_t slots, uint32_t experts) {
     return cut < slots ? cut : slots;
 }
 
-// one CTA: each expert's first sorted position (exclusive scan of the counts) into `cursor`, the tiles (expert, first
-// position, rows, 0) in expert order and their number
-__global__ void __launch_bounds__(1024) route_plan_kernel(const uint32_t* counts, uint32_t experts, uint32_t* cursor, int4* tiles,
-                                                          uint32_t* n_tiles) {
-    __shared__ uint32_t s_scan[2][1024];
-    __shared__ uint32_t base[2];
-    const uint32_t tid = threadIdx.x;
-    if (tid < 2u) base[tid] = 0;
-    __syncthreads();
-    // experts are walked in chunks of 1024 with running bases
-    for (uint32_t e0 = 0; e0 < experts; e0 += 1024u) {
-        const uint32_t e = e0 + tid;
-        const uint32_t c = e < experts ? counts[e] : 0u, h = tile_height(c), cuts = (c + h - 1u) / h;
-        s_scan[0][tid] = c, s_scan[1][tid] = cuts;
-        __syncthreads();
-        for (uint32_t off = 1; off < 1024u; off <<= 1) {  // inclusive Hillis-Steele scans
-            const uint32_t add0 = tid >= off ? s_scan[0][tid - off] : 0u, add1 = tid >= off ? s_scan[1][tid - off] : 0u;
-            __syncthreads();
-            s_scan[0][tid] += add0, s_scan[1][tid] += add1;
-            __syncthreads();
-        }
-        if (e < experts) {
-            const uint32_t first = base[0] + s_scan[0][tid] - c, at = base[1] + s_scan[1][tid] - cuts;
-            cursor[e] = first;
-            for (uint32_t i = 0; i < cuts; ++i) {
-                const uint32_t lo = i * h, r = c - lo < h ? c - lo : h;
-                tiles[at + i] = make_int4((int)e, (int)(first + lo), (int)r, 0);
-            }
-        }
-        __syncthreads();
-        if (tid < 2u) base[tid] += s_scan[tid][1023];
+// Where the router's expert ids lie: one bank (bank_of null: the id is the expert), or several banks of one geometry at rates
+// of their own (layer expert g is expert local_of[g] of bank bank_of[g]). Experts are numbered bank by bank: bank b's from
+// base[b] on.
+struct ExpertMap {
+    const int64_t *bank_of, *local_of;
+    uint32_t base[kMixedBanksMax + 1];
+    uint32_t banks, ids;  // banks; router ids (out-of-range ones are clamped)
+    __device__ uint32_t number(uint32_t id) const {
+        id = min(id, ids - 1u);
+        return bank_of ? base[bank_of[id]] + (uint32_t)local_of[id] : id;
+    }
+    // the bank of an expert number, and the number inside it
+    __device__ uint32_t bank(uint32_t e) const {
+        uint32_t b = 0;
+        while (b + 1u < banks && e >= base[b + 1u]) ++b;
+        return b;
+    }
+};
+
+// One launch counts the row-slots of every expert and remembers each slot's rank among its expert's (a block counts in shared
+// memory and reserves its ranks with one atomic an expert); the last block to finish lays out the experts: first[e] the
+// expert's first sorted position, tiles (expert inside its bank, first position, rows, 0) in expert order, range[b] .. range[b +
+// 1] bank b's tiles. counts and `ticket` are zero before the launch. (Counting, laying out and a second pass of atomics to
+// scatter were three launches and 20 us.)
+constexpr uint32_t kRouteThreads = 1024, kRouteSlots = 4096, kRouteExperts = 8192;
+__global__ void __launch_bounds__(kRouteThreads) route_plan_kernel(const uint32_t* inds, uint32_t slots, const __grid_constant__ ExpertMap map,
+                                                                   uint32_t* counts, uint32_t* ticket, uint32_t* rank, uint32_t* first,
+                                                                   int4* tiles, uint32_t* range) {
+    extern __shared__ uint32_t hist[];  // one counter an expert, then its base in this block's ranks; empty past kRouteExperts
+    __shared__ uint32_t s_sum[2][32], s_base[2], s_last;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, experts = map.base[map.banks];
+    const bool shared_hist = experts <= kRouteExperts;
+    const uint32_t lo = blockIdx.x * kRouteSlots;
+    uint32_t mine_e[kRouteSlots / kRouteThreads], mine_r[kRouteSlots / kRouteThreads];
+    if (shared_hist) {
+        for (uint32_t e = tid; e < experts; e += kRouteThreads) hist[e] = 0u;
         __syncthreads();
     }
-    if (tid == 0) *n_tiles = base[1];
+#pragma unroll
+    for (uint32_t i = 0; i < kRouteSlots / kRouteThreads; ++i) {
+        const uint32_t s = lo + i * kRouteThreads + tid;
+        if (s >= slots) break;
+        mine_e[i] = map.number(inds[s]);
+        mine_r[i] = atomicAdd(shared_hist ? &hist[mine_e[i]] : &counts[mine_e[i]], 1u);
+    }
+    if (shared_hist) {
+        __syncthreads();
+        for (uint32_t e = tid; e < experts; e += kRouteThreads)
+            if (hist[e]) hist[e] = atomicAdd(&counts[e], hist[e]);
+        __syncthreads();
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kRouteSlots / kRouteThreads; ++i) {
+        const uint32_t s = lo + i * kRouteThreads + tid;
+        if (s >= slots) break;
+        rank[s] = mine_r[i] + (shared_hist ? hist[mine_e[i]] : 0u);
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1u;
+    if (tid < 2u) s_base[tid] = 0u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (uint32_t e0 = 0; e0 < experts; e0 += kRouteThreads) {  // experts in runs of a thread each, with running bases
+        const uint32_t e = e0 + tid, c = e < experts ? __ldcg(&counts[e]) : 0u, h = tile_height(c), cuts = (c + h - 1u) / h;
+        uint32_t in0 = c, in1 = cuts;  // inclusive scans: inside a warp, then over the warps' sums
+#pragma unroll
+        for (uint32_t off = 1; off < 32u; off <<= 1) {
+            const uint32_t a0 = __shfl_up_sync(0xFFFFFFFFu, in0, off), a1 = __shfl_up_sync(0xFFFFFFFFu, in1, off);
+            if (lane >= off) in0 += a0, in1 += a1;
+        }
+        if (lane == 31u) s_sum[0][warp] = in0, s_sum[1][warp] = in1;
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t t0 = s_sum[0][lane], t1 = s_sum[1][lane];
+#pragma unroll
+            for (uint32_t off = 1; off < 32u; off <<= 1) {
+                const uint32_t a0 = __shfl_up_sync(0xFFFFFFFFu, t0, off), a1 = __shfl_up_sync(0xFFFFFFFFu, t1, off);
+                if (lane >= off) t0 += a0, t1 += a1;
+            }
+            s_sum[0][lane] = t0, s_sum[1][lane] = t1;
+        }
+        __syncthreads();
+        const uint32_t pos = s_base[0] + in0 - c + (warp ? s_sum[0][warp - 1u] : 0u);
+        const uint32_t at = s_base[1] + in1 - cuts + (warp ? s_sum[1][warp - 1u] : 0u);
+        if (e < experts) {
+            first[e] = pos;
+            const uint32_t b = map.bank(e);
+            for (uint32_t i = 0; i < cuts; ++i) {
+                const uint32_t r0 = i * h, r = c - r0 < h ? c - r0 : h;
+                tiles[at + i] = make_int4((int)(e - map.base[b]), (int)(pos + r0), (int)r, 0);
+            }
+            for (uint32_t k = 0; k < map.banks; ++k)
+                if (map.base[k] == e) range[k] = at;
+        }
+        __syncthreads();
+        if (tid < 2u) s_base[tid] += s_sum[tid][31];
+        __syncthreads();
+    }
+    if (tid <= map.banks && map.base[tid] >= experts) range[tid] = s_base[1];
 }
 
-__global__ void route_scatter_kernel(const uint32_t* inds, uint32_t slots, uint32_t experts, uint32_t* cursor,
-                                     uint32_t* order, uint32_t* inv) {
+// every slot's sorted position (inv), and per position the x row it reads and its (bank << 24 | expert inside the bank)
+__global__ void route_scatter_kernel(const uint32_t* inds, uint32_t slots, const __grid_constant__ ExpertMap map, const uint32_t* rank,
+                                     const uint32_t* first, const uint32_t* row_map, uint32_t topk, uint2* where, uint32_t* inv) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= slots) return;
-    const uint32_t p = atomicAdd(&cursor[min(inds[s], experts - 1u)], 1u);
-    order[p] = s;
+    const uint32_t e = map.number(inds[s]), p = first[e] + rank[s], b = map.bank(e);
+    where[p] = make_uint2(row_map ? row_map[s] : s / topk, (b << 24) | (e - map.base[b]));
     inv[s] = p;
 }
 
@@ -103,55 +167,55 @@ __device__ __forceinline__ bool my_position(uint32_t count, uint32_t lane, uint3
     return true;
 }
 
-// grid (spread, ceil(P / 64)), 256 threads. Dense: position = row, suh shared. Routed: position p -> slot order[p] -> row
-// slot / topk, suh of the slot's expert; the second op (up) reuses the row with its own suh.
+// grid (spread, ceil(P / 64)), 256 threads. Dense and one-expert calls (where null): positions are the call's rows. Routed: position p reads row
+// where[p].x with the scales of its expert (where[p].y); the second op (up) reuses the row with its own suh.
 struct PrepArgs {
     const void* x;
     int x_dt;
-    const __half* suh[2];
-    uint32_t K, positions, topk, experts, ops;
-    const uint32_t *order, *inds;  // null for a dense linear
-    const uint32_t* row_map;       // routed: the x row of each row-slot when the call gathers rows, else slot / topk
-    __half* xp;                    // [ops][positions][K]
+    const __half* suh[2][kMixedBanksMax];  // per op and bank, expert-major
+    uint32_t K, positions, ops;
+    const uint2* where;
+    const uint32_t* row_map;  // where null: position p reads row row_map[p], or row p / topk
+    uint32_t topk;
+    __half* xp;  // [ops][positions][K]
 };
-__global__ void __launch_bounds__(256, 3) prep_rows_kernel(const PrepArgs a) {
+__global__ void __launch_bounds__(256, 3) prep_rows_kernel(const __grid_constant__ PrepArgs a) {
     const uint32_t lane = threadIdx.x & 31u, q = lane & 3u;
     uint32_t p;
     bool live;
     if (!my_position(a.positions, lane, p, live)) return;
-    uint32_t row = p, e = 0;
-    if (a.order) {
-        const uint32_t slot = a.order[p];
-        row = a.row_map ? a.row_map[slot] : slot / a.topk;
-        e = min(a.inds[slot], a.experts - 1u);
+    uint32_t row, e = 0, bank = 0;
+    if (a.where) {
+        const uint2 w = a.where[p];
+        row = w.x, bank = w.y >> 24, e = w.y & 0xFFFFFFu;
+    } else {
+        row = a.row_map ? a.row_map[p] : p / a.topk;
     }
+    const __half* suh[2];
+#pragma unroll
+    for (int op = 0; op < 2; ++op) suh[op] = a.suh[op][bank] + (size_t)e * a.K;
+    const bool wide_x = aligned16(a.x), wide_s = aligned16(suh[0]) && aligned16(suh[1]);
     const HadB hb = had_b(lane);
     for (uint32_t blk = blockIdx.x; blk < (a.K >> 7); blk += gridDim.x) {
-        const uint32_t col = blk * 128u + 4u * q;
-        float xv[8][4];
+        const uint32_t col = blk * 128u + 8u * q;
+        uint32_t x[4][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) load_act4(a.x, a.x_dt, (size_t)row * a.K + col + 16u * i, xv[i]);
+        for (int s = 0; s < 4; ++s) load_half8(a.x, a.x_dt, wide_x, (size_t)row * a.K + col + 32u * s, x[s]);
+#pragma unroll 1
         for (uint32_t op = 0; op < a.ops; ++op) {
-            const __half* suh = (op ? a.suh[1] : a.suh[0]) + (size_t)e * a.K + col;
-            float v[8][4], out[8][4];
-            bool unit = true;
+            const __half* sp = (op ? suh[1] : suh[0]) + col;
+            uint32_t w[4][4], sc[4][4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                float sc[4];
-                load_half4(suh + 16 * i, sc);
-                unit = unit && all_unit(sc);
+            for (int s = 0; s < 4; ++s) {
+                load_16b(sp + 32 * s, wide_s, sc[s]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) v[i][j] = round_half(xv[i][j]) * sc[j];
+                for (int j = 0; j < 4; ++j) w[s][j] = x[s][j];
             }
-            h128_split(v, __all_sync(0xFFFFFFFFu, unit) != 0, hb, out);
+            rotate_block(w, sc, hb);
             if (live) {
-                const size_t o = ((size_t)op * a.positions + p) * a.K + col;
+                uint4* o = reinterpret_cast<uint4*>(a.xp + ((size_t)op * a.positions + p) * a.K + col);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) out[i][j] *= kHadScale;
-                    store_act4(a.xp, kF16, o + 16u * i, out[i]);
-                }
+                for (int s = 0; s < 4; ++s) o[4 * s] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
             }
         }
     }
@@ -171,53 +235,54 @@ __device__ __forceinline__ float swiglu_f32(float g, float u, float limit, int c
 // down projection's prepare, per sorted position
 struct MidArgs {
     const __half* z;  // [2][P][inter]: finished gate, finished up
-    const __half* down_suh;
-    const uint32_t *order, *inds;
-    uint32_t positions, inter, experts;
+    const __half* down_suh[kMixedBanksMax];
+    const uint2* where;  // or null: one expert
+    uint32_t positions, inter;
     float limit;
     int clamp_at;
     __half* hd;  // [P][inter]
 };
-__global__ void __launch_bounds__(256, 3) mid_kernel(const MidArgs a) {
+__global__ void __launch_bounds__(256, 3) mid_kernel(const __grid_constant__ MidArgs a) {
     const uint32_t lane = threadIdx.x & 31u, q = lane & 3u;
     uint32_t p;
     bool live;
     if (!my_position(a.positions, lane, p, live)) return;
-    const uint32_t e = min(a.inds[a.order[p]], a.experts - 1u);
+    const uint32_t id = a.where ? a.where[p].y : 0u;
+    const __half* suh = a.down_suh[id >> 24] + (size_t)(id & 0xFFFFFFu) * a.inter;
+    const bool wide_s = aligned16(suh);
     const HadB hb = had_b(lane);
     for (uint32_t blk = blockIdx.x; blk < (a.inter >> 7); blk += gridDim.x) {
-        const size_t eo = (size_t)e * a.inter + blk * 128u + 4u * q, zo = (size_t)p * a.inter + blk * 128u + 4u * q;
-        float g[8][4], u[8][4];
+        const uint32_t col = blk * 128u + 8u * q;
+        const size_t zo = (size_t)p * a.inter + col;
+        uint32_t g[4][4], u[4][4], sc[4][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            load_half4(a.z + zo + 16 * i, g[i]);
-            load_half4(a.z + (size_t)a.positions * a.inter + zo + 16 * i, u[i]);
+        for (int s = 0; s < 4; ++s) {
+            load_16b(a.z + zo + 32 * s, true, g[s]);
+            load_16b(a.z + (size_t)a.positions * a.inter + zo + 32 * s, true, u[s]);
         }
-        bool unit = true;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            float sd[4];
-            load_half4(a.down_suh + eo + 16 * i, sd);
-            unit = unit && all_unit(sd);
+        for (int s = 0; s < 4; ++s)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) g[i][j] = round_half(swiglu_f32(g[i][j], u[i][j], a.limit, a.clamp_at)) * sd[j];
-        }
-        h128_split(g, __all_sync(0xFFFFFFFFu, unit) != 0, hb, u);
-        if (live)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) u[i][j] *= kHadScale;
-                store_act4(a.hd, kF16, zo + 16u * i, u[i]);
+            for (int j = 0; j < 4; ++j) {
+                const float2 gv = unpack_half2(g[s][j]), uv = unpack_half2(u[s][j]);
+                g[s][j] = pack_half2(swiglu_f32(gv.x, uv.x, a.limit, a.clamp_at), swiglu_f32(gv.y, uv.y, a.limit, a.clamp_at));
             }
+#pragma unroll
+        for (int s = 0; s < 4; ++s) load_16b(suh + col + 32 * s, wide_s, sc[s]);  // (with the loads above it cost spills)
+        rotate_block(g, sc, hb);
+        if (live) {
+            uint4* o = reinterpret_cast<uint4*>(a.hd + zo);
+#pragma unroll
+            for (int s = 0; s < 4; ++s) o[4 * s] = make_uint4(g[s][0], g[s][1], g[s][2], g[s][3]);
+        }
     }
 }
 
-// grid (spread, ceil(rows / 64)): per row, the score-weighted sum of its slots' finished down outputs (through inv) in
+// grid (spread, ceil(rows / 8)): per row, the score-weighted sum of its slots' finished down outputs (through inv) in
 // slot order, then the optional shared-expert add in the output dtype
 struct FinArgs {
     const __half* zd;  // [P][hidden]: each sorted position's finished down output (the per-slot v)
-    const uint32_t* inv;
+    const uint32_t* inv;  // or null: slot s's is row s
     const void* scores;
     int score_dt;
     const void* shared;
@@ -226,38 +291,51 @@ struct FinArgs {
     uint32_t rows, hidden, topk;
 };
 __global__ void __launch_bounds__(256) moe_fin_kernel(const FinArgs a) {
-    // a warp a row, a lane four consecutive elements of a 128-block: every slot's 256 bytes are one coalesced read
+    // A warp a row, a lane eight consecutive elements of two 128-blocks: a slot's 512 bytes are one coalesced read, eight slots'
+    // in flight at once (four 8-byte reads a lane left the kernel waiting on memory: 49 us where its bytes take 28).
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t row = blockIdx.y * 8u + warp;
     if (row >= a.rows) return;
-    for (uint32_t blk = blockIdx.x; blk < (a.hidden >> 7); blk += gridDim.x) {
-        const uint32_t col = blk * 128u + 4u * lane;
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (uint32_t k0 = 0; k0 < a.topk; k0 += 4u) {  // four slots' loads in flight, the sum still in slot order
-            float w[4], v[4][4];
+    for (uint32_t col = (blockIdx.x * 32u + lane) * 8u; col < a.hidden; col += gridDim.x * 256u) {
+        float acc[8] = {};
+        for (uint32_t k0 = 0; k0 < a.topk; k0 += 8u) {
+            uint4 v[8];
+            float w[8];
 #pragma unroll
-            for (uint32_t i = 0; i < 4u; ++i) {
+            for (uint32_t i = 0; i < 8u; ++i) {
                 const uint32_t k = k0 + i < a.topk ? k0 + i : a.topk - 1u;
                 const size_t slot = (size_t)row * a.topk + k;
+                if (k0 + i >= a.topk) break;
                 w[i] = load_act(a.scores, a.score_dt, slot);
-                load_half4(a.zd + (size_t)a.inv[slot] * a.hidden + col, v[i]);
+                v[i] = *reinterpret_cast<const uint4*>(a.zd + (size_t)(a.inv ? a.inv[slot] : (uint32_t)slot) * a.hidden + col);
             }
 #pragma unroll
-            for (uint32_t i = 0; i < 4u; ++i)
-                if (k0 + i < a.topk)
+            for (uint32_t i = 0; i < 8u; ++i) {
+                if (k0 + i >= a.topk) break;
+                const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[j] = __fadd_rn(acc[j], __fmul_rn(w[i], v[i][j]));
+                for (int j = 0; j < 4; ++j) {
+                    const float2 f = unpack_half2(u[j]);
+                    acc[2 * j] = __fadd_rn(acc[2 * j], __fmul_rn(w[i], f.x));
+                    acc[2 * j + 1] = __fadd_rn(acc[2 * j + 1], __fmul_rn(w[i], f.y));
+                }
+            }
         }
-        const size_t o = (size_t)row * a.hidden + col;
-        if (a.shared) {
-            float t[4], sh[4];
-            store_act4(a.y, a.y_dt, o, acc);  // the routed output's rounding point
-            load_act4(a.y, a.y_dt, o, t);
-            load_act4(a.shared, a.y_dt, o, sh);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[j] = __fadd_rn(t[j], sh[j]);
+        for (int half = 0; half < 2; ++half) {
+            float f[4] = {acc[4 * half], acc[4 * half + 1], acc[4 * half + 2], acc[4 * half + 3]};
+            const size_t o = (size_t)row * a.hidden + col + 4u * half;
+            if (a.shared) {
+                float sh[4];
+                load_act4(a.shared, a.y_dt, o, sh);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {  // the routed output's rounding point, then the add in f32
+                    const float t = a.y_dt == kF32 ? f[j] : a.y_dt == kF16 ? round_half(f[j]) : __bfloat162float(__float2bfloat16_rn(f[j]));
+                    f[j] = __fadd_rn(t, sh[j]);
+                }
+            }
+            store_act4(a.y, a.y_dt, o, f);
         }
-        store_act4(a.y, a.y_dt, o, acc);
     }
 }
 
@@ -395,11 +473,10 @@ cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cuda
     PrepArgs pa = {};
     pa.x = p.x;
     pa.x_dt = p.x_dt;
-    pa.suh[0] = pa.suh[1] = static_cast<const __half*>(p.suh);
+    pa.suh[0][0] = pa.suh[1][0] = static_cast<const __half*>(p.suh);
     pa.K = p.in;
     pa.positions = p.rows;
     pa.topk = 1;
-    pa.experts = 1;
     pa.xp = xp;
     pa.ops = 1;
     prep_rows_kernel<<<dim3(spread(p.rows, p.in / 128u), (p.rows + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream>>>(pa);
@@ -459,9 +536,9 @@ cudaError_t launch_plain_linear(const void* x, int dt, uint32_t rows, const void
 
 namespace {
 struct MoeWs {
-    uint32_t *counts, *cursor, *order, *inv;
+    uint32_t *counts, *first, *rank, *inv, *range;
+    uint2* where;
     int4* tiles;
-    uint32_t* n_tiles;
     __half *xp, *zgu, *hd, *zd;
     size_t total;
 };
@@ -473,12 +550,13 @@ MoeWs carve_moe(uint8_t* base, size_t slots, uint32_t experts, uint32_t hidden, 
         off += up256(bytes);
         return p;
     };
-    w.counts = reinterpret_cast<uint32_t*>(take((size_t)experts * 4u));
-    w.cursor = reinterpret_cast<uint32_t*>(take((size_t)experts * 4u));
-    w.order = reinterpret_cast<uint32_t*>(take(slots * 4u));
+    w.counts = reinterpret_cast<uint32_t*>(take(((size_t)experts + 1u) * 4u));  // and the ticket
+    w.first = reinterpret_cast<uint32_t*>(take((size_t)experts * 4u));
+    w.rank = reinterpret_cast<uint32_t*>(take(slots * 4u));
     w.inv = reinterpret_cast<uint32_t*>(take(slots * 4u));
+    w.where = reinterpret_cast<uint2*>(take(slots * 8u));
     w.tiles = reinterpret_cast<int4*>(take(routed_tiles_max(slots, experts) * 16u));
-    w.n_tiles = reinterpret_cast<uint32_t*>(take(4u));
+    w.range = reinterpret_cast<uint32_t*>(take((kMixedBanksMax + 1u) * 4u));
     w.xp = reinterpret_cast<__half*>(take(2u * slots * hidden * 2u));
     w.zgu = reinterpret_cast<__half*>(take(2u * slots * inter * 2u));
     w.hd = reinterpret_cast<__half*>(take(slots * inter * 2u));
@@ -493,83 +571,125 @@ size_t prefill_moe_workspace(size_t rows, uint32_t topk, uint32_t experts, uint3
     return carve_moe(nullptr, rows * topk, experts, hidden, inter).total;
 }
 
-cudaError_t launch_prefill_moe(const MoeArgs& a, void* workspace, int codebook, cudaStream_t stream, int* launches) {
+cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* workspace, int codebook, cudaStream_t stream,
+                               int* launches) {
     const size_t slots = (size_t)a.rows * a.topk;
     const uint32_t S = (uint32_t)slots, H = a.hidden, I = a.inter;
-    MoeWs w = carve_moe(static_cast<uint8_t*>(workspace), slots, a.experts, H, I);
+    const MoeWs w = carve_moe(static_cast<uint8_t*>(workspace), slots, a.experts, H, I);
     const uint32_t* inds = static_cast<const uint32_t*>(a.inds);
-    cudaError_t rc = cudaMemsetAsync(w.counts, 0, (size_t)a.experts * 4u, stream);
-    if (rc != cudaSuccess) return rc;
-    route_count_kernel<<<(S + 255u) / 256u, 256, 0, stream>>>(inds, S, a.experts, w.counts);
-    route_plan_kernel<<<1, 1024, 0, stream>>>(w.counts, a.experts, w.cursor, w.tiles, w.n_tiles);
-    route_scatter_kernel<<<(S + 255u) / 256u, 256, 0, stream>>>(inds, S, a.experts, w.cursor, w.order, w.inv);
-
+    MixedBanks one;
+    if (!mixed) {
+        one.count = 1;
+        one.n[0] = a.n;
+        one.bank[0] = {a.gate_t, a.up_t, a.down_t, a.gate_suh, a.gate_svh, a.up_suh, a.up_svh, a.down_suh, a.down_svh, a.experts};
+    }
+    const MixedBanks& banks = mixed ? *mixed : one;
+    // one expert (a shared expert's chain): the slots are in order as they stand, the chain is a dense one
+    const bool routed = a.experts > 1u;
+    cudaError_t rc;
+    if (routed) {
+        ExpertMap map = {};
+        map.banks = banks.count;
+        map.ids = mixed ? mixed->ids : a.experts;
+        map.bank_of = mixed ? mixed->bank_of : nullptr;
+        map.local_of = mixed ? mixed->local_of : nullptr;
+        for (uint32_t b = 0; b < banks.count; ++b) map.base[b + 1u] = map.base[b] + banks.bank[b].experts;
+        rc = cudaMemsetAsync(w.counts, 0, ((size_t)a.experts + 1u) * 4u, stream);
+        if (rc != cudaSuccess) return rc;
+        route_plan_kernel<<<(S + kRouteSlots - 1u) / kRouteSlots, kRouteThreads, a.experts <= kRouteExperts ? a.experts * 4u : 0u, stream>>>(
+            inds, S, map, w.counts, w.counts + a.experts, w.rank, w.first, w.tiles, w.range);
+        route_scatter_kernel<<<(S + 255u) / 256u, 256, 0, stream>>>(inds, S, map, w.rank, w.first, a.row_map, a.topk, w.where, w.inv);
+        *launches += 2;
+    }
     PrepArgs pa = {};
     pa.x = a.x;
     pa.x_dt = a.x_dt;
-    pa.suh[0] = static_cast<const __half*>(a.gate_suh);
-    pa.suh[1] = static_cast<const __half*>(a.up_suh);
+    MidArgs m = {};
+    for (uint32_t b = 0; b < banks.count; ++b) {
+        pa.suh[0][b] = static_cast<const __half*>(banks.bank[b].gate_suh);
+        pa.suh[1][b] = static_cast<const __half*>(banks.bank[b].up_suh);
+        m.down_suh[b] = static_cast<const __half*>(banks.bank[b].down_suh);
+    }
     pa.K = H;
     pa.positions = S;
-    pa.topk = a.topk;
-    pa.experts = a.experts;
-    pa.order = w.order;
-    pa.inds = inds;
+    pa.where = m.where = routed ? w.where : nullptr;
     pa.row_map = a.row_map;
+    pa.topk = a.topk;
     pa.xp = w.xp;
     pa.ops = 2;
     prep_rows_kernel<<<dim3(spread(S, H / 128u), (S + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream>>>(pa);
 
-    // two 128-output blocks a unit of work: a tile of up to 128 rows runs both on one copy of its rows
-    const size_t max_tiles = routed_tiles_max(slots, a.experts);
-    auto units = [&](uint32_t outs, uint32_t ops) {
-        const size_t u = max_tiles * ops * ((outs / 128u + 1u) / 2u);
-        return (uint32_t)(u < (1u << 20) ? u : 1u << 20);
+    // A unit of work is two 128-output blocks where tiles of up to 128 rows are the rule (both run on one copy of the rows) and
+    // there are units enough for every multiprocessor; else one.
+    auto gemm = [&](DecodeGemmArgs& g, const __half* rows, uint64_t rows_total) -> cudaError_t {
+        const uint32_t ncol = g.N / 128u;
+        g.mask = a.mask;
+        g.op_rows = S;
+        g.err = a.err;
+        const bool down = g.ops == 1u;
+        for (uint32_t b = 0; b < banks.count; ++b) {
+            const BankTab& t = banks.bank[b];
+            if (t.experts == 0u) continue;
+            g.n = banks.n[b];
+            g.svh[0] = static_cast<const __half*>(down ? t.down_svh : t.gate_svh);  // the epilogue finishes with the tile's expert's scales
+            g.svh[1] = static_cast<const __half*>(t.up_svh);
+            g.svh_stride = g.N;
+            size_t units;
+            if (routed) {
+                const size_t tiles = routed_tiles_max(slots, t.experts);
+                g.pair = slots <= (size_t)160u * a.experts && tiles * g.ops * ((ncol + 1u) / 2u) >= 2u * one_wave_ctas() ? 2u : 1u;
+                g.tiles = w.tiles;
+                g.range = w.range + b;
+                units = tiles * g.ops * ((ncol + g.pair - 1u) / g.pair);
+            } else {
+                g.pair = 1;
+                g.dense_rows = S;
+                g.tile_rows = dense_tile_rows(S, g.K, ncol * g.ops);
+                g.dense_tiles = (S + g.tile_rows - 1u) / g.tile_rows;
+                units = (size_t)g.dense_tiles * g.ops * ncol;
+            }
+            GemmMaps maps;
+            if (!make_gemm_maps(&maps, rows, rows_total, g.K, down ? t.down_t : t.gate_t, down ? nullptr : t.up_t, g.N, g.n, t.experts))
+                return cudaErrorNotSupported;
+            const cudaError_t e = launch_decode_gemm(maps, g, (uint32_t)(units < (1u << 20) ? units : 1u << 20), codebook, stream);
+            if (e != cudaSuccess) return e;
+            *launches += 1;
+        }
+        return cudaSuccess;
     };
-    GemmMaps maps;
-    if (!make_gemm_maps(&maps, w.xp, 2u * slots, H, a.gate_t, a.up_t, I, a.n, a.experts)) return cudaErrorNotSupported;
-    DecodeGemmArgs g = {};
-    g.K = H;
-    g.N = I;
-    g.n = a.n;
-    g.mask = a.mask;
-    g.ops = 2;
-    g.op_rows = S;
-    g.tiles = w.tiles;
-    g.n_tiles = w.n_tiles;
-    g.pair = 2;
-    g.z = w.zgu;
-    g.z_op_stride = slots * I;
-    g.svh[0] = static_cast<const __half*>(a.gate_svh);  // the epilogue finishes gate and up with the tile's expert's scales
-    g.svh[1] = static_cast<const __half*>(a.up_svh);
-    g.svh_stride = I;
-    g.err = a.err;
-    rc = launch_decode_gemm(maps, g, units(I, 2u), codebook, stream);
+    DecodeGemmArgs gu = {};
+    gu.K = H;
+    gu.N = I;
+    gu.ops = 2;
+    gu.z = w.zgu;
+    gu.z_op_stride = slots * I;
+    rc = gemm(gu, w.xp, 2u * slots);
     if (rc != cudaSuccess) return rc;
 
-    MidArgs m = {w.zgu, static_cast<const __half*>(a.down_suh), w.order, inds, S, I, a.experts, a.limit, a.clamp_at, w.hd};
+    m.z = w.zgu;
+    m.positions = S;
+    m.inter = I;
+    m.limit = a.limit;
+    m.clamp_at = a.clamp_at;
+    m.hd = w.hd;
     mid_kernel<<<dim3(spread(S, I / 128u), (S + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream>>>(m);
 
-    if (!make_gemm_maps(&maps, w.hd, slots, I, a.down_t, nullptr, H, a.n, a.experts)) return cudaErrorNotSupported;
-    DecodeGemmArgs d = g;
+    DecodeGemmArgs d = {};
     d.K = I;
     d.N = H;
     d.ops = 1;
-    d.z = w.zd;
-    d.z_op_stride = 0;
-    d.svh[0] = d.svh[1] = static_cast<const __half*>(a.down_svh);  // each slot's finished down output, the per-slot v
-    d.svh_stride = H;
-    rc = launch_decode_gemm(maps, d, units(H, 1u), codebook, stream);
+    d.z = w.zd;  // each slot's finished down output, the per-slot v
+    rc = gemm(d, w.hd, slots);
     if (rc != cudaSuccess) return rc;
 
-    FinArgs f = {w.zd, w.inv, a.scores, a.score_dt, a.shared, a.y, a.y_dt, a.rows, H, a.topk};
+    FinArgs f = {w.zd, routed ? w.inv : nullptr, a.scores, a.score_dt, a.shared, a.y, a.y_dt, a.rows, H, a.topk};
     if (a.shared_ready) {  // only this launch reads `shared`
         rc = cudaStreamWaitEvent(stream, static_cast<cudaEvent_t>(a.shared_ready), 0);
         if (rc != cudaSuccess) return rc;
     }
-    const uint32_t fin_groups = (a.rows + 7u) / 8u, fin_want = (1184u + fin_groups - 1u) / fin_groups;
-    moe_fin_kernel<<<dim3(fin_want < H / 128u ? fin_want : H / 128u, fin_groups), 256, 0, stream>>>(f);
-    *launches += 8;
+    const uint32_t fin_groups = (a.rows + 7u) / 8u, fin_want = (1184u + fin_groups - 1u) / fin_groups, fin_cols = (H + 255u) / 256u;
+    moe_fin_kernel<<<dim3(fin_want < fin_cols ? fin_want : fin_cols, fin_groups), 256, 0, stream>>>(f);
+    *launches += 3;
     return cudaGetLastError();
 }
 
