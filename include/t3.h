@@ -172,6 +172,17 @@ int t3_moe_swiglu_rows(const void* x, int x_dtype, size_t x_rows, const void* ro
 int t3_moe_clamped_banked(const void* x, int x_dtype, size_t rows, const t3_bank* banks, const void* ids, t3_decode dec,
                           int limit, void* y, int y_dtype, void* workspace, size_t workspace_bytes, void* stream);
 
+/* A routed layer whose experts have rates of their own, more than 32 rows (the reference serves one rate per bank,
+ * src/root.zig:841): `count` banks of one geometry (1..T3_MIXED_BANKS_MAX), each at its own rate; layer expert g (0 .. ids - 1, the
+ * router's numbering) is expert local_of[g] of bank bank_of[g] (device int64 arrays, every entry in range: not checked). One
+ * sort, one prepare and one merge for the whole layer: y is, bit for bit, what one bank of those experts would give. `shared` as
+ * in t3_moe_with_shared, or null. Up to 32 rows: Exl3EngineNotImplemented. */
+#define T3_MIXED_BANKS_MAX 8
+size_t t3_moe_mixed_workspace_bytes(size_t rows, int topk, const t3_bank* banks, int count);
+int t3_moe_mixed(const void* x, int x_dtype, size_t rows, const t3_bank* banks, int count, const void* bank_of, const void* local_of,
+                 int ids, const void* inds, const void* scores, int scores_dtype, int topk, t3_decode dec, const void* shared, void* y,
+                 void* workspace, size_t workspace_bytes, void* stream);
+
 /* t3_moe_with_shared for a shared-expert output that another stream is still computing: `shared_ready` is a cudaEvent_t
  * recorded on that stream after `shared` was written. Only the call's last launch (the one that adds `shared`) waits for
  * the event, so the routed experts' launches run beside the shared expert's. The reference's moeWithShared

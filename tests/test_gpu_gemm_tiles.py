@@ -47,3 +47,22 @@ def test_routed_tile_edges(case):
     ref = ob.moe_rows(obank, host_f32(x)[sample], inds[sample].reshape(-1, 1), np.ones((len(sample), 1), np.float32), cb, 16, 0.0, 0)
     check_moe(host_f32(y).reshape(rows, hidden)[sample], ref, dt, ("routed tile edges", case))
     assert t3.device_error() == 0
+
+
+@pytest.mark.parametrize("rows,dt", [(33, "f16"), (300, "bf16")])
+def test_mixed_banks_give_the_one_bank_bytes(rows, dt):
+    """Experts dealt over three banks (one of them with a single expert) at one rate: the bytes of the undivided bank."""
+    H, I, E, topk, n = 384, 256, 11, 4, 48
+    bank, _ = make_bank(2300, E, H, I, n)
+    bank_of = torch.tensor([0, 2, 0, 2, 2, 0, 1, 0, 2, 0, 2])
+    local_of = torch.zeros_like(bank_of)
+    for b in range(3):
+        local_of[bank_of == b] = torch.arange(int((bank_of == b).sum()))
+    pick = lambda p, b: t3.Proj(*(v[(bank_of == b).to(v.device)].contiguous() for v in (p.trellis.view(torch.int16), p.suh, p.svh)))
+    banks = [t3.Bank(pick(bank.gate, b), pick(bank.up, b), pick(bank.down, b)) for b in range(3)]
+    inds, scores = synth.routing(2301, rows, E, topk)
+    x, di, ds = x_as(synth.activations(2302, rows, H), dt), dev(inds), dev(scores)
+    whole = t3.moe(x.view(1, rows, H), bank, di.view(1, rows, topk), ds.view(1, rows, topk))
+    mixed = t3.moe_mixed(x, banks, bank_of.cuda(), local_of.cuda(), di, ds)
+    assert torch.equal(whole.view(rows, H), mixed)
+    assert t3.device_error() == 0

@@ -85,6 +85,8 @@ SYMBOLS = {
     "t3_moe_clamped": (_i, [_vp, _i, _sz, C.POINTER(_Bank), _vp, _vp, _i, _i, _Decode, _i, _vp, _vp, _sz, _vp]),
     "t3_moe_with_shared": (_i, [_vp, _i, _sz, C.POINTER(_Bank), _vp, _vp, _i, _i, _Decode, _vp, _vp, _vp, _sz, _vp]),
     "t3_moe_swiglu_rows": (_i, [_vp, _i, _sz, _vp, _sz, C.POINTER(_Bank), _vp, _vp, _i, _Decode, _i, _i, _vp, _i, _vp, _sz, _vp]),
+    "t3_moe_mixed_workspace_bytes": (_sz, [_sz, _i, C.POINTER(_Bank), _i]),
+    "t3_moe_mixed": (_i, [_vp, _i, _sz, C.POINTER(_Bank), _i, _vp, _vp, _i, _vp, _vp, _i, _i, _Decode, _vp, _vp, _vp, _sz, _vp]),
     "t3_moe_with_shared_after": (_i, [_vp, _i, _sz, C.POINTER(_Bank), _vp, _vp, _i, _i, _Decode, _vp, _vp, _vp, _vp, _sz, _vp]),
     "t3_moe_merge": (_i, [_vp, _vp, _i, _sz, _i, _i, _vp, _vp, _i, _vp]),
     "t3_moe_merge_mapped": (_i, [_vp, _vp, _vp, _i, _sz, _i, _i, _vp, _vp, _i, _vp]),
@@ -421,6 +423,38 @@ def moe_swiglu_rows(x: torch.Tensor, rows: torch.Tensor, bank: Bank, inds: torch
     _check(L.t3_moe_swiglu_rows(x.data_ptr(), _DTYPES[x.dtype], x.shape[0], rows.data_ptr(), S, C.byref(cb), inds.data_ptr(),
                                 scores.data_ptr(), _DTYPES[scores.dtype], dec._c(), limit, clamp_at, y.data_ptr(),
                                 _DTYPES[out_dtype], ws.data_ptr(), ws_bytes, _stream_ptr(x)))
+    return y
+
+
+MIXED_BANKS_MAX = 8
+
+
+def moe_mixed(x: torch.Tensor, banks, bank_of: torch.Tensor, local_of: torch.Tensor, inds: torch.Tensor, scores: torch.Tensor,
+              dec: Decode = Decode.mul1, shared: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """A routed layer whose experts have rates of their own (t3_moe_mixed), more than 32 rows: x [rows, hidden], banks up to
+    MIXED_BANKS_MAX `Bank`s of one geometry, layer expert g = expert local_of[g] of bank bank_of[g] (int64), inds / scores
+    [rows, topk]; y [rows, hidden] in x's dtype."""
+    _need_cuda(x, bank_of, local_of, inds, scores)
+    if x.dim() != 2 or inds.dim() != 2 or inds.shape != scores.shape or inds.shape[0] != x.shape[0] or x.shape[1] % 128:
+        raise Exl3Error(1, "BadExl3Shape")
+    if bank_of.dim() != 1 or bank_of.shape != local_of.shape or not 1 <= len(banks) <= MIXED_BANKS_MAX:
+        raise Exl3Error(1, "BadExl3Shape")
+    if (x.dtype not in _DTYPES or inds.dtype not in (torch.int32, torch.uint32) or scores.dtype not in _DTYPES
+            or bank_of.dtype != torch.int64 or local_of.dtype != torch.int64):
+        raise Exl3Error(2, "BadExl3Dtype")
+    if shared is not None:
+        _need_cuda(shared)
+        if shared.dtype != x.dtype or shared.numel() != x.numel():
+            raise Exl3Error(1, "BadExl3Shape")
+    cbs = (_Bank * len(banks))(*[_bank_c(b, x.shape[1]) for b in banks])
+    rows, topk = inds.shape
+    L = lib()
+    ws_bytes = L.t3_moe_mixed_workspace_bytes(rows, topk, cbs, len(banks))
+    ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=x.device)
+    y = torch.empty_like(x)
+    _check(L.t3_moe_mixed(x.data_ptr(), _DTYPES[x.dtype], rows, cbs, len(banks), bank_of.data_ptr(), local_of.data_ptr(), bank_of.numel(),
+                          inds.data_ptr(), scores.data_ptr(), _DTYPES[scores.dtype], topk, dec._c(),
+                          shared.data_ptr() if shared is not None else None, y.data_ptr(), ws.data_ptr(), ws_bytes, _stream_ptr(x)))
     return y
 
 

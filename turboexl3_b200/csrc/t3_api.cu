@@ -849,6 +849,70 @@ int t3_moe_clamped(const void* x, int x_dtype, size_t rows, const t3_bank* bank,
                     nullptr, y, workspace, workspace_bytes, stream);
 }
 
+size_t t3_moe_mixed_workspace_bytes(size_t rows, int topk, const t3_bank* banks, int count) {
+    if (!banks || count < 1 || count > T3_MIXED_BANKS_MAX || topk <= 0) return 0;
+    size_t experts = 0;
+    for (int b = 0; b < count; ++b) experts += banks[b].experts > 0 ? (size_t)banks[b].experts : 0u;
+    if (experts == 0 || banks[0].hidden <= 0 || banks[0].inter <= 0) return 0;
+    return prefill_moe_workspace(rows, (uint32_t)topk, (uint32_t)experts, (uint32_t)banks[0].hidden, (uint32_t)banks[0].inter);
+}
+
+int t3_moe_mixed(const void* x, int x_dtype, size_t rows, const t3_bank* banks, int count, const void* bank_of, const void* local_of,
+                 int ids, const void* inds, const void* scores, int scores_dtype, int topk, t3_decode dec, const void* shared, void* y,
+                 void* workspace, size_t workspace_bytes, void* stream) {
+    if (!x || !banks || !bank_of || !local_of || !inds || !scores || !y) return T3_NULL_POINTER;
+    if (count < 1 || count > T3_MIXED_BANKS_MAX || ids < 1 || rows < 1 || rows > (size_t)1 << 30 || topk <= 0 || topk > T3_REDUCE_MAX_TOPK)
+        return T3_BAD_EXL3_SHAPE;
+    MixedBanks mixed = {};
+    size_t experts = 0;
+    for (int b = 0; b < count; ++b) {
+        const t3_bank& k = banks[b];
+        if (int rc = validate_bank(&k, banks[0].hidden)) return rc;
+        if (k.inter != banks[0].inter) return T3_BAD_EXL3_SHAPE;
+        mixed.bank[b] = {static_cast<const uint8_t*>(k.gate.trellis), static_cast<const uint8_t*>(k.up.trellis),
+                         static_cast<const uint8_t*>(k.down.trellis), k.gate.suh, k.gate.svh, k.up.suh, k.up.svh, k.down.suh, k.down.svh,
+                         (uint32_t)k.experts};
+        mixed.n[b] = (uint32_t)k.n_gate;
+        experts += (size_t)k.experts;
+    }
+    if (experts > 1u << 24) return T3_BAD_EXL3_SHAPE;
+    if (!dtype_ok(x_dtype) || !dtype_ok(scores_dtype)) return T3_BAD_EXL3_DTYPE;
+    uint32_t mask;
+    if (int rc = decode_mask(dec, mask)) return rc;
+    if (rows <= T3_DECODE_ROWS_MAX) return T3_ENGINE_NOT_IMPLEMENTED;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        if (!g_cfg.prefill) return T3_ENGINE_NOT_IMPLEMENTED;
+    }
+    const size_t slots = rows * (size_t)topk, wide = (size_t)(banks[0].hidden > banks[0].inter ? banks[0].hidden : banks[0].inter);
+    if (rows > kPrefillMoeRowsMax || slots > kPrefillSlotsMax || slots > 0x7FFFFFFFu / wide) return T3_BAD_EXL3_SHAPE;
+    if (!workspace || workspace_bytes < t3_moe_mixed_workspace_bytes(rows, topk, banks, count)) return T3_WORKSPACE_TOO_SMALL;
+    mixed.count = (uint32_t)count;
+    mixed.ids = (uint32_t)ids;
+    mixed.bank_of = static_cast<const int64_t*>(bank_of);
+    mixed.local_of = static_cast<const int64_t*>(local_of);
+    MoeArgs a = {};
+    a.x = x;
+    a.x_dt = a.y_dt = x_dtype;
+    a.inds = inds;
+    a.scores = scores;
+    a.score_dt = scores_dtype;
+    a.experts = (uint32_t)experts;
+    a.hidden = (uint32_t)banks[0].hidden;
+    a.inter = (uint32_t)banks[0].inter;
+    a.topk = (uint32_t)topk;
+    a.rows = (uint32_t)rows;
+    a.mask = mask;
+    a.y = y;
+    a.shared = shared;
+    a.err = dev_error_ptr();
+    for (int b = 0; b < count; ++b) note_engine(2, ((uint64_t)a.hidden << 32) | a.inter, (uint64_t)banks[b].experts, mixed.n[b], a.topk);
+    int launches = 0;
+    const cudaError_t rc = launch_prefill_moe(a, &mixed, workspace, dec.codebook, static_cast<cudaStream_t>(stream), &launches);
+    g_launches.fetch_add((uint64_t)launches, std::memory_order_relaxed);
+    return cuda_status(rc);
+}
+
 int t3_moe_clamped_banked(const void* x, int x_dtype, size_t rows, const t3_bank* banks, const void* ids, t3_decode dec,
                           int limit, void* y, int y_dtype, void* workspace, size_t workspace_bytes, void* stream) {
     if (!x || !banks || !ids || !y) return T3_NULL_POINTER;

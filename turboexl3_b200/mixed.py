@@ -3,9 +3,10 @@
 The reference serves one rate per bank (moe requires gate, up and down of a bank to share n: src/root.zig:841, and a
 bank's geometry carries a single rate: src/core/decode.zig Geometry.rate), so a layer whose experts were quantised at
 different bit widths is held as one sub-bank per rate. This module routes such a layer: every row-slot goes to the sub-bank
-that holds its expert, each sub-bank runs its slots at top-1 with score 1 (the finished down projection `v`, f16, exactly
-what the single-bank chain feeds its merge), and the score-weighted sum runs once over all slots in slot order
-(`t3.moe_merge`) — so the result is the one a single bank of those experts would give, whatever the bucketing.
+that holds its expert (the finished down projection `v`, f16, exactly what the single-bank chain feeds its merge), and the
+score-weighted sum runs once over all slots in slot order — so the result is the one a single bank of those experts would
+give, whatever the bucketing. Past 32 rows the whole layer is one native call (`api.moe_mixed`); decode rows, more than eight
+rates and injected stand-ins run each sub-bank's slots at top-1 with score 1 and merge with `t3.moe_merge`.
 """
 from __future__ import annotations
 
@@ -61,12 +62,18 @@ def mixed_rate_moe(x: torch.Tensor, banks: Sequence, buckets: RateBuckets, inds:
     """x [rows, hidden]; banks[b] = the sub-bank of rate buckets.rates[b]; inds/scores [rows, topk] with the layer's
     expert ids. Returns y [rows, hidden] in x's dtype. expert_fn(x_rows, bank, local_expert) -> v and
     merge_fn(v [rows, topk, hidden], scores) -> y default to the engine; tests inject host stand-ins."""
+    from . import api
+    rows, topk = inds.shape
+    if (expert_fn is None and merge_fn is None and rows > api.DECODE_ROWS_MAX and 0 < len(banks) <= api.MIXED_BANKS_MAX
+            and inds.dtype in (torch.int32, torch.uint32) and x.is_contiguous() and x.dim() == 2
+            and rows * topk * max(x.shape[1], banks[0].down.suh.shape[1]) < 1 << 31):  # the native call's index range
+        # one sort, one prepare and one merge for the layer, a GEMM pair a bank
+        return api.moe_mixed(x, banks, buckets.bank_of.to(x.device), buckets.local_of.to(x.device), inds.contiguous(),
+                             scores.contiguous(), dec, shared)
     if expert_fn is None:
         expert_fn = lambda xr, bank, er: expert_rows(xr, bank, er, dec)
     if merge_fn is None:
-        from . import api
         merge_fn = lambda vv, sc: api.moe_merge(vv, sc.contiguous(), x.dtype, shared)
-    rows, topk = inds.shape
     flat = inds.reshape(-1).to(torch.int64)
     bank_of, local_of = buckets.bank_of.to(flat.device), buckets.local_of.to(flat.device)
     slot_bank = bank_of[flat]
