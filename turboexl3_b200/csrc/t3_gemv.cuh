@@ -14,6 +14,8 @@
 // (src/kernels/hip/dense/dense.hip:49-145).
 #pragma once
 
+#include <type_traits>
+
 #include <cooperative_groups.h>
 
 #include "t3_common.cuh"
@@ -205,25 +207,30 @@ __device__ __forceinline__ void consume_slab(const uint8_t* ring, uint64_t* full
         if (CB == kProbeStream) {
             // timing probe: the stage has landed, nothing reads it
         } else if (N > 0) {
-            // the stage's four tiles of this warp, two at a time: words, then decodes, then tensor-core steps, so the
-            // dependent chains of two tiles overlap and the registers of four are never needed at once
+            // the stage's tiles of this warp, a batch at a time: words, then decodes, then tensor-core steps, so the dependent
+            // chains of a batch overlap and the registers of all are never needed at once. Full-width codewords (all packs but
+            // those with a narrower search width) take their windows without a mask: see decode_raw.
             uint32_t wa[kRaw];
 #pragma unroll
             for (uint32_t w = 0; w < kRaw; ++w) wa[w] = st + woff[w];
+            auto stage = [&](auto full) {
 #pragma unroll
-            for (uint32_t h = 0; h < kBatch; h += kHalfBatch) {
-                if (h >= tiles) break;
-                uint32_t raw[kHalfBatch][kRaw];
+                for (uint32_t h = 0; h < kBatch; h += kHalfBatch) {
+                    if (h >= tiles) break;
+                    uint32_t raw[kHalfBatch][kRaw];
 #pragma unroll
-                for (uint32_t i = 0; i < kHalfBatch; ++i)
+                    for (uint32_t i = 0; i < kHalfBatch; ++i)
 #pragma unroll
-                    for (uint32_t w = 0; w < kRaw; ++w) raw[i][w] = lds_u32(wa[w] + (h + i) * kKGroups * row_bytes);
-                uint32_t b[kHalfBatch][4];
+                        for (uint32_t w = 0; w < kRaw; ++w) raw[i][w] = lds_u32(wa[w] + (h + i) * kKGroups * row_bytes);
+                    uint32_t b[kHalfBatch][4];
 #pragma unroll
-                for (uint32_t i = 0; i < kHalfBatch; ++i) decode_raw<NP, CB>(raw[i], plan, mask, b[i]);
+                    for (uint32_t i = 0; i < kHalfBatch; ++i) decode_raw<NP, CB, decltype(full)::value>(raw[i], plan, mask, b[i]);
 #pragma unroll
-                for (uint32_t i = 0; i < kHalfBatch; ++i) mma_tile<RM>(acc, xs + (h + i) * kKGroups * 32u, ro, b[i]);
-            }
+                    for (uint32_t i = 0; i < kHalfBatch; ++i) mma_tile<RM>(acc, xs + (h + i) * kKGroups * 32u, ro, b[i]);
+                }
+            };
+            if (mask == 0xFFFFu) stage(std::true_type());
+            else stage(std::false_type());
         } else {
             const uint8_t* stp = ring + (st - ring0);
 #pragma unroll 1
