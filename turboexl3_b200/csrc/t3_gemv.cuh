@@ -175,7 +175,9 @@ __device__ __forceinline__ void mma_tile(float (&acc)[RowCap<RM>::kMB][2][4], ui
 // A full stage holds kStageRows tk rows, a warp's share of it kBatch tiles taken two at a time, and with the rate
 // a template constant every shared-memory offset inside a stage is an immediate.
 // HB: tiles whose words and fragments are in registers together (the routed kernels keep two: four spill there).
-template <int N, int CB, int RM, int HB = 2>
+// WINDOWS: full-width codewords at the rates whose windows are byte permutations take them so (decode_raw's FULL; the dense kernel:
+// 16384 -> 7168 at K4 38.9 -> 37.0 us; in the routed kernels, out of registers already, the second copy of the loop cost 2 %).
+template <int N, int CB, int RM, int HB = 2, bool WINDOWS = false>
 __device__ __forceinline__ void consume_slab(const uint8_t* ring, uint64_t* full, uint64_t* empty, uint32_t nrows,
                                              uint32_t n_rt, uint32_t mask, Ring rc, const __half* xp, uint32_t xstride,
                                              uint32_t live_rows, RingPos& pos, uint32_t tcol, uint32_t kg, uint32_t lane,
@@ -208,8 +210,7 @@ __device__ __forceinline__ void consume_slab(const uint8_t* ring, uint64_t* full
             // timing probe: the stage has landed, nothing reads it
         } else if (N > 0) {
             // the stage's tiles of this warp, a batch at a time: words, then decodes, then tensor-core steps, so the dependent
-            // chains of a batch overlap and the registers of all are never needed at once. Full-width codewords (all packs but
-            // those with a narrower search width) take their windows without a mask: see decode_raw.
+            // chains of a batch overlap and the registers of all are never needed at once
             uint32_t wa[kRaw];
 #pragma unroll
             for (uint32_t w = 0; w < kRaw; ++w) wa[w] = st + woff[w];
@@ -229,7 +230,7 @@ __device__ __forceinline__ void consume_slab(const uint8_t* ring, uint64_t* full
                     for (uint32_t i = 0; i < kHalfBatch; ++i) mma_tile<RM>(acc, xs + (h + i) * kKGroups * 32u, ro, b[i]);
                 }
             };
-            if (mask == 0xFFFFu) stage(std::true_type());
+            if (WINDOWS && (N == 32 || N == 64 || N == 128) && mask == 0xFFFFu) stage(std::true_type());
             else stage(std::false_type());
         } else {
             const uint8_t* stp = ring + (st - ring0);
