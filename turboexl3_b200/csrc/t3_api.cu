@@ -64,6 +64,11 @@ uint32_t* dev_error_ptr() {
     return g_err_ptr[dev];
 }
 
+t3_config config() {
+    std::lock_guard<std::mutex> lock(g_mu);
+    return g_cfg;
+}
+
 uint32_t pow2_at_most(uint32_t v, uint32_t cap) {
     uint32_t s = 1;
     while (s * 2u <= v && s * 2u <= cap) s *= 2u;
@@ -365,7 +370,7 @@ int t3_linear_resident(const void* x, int x_dtype, size_t rows, const void* w_ha
     if (rows > kPrefillDenseRowsMax) return T3_BAD_EXL3_SHAPE;
     if (!workspace || workspace_bytes < t3_linear_workspace_bytes(rows, in_dim, out_dim, 16)) return T3_WORKSPACE_TOO_SMALL;
     PrefillLinearArgs p = {x, y, nullptr, w_hat_t, suh, svh, (uint32_t)rows, (uint32_t)in_dim, (uint32_t)out_dim, 16u, 0xFFFFu,
-                           x_dtype, workspace, dev_error_ptr()};
+                           x_dtype, workspace, dev_error_ptr(), !config().no_overlap};
     note_engine(2, (uint64_t)in_dim, (uint64_t)out_dim, 0, 1);
     int launches = 0;
     const cudaError_t rc = launch_prefill_linear(p, kMul1, static_cast<cudaStream_t>(stream), &launches);
@@ -397,7 +402,7 @@ int t3_linear_unrot(const void* x, int x_dtype, size_t rows, const void* w_std_t
     note_engine(2, (uint64_t)in_dim, (uint64_t)out_dim, 0, 2);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return cuda_status(launch_plain_linear(x, x_dtype, (uint32_t)rows, w_std_t, (uint32_t)in_dim, (uint32_t)out_dim, y,
-                                           dev_error_ptr(), static_cast<cudaStream_t>(stream)));
+                                           dev_error_ptr(), !config().no_overlap, static_cast<cudaStream_t>(stream)));
 }
 
 int t3_codebook_table(t3_decode dec, void* out, void* stream) {
@@ -509,11 +514,7 @@ size_t t3_linear_workspace_bytes(size_t rows, int in_dim, int out_dim, int n) {
     // Decode rows. Up to 8 rows of an ordinary linear: nothing (the kernel keeps everything on chip). 9 to 32 rows: the rows
     // rotated once ahead of the GEMV. Linears of 24 MB of codes and up: the K slices' partial sums, when a slice count that
     // fills the multiprocessors evenly exists for the shape. All optional: a call without it takes the cluster kernel.
-    t3_config cfg;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        cfg = g_cfg;
-    }
+    const t3_config cfg = config();
     DenseArgs a = {};
     a.in = (uint32_t)in_dim, a.out = (uint32_t)out_dim, a.n = (uint32_t)n, a.rows = (uint32_t)rows;
     if (plan_dense(a, cfg, true) != T3_OK) return 0;
@@ -530,18 +531,14 @@ int t3_linear(const void* x, int x_dtype, size_t rows, const void* trellis, cons
     if (!dtype_ok(x_dtype)) return T3_BAD_EXL3_DTYPE;
     uint32_t mask;
     if (int rc = decode_mask(dec, mask)) return rc;
-    t3_config cfg;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        cfg = g_cfg;
-    }
+    const t3_config cfg = config();
     if (rows > T3_DECODE_ROWS_MAX) {
         if (!cfg.prefill) return T3_ENGINE_NOT_IMPLEMENTED;
         if (rows > 0x7FFFFFFFu / (size_t)(in_dim > out_dim ? in_dim : out_dim)) return T3_BAD_EXL3_SHAPE;
         if (rows > kPrefillDenseRowsMax) return T3_BAD_EXL3_SHAPE;  // the prepare launch's row groups are a grid dimension
         if (!workspace || workspace_bytes < t3_linear_workspace_bytes(rows, in_dim, out_dim, n)) return T3_WORKSPACE_TOO_SMALL;
         PrefillLinearArgs p = {x, y, static_cast<const uint8_t*>(trellis), nullptr, suh, svh, (uint32_t)rows, (uint32_t)in_dim,
-                               (uint32_t)out_dim, (uint32_t)n, mask, x_dtype, workspace, dev_error_ptr()};
+                               (uint32_t)out_dim, (uint32_t)n, mask, x_dtype, workspace, dev_error_ptr(), !cfg.no_overlap};
         note_engine(2, (uint64_t)in_dim, (uint64_t)out_dim, (uint64_t)n, 0);
         int launches = 0;
         const cudaError_t rc = launch_prefill_linear(p, dec.codebook, static_cast<cudaStream_t>(stream), &launches);
@@ -602,11 +599,7 @@ int t3_plan_linear(size_t rows, int in_dim, int out_dim, int n, t3_decode dec, t
     if (int rc = decode_mask(dec, mask)) return -rc;
     if (rows > T3_DECODE_ROWS_MAX) return -T3_ENGINE_NOT_IMPLEMENTED;  // the plan covers the decode-row kernels
     if (max_launches < 1) return -T3_BAD_EXL3_SHAPE;
-    t3_config cfg;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        cfg = g_cfg;
-    }
+    const t3_config cfg = config();
     DenseArgs a = {};
     a.in = (uint32_t)in_dim, a.out = (uint32_t)out_dim, a.n = (uint32_t)n, a.rows = (uint32_t)rows;
     if (int rc = plan_dense(a, cfg, true)) return -rc;
@@ -720,11 +713,7 @@ int moe_call(const void* x, int x_dtype, size_t rows, const t3_bank* bank, const
     if (clamp_at != T3_CLAMP_GATE_IN && clamp_at != T3_CLAMP_SILU_OUT) return T3_INVALID_CLAMP;
     uint32_t mask;
     if (int rc = decode_mask(dec, mask)) return rc;
-    t3_config cfg;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        cfg = g_cfg;
-    }
+    const t3_config cfg = config();
     if (rows > T3_DECODE_ROWS_MAX && !cfg.prefill) return T3_ENGINE_NOT_IMPLEMENTED;  // src/root.zig:850-852
     // the prefill chain's launches carry row groups in a grid dimension (65535 at most): 8 rows a group in the last launch,
     // 64 row-slots a group in the prepare and the middle
@@ -762,6 +751,7 @@ int moe_call(const void* x, int x_dtype, size_t rows, const t3_bank* bank, const
     a.shared = shared;
     a.y_dt = x_dtype;
     a.shared_ready = shared_ready;
+    a.overlap = !cfg.no_overlap;
     a.err = dev_error_ptr();
     note_engine(rows > T3_DECODE_ROWS_MAX ? 2 : 0, ((uint64_t)a.hidden << 32) | a.inter, a.experts, a.n, a.topk);
     if (rows > T3_DECODE_ROWS_MAX) {
@@ -788,11 +778,7 @@ int t3_plan_moe(size_t rows, int topk, const t3_bank* bank, t3_decode dec, t3_la
     if (rows > T3_DECODE_ROWS_MAX) return -T3_ENGINE_NOT_IMPLEMENTED;  // the plan covers the decode-row kernels
     const int count = topk == 1 ? 2 : 3;
     if (max_launches < count) return -T3_BAD_EXL3_SHAPE;
-    t3_config cfg;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        cfg = g_cfg;
-    }
+    const t3_config cfg = config();
     MoeArgs a = {};
     a.experts = (uint32_t)bank->experts, a.hidden = (uint32_t)bank->hidden, a.inter = (uint32_t)bank->inter;
     a.topk = (uint32_t)topk, a.rows = (uint32_t)rows, a.n = (uint32_t)bank->n_gate;
@@ -880,10 +866,8 @@ int t3_moe_mixed(const void* x, int x_dtype, size_t rows, const t3_bank* banks, 
     uint32_t mask;
     if (int rc = decode_mask(dec, mask)) return rc;
     if (rows <= T3_DECODE_ROWS_MAX) return T3_ENGINE_NOT_IMPLEMENTED;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        if (!g_cfg.prefill) return T3_ENGINE_NOT_IMPLEMENTED;
-    }
+    const t3_config cfg = config();
+    if (!cfg.prefill) return T3_ENGINE_NOT_IMPLEMENTED;
     const size_t slots = rows * (size_t)topk, wide = (size_t)(banks[0].hidden > banks[0].inter ? banks[0].hidden : banks[0].inter);
     if (rows > kPrefillMoeRowsMax || slots > kPrefillSlotsMax || slots > 0x7FFFFFFFu / wide) return T3_BAD_EXL3_SHAPE;
     if (!workspace || workspace_bytes < t3_moe_mixed_workspace_bytes(rows, topk, banks, count)) return T3_WORKSPACE_TOO_SMALL;
@@ -905,6 +889,7 @@ int t3_moe_mixed(const void* x, int x_dtype, size_t rows, const t3_bank* banks, 
     a.mask = mask;
     a.y = y;
     a.shared = shared;
+    a.overlap = !cfg.no_overlap;
     a.err = dev_error_ptr();
     for (int b = 0; b < count; ++b) note_engine(2, ((uint64_t)a.hidden << 32) | a.inter, (uint64_t)banks[b].experts, mixed.n[b], a.topk);
     int launches = 0;
@@ -930,11 +915,7 @@ int t3_moe_clamped_banked(const void* x, int x_dtype, size_t rows, const t3_bank
     uint32_t mask;
     if (int rc = decode_mask(dec, mask)) return rc;
     if (!workspace || workspace_bytes < t3_moe_workspace_bytes(rows < 32 ? rows : 32, 1, &banks[0])) return T3_WORKSPACE_TOO_SMALL;
-    t3_config cfg;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        cfg = g_cfg;
-    }
+    const t3_config cfg = config();
     const t3_bank* bank = &banks[0];
     MoeArgs a = {};
     a.x_dt = x_dtype;
@@ -1047,11 +1028,7 @@ int t3_moe_swiglu_rows(const void* x, int x_dtype, size_t x_rows, const void* ro
     if (x_rows < 1 || slots < 1 || slots > (size_t)1 << 30) return T3_BAD_EXL3_SHAPE;
     if (int rc = validate_bank(bank, bank ? bank->hidden : 0)) return rc;
     if (!dtype_ok(x_dtype) || !dtype_ok(scores_dtype) || !dtype_ok(y_dtype)) return T3_BAD_EXL3_DTYPE;
-    t3_config cfg;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        cfg = g_cfg;
-    }
+    const t3_config cfg = config();
     if (!cfg.prefill || slots <= T3_DECODE_ROWS_MAX) return T3_ENGINE_NOT_IMPLEMENTED;  // src/root.zig:1059,1066
     if (slots > kPrefillMoeRowsMax) return T3_BAD_EXL3_SHAPE;  // row groups of the last launch are a grid dimension
     if (bank->n_gate != bank->n_down) return T3_ENGINE_NOT_IMPLEMENTED;                 // src/root.zig:1074
@@ -1086,6 +1063,7 @@ int t3_moe_swiglu_rows(const void* x, int x_dtype, size_t x_rows, const void* ro
     a.y = y;
     a.y_dt = y_dtype;
     a.row_map = static_cast<const uint32_t*>(row_map);
+    a.overlap = !config().no_overlap;
     a.err = dev_error_ptr();
     note_engine(2, ((uint64_t)a.hidden << 32) | a.inter, a.experts, a.n, 1);
     int launches = 0;

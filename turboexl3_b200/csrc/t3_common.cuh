@@ -409,4 +409,10 @@ static __device__ __noinline__ void report(uint32_t* err, uint32_t bit) {
     if (err) atomicOr(err, bit);
 }
 
+// Programmatic dependent launch: `pdl_trigger` lets the next kernel of the stream start its own prologue (its weight
+// copies do not depend on this kernel); `pdl_wait` blocks until the previous kernel of the stream has completed and its
+// writes are visible. Both are no-ops for a launch without the attribute.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 }  // namespace t3

@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         mbar_init_fence();
     }
     if (warp == kMmaWarp) tmem_alloc(tmem_slot, kTmemCols);
+    if (tid == 32u) pdl_trigger();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -362,7 +363,9 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
             return true;
         });
     } else if (warp == kRowWarp) {
-        // ---- row ring: 64 inputs of the tile's rows a slot
+        // ---- row ring: 64 inputs of the tile's rows a slot. The rows are the previous kernel's output; the other roles' inputs
+        // are not, so the codes stream in and the first stages decode while that kernel finishes.
+        pdl_wait();
         Ring<kSlots> ring;
         for_each_sub(a, [&](const Sub& s) {
             const int row0 = (int)(s.op * a.op_rows + s.first);
@@ -614,22 +617,8 @@ cudaError_t launch_one(const GemmMaps& maps, const DecodeGemmArgs& a, uint32_t u
     static std::atomic<uint64_t> ready{0};  // devices (by ordinal) on which the kernel may use its shared memory
     const cudaError_t rc = allow_smem_once(ready, reinterpret_cast<const void*>(fn), bytes(NN > 0 ? NN : 128));
     if (rc != cudaSuccess) return rc;
-    if (a.ksplit <= 1u) {
-        fn<<<units < sms ? units : sms, kThreads, bytes(a.n), stream>>>(maps, a);
-        return cudaGetLastError();
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(a.ksplit, units, 1);
-    cfg.blockDim = dim3(kThreads, 1, 1);
-    cfg.dynamicSmemBytes = bytes(a.n);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = a.ksplit;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, fn, maps, a);
+    if (a.ksplit <= 1u) return launch_overlapped(fn, dim3(units < sms ? units : sms), kThreads, bytes(a.n), stream, a.overlap != 0, 1u, maps, a);
+    return launch_overlapped(fn, dim3(a.ksplit, units), kThreads, bytes(a.n), stream, a.overlap != 0, a.ksplit, maps, a);
 }
 
 }  // namespace

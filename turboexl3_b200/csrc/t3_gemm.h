@@ -49,6 +49,9 @@ struct DecodeGemmArgs {
     uint32_t kept;              // codes[0] is a kept weight: f16 (or bf16) [N, K], boxes of 64 inputs x 128 outputs; nothing is decoded
     uint32_t bf16;              // kept weight and rows are bf16
     uint32_t* err;
+    int overlap;                // launch with the programmatic-dependent-launch attribute: the rows (and nothing else that is read
+                                // here but weights and, routed, the tiles) are the stream's previous kernel's output, and that
+                                // kernel lets this one start only after its own wait
 };
 
 // max_units: an upper bound of the launch's units of work (the kernel is persistent; a smaller grid serves a small call)

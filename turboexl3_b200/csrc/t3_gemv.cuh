@@ -77,12 +77,6 @@ __device__ __forceinline__ uint8_t* aligned_smem(uint8_t* raw) {
     return raw + (((a + 127u) & ~127u) - a);
 }
 
-// Programmatic dependent launch: `pdl_trigger` lets the next kernel of the stream start its own prologue (its weight
-// copies do not depend on this kernel); `pdl_wait` blocks until the previous kernel of the stream has completed and its
-// writes are visible. Both are no-ops for a launch without the attribute.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // ---- producer -----------------------------------------------------------------------------------------------------
 
 // Where a warp stands in the ring: the slot it uses next and how many times it has gone round (kept as running counters:

@@ -86,6 +86,33 @@ inline cudaError_t allow_smem_once(std::atomic<uint64_t>& ready, const void* ker
     return rc;
 }
 
+// A launch that may start while the stream's previous kernel is still running (`overlap`; the kernel orders itself with pdl_wait,
+// see t3_common.cuh), of one CTA or a cluster of `cluster` along grid x.
+template <typename... Params>
+cudaError_t launch_overlapped(void (*fn)(Params...), dim3 grid, uint32_t block, uint32_t smem, cudaStream_t stream, bool overlap,
+                              uint32_t cluster, const Params&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (overlap) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1u) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
 // remembers, per host thread, the kernel a decode-row launch is about to run (t3_last_kernel_symbol names it)
 void note_symbol(const void* kernel);
 
@@ -121,6 +148,7 @@ struct PrefillLinearArgs {
     int x_dt;
     void* workspace;  // prefill_linear_workspace bytes
     uint32_t* err;
+    int overlap;      // launch with the programmatic-dependent-launch attribute
 };
 size_t prefill_linear_workspace(size_t rows, uint32_t in, uint32_t out);
 cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cudaStream_t stream, int* launches);
@@ -145,7 +173,7 @@ cudaError_t launch_dequant(const uint8_t* trellis, uint32_t in, uint32_t out, ui
 cudaError_t launch_unrot(void* w_t, const void* suh, const void* svh, uint32_t in, uint32_t out, int dt, cudaStream_t stream);
 // y = x W_std (x and the weight in the same 16-bit dtype, f32 accumulation, one rounding): the plain tensor-core GEMM
 cudaError_t launch_plain_linear(const void* x, int dt, uint32_t rows, const void* w_std_t, uint32_t in, uint32_t out, void* y,
-                                uint32_t* err, cudaStream_t stream);
+                                uint32_t* err, bool overlap, cudaStream_t stream);
 // the expert-parallel dispatch plan of one rank's routing (see ep_plan_kernel); world 1..8, experts a multiple of world
 cudaError_t launch_ep_plan(const uint32_t* inds, uint32_t rows, uint32_t topk, uint32_t experts, uint32_t world, uint32_t* order,
                            uint32_t* where, uint32_t* send_rows, void* meta, int* counts, cudaStream_t stream);

@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(kRouteThreads) route_plan_kernel(const uint32_
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, experts = map.base[map.banks];
     const bool shared_hist = experts <= kRouteExperts;
     const uint32_t lo = blockIdx.x * kRouteSlots;
+    pdl_trigger();
     uint32_t mine_e[kRouteSlots / kRouteThreads], mine_r[kRouteSlots / kRouteThreads];
     if (shared_hist) {
         for (uint32_t e = tid; e < experts; e += kRouteThreads) hist[e] = 0u;
@@ -140,6 +141,8 @@ __global__ void __launch_bounds__(kRouteThreads) route_plan_kernel(const uint32_
 __global__ void route_scatter_kernel(const uint32_t* inds, uint32_t slots, const __grid_constant__ ExpertMap map, const uint32_t* rank,
                                      const uint32_t* first, const uint32_t* row_map, uint32_t topk, uint2* where, uint32_t* inv) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     if (s >= slots) return;
     const uint32_t e = map.number(inds[s]), p = first[e] + rank[s], b = map.bank(e);
     where[p] = make_uint2(row_map ? row_map[s] : s / topk, (b << 24) | (e - map.base[b]));
@@ -183,6 +186,8 @@ __global__ void __launch_bounds__(256, 3) prep_rows_kernel(const __grid_constant
     const uint32_t lane = threadIdx.x & 31u, q = lane & 3u;
     uint32_t p;
     bool live;
+    pdl_wait();
+    pdl_trigger();  // after the wait: the GEMM that follows reads the tiles ahead of its own
     if (!my_position(a.positions, lane, p, live)) return;
     uint32_t row, e = 0, bank = 0;
     if (a.where) {
@@ -246,6 +251,8 @@ __global__ void __launch_bounds__(256, 3) mid_kernel(const __grid_constant__ Mid
     const uint32_t lane = threadIdx.x & 31u, q = lane & 3u;
     uint32_t p;
     bool live;
+    pdl_wait();
+    pdl_trigger();  // after the wait: the GEMM that follows reads the tiles ahead of its own
     if (!my_position(a.positions, lane, p, live)) return;
     const uint32_t id = a.where ? a.where[p].y : 0u;
     const __half* suh = a.down_suh[id >> 24] + (size_t)(id & 0xFFFFFFu) * a.inter;
@@ -295,6 +302,8 @@ __global__ void __launch_bounds__(256) moe_fin_kernel(const FinArgs a) {
     // in flight at once (four 8-byte reads a lane left the kernel waiting on memory: 49 us where its bytes take 28).
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t row = blockIdx.y * 8u + warp;
+    pdl_wait();
+    pdl_trigger();
     if (row >= a.rows) return;
     for (uint32_t col = (blockIdx.x * 32u + lane) * 8u; col < a.hidden; col += gridDim.x * 256u) {
         float acc[8] = {};
@@ -419,21 +428,21 @@ cudaError_t launch_decode_gemm(const GemmMaps& maps, const DecodeGemmArgs& a, ui
 // K slices of a dense linear of few rows: a call of up to 512 rows is one or two tiles of rows, out / 128 CTAs each, every one
 // decoding all of its 128 columns' weights (a 6144 -> 2048 linear would run on 16 CTAs). Such calls cut K into slices, a CTA a
 // slice, that meet in global memory (see DecodeGemmArgs::ksplit). Two arms, 33..256 rows and 257..512, each with a slice count
-// that follows the geometry alone, so a row's bytes do not depend on the call's row count within an arm. The count: what fills two CTAs a multiprocessor at the arm's most
-// tiles, eight at most (the tile's last arriver reads every slice), four K stages a slice at least — eight where K is short
-// (under 64 stages), and there only while every CTA has a multiprocessor to itself and only in the first arm: with short K
-// the slab's traffic and two CTAs sharing a multiprocessor cost what the slices save (measured: 2048 -> 6144 at 256 rows
-// 35 us in three slices against 29, 2048 -> 2048 at 512 rows 32 us in four against 28).
+// that follows the geometry alone, so a row's bytes do not depend on the call's row count within an arm. The count: the most
+// (eight at most) whose clusters are all resident at once — a second wave doubles the call: 6144 -> 2048 at 200 rows took 33 us
+// in eight slices, of which fifteen clusters fit and sixteen are needed, against 18 in six — four 64-input steps a slice at
+// least, eight where K is short (under 64 steps), and there only in the first arm and while the slab's traffic is small.
 uint32_t prefill_ksplit(size_t rows, uint32_t in, uint32_t out) {
     if (rows > 512u) return 1u;
+    // clusters of 1 .. 8 CTAs of this shared memory that are resident at once on 148 multiprocessors
+    static const uint32_t resident[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
     const uint32_t ncol = out / 128u, ksteps = in / 64u, sms = one_wave_ctas();
     const bool long_k = ksteps >= 64u;
-    const uint32_t mtiles = rows <= 256u ? 2u : 4u;
+    const uint32_t mtiles = rows <= 256u ? 2u : 4u, units = ncol * mtiles / 2u;
     if (mtiles == 4u && !long_k) return 1u;
-    uint32_t s = (2u * sms) / (mtiles * ncol);
-    s = s < 8u ? s : 8u;
-    const uint32_t by_k = long_k ? ksteps / 4u : ksteps / 8u;
-    s = s < by_k ? s : by_k;
+    const uint32_t by_slab = (2u * sms) / (mtiles * ncol), by_k = long_k ? ksteps / 4u : ksteps / 8u;
+    uint32_t s = 8;
+    while (s > 1u && (s > by_slab || s > by_k || units > resident[s] * sms / 148u)) --s;
     if (s < 2u) return 1u;
     if (!long_k && mtiles * ncol * s > sms) return 1u;
     return s;
@@ -479,7 +488,9 @@ cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cuda
     pa.topk = 1;
     pa.xp = xp;
     pa.ops = 1;
-    prep_rows_kernel<<<dim3(spread(p.rows, p.in / 128u), (p.rows + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream>>>(pa);
+    cudaError_t rc = launch_overlapped(prep_rows_kernel, dim3(spread(p.rows, p.in / 128u), (p.rows + kRowsPerCta - 1u) / kRowsPerCta), 256, 0,
+                                       stream, p.overlap != 0, 1, pa);
+    if (rc != cudaSuccess) return rc;
     const uint32_t ncol = p.out / 128u, ksplit = prefill_ksplit(p.rows, p.in, p.out);
     GemmMaps maps;
     const bool mapped = p.resident ? make_row_maps(&maps, xp, p.rows, p.in) && make_a_map(&maps.codes[0], p.resident, p.out, p.in, 128u)
@@ -502,7 +513,8 @@ cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cuda
     d.part = reinterpret_cast<float*>(ws + up256((size_t)p.rows * p.in * 2u));  // a sliced call's slab, behind the prepared rows
     d.kept = p.resident != nullptr;
     d.err = p.err;
-    const cudaError_t rc = launch_decode_gemm(maps, d, d.dense_tiles * ncol, codebook, stream);
+    d.overlap = p.overlap;
+    rc = launch_decode_gemm(maps, d, d.dense_tiles * ncol, codebook, stream);
     if (rc == cudaSuccess) *launches += 2;  // the output rotation runs in the GEMM's epilogue
     return rc;
 }
@@ -513,7 +525,7 @@ cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cuda
 // dtype), the epilogue rounds the f32 accumulators once into y (dense.residentPlain, src/core/dense.zig:1261-1263: "one
 // matmul of x against its resident W_std in x's dtype").
 cudaError_t launch_plain_linear(const void* x, int dt, uint32_t rows, const void* w_std_t, uint32_t in, uint32_t out, void* y,
-                                uint32_t* err, cudaStream_t stream) {
+                                uint32_t* err, bool overlap, cudaStream_t stream) {
     GemmMaps maps;
     if (!make_row_maps(&maps, x, rows, in) || !make_a_map(&maps.codes[0], w_std_t, out, in, 128u)) return cudaErrorNotSupported;
     DecodeGemmArgs d = {};
@@ -529,6 +541,7 @@ cudaError_t launch_plain_linear(const void* x, int dt, uint32_t rows, const void
     d.kept = 1;
     d.bf16 = dt == (int)kBf16;
     d.err = err;
+    d.overlap = overlap;
     return launch_decode_gemm(maps, d, d.dense_tiles * (out / 128u), kMul1, stream);
 }
 
@@ -585,7 +598,7 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
     }
     const MixedBanks& banks = mixed ? *mixed : one;
     // one expert (a shared expert's chain): the slots are in order as they stand, the chain is a dense one
-    const bool routed = a.experts > 1u;
+    const bool routed = a.experts > 1u, overlap = a.overlap != 0;
     cudaError_t rc;
     if (routed) {
         ExpertMap map = {};
@@ -598,7 +611,9 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
         if (rc != cudaSuccess) return rc;
         route_plan_kernel<<<(S + kRouteSlots - 1u) / kRouteSlots, kRouteThreads, a.experts <= kRouteExperts ? a.experts * 4u : 0u, stream>>>(
             inds, S, map, w.counts, w.counts + a.experts, w.rank, w.first, w.tiles, w.range);
-        route_scatter_kernel<<<(S + 255u) / 256u, 256, 0, stream>>>(inds, S, map, w.rank, w.first, a.row_map, a.topk, w.where, w.inv);
+        rc = launch_overlapped(route_scatter_kernel, dim3((S + 255u) / 256u), 256, 0, stream, overlap, 1, inds, S, map,
+                               static_cast<const uint32_t*>(w.rank), static_cast<const uint32_t*>(w.first), a.row_map, a.topk, w.where, w.inv);
+        if (rc != cudaSuccess) return rc;
         *launches += 2;
     }
     PrepArgs pa = {};
@@ -617,7 +632,8 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
     pa.topk = a.topk;
     pa.xp = w.xp;
     pa.ops = 2;
-    prep_rows_kernel<<<dim3(spread(S, H / 128u), (S + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream>>>(pa);
+    rc = launch_overlapped(prep_rows_kernel, dim3(spread(S, H / 128u), (S + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream, overlap, 1, pa);
+    if (rc != cudaSuccess) return rc;
 
     // A unit of work is two 128-output blocks where tiles of up to 128 rows are the rule (both run on one copy of the rows) and
     // there are units enough for every multiprocessor; else one.
@@ -626,6 +642,7 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
         g.mask = a.mask;
         g.op_rows = S;
         g.err = a.err;
+        g.overlap = a.overlap;
         const bool down = g.ops == 1u;
         for (uint32_t b = 0; b < banks.count; ++b) {
             const BankTab& t = banks.bank[b];
@@ -672,7 +689,8 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
     m.limit = a.limit;
     m.clamp_at = a.clamp_at;
     m.hd = w.hd;
-    mid_kernel<<<dim3(spread(S, I / 128u), (S + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream>>>(m);
+    rc = launch_overlapped(mid_kernel, dim3(spread(S, I / 128u), (S + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream, overlap, 1, m);
+    if (rc != cudaSuccess) return rc;
 
     DecodeGemmArgs d = {};
     d.K = I;
@@ -688,7 +706,9 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
         if (rc != cudaSuccess) return rc;
     }
     const uint32_t fin_groups = (a.rows + 7u) / 8u, fin_want = (1184u + fin_groups - 1u) / fin_groups, fin_cols = (H + 255u) / 256u;
-    moe_fin_kernel<<<dim3(fin_want < fin_cols ? fin_want : fin_cols, fin_groups), 256, 0, stream>>>(f);
+    rc = launch_overlapped(moe_fin_kernel, dim3(fin_want < fin_cols ? fin_want : fin_cols, fin_groups), 256, 0, stream,
+                           overlap && !a.shared_ready, 1, f);
+    if (rc != cudaSuccess) return rc;
     *launches += 3;
     return cudaGetLastError();
 }
