@@ -642,7 +642,7 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
         g.mask = a.mask;
         g.op_rows = S;
         g.err = a.err;
-        g.overlap = a.overlap;
+        g.overlap = routed ? 0 : a.overlap;
         const bool down = g.ops == 1u;
         for (uint32_t b = 0; b < banks.count; ++b) {
             const BankTab& t = banks.bank[b];
