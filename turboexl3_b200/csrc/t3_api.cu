@@ -648,12 +648,15 @@ int validate_bank(const t3_bank* b, int hidden_of_x) {
 // top-k set.
 int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     const size_t slots = (size_t)a.rows * a.topk;
-    // Rows one pass over an expert's weights serves. Sized from the geometry's expected members an expert (rows * topk /
-    // experts, with headroom), not from the row count: with many experts a 32-row call still has one or two rows an
-    // expert, and a 32-row pass would pay four times the shared memory and twice the tensor-core steps for nothing. An
-    // expert with more members than this takes further passes over its weights. A row's bytes do not depend on it.
+    // Members of an expert one CTA's decode of its weights serves. Sized from the geometry's expected members an expert (rows *
+    // topk / experts, with headroom), not from the row count: with many experts a 32-row call still has one or two rows an
+    // expert, and a 32-row pass would pay four times the shared memory and twice the tensor-core steps for nothing. An expert
+    // with more members is served by several CTAs at once, so where those all find a place (few experts: a shared expert's
+    // chain) eight members a CTA is the quickest: 29 rows on one expert of 2048 x 512 took 61 us in one CTA a block, most of it
+    // the 29 prepares and finishes. A row's bytes do not depend on it.
     const uint32_t expect = (uint32_t)((4u * slots + a.experts - 1u) / a.experts) + 4u;
-    const uint32_t rm = row_cap_for(expect < a.rows ? expect : a.rows);
+    uint32_t rm = row_cap_for(expect < a.rows ? expect : a.rows);
+    if ((uint64_t)(a.experts + slots / 8u) * (a.inter / 128u) * 2u <= one_wave() / 2u) rm = 8u;
     a.row_cap = rm;
     a.overlap = !cfg.no_overlap;
     // The K splits depend on hidden and inter only (sized as if a row had eight slots), never on the row count, the top-k

@@ -239,35 +239,44 @@ __device__ __forceinline__ uint32_t canon_id(const MoeArgs& a, uint32_t id) {
 // The arrays of the bank a canonical id names (bank 0: the call's own)
 #define T3_BANK_FIELD(a, id, f) (!(a).banked || ((id) >> 24) == 0u ? (a).f : (((id) >> 24) == 1u ? (a).ext[0].f : (a).ext[1].f))
 
-// Row-slot j's expert and every row-slot of the call on that expert, ascending, into `members`; skip = an earlier
-// row-slot already owns this expert (its CTAs do the work), or the row-slot runs no expert. All threads of the CTA must
-// call this.
-__device__ __forceinline__ Members find_members(const MoeArgs& a, uint32_t j, uint32_t* s_inds, uint16_t* members,
-                                                uint32_t* s_count) {
-    const uint32_t tid = threadIdx.x, slots = a.rows * a.topk;
+// Row-slot j's expert and the row-slots it serves. The row-slots on one expert, in ascending order, are cut into runs of RM, a
+// run's first row-slot serves the run (its CTAs decode the expert's weights for all of them) and the others skip: an expert with
+// more than RM members is served by several CTAs at once. One ballot a 32 row-slots and one barrier (finding the members took
+// four, a fifth of a down CTA's life); `members` is written before the next __syncthreads. All threads of the CTA call this.
+template <int RM>
+__device__ __forceinline__ Members find_members(const MoeArgs& a, uint32_t j, uint16_t* members, uint32_t* masks) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, slots = a.rows * a.topk, chunks = (slots + 31u) / 32u;
     const uint32_t* inds = static_cast<const uint32_t*>(a.inds);
-    for (uint32_t s = tid; s < slots; s += blockDim.x) s_inds[s] = canon_id(a, inds[s]);
-    __syncthreads();
+    constexpr uint32_t kWarps = kGemvThreads / 32u, kTurns = (kMaxSlots / 32u + kWarps - 1u) / kWarps;
     Members m;
-    m.expert = s_inds[j];
-    int earlier = a.banked && m.expert == kSkipId;
-    for (uint32_t s = tid; s < j; s += blockDim.x) earlier |= (s_inds[s] == m.expert);
-    m.skip = __syncthreads_or(earlier) != 0;
-    m.count = 0;
-    if (m.skip) return m;
-    if (tid < 32u) {
-        uint32_t count = 0;
-        for (uint32_t base = j & ~31u; base < slots; base += 32u) {
-            const uint32_t s = base + tid;
-            const bool hit = s >= j && s < slots && s_inds[s] == m.expert;
-            const uint32_t votes = __ballot_sync(0xFFFFFFFFu, hit);
-            if (hit) members[count + __popc(votes & ((1u << tid) - 1u))] = (uint16_t)s;
-            count += __popc(votes);
-        }
-        if (tid == 0) *s_count = count;
+    m.expert = canon_id(a, inds[j]);
+    uint32_t mine[kTurns];  // this warp's ballots
+#pragma unroll
+    for (uint32_t i = 0; i < kTurns; ++i) {
+        const uint32_t chunk = warp + i * kWarps, s = chunk * 32u + lane;
+        mine[i] = chunk < chunks ? __ballot_sync(0xFFFFFFFFu, s < slots && canon_id(a, inds[min(s, slots - 1u)]) == m.expert) : 0u;
+        if (chunk < chunks && lane == 0) masks[chunk] = mine[i];
     }
     __syncthreads();
-    m.count = *s_count;
+    // lane c: members in chunk c and, after the scan, up to its end
+    const uint32_t mask = lane < chunks ? masks[lane] : 0u;
+    uint32_t upto = __popc(mask);
+#pragma unroll
+    for (uint32_t off = 1; off < 32u; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, upto, off);
+        if (lane >= off) upto += v;
+    }
+    const uint32_t before = upto - __popc(mask), total = __shfl_sync(0xFFFFFFFFu, upto, 31);
+    const uint32_t ordinal = __shfl_sync(0xFFFFFFFFu, before + __popc(mask & ((1u << (j & 31u)) - 1u)), j >> 5);
+    m.skip = ordinal % RM != 0u || (a.banked && m.expert == kSkipId);
+    m.count = min((uint32_t)RM, total - ordinal);
+#pragma unroll
+    for (uint32_t i = 0; i < kTurns; ++i) {
+        const uint32_t chunk = warp + i * kWarps;
+        if (chunk >= chunks) break;
+        const uint32_t at = __shfl_sync(0xFFFFFFFFu, before, chunk) + __popc(mine[i] & ((1u << lane) - 1u)) - ordinal;
+        if (((mine[i] >> lane) & 1u) && at < (uint32_t)RM) members[at] = (uint16_t)(chunk * 32u + lane);
+    }
     return m;
 }
 
@@ -289,17 +298,15 @@ template <int N, int RM>
 __device__ __forceinline__ void moe_gate_up_body(const MoeArgs& a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* smem = aligned_smem(smem_raw);
-    __shared__ uint32_t s_inds[kMaxSlots];
-    __shared__ uint16_t s_members[kMaxSlots];
-    __shared__ uint32_t s_count;
+    __shared__ uint32_t s_masks[kMaxSlots / 32u];
+    __shared__ uint16_t s_members[RM];
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank(), csize = 2u * a.split_gu, ib = blockIdx.y, j = blockIdx.z;
     const uint32_t proj = rank & 1u, kpart = rank >> 1;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t H = a.hidden, I = a.inter;
     pdl_wait();     // the routing (and x) may be the previous kernel's output
-    pdl_trigger();  // after the wait: the down launch reads the routing ahead of its own wait
-    const Members mem = find_members(a, j, s_inds, s_members, &s_count);
+    const Members mem = find_members<RM>(a, j, s_members, s_masks);
     if (mem.skip) return;
     const uint32_t id = mem.expert, e = a.banked ? id & 0xFFFFFFu : id;
 
@@ -326,47 +333,43 @@ __device__ __forceinline__ void moe_gate_up_body(const MoeArgs& a) {
     }
     const uint32_t owned = rows_owned(RM, csize);
     RingPos pos;
-    for (uint32_t m0 = 0; m0 < mem.count; m0 += RM) {
-        const uint32_t mcount = min((uint32_t)RM, mem.count - m0);
-        if (warp == kConsumerWarps) {
-            produce_slab(c.ring, c.full, c.empty, wsrc, (size_t)out_tiles * tile_bytes, nrows, row_bytes, rc, pos, lane, a.err);
-        } else {
-            for (uint32_t i = mcount * xstride + tid; i < RM * xstride; i += kConsumerThreads) c.xp[i] = __float2half_rn(0.0f);
-            for (uint32_t task = warp; task < mcount * nblk; task += kConsumerWarps) {
-                const uint32_t m = task / nblk, b = task - m * nblk;
-                const uint32_t row = s_members[m0 + m] / a.topk, k0 = (b0 + b) * 128u;
-                prepare_block(a.x, a.x_dt, (size_t)row * H + k0, suh + k0, c.xp + m * xstride + b * 128u, lane);
-            }
-            named_sync(1, kConsumerThreads);
-            gemv_and_push<N, RM>(cluster, c, nrows, a.n, a.mask, rc, xstride, RM, pos, mcount, rank, csize, warp, lane, a.err);
+    const uint32_t count = mem.count;
+    if (warp == kConsumerWarps) {
+        produce_slab(c.ring, c.full, c.empty, wsrc, (size_t)out_tiles * tile_bytes, nrows, row_bytes, rc, pos, lane, a.err);
+        pdl_trigger();  // after the wait: the down launch reads the routing ahead of its own wait
+    } else {
+        for (uint32_t task = warp; task < count * nblk; task += kConsumerWarps) {
+            const uint32_t m = task / nblk, b = task - m * nblk;
+            const uint32_t row = s_members[m] / a.topk, k0 = (b0 + b) * 128u;
+            prepare_block(a.x, a.x_dt, (size_t)row * H + k0, suh + k0, c.xp + m * xstride + b * 128u, lane);
         }
-        cluster_arrive();
-        const bool last = m0 + RM >= mem.count;
-        if (last && rank >= mcount) return;
-        cluster_wait();
-        if (warp < kConsumerWarps) {
-            const size_t eo = (size_t)e * I + ib * 128u;
-            for (uint32_t i = warp; i * csize + rank < mcount; i += kConsumerWarps) {
-                const uint32_t m = i * csize + rank;
-                float g[4], u[4];
-                float sg[4], su[4], sd[4];
-                load_scales(static_cast<const __half*>(T3_BANK_FIELD(a, id, gate_svh)) + eo, lane, sg);
-                load_scales(static_cast<const __half*>(T3_BANK_FIELD(a, id, up_svh)) + eo, lane, su);
-                load_scales(static_cast<const __half*>(T3_BANK_FIELD(a, id, down_suh)) + eo, lane, sd);
-                gather_owned(c.recv, owned, i, 0, 2, a.split_gu, lane, g);
-                gather_owned(c.recv, owned, i, 1, 2, a.split_gu, lane, u);
-                finish_block(g, sg, lane);
-                finish_block(u, su, lane);
-                float d[4];
+        named_sync(1, kConsumerThreads);
+        gemv_and_push<N, RM>(cluster, c, nrows, a.n, a.mask, rc, xstride, count, pos, count, rank, csize, warp, lane, a.err);
+    }
+    cluster_arrive();
+    if (rank >= count) return;
+    cluster_wait();
+    if (warp < kConsumerWarps) {
+        const size_t eo = (size_t)e * I + ib * 128u;
+        for (uint32_t i = warp; i * csize + rank < count; i += kConsumerWarps) {
+            const uint32_t m = i * csize + rank;
+            float g[4], u[4];
+            float sg[4], su[4], sd[4];
+            load_scales(static_cast<const __half*>(T3_BANK_FIELD(a, id, gate_svh)) + eo, lane, sg);
+            load_scales(static_cast<const __half*>(T3_BANK_FIELD(a, id, up_svh)) + eo, lane, su);
+            load_scales(static_cast<const __half*>(T3_BANK_FIELD(a, id, down_suh)) + eo, lane, sd);
+            gather_owned(c.recv, owned, i, 0, 2, a.split_gu, lane, g);
+            gather_owned(c.recv, owned, i, 1, 2, a.split_gu, lane, u);
+            finish_block(g, sg, lane);
+            finish_block(u, su, lane);
+            float d[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) d[q] = round_half(swiglu(g[q], u[q], a.limit, a.clamp_at)) * sd[q];
-                h128_warp(d, lane);
-                __half* hd = static_cast<__half*>(a.hd) + (size_t)s_members[m0 + m] * I + ib * 128u;
+            for (int q = 0; q < 4; ++q) d[q] = round_half(swiglu(g[q], u[q], a.limit, a.clamp_at)) * sd[q];
+            h128_warp(d, lane);
+            __half* hd = static_cast<__half*>(a.hd) + (size_t)s_members[m] * I + ib * 128u;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) hd[lane + 32u * q] = __float2half_rn(d[q] * kHadScale);
-            }
+            for (int q = 0; q < 4; ++q) hd[lane + 32u * q] = __float2half_rn(d[q] * kHadScale);
         }
-        if (!last) cluster.sync();  // the next pass overwrites the receive tiles
     }
 }
 
@@ -376,15 +379,14 @@ template <int N, int RM>
 __device__ __forceinline__ void moe_down_body(const MoeArgs& a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* smem = aligned_smem(smem_raw);
-    __shared__ uint32_t s_inds[kMaxSlots];
-    __shared__ uint16_t s_members[kMaxSlots];
-    __shared__ uint32_t s_count;
+    __shared__ uint32_t s_masks[kMaxSlots / 32u];
+    __shared__ uint16_t s_members[RM];
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank(), csize = a.split_d, hb = blockIdx.y, j = blockIdx.z;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t H = a.hidden, I = a.inter;
     // the routing was complete before the gate|up launch started, so it can be read ahead of pdl_wait
-    const Members mem = find_members(a, j, s_inds, s_members, &s_count);
+    const Members mem = find_members<RM>(a, j, s_members, s_masks);
     if (mem.skip) return;
     const uint32_t id = mem.expert, e = a.banked ? id & 0xFFFFFFu : id;
 
@@ -403,62 +405,57 @@ __device__ __forceinline__ void moe_down_body(const MoeArgs& a) {
     if (warp == 0) prefetch_l2(static_cast<const __half*>(T3_BANK_FIELD(a, id, down_svh)) + (size_t)e * H + hb * 128u, 256u, lane);
     const uint32_t owned = rows_owned(RM, csize);
     RingPos pos;
-    for (uint32_t m0 = 0; m0 < mem.count; m0 += RM) {
-        const uint32_t mcount = min((uint32_t)RM, mem.count - m0);
-        if (warp == kConsumerWarps) {
-            produce_slab(c.ring, c.full, c.empty, wsrc, (size_t)out_tiles * tile_bytes, nrows, row_bytes, rc, pos, lane, a.err);
-            pdl_trigger();
-        } else {
-            pdl_trigger();
-            pdl_wait();  // hd is the gate|up launch's output
-            for (uint32_t i = mcount * xstride + tid; i < RM * xstride; i += kConsumerThreads) c.xp[i] = __float2half_rn(0.0f);
-            for (uint32_t task = warp; task < mcount * nblk; task += kConsumerWarps) {
-                const uint32_t m = task / nblk, b = task - m * nblk;
-                const __half* src = static_cast<const __half*>(a.hd) + (size_t)s_members[m0 + m] * I + (b0 + b) * 128u;
-                __half* dst = c.xp + m * xstride + b * 128u;
+    const uint32_t count = mem.count;
+    if (warp == kConsumerWarps) {
+        produce_slab(c.ring, c.full, c.empty, wsrc, (size_t)out_tiles * tile_bytes, nrows, row_bytes, rc, pos, lane, a.err);
+        pdl_trigger();
+    } else {
+        pdl_trigger();
+        pdl_wait();  // hd is the gate|up launch's output
+        for (uint32_t task = warp; task < count * nblk; task += kConsumerWarps) {
+            const uint32_t m = task / nblk, b = task - m * nblk;
+            const __half* src = static_cast<const __half*>(a.hd) + (size_t)s_members[m] * I + (b0 + b) * 128u;
+            __half* dst = c.xp + m * xstride + b * 128u;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t i = lane + 32u * q;
+                dst[(i & ~15u) | lane_order16(i & 15u)] = src[i];
+            }
+        }
+        named_sync(1, kConsumerThreads);
+        gemv_and_push<N, RM>(cluster, c, nrows, a.n, a.mask, rc, xstride, count, pos, count, rank, csize, warp, lane, a.err);
+    }
+    cluster_arrive();
+    if (rank >= count) return;
+    cluster_wait();
+    if (warp < kConsumerWarps) {
+        for (uint32_t i = warp; i * csize + rank < count; i += kConsumerWarps) {
+            const uint32_t m = i * csize + rank;
+            float v[4], sv[4];
+            load_scales(static_cast<const __half*>(T3_BANK_FIELD(a, id, down_svh)) + (size_t)e * H + hb * 128u, lane, sv);
+            gather_owned(c.recv, owned, i, 0, 1, csize, lane, v);
+            finish_block(v, sv, lane);
+            const uint32_t slot = s_members[m];
+            if (a.topk == 1u) {
+                // One slot a row: the merge has nothing to gather, so the weighted value (and the shared-expert add)
+                // is stored here and the merge launch is skipped. The arithmetic is the merge kernel's, 0 + w v included.
+                const float w = a.scores ? load_act(a.scores, a.score_dt, slot) : 1.0f;
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const uint32_t i = lane + 32u * q;
-                    dst[(i & ~15u) | lane_order16(i & 15u)] = src[i];
-                }
-            }
-            named_sync(1, kConsumerThreads);
-            gemv_and_push<N, RM>(cluster, c, nrows, a.n, a.mask, rc, xstride, RM, pos, mcount, rank, csize, warp, lane, a.err);
-        }
-        cluster_arrive();
-        const bool last = m0 + RM >= mem.count;
-        if (last && rank >= mcount) return;
-        cluster_wait();
-        if (warp < kConsumerWarps) {
-            for (uint32_t i = warp; i * csize + rank < mcount; i += kConsumerWarps) {
-                const uint32_t m = i * csize + rank;
-                float v[4], sv[4];
-                load_scales(static_cast<const __half*>(T3_BANK_FIELD(a, id, down_svh)) + (size_t)e * H + hb * 128u, lane, sv);
-                gather_owned(c.recv, owned, i, 0, 1, csize, lane, v);
-                finish_block(v, sv, lane);
-                const uint32_t slot = s_members[m0 + m];
-                if (a.topk == 1u) {
-                    // One slot a row: the merge has nothing to gather, so the weighted value (and the shared-expert add)
-                    // is stored here and the merge launch is skipped. The arithmetic is the merge kernel's, 0 + w v included.
-                    const float w = a.scores ? load_act(a.scores, a.score_dt, slot) : 1.0f;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const size_t o = (size_t)slot * H + hb * 128u + lane + 32u * q;
-                        float acc = __fadd_rn(0.0f, __fmul_rn(w, v[q]));
-                        if (a.shared) {
-                            store_act(a.y, a.y_dt, o, acc);
-                            acc = __fadd_rn(load_act(a.y, a.y_dt, o), load_act(a.shared, a.y_dt, o));
-                        }
+                    const size_t o = (size_t)slot * H + hb * 128u + lane + 32u * q;
+                    float acc = __fadd_rn(0.0f, __fmul_rn(w, v[q]));
+                    if (a.shared) {
                         store_act(a.y, a.y_dt, o, acc);
+                        acc = __fadd_rn(load_act(a.y, a.y_dt, o), load_act(a.shared, a.y_dt, o));
                     }
-                    continue;
+                    store_act(a.y, a.y_dt, o, acc);
                 }
-                __half* vo = static_cast<__half*>(a.v) + (size_t)slot * H + hb * 128u;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) vo[lane + 32u * q] = __float2half_rn(v[q]);
+                continue;
             }
+            __half* vo = static_cast<__half*>(a.v) + (size_t)slot * H + hb * 128u;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) vo[lane + 32u * q] = __float2half_rn(v[q]);
         }
-        if (!last) cluster.sync();
     }
 }
 
