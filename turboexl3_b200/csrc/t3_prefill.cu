@@ -513,7 +513,7 @@ cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cuda
     d.part = reinterpret_cast<float*>(ws + up256((size_t)p.rows * p.in * 2u));  // a sliced call's slab, behind the prepared rows
     d.kept = p.resident != nullptr;
     d.err = p.err;
-    d.overlap = p.overlap;
+    d.overlap = p.rows <= 512u && p.overlap;  // a call of few rows is short: its set-up counts. Larger ones ran 2 % slower overlapped
     rc = launch_decode_gemm(maps, d, d.dense_tiles * ncol, codebook, stream);
     if (rc == cudaSuccess) *launches += 2;  // the output rotation runs in the GEMM's epilogue
     return rc;
