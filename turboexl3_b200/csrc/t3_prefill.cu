@@ -151,26 +151,27 @@ __global__ void route_scatter_kernel(const uint32_t* inds, uint32_t slots, const
 
 // ---- prepare / mid / finish ------------------------------------------------------------------------------------------
 
-constexpr uint32_t kRowsPerCta = 64;  // 8 warps x 8 positions
-
-// how many CTAs share a position group's 128-blocks, so that small calls still fill the GPU
-uint32_t spread(uint32_t positions, uint32_t nblk) {
-    const uint32_t groups = (positions + kRowsPerCta - 1u) / kRowsPerCta;
-    const uint32_t want = (1184u + groups - 1u) / groups;
-    return want < 1u ? 1u : (want > nblk ? nblk : want);
+// multiprocessors of the device (a decode GEMM CTA fits each)
+uint32_t one_wave_ctas() {
+    static int sms = [] {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            n = 148;
+        return n;
+    }();
+    return (uint32_t)sms;
 }
 
-// this lane's position in a warp's group of eight; returns false when the whole warp is past the end
-__device__ __forceinline__ bool my_position(uint32_t count, uint32_t lane, uint32_t& p, bool& live) {
-    const uint32_t first = (blockIdx.y * 8u + (threadIdx.x >> 5)) * 8u;
-    if (first >= count) return false;
-    const uint32_t mine = first + (lane >> 2);
-    live = mine < count;
-    p = live ? mine : count - 1u;
-    return true;
+// The prepares work on (position, 128-block) pairs, eight consecutive pairs a warp: a position's blocks lie side by side in
+// memory, so a warp reads and writes runs of up to 2 KB (with eight positions' same block a warp, 256 bytes a row, the
+// prepare of 65536 slots of 7168 x 2 wrote at 2.5 TB/s). A few CTAs a multiprocessor walk the pairs.
+constexpr uint32_t kPairsPerCta = 64;  // 8 warps x 8 pairs
+uint32_t pair_ctas(size_t positions, uint32_t nblk) {
+    const size_t want = (positions * nblk + kPairsPerCta - 1u) / kPairsPerCta, most = (size_t)one_wave_ctas() * 12u;
+    return (uint32_t)(want < most ? want : most);
 }
 
-// grid (spread, ceil(P / 64)), 256 threads. Dense and one-expert calls (where null): positions are the call's rows. Routed: position p reads row
+// 256 threads. Dense and one-expert calls (where null): positions are the call's rows. Routed: position p reads row
 // where[p].x with the scales of its expert (where[p].y); the second op (up) reuses the row with its own suh.
 struct PrepArgs {
     const void* x;
@@ -183,38 +184,33 @@ struct PrepArgs {
     __half* xp;  // [ops][positions][K]
 };
 __global__ void __launch_bounds__(256, 3) prep_rows_kernel(const __grid_constant__ PrepArgs a) {
-    const uint32_t lane = threadIdx.x & 31u, q = lane & 3u;
-    uint32_t p;
-    bool live;
+    const uint32_t lane = threadIdx.x & 31u, q = lane & 3u, nblk = a.K >> 7;
+    const uint32_t pairs = a.positions * nblk;  // (the callers keep positions x width under 2^31)
     pdl_wait();
     pdl_trigger();  // after the wait: the GEMM that follows reads the tiles ahead of its own
-    if (!my_position(a.positions, lane, p, live)) return;
-    uint32_t row, e = 0, bank = 0;
-    if (a.where) {
-        const uint2 w = a.where[p];
-        row = w.x, bank = w.y >> 24, e = w.y & 0xFFFFFFu;
-    } else {
-        row = a.row_map ? a.row_map[p] : p / a.topk;
-    }
-    const __half* suh[2];
-#pragma unroll
-    for (int op = 0; op < 2; ++op) suh[op] = a.suh[op][bank] + (size_t)e * a.K;
-    const bool wide_x = aligned16(a.x), wide_s = aligned16(suh[0]) && aligned16(suh[1]);
+    const bool wide_x = aligned16(a.x);
     const HadB hb = had_b(lane);
-    for (uint32_t blk = blockIdx.x; blk < (a.K >> 7); blk += gridDim.x) {
-        const uint32_t col = blk * 128u + 8u * q;
-        uint32_t x[4][4];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) load_half8(a.x, a.x_dt, wide_x, (size_t)row * a.K + col + 32u * s, x[s]);
+    for (uint32_t f0 = (blockIdx.x * 8u + (threadIdx.x >> 5)) * 8u; f0 < pairs; f0 += gridDim.x * kPairsPerCta) {
+        const bool live = f0 + (lane >> 2) < pairs;
+        const uint32_t f = live ? f0 + (lane >> 2) : pairs - 1u;
+        const uint32_t p = f / nblk, col = (f - p * nblk) * 128u + 8u * q;
+        uint32_t row, e = 0, bank = 0;
+        if (a.where) {
+            const uint2 w = a.where[p];
+            row = w.x, bank = w.y >> 24, e = w.y & 0xFFFFFFu;
+        } else {
+            row = a.row_map ? a.row_map[p] : p / a.topk;
+        }
 #pragma unroll 1
         for (uint32_t op = 0; op < a.ops; ++op) {
-            const __half* sp = (op ? suh[1] : suh[0]) + col;
+            // the row is read again for the second op (from L1): kept in registers over the first one's rotation it spilled
+            const __half* sp = (op ? a.suh[1][bank] : a.suh[0][bank]) + (size_t)e * a.K + col;
+            const bool wide_s = aligned16(sp);
             uint32_t w[4][4], sc[4][4];
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
+                load_half8(a.x, a.x_dt, wide_x, (size_t)row * a.K + col + 32u * s, w[s]);
                 load_16b(sp + 32 * s, wide_s, sc[s]);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) w[s][j] = x[s][j];
             }
             rotate_block(w, sc, hb);
             if (live) {
@@ -236,7 +232,7 @@ __device__ __forceinline__ float swiglu_f32(float g, float u, float limit, int c
     return s * u;
 }
 
-// grid (spread, ceil(P / 64)): SwiGLU of the finished gate and up values (the GEMM's epilogue finished them) and the
+// SwiGLU of the finished gate and up values (the GEMM's epilogue finished them) and the
 // down projection's prepare, per sorted position
 struct MidArgs {
     const __half* z;  // [2][P][inter]: finished gate, finished up
@@ -248,18 +244,18 @@ struct MidArgs {
     __half* hd;  // [P][inter]
 };
 __global__ void __launch_bounds__(256, 3) mid_kernel(const __grid_constant__ MidArgs a) {
-    const uint32_t lane = threadIdx.x & 31u, q = lane & 3u;
-    uint32_t p;
-    bool live;
+    const uint32_t lane = threadIdx.x & 31u, q = lane & 3u, nblk = a.inter >> 7;
+    const uint32_t pairs = a.positions * nblk;
     pdl_wait();
     pdl_trigger();  // after the wait: the GEMM that follows reads the tiles ahead of its own
-    if (!my_position(a.positions, lane, p, live)) return;
-    const uint32_t id = a.where ? a.where[p].y : 0u;
-    const __half* suh = a.down_suh[id >> 24] + (size_t)(id & 0xFFFFFFu) * a.inter;
-    const bool wide_s = aligned16(suh);
     const HadB hb = had_b(lane);
-    for (uint32_t blk = blockIdx.x; blk < (a.inter >> 7); blk += gridDim.x) {
-        const uint32_t col = blk * 128u + 8u * q;
+    for (uint32_t f0 = (blockIdx.x * 8u + (threadIdx.x >> 5)) * 8u; f0 < pairs; f0 += gridDim.x * kPairsPerCta) {
+        const bool live = f0 + (lane >> 2) < pairs;
+        const uint32_t f = live ? f0 + (lane >> 2) : pairs - 1u;
+        const uint32_t p = f / nblk, col = (f - p * nblk) * 128u + 8u * q;
+        const uint32_t id = a.where ? a.where[p].y : 0u;
+        const __half* suh = a.down_suh[id >> 24] + (size_t)(id & 0xFFFFFFu) * a.inter + col;
+        const bool wide_s = aligned16(suh);
         const size_t zo = (size_t)p * a.inter + col;
         uint32_t g[4][4], u[4][4], sc[4][4];
 #pragma unroll
@@ -275,7 +271,7 @@ __global__ void __launch_bounds__(256, 3) mid_kernel(const __grid_constant__ Mid
                 g[s][j] = pack_half2(swiglu_f32(gv.x, uv.x, a.limit, a.clamp_at), swiglu_f32(gv.y, uv.y, a.limit, a.clamp_at));
             }
 #pragma unroll
-        for (int s = 0; s < 4; ++s) load_16b(suh + col + 32 * s, wide_s, sc[s]);  // (with the loads above it cost spills)
+        for (int s = 0; s < 4; ++s) load_16b(suh + 32 * s, wide_s, sc[s]);  // (with the loads above it cost spills)
         rotate_block(g, sc, hb);
         if (live) {
             uint4* o = reinterpret_cast<uint4*>(a.hd + zo);
@@ -285,7 +281,7 @@ __global__ void __launch_bounds__(256, 3) mid_kernel(const __grid_constant__ Mid
     }
 }
 
-// grid (spread, ceil(rows / 8)): per row, the score-weighted sum of its slots' finished down outputs (through inv) in
+// grid (column runs, ceil(rows / 8)): per row, the score-weighted sum of its slots' finished down outputs (through inv) in
 // slot order, then the optional shared-expert add in the output dtype
 struct FinArgs {
     const __half* zd;  // [P][hidden]: each sorted position's finished down output (the per-slot v)
@@ -299,37 +295,42 @@ struct FinArgs {
 };
 __global__ void __launch_bounds__(256) moe_fin_kernel(const FinArgs a) {
     // A warp a row, a lane eight consecutive elements of two 128-blocks: a slot's 512 bytes are one coalesced read, eight slots'
-    // in flight at once (four 8-byte reads a lane left the kernel waiting on memory: 49 us where its bytes take 28).
+    // in flight at once (four 8-byte reads a lane left the kernel waiting on memory: 49 us where its bytes take 28). Lane k holds
+    // slot k's weight and place for the whole row (top-k is 32 at most).
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t row = blockIdx.y * 8u + warp;
     pdl_wait();
     pdl_trigger();
     if (row >= a.rows) return;
-    for (uint32_t col = (blockIdx.x * 32u + lane) * 8u; col < a.hidden; col += gridDim.x * 256u) {
+    const size_t slot = (size_t)row * a.topk + min(lane, a.topk - 1u);
+    const float my_w = load_act(a.scores, a.score_dt, slot);
+    const uint32_t my_at = a.inv ? a.inv[slot] : (uint32_t)slot;
+    for (uint32_t c0 = blockIdx.x * 256u; c0 < a.hidden; c0 += gridDim.x * 256u) {
+        const uint32_t col = c0 + lane * 8u;
+        const bool in = col < a.hidden;  // the last run may be one 128-block
         float acc[8] = {};
         for (uint32_t k0 = 0; k0 < a.topk; k0 += 8u) {
             uint4 v[8];
-            float w[8];
 #pragma unroll
             for (uint32_t i = 0; i < 8u; ++i) {
-                const uint32_t k = k0 + i < a.topk ? k0 + i : a.topk - 1u;
-                const size_t slot = (size_t)row * a.topk + k;
-                if (k0 + i >= a.topk) break;
-                w[i] = load_act(a.scores, a.score_dt, slot);
-                v[i] = *reinterpret_cast<const uint4*>(a.zd + (size_t)(a.inv ? a.inv[slot] : (uint32_t)slot) * a.hidden + col);
+                const uint32_t at = __shfl_sync(0xFFFFFFFFu, my_at, (k0 + i) & 31u);
+                v[i] = make_uint4(0u, 0u, 0u, 0u);
+                if (in && k0 + i < a.topk) v[i] = __ldcs(reinterpret_cast<const uint4*>(a.zd + (size_t)at * a.hidden + col));
             }
 #pragma unroll
             for (uint32_t i = 0; i < 8u; ++i) {
                 if (k0 + i >= a.topk) break;
+                const float w = __shfl_sync(0xFFFFFFFFu, my_w, (k0 + i) & 31u);
                 const uint32_t u[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 f = unpack_half2(u[j]);
-                    acc[2 * j] = __fadd_rn(acc[2 * j], __fmul_rn(w[i], f.x));
-                    acc[2 * j + 1] = __fadd_rn(acc[2 * j + 1], __fmul_rn(w[i], f.y));
+                    acc[2 * j] = __fadd_rn(acc[2 * j], __fmul_rn(w, f.x));
+                    acc[2 * j + 1] = __fadd_rn(acc[2 * j + 1], __fmul_rn(w, f.y));
                 }
             }
         }
+        if (!in) continue;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             float f[4] = {acc[4 * half], acc[4 * half + 1], acc[4 * half + 2], acc[4 * half + 3]};
@@ -402,17 +403,6 @@ bool make_gemm_maps(GemmMaps* maps, const void* rows_base, uint64_t rows, uint32
 }
 
 size_t up256(size_t v) { return (v + 255u) & ~(size_t)255u; }
-
-// multiprocessors of the device (a decode GEMM CTA fits each)
-uint32_t one_wave_ctas() {
-    static int sms = [] {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            n = 148;
-        return n;
-    }();
-    return (uint32_t)sms;
-}
 
 }  // namespace
 
@@ -488,7 +478,7 @@ cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cuda
     pa.topk = 1;
     pa.xp = xp;
     pa.ops = 1;
-    cudaError_t rc = launch_overlapped(prep_rows_kernel, dim3(spread(p.rows, p.in / 128u), (p.rows + kRowsPerCta - 1u) / kRowsPerCta), 256, 0,
+    cudaError_t rc = launch_overlapped(prep_rows_kernel, dim3(pair_ctas(p.rows, p.in / 128u)), 256, 0,
                                        stream, p.overlap != 0, 1, pa);
     if (rc != cudaSuccess) return rc;
     const uint32_t ncol = p.out / 128u, ksplit = prefill_ksplit(p.rows, p.in, p.out);
@@ -632,7 +622,7 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
     pa.topk = a.topk;
     pa.xp = w.xp;
     pa.ops = 2;
-    rc = launch_overlapped(prep_rows_kernel, dim3(spread(S, H / 128u), (S + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream, overlap, 1, pa);
+    rc = launch_overlapped(prep_rows_kernel, dim3(pair_ctas(S, H / 128u)), 256, 0, stream, overlap, 1, pa);
     if (rc != cudaSuccess) return rc;
 
     // A unit of work is two 128-output blocks where tiles of up to 128 rows are the rule (both run on one copy of the rows) and
@@ -689,7 +679,7 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
     m.limit = a.limit;
     m.clamp_at = a.clamp_at;
     m.hd = w.hd;
-    rc = launch_overlapped(mid_kernel, dim3(spread(S, I / 128u), (S + kRowsPerCta - 1u) / kRowsPerCta), 256, 0, stream, overlap, 1, m);
+    rc = launch_overlapped(mid_kernel, dim3(pair_ctas(S, I / 128u)), 256, 0, stream, overlap, 1, m);
     if (rc != cudaSuccess) return rc;
 
     DecodeGemmArgs d = {};
