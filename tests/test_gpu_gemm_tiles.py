@@ -63,6 +63,6 @@ def test_mixed_banks_give_the_one_bank_bytes(rows, dt):
     inds, scores = synth.routing(2301, rows, E, topk)
     x, di, ds = x_as(synth.activations(2302, rows, H), dt), dev(inds), dev(scores)
     whole = t3.moe(x.view(1, rows, H), bank, di.view(1, rows, topk), ds.view(1, rows, topk))
-    mixed = t3.moe_mixed(x, banks, bank_of.cuda(), local_of.cuda(), di, ds)
+    mixed = t3.api.moe_mixed(x, banks, bank_of.cuda(), local_of.cuda(), di, ds)
     assert torch.equal(whole.view(rows, H), mixed)
     assert t3.device_error() == 0

@@ -239,16 +239,20 @@ __device__ __forceinline__ void finish_part(uint32_t taddr, uint32_t cols, float
     }
 }
 
-// A part's 16-bit rows from its buffer to y, 256 bytes a row (`warp` of the epilogue's eight)
+// A part's 16-bit rows from its buffer to y, 256 bytes a row (`warp` of the epilogue's eight); a caller's y may be aligned to 8
+// bytes only
 __device__ __forceinline__ void store_part(uint32_t buffer, uint16_t* y, size_t N, uint32_t rows, uint32_t warp, uint32_t lane) {
     const uint32_t j = lane & 15u;
+    const bool wide = aligned16(y);
 #pragma unroll 4
     for (uint32_t r = 2u * warp + (lane >> 4); r < rows; r += 2u * kEpiWarps) {
         uint4 w;
         asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                      : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
                      : "r"(buffer + (j >> 3) * 16384u + r * 128u + (((j & 7u) ^ (r & 7u)) << 4)));
-        *reinterpret_cast<uint4*>(y + r * N + 8u * j) = w;
+        uint16_t* at = y + r * N + 8u * j;
+        if (wide) *reinterpret_cast<uint4*>(at) = w;
+        else reinterpret_cast<uint2*>(at)[0] = make_uint2(w.x, w.y), reinterpret_cast<uint2*>(at)[1] = make_uint2(w.z, w.w);
     }
 }
 

@@ -17,7 +17,6 @@
 namespace t3 {
 namespace {
 
-
 // ---- route ---------------------------------------------------------------------------------------------------------
 
 // How an expert's c rows are cut into tiles: as few as hold them (a tile decodes its expert's weights once whatever its rows,
