@@ -212,54 +212,6 @@ __device__ __forceinline__ void h128_mma(const uint32_t (&a)[8][2], const uint32
                 }
 }
 
-// format.prepareInput's rotation of a block: w (f16 pairs, w[s][p] = elements 8 (4 s + q) + 2 p, + 1 of this quad's position) times
-// the scales sc (f16, the same elements), H128, / sqrt(128), rounded to f16; in place. Sign scales (the usual suh) are a sign
-// flip of the f16 values; with any other a product is taken in f32 and split into an f16 part and the f16 of what is left, so
-// that the sums see the f32 products.
-__device__ __forceinline__ void rotate_block(uint32_t (&w)[4][4], const uint32_t (&sc)[4][4], const HadB& hb) {
-    uint32_t a[8][2], lo[8][2], odd = 0, rest = 0;
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-#pragma unroll
-        for (int p = 0; p < 4; ++p) odd |= (sc[s][p] & 0x7FFF7FFFu) ^ 0x3C003C00u;
-    float2 out[8][2];
-    if (__any_sync(0xFFFFFFFFu, odd != 0u) == 0) {
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t u = w[2 * h][p] ^ (sc[2 * h][p] & 0x80008000u), v = w[2 * h + 1][p] ^ (sc[2 * h + 1][p] & 0x80008000u);
-                a[2 * p][h] = pack_lo(u, v);
-                a[2 * p + 1][h] = pack_hi(u, v);
-            }
-        h128_mma(a, a, false, hb, out);
-    } else {
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float2 x0 = unpack_half2(w[2 * h][p]), x1 = unpack_half2(w[2 * h + 1][p]);
-                const float2 c0 = unpack_half2(sc[2 * h][p]), c1 = unpack_half2(sc[2 * h + 1][p]);
-                const float v[2][2] = {{x0.x * c0.x, x1.x * c1.x}, {x0.y * c0.y, x1.y * c1.y}};
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    a[2 * p + i][h] = pack_half2(v[i][0], v[i][1]);
-                    lo[2 * p + i][h] = pack_half2(v[i][0] - round_half(v[i][0]), v[i][1] - round_half(v[i][1]));
-                    rest |= lo[2 * p + i][h] & 0x7FFF7FFFu;
-                }
-            }
-        h128_mma(a, lo, __any_sync(0xFFFFFFFFu, rest != 0u) != 0, hb, out);
-    }
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const float2 e = mul2(out[2 * p][t], kHadScale), f = mul2(out[2 * p + 1][t], kHadScale);
-            w[2 * t][p] = pack_half2(e.x, f.x);
-            w[2 * t + 1][p] = pack_half2(e.y, f.y);
-        }
-}
-
 // sixteen bytes as four words; `wide`: p is 16-byte aligned, else it is to 8 bytes
 __device__ __forceinline__ void load_16b(const void* p, bool wide, uint32_t (&w)[4]) {
     if (wide) {
@@ -271,6 +223,64 @@ __device__ __forceinline__ void load_16b(const void* p, bool wide, uint32_t (&w)
     }
 }
 __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
+
+// format.prepareInput's rotation of a block: w (f16 pairs, w[s][p] = elements 8 (4 s + q) + 2 p, + 1 of this quad's position) times
+// the scales at sp (f16, this lane's first element; `wide`: 16-byte aligned), H128, / sqrt(128), rounded to f16; in place. Sign
+// scales (the usual suh) are a sign flip of the f16 values, and need no registers past it; with any other a product is taken in
+// f32 and split into an f16 part and the f16 of what is left, so that the sums see the f32 products.
+__device__ __forceinline__ void rotate_block(uint32_t (&w)[4][4], const __half* sp, bool wide, const HadB& hb) {
+    uint32_t a[8][2], odd = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        uint32_t sc[4];
+        load_16b(sp + 32 * s, wide, sc);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            odd |= (sc[p] & 0x7FFF7FFFu) ^ 0x3C003C00u;
+            w[s][p] ^= sc[p] & 0x80008000u;
+        }
+    }
+    float2 out[8][2];
+    if (__any_sync(0xFFFFFFFFu, odd != 0u) == 0) {
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                a[2 * p][h] = pack_lo(w[2 * h][p], w[2 * h + 1][p]);
+                a[2 * p + 1][h] = pack_hi(w[2 * h][p], w[2 * h + 1][p]);
+            }
+        h128_mma(a, a, false, hb, out);
+    } else {
+        uint32_t lo[8][2], rest = 0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint32_t sc[2][4];
+            load_16b(sp + 64 * h, wide, sc[0]);
+            load_16b(sp + 64 * h + 32, wide, sc[1]);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const float2 x0 = unpack_half2(w[2 * h][p]), x1 = unpack_half2(w[2 * h + 1][p]);  // the signs are in already
+                const float2 c0 = unpack_half2(sc[0][p] & 0x7FFF7FFFu), c1 = unpack_half2(sc[1][p] & 0x7FFF7FFFu);
+                const float v[2][2] = {{x0.x * c0.x, x1.x * c1.x}, {x0.y * c0.y, x1.y * c1.y}};
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    a[2 * p + i][h] = pack_half2(v[i][0], v[i][1]);
+                    lo[2 * p + i][h] = pack_half2(v[i][0] - round_half(v[i][0]), v[i][1] - round_half(v[i][1]));
+                    rest |= lo[2 * p + i][h] & 0x7FFF7FFFu;
+                }
+            }
+        }
+        h128_mma(a, lo, __any_sync(0xFFFFFFFFu, rest != 0u) != 0, hb, out);
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const float2 e = mul2(out[2 * p][t], kHadScale), f = mul2(out[2 * p + 1][t], kHadScale);
+            w[2 * t][p] = pack_half2(e.x, f.x);
+            w[2 * t + 1][p] = pack_half2(e.y, f.y);
+        }
+}
 
 // eight consecutive elements i .. i + 7 (i a multiple of 8) of an activation array, each rounded to f16
 __device__ __forceinline__ void load_half8(const void* p, int dt, bool wide, size_t i, uint32_t (&w)[4]) {

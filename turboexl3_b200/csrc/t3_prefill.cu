@@ -182,7 +182,7 @@ struct PrepArgs {
     uint32_t topk;
     __half* xp;  // [ops][positions][K]
 };
-__global__ void __launch_bounds__(256, 3) prep_rows_kernel(const __grid_constant__ PrepArgs a) {
+__global__ void __launch_bounds__(256, 4) prep_rows_kernel(const __grid_constant__ PrepArgs a) {
     const uint32_t lane = threadIdx.x & 31u, q = lane & 3u, nblk = a.K >> 7;
     const uint32_t pairs = a.positions * nblk;  // (the callers keep positions x width under 2^31)
     pdl_wait();
@@ -205,13 +205,10 @@ __global__ void __launch_bounds__(256, 3) prep_rows_kernel(const __grid_constant
             // the row is read again for the second op (from L1): kept in registers over the first one's rotation it spilled
             const __half* sp = (op ? a.suh[1][bank] : a.suh[0][bank]) + (size_t)e * a.K + col;
             const bool wide_s = aligned16(sp);
-            uint32_t w[4][4], sc[4][4];
+            uint32_t w[4][4];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                load_half8(a.x, a.x_dt, wide_x, (size_t)row * a.K + col + 32u * s, w[s]);
-                load_16b(sp + 32 * s, wide_s, sc[s]);
-            }
-            rotate_block(w, sc, hb);
+            for (int s = 0; s < 4; ++s) load_half8(a.x, a.x_dt, wide_x, (size_t)row * a.K + col + 32u * s, w[s]);
+            rotate_block(w, sp, wide_s, hb);
             if (live) {
                 uint4* o = reinterpret_cast<uint4*>(a.xp + ((size_t)op * a.positions + p) * a.K + col);
 #pragma unroll
@@ -242,7 +239,7 @@ struct MidArgs {
     int clamp_at;
     __half* hd;  // [P][inter]
 };
-__global__ void __launch_bounds__(256, 3) mid_kernel(const __grid_constant__ MidArgs a) {
+__global__ void __launch_bounds__(256, 4) mid_kernel(const __grid_constant__ MidArgs a) {
     const uint32_t lane = threadIdx.x & 31u, q = lane & 3u, nblk = a.inter >> 7;
     const uint32_t pairs = a.positions * nblk;
     pdl_wait();
@@ -256,7 +253,7 @@ __global__ void __launch_bounds__(256, 3) mid_kernel(const __grid_constant__ Mid
         const __half* suh = a.down_suh[id >> 24] + (size_t)(id & 0xFFFFFFu) * a.inter + col;
         const bool wide_s = aligned16(suh);
         const size_t zo = (size_t)p * a.inter + col;
-        uint32_t g[4][4], u[4][4], sc[4][4];
+        uint32_t g[4][4], u[4][4];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
             load_16b(a.z + zo + 32 * s, true, g[s]);
@@ -269,9 +266,7 @@ __global__ void __launch_bounds__(256, 3) mid_kernel(const __grid_constant__ Mid
                 const float2 gv = unpack_half2(g[s][j]), uv = unpack_half2(u[s][j]);
                 g[s][j] = pack_half2(swiglu_f32(gv.x, uv.x, a.limit, a.clamp_at), swiglu_f32(gv.y, uv.y, a.limit, a.clamp_at));
             }
-#pragma unroll
-        for (int s = 0; s < 4; ++s) load_16b(suh + 32 * s, wide_s, sc[s]);  // (with the loads above it cost spills)
-        rotate_block(g, sc, hb);
+        rotate_block(g, suh, wide_s, hb);
         if (live) {
             uint4* o = reinterpret_cast<uint4*>(a.hd + zo);
 #pragma unroll
