@@ -239,6 +239,10 @@ __device__ __forceinline__ uint32_t canon_id(const MoeArgs& a, uint32_t id) {
 // The arrays of the bank a canonical id names (bank 0: the call's own)
 #define T3_BANK_FIELD(a, id, f) (!(a).banked || ((id) >> 24) == 0u ? (a).f : (((id) >> 24) == 1u ? (a).ext[0].f : (a).ext[1].f))
 
+// A bank of one expert (a shared expert's): every row-slot runs it whatever its id says, so nothing waits for the routing and the
+// weights may start before the stream's previous kernel is done.
+__device__ __forceinline__ bool one_expert(const MoeArgs& a) { return a.experts == 1u && !a.banked; }
+
 // Row-slot j's expert and the row-slots it serves. The row-slots on one expert, in ascending order, are cut into runs of RM, a
 // run's first row-slot serves the run (its CTAs decode the expert's weights for all of them) and the others skip: an expert with
 // more than RM members is served by several CTAs at once. One ballot a 32 row-slots and one barrier (finding the members took
@@ -249,6 +253,13 @@ __device__ __forceinline__ Members find_members(const MoeArgs& a, uint32_t j, ui
     const uint32_t* inds = static_cast<const uint32_t*>(a.inds);
     constexpr uint32_t kWarps = kGemvThreads / 32u, kTurns = (kMaxSlots / 32u + kWarps - 1u) / kWarps;
     Members m;
+    if (one_expert(a)) {
+        m.expert = 0u;
+        m.skip = j % RM != 0u;
+        m.count = min((uint32_t)RM, slots - j);
+        if (threadIdx.x < m.count) members[threadIdx.x] = (uint16_t)(j + threadIdx.x);
+        return m;
+    }
     m.expert = canon_id(a, inds[j]);
     uint32_t mine[kTurns];  // this warp's ballots
 #pragma unroll
@@ -305,7 +316,8 @@ __device__ __forceinline__ void moe_gate_up_body(const MoeArgs& a) {
     const uint32_t proj = rank & 1u, kpart = rank >> 1;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t H = a.hidden, I = a.inter;
-    pdl_wait();     // the routing (and x) may be the previous kernel's output
+    const bool known = one_expert(a);
+    if (!known) pdl_wait();  // the routing (and x) may be the previous kernel's output
     const Members mem = find_members<RM>(a, j, s_members, s_masks);
     if (mem.skip) return;
     const uint32_t id = mem.expert, e = a.banked ? id & 0xFFFFFFu : id;
@@ -336,8 +348,9 @@ __device__ __forceinline__ void moe_gate_up_body(const MoeArgs& a) {
     const uint32_t count = mem.count;
     if (warp == kConsumerWarps) {
         produce_slab(c.ring, c.full, c.empty, wsrc, (size_t)out_tiles * tile_bytes, nrows, row_bytes, rc, pos, lane, a.err);
-        pdl_trigger();  // after the wait: the down launch reads the routing ahead of its own wait
+        pdl_trigger();  // after the wait: the down launch reads the routing (if it needs it) ahead of its own wait
     } else {
+        if (known) pdl_wait();
         for (uint32_t task = warp; task < count * nblk; task += kConsumerWarps) {
             const uint32_t m = task / nblk, b = task - m * nblk;
             const uint32_t row = s_members[m] / a.topk, k0 = (b0 + b) * 128u;
