@@ -69,12 +69,6 @@ t3_config config() {
     return g_cfg;
 }
 
-uint32_t pow2_at_most(uint32_t v, uint32_t cap) {
-    uint32_t s = 1;
-    while (s * 2u <= v && s * 2u <= cap) s *= 2u;
-    return s;
-}
-
 // CTAs that fit on the device at once (two GEMV CTAs a multiprocessor)
 uint32_t one_wave() {
     static std::atomic<uint32_t> ctas[64];  // per device ordinal; 0 = not asked yet

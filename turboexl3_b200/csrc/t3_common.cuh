@@ -60,25 +60,6 @@ __device__ __forceinline__ void h128_warp(float (&v)[4], uint32_t lane) {
     v[3] = d01 - d23;
 }
 
-// The same transform for a lane that holds four CONSECUTIVE elements 4 L .. 4 L + 3 (so a warp's loads and stores of a
-// 128-block are one contiguous 256- or 512-byte run): index bits 0-1 inside the lane, bits 2-6 across lanes.
-__device__ __forceinline__ void h128_warp_v4(float (&v)[4], uint32_t lane) {
-    const float s01 = v[0] + v[1], d01 = v[0] - v[1], s23 = v[2] + v[3], d23 = v[2] - v[3];
-    v[0] = s01 + s23;
-    v[1] = d01 + d23;
-    v[2] = s01 - s23;
-    v[3] = d01 - d23;
-#pragma unroll
-    for (uint32_t bit = 1; bit < 32u; bit <<= 1) {
-        const bool upper = (lane & bit) != 0u;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float other = __shfl_xor_sync(0xFFFFFFFFu, v[j], bit);
-            v[j] = upper ? other - v[j] : v[j] + other;
-        }
-    }
-}
-
 // four consecutive elements i .. i + 3 (i a multiple of 4) of an activation array as f32, one vector load
 __device__ __forceinline__ void load_act4(const void* p, int dt, size_t i, float (&v)[4]) {
     if (dt == kF32) {
@@ -96,8 +77,6 @@ __device__ __forceinline__ void load_act4(const void* p, int dt, size_t i, float
         }
     }
 }
-
-__device__ __forceinline__ void load_half4(const __half* p, float (&v)[4]) { load_act4(p, kF16, 0, v); }
 
 // four consecutive elements stored in dtype dt (round to nearest even), one vector store
 __device__ __forceinline__ void store_act4(void* p, int dt, size_t i, const float (&v)[4]) {
@@ -307,10 +286,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t arrivals) {
 // makes freshly initialised barriers visible to the copy engine and to the cluster
 __device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 __device__ __forceinline__ void mbar_arrive_expect_tx_addr(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -325,18 +300,6 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t addr, uint32_t parity) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    return done;
-}
-// whether the phase has completed, without waiting at all
-__device__ __forceinline__ uint32_t mbar_test(uint32_t addr, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done)
         : "r"(addr), "r"(parity)
@@ -413,10 +376,6 @@ __device__ __forceinline__ void named_sync(uint32_t id, uint32_t threads) {
 // weight-side vectors whose first use sits behind a wait, so that the use finds them in L2 and not in DRAM
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes, uint32_t lane) {
     if (lane * 128u < bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t*>(p) + lane * 128u));
-}
-
-static __device__ __noinline__ void report(uint32_t* err, uint32_t bit) {
-    if (err) atomicOr(err, bit);
 }
 
 // Programmatic dependent launch: `pdl_trigger` lets the next kernel of the stream start its own prologue (its weight

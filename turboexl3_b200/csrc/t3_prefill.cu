@@ -432,8 +432,8 @@ uint32_t prefill_ksplit(size_t rows, uint32_t in, uint32_t out) {
     return s;
 }
 
-// the prepared rows (the GEMM's epilogue finishes into y, so the inner products of an unsliced call never reach memory);
-// for a sliced call the slices' partial sums and the tiles' arrival counters as well
+// the prepared rows (the GEMM's epilogue finishes into y, so the inner products of an unsliced call never reach memory); for a
+// sliced call the slices' partial sums as well (sized in whole 128-row tiles and a word a tile, as callers of this size expect)
 size_t prefill_linear_workspace(size_t rows, uint32_t in, uint32_t out) {
     size_t bytes = up256(rows * in * 2u);
     const uint32_t s = prefill_ksplit(rows, in, out);
