@@ -438,10 +438,10 @@ struct DenseWs {
 // CTA repeats the rotation of its whole slice for every row before its first tensor-core step).
 bool prep_ahead(uint32_t rows, uint32_t slice_max) { return rows > kFusedRows || rows * (slice_max / 128u) > 2u * kConsumerWarps; }
 
-DenseWs dense_ws(uint32_t rows, uint32_t in, uint32_t out, uint32_t global_split, uint32_t slice_max) {
+DenseWs dense_ws(uint32_t rows, uint32_t in, uint32_t out, uint32_t global_split, bool ahead) {
     DenseWs w;
     w.xp = 0;
-    w.part = prep_ahead(rows, slice_max) ? align256((size_t)rows * in * 2u) : 0u;
+    w.part = ahead ? align256((size_t)rows * in * 2u) : 0u;
     w.counters = w.part + (global_split ? align256((size_t)(out / 128u) * global_split * rows * 512u) : 0u);
     w.total = w.counters + (global_split ? align256((size_t)(out / 128u) * 4u) : 0u);
     return w;
@@ -501,7 +501,11 @@ void fill_launch(t3_launch* l, const char* symbol, const char* group, dim3 grid,
 }  // namespace
 
 
-size_t t3_linear_workspace_bytes(size_t rows, int in_dim, int out_dim, int n) {
+}  // extern "C"
+
+namespace t3 {
+
+size_t linear_workspace(size_t rows, int in_dim, int out_dim, int n, bool far_x) {
     if (in_dim <= 0 || out_dim <= 0 || rows < 1) return 0;
     if (rows > T3_DECODE_ROWS_MAX) return prefill_linear_workspace(rows, (uint32_t)in_dim, (uint32_t)out_dim);
     if (in_dim % 128 != 0 || out_dim % 128 != 0 || !rate_ok(n)) return 0;
@@ -512,12 +516,12 @@ size_t t3_linear_workspace_bytes(size_t rows, int in_dim, int out_dim, int n) {
     DenseArgs a = {};
     a.in = (uint32_t)in_dim, a.out = (uint32_t)out_dim, a.n = (uint32_t)n, a.rows = (uint32_t)rows;
     if (plan_dense(a, cfg, true) != T3_OK) return 0;
-    return dense_ws(a.rows, a.in, a.out, a.part ? a.split : 0u, a.slice_max).total;
+    return dense_ws(a.rows, a.in, a.out, a.part ? a.split : 0u, far_x || prep_ahead(a.rows, a.slice_max)).total;
 }
 
-int t3_linear(const void* x, int x_dtype, size_t rows, const void* trellis, const void* suh, const void* svh,
+int linear_call(const void* x, int x_dtype, size_t rows, const void* trellis, const void* suh, const void* svh,
               int in_dim, int out_dim, int n, t3_decode dec, void* y, void* workspace, size_t workspace_bytes,
-              void* stream) {
+              void* stream, bool far_x) {
     if (!x || !trellis || !suh || !svh || !y) return T3_NULL_POINTER;
     if (in_dim <= 0 || out_dim <= 0 || in_dim % 128 != 0 || out_dim % 128 != 0 || !rate_ok(n) || rows < 1 ||
         rows > (size_t)1 << 30)
@@ -530,7 +534,7 @@ int t3_linear(const void* x, int x_dtype, size_t rows, const void* trellis, cons
         if (!cfg.prefill) return T3_ENGINE_NOT_IMPLEMENTED;
         if (rows > 0x7FFFFFFFu / (size_t)(in_dim > out_dim ? in_dim : out_dim)) return T3_BAD_EXL3_SHAPE;
         if (rows > kPrefillDenseRowsMax) return T3_BAD_EXL3_SHAPE;  // the prepare launch's row groups are a grid dimension
-        if (!workspace || workspace_bytes < t3_linear_workspace_bytes(rows, in_dim, out_dim, n)) return T3_WORKSPACE_TOO_SMALL;
+        if (!workspace || workspace_bytes < linear_workspace(rows, in_dim, out_dim, n, far_x)) return T3_WORKSPACE_TOO_SMALL;
         PrefillLinearArgs p = {x, y, static_cast<const uint8_t*>(trellis), nullptr, suh, svh, (uint32_t)rows, (uint32_t)in_dim,
                                (uint32_t)out_dim, (uint32_t)n, mask, x_dtype, workspace, dev_error_ptr(), !cfg.no_overlap};
         note_engine(2, (uint64_t)in_dim, (uint64_t)out_dim, (uint64_t)n, 0);
@@ -552,11 +556,13 @@ int t3_linear(const void* x, int x_dtype, size_t rows, const void* trellis, cons
     note_engine(1, (uint64_t)in_dim, (uint64_t)out_dim, (uint64_t)n, 0);
     a.rows = (uint32_t)rows;
     if (int rc = plan_dense(a, cfg, workspace != nullptr)) return rc;
-    DenseWs ws = dense_ws(a.rows, a.in, a.out, a.part ? a.split : 0u, a.slice_max);
+    bool ahead = far_x || prep_ahead(a.rows, a.slice_max);
+    DenseWs ws = dense_ws(a.rows, a.in, a.out, a.part ? a.split : 0u, ahead);
     bool has_ws = workspace != nullptr && workspace_bytes >= ws.total;
     if (a.part && !has_ws) {  // too small for the global exchange: the cluster kernel, with the rotated rows if those fit
         if (int rc = plan_dense(a, cfg, false)) return rc;
-        ws = dense_ws(a.rows, a.in, a.out, 0u, a.slice_max);
+        ahead = far_x || prep_ahead(a.rows, a.slice_max);
+        ws = dense_ws(a.rows, a.in, a.out, 0u, ahead);
         has_ws = workspace != nullptr && workspace_bytes >= ws.total;
     }
     a.err = dev_error_ptr();
@@ -568,7 +574,7 @@ int t3_linear(const void* x, int x_dtype, size_t rows, const void* trellis, cons
     }
     a.x = x;
     a.y = y;
-    if (prep_ahead(a.rows, a.slice_max) && !cfg.probe && has_ws) {
+    if (ahead && !cfg.probe && has_ws) {
         a.xp_g = workspace;
         g_launches.fetch_add(1, std::memory_order_relaxed);
         if (int rc = cuda_status(launch_dense_prep(a, static_cast<cudaStream_t>(stream)))) return rc;
@@ -578,6 +584,18 @@ int t3_linear(const void* x, int x_dtype, size_t rows, const void* trellis, cons
         return cuda_status(launch_dense_gemv(a, 1 + cfg.probe, static_cast<cudaStream_t>(stream)));
     }
     return cuda_status(launch_dense_gemv(a, dec.codebook, static_cast<cudaStream_t>(stream)));
+}
+
+}  // namespace t3
+
+extern "C" {
+
+size_t t3_linear_workspace_bytes(size_t rows, int in_dim, int out_dim, int n) { return linear_workspace(rows, in_dim, out_dim, n, false); }
+
+int t3_linear(const void* x, int x_dtype, size_t rows, const void* trellis, const void* suh, const void* svh,
+              int in_dim, int out_dim, int n, t3_decode dec, void* y, void* workspace, size_t workspace_bytes,
+              void* stream) {
+    return linear_call(x, x_dtype, rows, trellis, suh, svh, in_dim, out_dim, n, dec, y, workspace, workspace_bytes, stream, false);
 }
 
 const char* t3_last_kernel_symbol(void) {

@@ -7,6 +7,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include "../../include/t3.h"
+
 namespace t3 {
 
 struct RingPlan {
@@ -161,6 +163,12 @@ struct MixedBanks {
     BankTab bank[kMixedBanksMax];
     uint32_t n[kMixedBanksMax];
 };
+// t3_linear and its workspace; far_x: x lies across the bus (a host array the kernels read in place), so at decode rows it is
+// rotated once by a launch of its own: read by every 128-output block instead, a row of 1536 crossed the bus 192 times for 24576
+// outputs
+size_t linear_workspace(size_t rows, int in_dim, int out_dim, int n, bool far_x);
+int linear_call(const void* x, int x_dtype, size_t rows, const void* trellis, const void* suh, const void* svh, int in_dim, int out_dim,
+                int n, t3_decode dec, void* y, void* workspace, size_t workspace_bytes, void* stream, bool far_x);
 // The routed chain at prefill rows: route -> prepare -> GEMM(gate|up) -> mid -> GEMM(down) -> finish
 size_t prefill_moe_workspace(size_t rows, uint32_t topk, uint32_t experts, uint32_t hidden, uint32_t inter);
 // mixed: the banks in the place of a's own (whose geometry, rows and clamp count; a.experts is the sum of the banks'), or null
