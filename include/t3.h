@@ -174,9 +174,9 @@ int t3_moe_clamped_banked(const void* x, int x_dtype, size_t rows, const t3_bank
 
 /* A routed layer whose experts have rates of their own, more than 32 rows (the reference serves one rate per bank,
  * src/root.zig:841): `count` banks of one geometry (1..T3_MIXED_BANKS_MAX), each at its own rate; layer expert g (0 .. ids - 1, the
- * router's numbering) is expert local_of[g] of bank bank_of[g] (device int64 arrays, every entry in range: not checked). One
- * sort, one prepare and one merge for the whole layer: y is, bit for bit, what one bank of those experts would give. `shared` as
- * in t3_moe_with_shared, or null. Up to 32 rows: Exl3EngineNotImplemented. */
+ * router's numbering) is expert local_of[g] of bank bank_of[g] (device int64 arrays; a bank, a number in its bank or a router
+ * id out of range is clamped into it). One sort, one prepare and one merge for the whole layer: y is, bit for bit, what one bank
+ * of those experts would give. `shared` as in t3_moe_with_shared, or null. Up to 32 rows: Exl3EngineNotImplemented. */
 #define T3_MIXED_BANKS_MAX 8
 size_t t3_moe_mixed_workspace_bytes(size_t rows, int topk, const t3_bank* banks, int count);
 int t3_moe_mixed(const void* x, int x_dtype, size_t rows, const t3_bank* banks, int count, const void* bank_of, const void* local_of,

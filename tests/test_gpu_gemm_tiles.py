@@ -7,7 +7,7 @@ import torch
 
 import turboexl3_b200 as t3
 from oracle import binding as ob
-from turboexl3_b200 import synth
+from turboexl3_b200 import mixed, synth
 
 from gpu_util import TORCH_DT, check, dev, host_f32, x_as
 from test_gpu_moe import check_moe, make_bank
@@ -49,20 +49,46 @@ def test_routed_tile_edges(case):
     assert t3.device_error() == 0
 
 
-@pytest.mark.parametrize("rows,dt", [(33, "f16"), (300, "bf16")])
-def test_mixed_banks_give_the_one_bank_bytes(rows, dt):
-    """Experts dealt over three banks (one of them with a single expert) at one rate: the bytes of the undivided bank."""
-    H, I, E, topk, n = 384, 256, 11, 4, 48
-    bank, _ = make_bank(2300, E, H, I, n)
+def split_bank(seed, E, H, I, n):
+    """A bank of 11 experts whole, and dealt over three banks (one of them with a single expert): bank, banks, bank_of, local_of."""
+    bank, _ = make_bank(seed, E, H, I, n)
     bank_of = torch.tensor([0, 2, 0, 2, 2, 0, 1, 0, 2, 0, 2])
     local_of = torch.zeros_like(bank_of)
     for b in range(3):
         local_of[bank_of == b] = torch.arange(int((bank_of == b).sum()))
     pick = lambda p, b: t3.Proj(*(v[(bank_of == b).to(v.device)].contiguous() for v in (p.trellis.view(torch.int16), p.suh, p.svh)))
-    banks = [t3.Bank(pick(bank.gate, b), pick(bank.up, b), pick(bank.down, b)) for b in range(3)]
+    return bank, [t3.Bank(pick(bank.gate, b), pick(bank.up, b), pick(bank.down, b)) for b in range(3)], bank_of, local_of
+
+
+@pytest.mark.parametrize("rows,dt", [(33, "f16"), (300, "bf16")])
+def test_mixed_banks_give_the_one_bank_bytes(rows, dt):
+    H, I, E, topk, n = 384, 256, 11, 4, 48
+    bank, banks, bank_of, local_of = split_bank(2300, E, H, I, n)
     inds, scores = synth.routing(2301, rows, E, topk)
     x, di, ds = x_as(synth.activations(2302, rows, H), dt), dev(inds), dev(scores)
     whole = t3.moe(x.view(1, rows, H), bank, di.view(1, rows, topk), ds.view(1, rows, topk))
     mixed = t3.api.moe_mixed(x, banks, bank_of.cuda(), local_of.cuda(), di, ds)
     assert torch.equal(whole.view(rows, H), mixed)
+    assert t3.device_error() == 0
+
+
+@pytest.mark.parametrize("rows", [5, 33, 300])
+def test_mixed_map_entries_out_of_range_are_clamped(rows):
+    """Banks, numbers in a bank and router ids past either end: the layer of the clamped map."""
+    H, I, E, topk, n = 256, 128, 11, 4, 48
+    _, banks, bank_of, local_of = split_bank(2310, E, H, I, n)
+    bad_bank, bad_local = bank_of.clone(), local_of.clone()
+    bad_bank[[0, 3, 6]] = torch.tensor([3, -1, 1 << 40])
+    bad_local[[0, 2, 9]] = torch.tensor([1 << 33, -7, 99])
+    good_bank = bad_bank.clamp(0, 2)
+    size = torch.tensor([b.gate.suh.shape[0] for b in banks])
+    good_local = torch.minimum(bad_local.clamp(min=0), size[good_bank] - 1)
+    inds, scores = synth.routing(2311, rows, E, topk)
+    x, di, ds = x_as(synth.activations(2312, rows, H), "f16"), dev(inds), dev(scores)
+    bad_inds = di.clone()
+    bad_inds[di == E - 1] = E + 1000
+    bad_inds[0, 0] = -1  # as u32: past every id
+    di[0, 0] = E - 1
+    layer = lambda bank, local, ids: mixed.mixed_rate_moe(x, banks, mixed.RateBuckets([n] * 3, bank, local, []), ids, ds, t3.Decode.mul1)
+    assert torch.equal(layer(bad_bank, bad_local, bad_inds), layer(good_bank, good_local, di))
     assert t3.device_error() == 0

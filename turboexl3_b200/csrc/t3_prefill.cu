@@ -34,14 +34,18 @@ size_t routed_tiles_max(size_t slots, uint32_t experts) {
 
 // Where the router's expert ids lie: one bank (bank_of null: the id is the expert), or several banks of one geometry at rates
 // of their own (layer expert g is expert local_of[g] of bank bank_of[g]). Experts are numbered bank by bank: bank b's from
-// base[b] on.
+// base[b] on. The ids and both arrays are the caller's: each is clamped into its range, since a number indexes the counters here
+// and the bank's arrays later.
 struct ExpertMap {
     const int64_t *bank_of, *local_of;
     uint32_t base[kMixedBanksMax + 1];
-    uint32_t banks, ids;  // banks; router ids (out-of-range ones are clamped)
+    uint32_t banks, ids;  // banks (none empty); router ids
+    static __device__ uint32_t clamped(int64_t v, uint32_t count) { return (uint32_t)min(max(v, (int64_t)0), (int64_t)count - 1); }
     __device__ uint32_t number(uint32_t id) const {
         id = min(id, ids - 1u);
-        return bank_of ? base[bank_of[id]] + (uint32_t)local_of[id] : id;
+        if (!bank_of) return id;
+        const uint32_t b = clamped(bank_of[id], banks);
+        return base[b] + clamped(local_of[id], base[b + 1u] - base[b]);
     }
     // the bank of an expert number, and the number inside it
     __device__ uint32_t bank(uint32_t e) const {

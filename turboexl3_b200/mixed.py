@@ -74,12 +74,13 @@ def mixed_rate_moe(x: torch.Tensor, banks: Sequence, buckets: RateBuckets, inds:
         expert_fn = lambda xr, bank, er: expert_rows(xr, bank, er, dec)
     if merge_fn is None:
         merge_fn = lambda vv, sc: api.moe_merge(vv, sc.contiguous(), x.dtype, shared)
-    flat = inds.reshape(-1).to(torch.int64)
-    bank_of, local_of = buckets.bank_of.to(flat.device), buckets.local_of.to(flat.device)
-    slot_bank = bank_of[flat]
+    bank_of, local_of = buckets.bank_of.to(inds.device), buckets.local_of.to(inds.device)
+    # a router id (read as u32), a bank and a number in its bank are clamped into range, as the native call clamps them
+    flat = (inds.reshape(-1).to(torch.int64) & 0xFFFFFFFF).clamp(max=bank_of.numel() - 1)
+    slot_bank = bank_of[flat].clamp(0, len(banks) - 1)
     v = torch.empty((rows * topk, x.shape[1]), dtype=torch.float16, device=x.device)
     for b, bank in enumerate(banks):
         sel = torch.nonzero(slot_bank == b).flatten()
         if sel.numel():
-            v[sel] = expert_fn(x[torch.div(sel, topk, rounding_mode="floor")], bank, local_of[flat[sel]]).to(v.dtype)
+            v[sel] = expert_fn(x[torch.div(sel, topk, rounding_mode="floor")], bank, local_of[flat[sel]].clamp(0, 0x7FFFFFFF)).to(v.dtype)
     return merge_fn(v.view(rows, topk, x.shape[1]), scores)
