@@ -135,3 +135,39 @@ def test_mixed_rate_buckets_route_every_slot_to_its_sub_bank():
     y = mixed.mixed_rate_moe(x, banks, b, inds, scores, None, expert_fn=expert_fn, merge_fn=merge_fn)
     want = ((x.float().unsqueeze(1) * (inds.float() + 1.0).unsqueeze(-1)).half().float() * scores.unsqueeze(-1)).sum(1)
     assert torch.allclose(y, want, rtol=0, atol=1e-6)
+
+
+@pytest.mark.parametrize("form,native", [("plain", True), ("int32 maps", True), ("strided maps", True), ("another inner width", False),
+                                         ("an empty bank", False), ("nine banks", False)])
+def test_mixed_rate_layer_takes_every_form_of_bank_and_map(form, native, monkeypatch):
+    """Which forms go to the one native call (what it is handed is what it takes), and that the others still run bank by bank."""
+    from types import SimpleNamespace as NS
+
+    from turboexl3_b200 import api, mixed
+    H, rows, topk = 128, 40, 2
+    sizes, widths = [4, 3, 4], [256, 256, 256]
+    if form == "another inner width":
+        widths[1] = 384
+    if form == "an empty bank":
+        sizes = [4, 0, 7]
+    if form == "nine banks":
+        sizes, widths = [2] * 9, [256] * 9
+    banks = [NS(down=NS(suh=torch.zeros((e, w)))) for e, w in zip(sizes, widths)]
+    bank_of = torch.repeat_interleave(torch.arange(len(sizes)), torch.tensor(sizes))
+    local_of = torch.cat([torch.arange(e) for e in sizes])
+    if form == "int32 maps":
+        bank_of, local_of = bank_of.int(), local_of.int()
+    if form == "strided maps":
+        bank_of, local_of = torch.stack([bank_of, local_of], 1).unbind(1)
+    calls = []
+
+    def moe_mixed(x, bs, bank, local, inds, scores, dec, shared):
+        assert bank.dtype == local.dtype == torch.int64 and bank.is_contiguous() and local.is_contiguous()
+        calls.append("native")
+
+    monkeypatch.setattr(api, "moe_mixed", moe_mixed)
+    monkeypatch.setattr(mixed, "expert_rows", lambda xr, bank, er, dec: calls.append("bank") or xr)
+    monkeypatch.setattr(api, "moe_merge", lambda v, scores, dtype, shared: calls.append("merge"))
+    inds = torch.arange(rows * topk, dtype=torch.int32).view(rows, topk) % len(bank_of)
+    mixed.mixed_rate_moe(torch.zeros((rows, H)), banks, mixed.RateBuckets([], bank_of, local_of, []), inds, torch.ones((rows, topk)), None)
+    assert calls == (["native"] if native else ["bank"] * sum(e > 0 for e in sizes) + ["merge"])

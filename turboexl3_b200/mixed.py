@@ -6,7 +6,8 @@ different bit widths is held as one sub-bank per rate. This module routes such a
 that holds its expert (the finished down projection `v`, f16, exactly what the single-bank chain feeds its merge), and the
 score-weighted sum runs once over all slots in slot order — so the result is the one a single bank of those experts would
 give, whatever the bucketing. Past 32 rows the whole layer is one native call (`api.moe_mixed`); decode rows, more than eight
-rates and injected stand-ins run each sub-bank's slots at top-1 with score 1 and merge with `t3.moe_merge`.
+rates, banks that are empty or differ in their inner width, and injected stand-ins run each sub-bank's slots at top-1 with
+score 1 and merge with `t3.moe_merge`.
 """
 from __future__ import annotations
 
@@ -66,10 +67,11 @@ def mixed_rate_moe(x: torch.Tensor, banks: Sequence, buckets: RateBuckets, inds:
     rows, topk = inds.shape
     if (expert_fn is None and merge_fn is None and rows > api.DECODE_ROWS_MAX and 0 < len(banks) <= api.MIXED_BANKS_MAX
             and inds.dtype in (torch.int32, torch.uint32) and x.is_contiguous() and x.dim() == 2
-            and rows * topk * max(x.shape[1], banks[0].down.suh.shape[1]) < 1 << 31):  # the native call's index range
+            and rows * topk * max(x.shape[1], banks[0].down.suh.shape[1]) < 1 << 31  # the native call's index range,
+            and all(b.down.suh.shape[0] > 0 and b.down.suh.shape[1] == banks[0].down.suh.shape[1] for b in banks)):  # its banks
         # one sort, one prepare and one merge for the layer, a GEMM pair a bank
-        return api.moe_mixed(x, banks, buckets.bank_of.to(x.device), buckets.local_of.to(x.device), inds.contiguous(),
-                             scores.contiguous(), dec, shared)
+        bank_of, local_of = (m.to(x.device, torch.int64).contiguous() for m in (buckets.bank_of, buckets.local_of))
+        return api.moe_mixed(x, banks, bank_of, local_of, inds.contiguous(), scores.contiguous(), dec, shared)
     if expert_fn is None:
         expert_fn = lambda xr, bank, er: expert_rows(xr, bank, er, dec)
     if merge_fn is None:
