@@ -6,6 +6,7 @@ import os
 import re
 
 import pytest
+import torch
 
 import turboexl3_b200 as t3
 from turboexl3_b200 import api
@@ -173,3 +174,12 @@ def test_launch_plans_name_kernels_and_shapes():
     assert chain[0]["grid"][1:] == (512 // 128, 40) and chain[1]["grid"][1:] == (2048 // 128, 40)
     assert chain[0]["cluster"] == chain[0]["grid"][0] and chain[2]["cluster"] == 1
     assert len(t3.plan_moe(2, 1, 1, 2048, 512, 48)) == 2  # one slot a row: the down launch stores y, no merge
+
+
+def test_a_shared_output_that_is_missing_or_not_ordered_is_refused():
+    """No `shared`, or an event that nobody has recorded (its handle is null): never a call without the add, or without the wait."""
+    from types import SimpleNamespace
+    x = torch.zeros((1, 1, 128))
+    for shared, event in ((None, None), (None, SimpleNamespace(cuda_event=FAKE)), (x, SimpleNamespace(cuda_event=0))):
+        with pytest.raises(t3.Exl3Error, match="NullPointer"):
+            t3.moe_with_shared(x, None, None, None, t3.Decode.mul1, shared, shared_ready=event)

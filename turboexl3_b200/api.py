@@ -571,4 +571,6 @@ def moe_with_shared(x, bank: Bank, inds, scores, dec: Decode, shared: torch.Tens
     """root.moeWithShared (src/root.zig:976-984). shared_ready: an event recorded on the stream that computes `shared`;
     only the call's last launch waits for it (t3_moe_with_shared_after)."""
     del verify_rows
+    if shared is None or (shared_ready is not None and not shared_ready.cuda_event):  # an event nobody has recorded has no handle
+        raise Exl3Error(14, "NullPointer")
     return _moe(x, bank, inds, scores, dec, 0, CLAMP_GATE_IN, shared, shared_ready=shared_ready)
