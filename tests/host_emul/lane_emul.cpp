@@ -3,9 +3,11 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 
 #include "../../oracle/t3_oracle.h"
 #include "../../turboexl3_b200/csrc/t3_lane.cuh"
+#include "../../turboexl3_b200/csrc/t3_slot.cuh"
 
 namespace {
 
@@ -123,6 +125,22 @@ extern "C" int lane_emul_lane_order() {
         bad += t3::lane_order16(2 * q + 1) != 4 * q + 1;
         bad += t3::lane_order16(2 * q + 8) != 4 * q + 2;
         bad += t3::lane_order16(2 * q + 9) != 4 * q + 3;
+    }
+    return bad;
+}
+
+// a sorted row-slot's bank and expert at the ends of their ranges: one bank of as many experts as an int counts, eight of 2^24
+extern "C" int lane_emul_slot_ids() {
+    int bad = 0;
+    for (uint32_t banks = 1; banks <= 8; ++banks) {
+        const t3::SlotId ids = {t3::SlotId::bits_for(banks)};
+        const uint32_t most = banks == 1 ? 0x7FFFFFFFu : 1u << 24;
+        for (uint32_t bank = 0; bank < banks; ++bank)
+            for (uint32_t e : {0u, 1u, 0xFFFFFFu, 0x1000000u, most - 1u}) {
+                if (e >= most) continue;
+                const uint32_t id = ids.pack(bank, e);
+                bad += ids.bank(id) != bank || ids.expert(id) != e;
+            }
     }
     return bad;
 }

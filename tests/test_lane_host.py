@@ -17,8 +17,8 @@ def emul():
     os.makedirs(out, exist_ok=True)
     so = os.path.join(out, "liblane_emul.so")
     srcs = [os.path.join(HERE, "host_emul", "lane_emul.cpp"), os.path.join(ROOT, "oracle", "t3_oracle.c")]
-    hdr = os.path.join(ROOT, "turboexl3_b200", "csrc", "t3_lane.cuh")
-    newest = max(os.path.getmtime(p) for p in srcs + [hdr])
+    hdrs = [os.path.join(ROOT, "turboexl3_b200", "csrc", h) for h in ("t3_lane.cuh", "t3_slot.cuh")]
+    newest = max(os.path.getmtime(p) for p in srcs + hdrs)
     if not os.path.exists(so) or os.path.getmtime(so) < newest:
         obj = os.path.join(out, "t3_oracle.o")
         subprocess.run(["gcc", "-O2", "-ffp-contract=off", "-fPIC", "-std=c11", "-c", srcs[1], "-o", obj], check=True)
@@ -45,3 +45,8 @@ def test_runtime_reader_every_rate(emul):
 
 def test_lane_order(emul):
     assert emul.lane_emul_lane_order() == 0
+
+
+def test_slot_ids_hold_every_bank_and_expert(emul):
+    """A bank of more than 2^24 experts keeps its ids whole (24 bits made the rest a bank that is not there)."""
+    assert emul.lane_emul_slot_ids() == 0

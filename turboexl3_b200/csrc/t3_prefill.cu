@@ -13,6 +13,7 @@
 #include "t3_common.cuh"
 #include "t3_gemm.h"
 #include "t3_internal.h"
+#include "t3_slot.cuh"
 
 namespace t3 {
 namespace {
@@ -140,15 +141,16 @@ __global__ void __launch_bounds__(kRouteThreads) route_plan_kernel(const uint32_
     if (tid <= map.banks && map.base[tid] >= experts) range[tid] = s_base[1];
 }
 
-// every slot's sorted position (inv), and per position the x row it reads and its (bank << 24 | expert inside the bank)
+// every slot's sorted position (inv), and per position the x row it reads and its bank and expert (SlotId)
 __global__ void route_scatter_kernel(const uint32_t* inds, uint32_t slots, const __grid_constant__ ExpertMap map, const uint32_t* rank,
-                                     const uint32_t* first, const uint32_t* row_map, uint32_t topk, uint2* where, uint32_t* inv) {
+                                     const uint32_t* first, const uint32_t* row_map, uint32_t topk, SlotId ids, uint2* where,
+                                     uint32_t* inv) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_wait();
     pdl_trigger();
     if (s >= slots) return;
     const uint32_t e = map.number(inds[s]), p = first[e] + rank[s], b = map.bank(e);
-    where[p] = make_uint2(row_map ? row_map[s] : s / topk, (b << 24) | (e - map.base[b]));
+    where[p] = make_uint2(row_map ? row_map[s] : s / topk, ids.pack(b, e - map.base[b]));
     inv[s] = p;
 }
 
@@ -182,6 +184,7 @@ struct PrepArgs {
     const __half* suh[2][kMixedBanksMax];  // per op and bank, expert-major
     uint32_t K, positions, ops;
     const uint2* where;
+    SlotId ids;               // how where[p].y is packed
     const uint32_t* row_map;  // where null: position p reads row row_map[p], or row p / topk
     uint32_t topk;
     __half* xp;  // [ops][positions][K]
@@ -200,7 +203,7 @@ __global__ void __launch_bounds__(256, 4) prep_rows_kernel(const __grid_constant
         uint32_t row, e = 0, bank = 0;
         if (a.where) {
             const uint2 w = a.where[p];
-            row = w.x, bank = w.y >> 24, e = w.y & 0xFFFFFFu;
+            row = w.x, bank = a.ids.bank(w.y), e = a.ids.expert(w.y);
         } else {
             row = a.row_map ? a.row_map[p] : p / a.topk;
         }
@@ -238,6 +241,7 @@ struct MidArgs {
     const __half* z;  // [2][P][inter]: finished gate, finished up
     const __half* down_suh[kMixedBanksMax];
     const uint2* where;  // or null: one expert
+    SlotId ids;
     uint32_t positions, inter;
     float limit;
     int clamp_at;
@@ -254,7 +258,7 @@ __global__ void __launch_bounds__(256, 4) mid_kernel(const __grid_constant__ Mid
         const uint32_t f = live ? f0 + (lane >> 2) : pairs - 1u;
         const uint32_t p = f / nblk, col = (f - p * nblk) * 128u + 8u * q;
         const uint32_t id = a.where ? a.where[p].y : 0u;
-        const __half* suh = a.down_suh[id >> 24] + (size_t)(id & 0xFFFFFFu) * a.inter + col;
+        const __half* suh = a.down_suh[a.ids.bank(id)] + (size_t)a.ids.expert(id) * a.inter + col;
         const bool wide_s = aligned16(suh);
         const size_t zo = (size_t)p * a.inter + col;
         uint32_t g[4][4], u[4][4];
@@ -587,6 +591,7 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
     const MixedBanks& banks = mixed ? *mixed : one;
     // one expert (a shared expert's chain): the slots are in order as they stand, the chain is a dense one
     const bool routed = a.experts > 1u, overlap = a.overlap != 0;
+    const SlotId ids = {SlotId::bits_for(banks.count)};
     cudaError_t rc;
     if (routed) {
         ExpertMap map = {};
@@ -600,7 +605,7 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
         route_plan_kernel<<<(S + kRouteSlots - 1u) / kRouteSlots, kRouteThreads, a.experts <= kRouteExperts ? a.experts * 4u : 0u, stream>>>(
             inds, S, map, w.counts, w.counts + a.experts, w.rank, w.first, w.tiles, w.range);
         rc = launch_overlapped(route_scatter_kernel, dim3((S + 255u) / 256u), 256, 0, stream, overlap, 1, inds, S, map,
-                               static_cast<const uint32_t*>(w.rank), static_cast<const uint32_t*>(w.first), a.row_map, a.topk, w.where, w.inv);
+                               static_cast<const uint32_t*>(w.rank), static_cast<const uint32_t*>(w.first), a.row_map, a.topk, ids, w.where, w.inv);
         if (rc != cudaSuccess) return rc;
         *launches += 2;
     }
@@ -616,6 +621,7 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
     pa.K = H;
     pa.positions = S;
     pa.where = m.where = routed ? w.where : nullptr;
+    pa.ids = m.ids = ids;
     pa.row_map = a.row_map;
     pa.topk = a.topk;
     pa.xp = w.xp;
