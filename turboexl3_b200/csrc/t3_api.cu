@@ -694,6 +694,16 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     }
     if (!plan_ring(rm, rm, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu) || !plan_ring(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d))
         return T3_ENGINE_NOT_IMPLEMENTED;
+    // When gate|up lets the down launch start: at once (its CTAs then fetch their first codes beside gate|up's) or when its own codes
+    // are all on the way. At once where gate|up leaves multiprocessors idle, unless down's CTAs would then double up on those while
+    // later they had a multiprocessor each: down's grid is past one a multiprocessor anyway, or both grids fit side by side. One
+    // layer of 512 experts of 2048 x 512 (80 and 160 CTAs) 32.7 -> 24.5 us, 128 experts at 3 rows (96 and 192) 33.2 -> 25.7, 32
+    // of 4096 x 1024 (64 and 64) 28.9 -> 23.3; against the rule 64 of 2048 x 2048 (128 and 64) 35.6 -> 40.9, 64 of 1024 x 256 (128
+    // and 128) 16.1 -> 16.8, and past one wave (two rows and more of the first) 1 % the other way. A one-expert chain, whose
+    // neighbour on the stream is another chain, keeps the late start (16 rows of 2048 x 512: 25.3 us against 31.8).
+    const uint32_t sms = one_wave() / 2u;
+    const uint64_t gu = (uint64_t)2u * a.split_gu * (a.inter / 128u) * slots, down = (uint64_t)a.split_d * (a.hidden / 128u) * slots;
+    a.down_early = a.experts > 1u && gu <= sms && (down > sms || gu + down <= sms);
     return T3_OK;
 }
 

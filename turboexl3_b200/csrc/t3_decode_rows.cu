@@ -318,6 +318,7 @@ __device__ __forceinline__ void moe_gate_up_body(const MoeArgs& a) {
     const uint32_t H = a.hidden, I = a.inter;
     const bool known = one_expert(a);
     if (!known) pdl_wait();  // the routing (and x) may be the previous kernel's output
+    if (a.down_early) pdl_trigger();  // after the wait: the down launch reads the routing ahead of its own
     const Members mem = find_members<RM>(a, j, s_members, s_masks);
     if (mem.skip) return;
     const uint32_t id = mem.expert, e = a.banked ? id & 0xFFFFFFu : id;
@@ -348,7 +349,7 @@ __device__ __forceinline__ void moe_gate_up_body(const MoeArgs& a) {
     const uint32_t count = mem.count;
     if (warp == kConsumerWarps) {
         produce_slab(c.ring, c.full, c.empty, wsrc, (size_t)out_tiles * tile_bytes, nrows, row_bytes, rc, pos, lane, a.err);
-        pdl_trigger();  // after the wait: the down launch reads the routing (if it needs it) ahead of its own wait
+        pdl_trigger();
     } else {
         if (known) pdl_wait();
         for (uint32_t task = warp; task < count * nblk; task += kConsumerWarps) {

@@ -71,6 +71,7 @@ struct MoeArgs {
     uint32_t split_gu, slice_max_gu;   // K slices of gate|up (cluster = 2 * split_gu), largest slice
     uint32_t split_d, slice_max_d;     // K slices of down
     RingPlan ring_gu, ring_d;
+    uint32_t down_early;               // gate|up lets the down launch start as soon as it has the routing (see plan_moe_decode)
     int overlap;
     uint32_t* err;
 };
