@@ -31,6 +31,22 @@ def test_dense_tile_edges(case):
     assert t3.device_error() == 0
 
 
+@pytest.mark.parametrize("in_dim,out_dim,n,dt", [(4096, 1024, 32, "f16"), (4096, 512, 48, "f32"), (2048, 2048, 64, "bf16")])
+def test_sliced_tile_heights(in_dim, out_dim, n, dt):
+    """Calls in K slices whose row tiles follow the clusters that are resident at once: one tile, several, ragged last ones; a row's
+    bytes do not depend on the height of its tile."""
+    trellis, suh, svh = synth.linear(2120 + n, in_dim, out_dim, n, scaled=True)
+    what = ob.reconstruct_inner(trellis, in_dim, out_dim, n, t3.MUL1, 16)
+    t, a, b = dev(trellis), dev(suh), dev(svh)
+    for rows, few in ((33, 33), (100, 33), (200, 100), (256, 200), (300, 257), (512, 300)):
+        x = x_as(synth.activations(2121, rows, in_dim), dt)
+        y = t3.linear(x, t, a, b)
+        sample = sorted({0, 15, 16, few - 1, rows // 2, rows - 1})
+        check(host_f32(y)[sample], ob.linear_rows_what(host_f32(x)[sample], what, suh, svh, in_dim, out_dim), dt, ("sliced tiles", in_dim, rows))
+        assert torch.equal(y[:few], t3.linear(x[:few].contiguous(), t, a, b))
+    assert t3.device_error() == 0
+
+
 @pytest.mark.parametrize("case", [(384, 128, 48, t3.MUL1, "f16"), (256, 384, 128, t3.MCG, "f32"), (128, 256, 20, t3.MUL1, "bf16")])
 def test_routed_tile_edges(case):
     """One expert for each height around the edges; every row goes to one expert at weight 1."""

@@ -417,6 +417,14 @@ cudaError_t launch_decode_gemm(const GemmMaps& maps, const DecodeGemmArgs& a, ui
 
 // ---- dense linear, more than 32 rows ---------------------------------------------------------------------------------
 
+// Clusters of `s` decode GEMM CTAs (one a multiprocessor) that are resident at once. Of B200's 148 multiprocessors, by cluster size:
+// what cudaOccupancyMaxActiveClusters gives for the kernel at every rate tried (n 16, 64, 128). Written down because a call's slice
+// count, hence its bytes and its workspace, follows from it and must be the same without a device.
+uint32_t resident_clusters(uint32_t s) {
+    static const uint32_t resident[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+    return resident[s] * one_wave_ctas() / 148u;
+}
+
 // K slices of a dense linear of few rows: a call of up to 512 rows is one or two tiles of rows, out / 128 CTAs each, every one
 // decoding all of its 128 columns' weights (a 6144 -> 2048 linear would run on 16 CTAs). Such calls cut K into slices, a CTA a
 // slice, that meet in global memory (see DecodeGemmArgs::ksplit). Two arms, 33..256 rows and 257..512, each with a slice count
@@ -426,15 +434,13 @@ cudaError_t launch_decode_gemm(const GemmMaps& maps, const DecodeGemmArgs& a, ui
 // least, eight where K is short (under 64 steps), and there only in the first arm and while the slab's traffic is small.
 uint32_t prefill_ksplit(size_t rows, uint32_t in, uint32_t out) {
     if (rows > 512u) return 1u;
-    // clusters of 1 .. 8 CTAs of this shared memory that are resident at once on 148 multiprocessors
-    static const uint32_t resident[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
     const uint32_t ncol = out / 128u, ksteps = in / 64u, sms = one_wave_ctas();
     const bool long_k = ksteps >= 64u;
     const uint32_t mtiles = rows <= 256u ? 2u : 4u, units = ncol * mtiles / 2u;
     if (mtiles == 4u && !long_k) return 1u;
     const uint32_t by_slab = (2u * sms) / (mtiles * ncol), by_k = long_k ? ksteps / 4u : ksteps / 8u;
     uint32_t s = 8;
-    while (s > 1u && (s > by_slab || s > by_k || units > resident[s] * sms / 148u)) --s;
+    while (s > 1u && (s > by_slab || s > by_k || units > resident_clusters(s))) --s;
     if (s < 2u) return 1u;
     if (!long_k && mtiles * ncol * s > sms) return 1u;
     return s;
@@ -452,17 +458,20 @@ size_t prefill_linear_workspace(size_t rows, uint32_t in, uint32_t out) {
     return bytes;
 }
 
-// Rows a tile of the dense decode GEMM holds: of the ways to cut the rows into equal tiles, the one whose rounds of tiles over
-// the multiprocessors take the least time. A tile's time, in cycles: per 64 inputs the decode of a 64 x 128 block (about 480
-// at the issue rate the decode warps reach) or its MMAs (2 a row), whichever is more, then the epilogue.
-uint32_t dense_tile_rows(uint32_t rows, uint32_t in, uint32_t ncol) {
-    const uint32_t sms = one_wave_ctas(), fewest = (rows + kGemmTileRows - 1u) / kGemmTileRows;
+// Rows a tile of the dense decode GEMM holds: of the ways to cut the rows into equal tiles, the one whose rounds of units (`units` a
+// tile, `at_once` of them resident: a CTA each, or a cluster of a sliced call) take the least time. A unit's time, in cycles: per 64
+// of its inputs the decode of a 64 x 128 block (about 480 at the issue rate the decode warps reach) or its MMAs (2 a row), whichever
+// is more, then the epilogue. (A sliced call's CTAs counted one by one, as if they needed no cluster, cut 4096 -> 1024 in eight
+// slices into two tiles, of whose sixteen clusters fifteen fit: 22.0 us at 200 rows, 20.4 at 100 and 27.7 at 512, against 14.9,
+// 12.6 and 19.2 in one round.)
+uint32_t dense_tile_rows(uint32_t rows, uint32_t inputs, uint32_t units, uint32_t at_once) {
+    const uint32_t fewest = (rows + kGemmTileRows - 1u) / kGemmTileRows;
     uint32_t best_h = kGemmTileRows;
     uint64_t best = ~0ull;
     for (uint32_t cuts = fewest; cuts <= 2u * fewest + 1u; ++cuts) {
         const uint32_t h = ((rows + cuts - 1u) / cuts + 15u) & ~15u, tiles = (rows + h - 1u) / h;
         const uint32_t step = 2u * h > 480u ? 2u * h : 480u;
-        const uint64_t cost = (((uint64_t)tiles * ncol + sms - 1u) / sms) * ((in / 64u) * step + 1500u + 10u * h);
+        const uint64_t cost = (((uint64_t)tiles * units + at_once - 1u) / at_once) * ((inputs / 64u) * step + 1500u + 10u * h);
         if (cost < best) best = cost, best_h = h;
     }
     return best_h;
@@ -495,7 +504,7 @@ cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cuda
     d.mask = p.mask;
     d.ops = 1;
     d.dense_rows = p.rows;
-    d.tile_rows = dense_tile_rows(p.rows, p.in, ncol * ksplit);
+    d.tile_rows = dense_tile_rows(p.rows, p.in / ksplit, ncol, resident_clusters(ksplit));
     d.dense_tiles = (p.rows + d.tile_rows - 1u) / d.tile_rows;
     d.pair = 1;
     d.svh[0] = d.svh[1] = static_cast<const __half*>(p.svh);
@@ -525,7 +534,7 @@ cudaError_t launch_plain_linear(const void* x, int dt, uint32_t rows, const void
     d.N = out;
     d.ops = 1;
     d.dense_rows = rows;
-    d.tile_rows = dense_tile_rows(rows, in, out / 128u);
+    d.tile_rows = dense_tile_rows(rows, in, out / 128u, one_wave_ctas());
     d.dense_tiles = (rows + d.tile_rows - 1u) / d.tile_rows;
     d.pair = 1;
     d.y = y;
@@ -655,7 +664,7 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
             } else {
                 g.pair = 1;
                 g.dense_rows = S;
-                g.tile_rows = dense_tile_rows(S, g.K, ncol * g.ops);
+                g.tile_rows = dense_tile_rows(S, g.K, ncol * g.ops, one_wave_ctas());
                 g.dense_tiles = (S + g.tile_rows - 1u) / g.tile_rows;
                 units = (size_t)g.dense_tiles * g.ops * ncol;
             }
