@@ -514,7 +514,11 @@ cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cuda
     d.part = reinterpret_cast<float*>(ws + up256((size_t)p.rows * p.in * 2u));  // a sliced call's slab, behind the prepared rows
     d.kept = p.resident != nullptr;
     d.err = p.err;
-    d.overlap = p.rows <= 512u && p.overlap;  // a call of few rows is short: its set-up counts. Larger ones ran 2 % slower overlapped
+    // Overlapped, the GEMM's set-up and first codes run beside the prepare, which counts in a short call; in a long one the GEMM's
+    // CTAs take the prepare's slots. Overlapped against not, 2048 -> 6144: 21.4 / 23.2 us at 520 rows, 51.5 / 52.8 at 2048, 71.1 / 71.3
+    // at 3072, 99.1 / 98.3 at 4096; 2048 -> 2048 17.8 / 20.4 .. 24.7 / 26.3 at 2048, 41.9 / 43.4 at 4096; 4096 -> 4096 K2 level at
+    // 2048, 1.5 % slower from 3072 on; 7168 -> 1536 and 6144 -> 2048 faster throughout (1-5 %).
+    d.overlap = p.rows <= 2048u && p.overlap;
     rc = launch_decode_gemm(maps, d, d.dense_tiles * ncol, codebook, stream);
     if (rc == cudaSuccess) *launches += 2;  // the output rotation runs in the GEMM's epilogue
     return rc;
