@@ -13,8 +13,10 @@ from gpu_util import bits16, dev
 pytestmark = pytest.mark.gpu
 
 
-# x read in place by the GEMV (15 blocks) / rotated ahead (16); y written in place (128 KB) / by the copy engine; and the staged path
-@pytest.mark.parametrize("in_dim,out_dim,rows", [(256, 1920, 1), (256, 2048, 1), (256, 2048, 32), (384, 24576, 3), (2176, 2048, 32)])
+# x read in place by the GEMV (up to 53 blocks of 256 inputs at one row) / rotated ahead (from 54 on, and past 8 rows); y written in
+# place (128 KB) / by the copy engine; and the staged path
+@pytest.mark.parametrize("in_dim,out_dim,rows", [(256, 1920, 1), (256, 2048, 1), (256, 6784, 1), (256, 6912, 1), (256, 2048, 32), (384, 24576, 3),
+                                                 (2176, 2048, 32)])
 def test_host_arrays_give_the_device_bytes(in_dim, out_dim, rows):
     trellis, suh, svh = synth.linear(2400 + rows, in_dim, out_dim, 32)
     block = tb.Block('{"format":"exl3","codebook":"mul1"}')

@@ -305,7 +305,14 @@ struct Staging {
     // past kMappedBytes is written to the device and copied by the engine, whose bursts then beat the kernels' 64-byte writes
     // (24576 outputs at 8 rows 74 -> 64 us; at 128 KB the two are level).
     static constexpr size_t kMappedBytes = 128u * 1024u, kMappedY = 1024u * 1024u;
-    static constexpr int kPrepareBlocks = 16;  // 128-output blocks from which x is worth a launch that reads it once (see linear_call)
+    // Whether a host x of `bytes` is rotated once by a launch of its own, or read in place by every 128-output block of the GEMV. In
+    // place the blocks' reads of the same rows queue up on the bus, so they cost more than their bytes: about bytes x blocks^2, and
+    // 1.4 MB of it is where the second launch (2-3 us) pays. In place / a launch, us: 256 -> 2048 at 1 row 18.7 / 19.6, 2048 -> 2048 at
+    // 1 row 21.7 / 22.1 (0.9 MB), 6144 -> 1024 at 2 rows 27.8 / 28.0 (1.3 MB), 256 -> 7168 at 1 row 21.4 / 20.0 (1.5 MB), 4096 ->
+    // 2048 at 1 row 27.5 / 26.4 (1.9 MB), 6144 -> 1024 at 4 rows 32.8 / 29.4 (2.6 MB), 512 -> 24576 at 1 row 56.3 / 26.9 (36 MB). (Of 130
+    // shapes from 256 to 16384 inputs the three on the wrong side of it are 16384 inputs to 1536 and 1792 at 1 row, 37.4 / 40.4 and
+    // 39.1 / 40.5, and to 1024 at 2 rows, 41.4 / 42.6.)
+    static bool prepare_ahead(size_t bytes, size_t blocks) { return bytes * blocks * (blocks - 1u) >= 1400u * 1024u; }
     void *hx = nullptr, *hy = nullptr, *hx_dev = nullptr, *hy_dev = nullptr;
     bool mapped() {
         if (hx && hy) return true;
@@ -374,7 +381,7 @@ t3_verdict table_matmul(const t3_weight* w, const t3_array* x, void* stream, t3_
     const bool decode_rows = rows <= T3_DECODE_ROWS_MAX;
     const bool in_place = !x->device && !out->device && decode_rows && xb <= Staging::kMappedBytes && yb <= Staging::kMappedY &&
                           g_staging.mapped();
-    const bool far_x = in_place && w->out_dim / 128 >= Staging::kPrepareBlocks, engine_y = in_place && yb > Staging::kMappedBytes;
+    const bool far_x = in_place && Staging::prepare_ahead(xb, (size_t)w->out_dim / 128u), engine_y = in_place && yb > Staging::kMappedBytes;
     if (engine_y && !g_staging.fit(g_staging.y, yb)) return refuse(T3_VERDICT_FAILED, "CudaError");
     const size_t wsb = t3::linear_workspace(rows, w->in_dim, w->out_dim, w->block, far_x);
     Staging::Buf& wsbuf = decode_rows ? sws.rows : sws.ws;
