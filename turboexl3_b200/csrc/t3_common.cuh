@@ -21,7 +21,6 @@ enum DevError : uint32_t {
     kErrFullWait = 1u,    // a consumer gave up waiting for a bulk copy to land
     kErrEmptyWait = 2u,   // the producer gave up waiting for a ring slot
     kErrMmaWait = 4u,     // a tensor-core completion never arrived
-    kErrTmemAlloc = 8u,   // tensor memory could not be allocated
 };
 
 __device__ __forceinline__ float round_half(float v) { return __half2float(__float2half_rn(v)); }

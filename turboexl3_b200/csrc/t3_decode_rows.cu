@@ -194,7 +194,6 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) store_act(a.y, a.x_dt, (size_t)row * a.out + blk * 128u + lane + 32u * j, v[j]);
             }
-            if (tid == 0) a.counters[blk] = 0u;  // as the next call on this workspace expects it
             return;
         }
         if (traced && tid == 0) a.trace[4] = clock64();

@@ -653,7 +653,6 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
         const bool down = g.ops == 1u;
         for (uint32_t b = 0; b < banks.count; ++b) {
             const BankTab& t = banks.bank[b];
-            if (t.experts == 0u) continue;
             g.n = banks.n[b];
             g.svh[0] = static_cast<const __half*>(down ? t.down_svh : t.gate_svh);  // the epilogue finishes with the tile's expert's scales
             g.svh[1] = static_cast<const __half*>(t.up_svh);

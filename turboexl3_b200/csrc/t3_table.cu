@@ -277,19 +277,13 @@ struct Staging {
         void* p = nullptr;
         size_t cap = 0;
     } x, y, inds, scores;
-    // ws: the prefill and routed workspaces (written before they are read). rows: the decode-row linear's workspace, which
-    // must start zero and is left zero-tagged by every call (t3_linear), so it is cleared when it is (re)allocated and
-    // nothing else ever writes it.
+    // ws: the prefill and routed workspaces. rows: the decode-row linear's, apart, so that a longer call that makes ws grow moves
+    // nothing a decode step runs on. Both are written before they are read.
     struct StreamWs {
         Buf ws, rows;
     };
     std::unordered_map<void*, StreamWs> per_stream;
     StreamWs& of(void* stream) { return per_stream[stream]; }
-    bool fit_zeroed(Buf& b, size_t bytes) {
-        if (bytes <= b.cap) return true;
-        if (!fit(b, bytes)) return false;
-        return cudaMemset(b.p, 0, b.cap) == cudaSuccess;
-    }
     bool fit(Buf& b, size_t bytes) {
         if (bytes <= b.cap) return true;
         cudaFree(b.p);
@@ -385,7 +379,7 @@ t3_verdict table_matmul(const t3_weight* w, const t3_array* x, void* stream, t3_
     if (engine_y && !g_staging.fit(g_staging.y, yb)) return refuse(T3_VERDICT_FAILED, "CudaError");
     const size_t wsb = t3::linear_workspace(rows, w->in_dim, w->out_dim, w->block, far_x);
     Staging::Buf& wsbuf = decode_rows ? sws.rows : sws.ws;
-    if (wsb && !(decode_rows ? g_staging.fit_zeroed(wsbuf, wsb) : g_staging.fit(wsbuf, wsb))) return refuse(T3_VERDICT_FAILED, "CudaError");
+    if (wsb && !g_staging.fit(wsbuf, wsb)) return refuse(T3_VERDICT_FAILED, "CudaError");
     if (in_place) {
         // decode rows on host arrays: the launches between two memcpys
         memcpy(g_staging.hx, x->data, xb);
