@@ -533,7 +533,7 @@ int linear_call(const void* x, int x_dtype, size_t rows, const void* trellis, co
     if (rows > T3_DECODE_ROWS_MAX) {
         if (!cfg.prefill) return T3_ENGINE_NOT_IMPLEMENTED;
         if (rows > 0x7FFFFFFFu / (size_t)(in_dim > out_dim ? in_dim : out_dim)) return T3_BAD_EXL3_SHAPE;
-        if (rows > kPrefillDenseRowsMax) return T3_BAD_EXL3_SHAPE;  // the prepare launch's row groups are a grid dimension
+        if (rows > kPrefillDenseRowsMax) return T3_BAD_EXL3_SHAPE;
         if (!workspace || workspace_bytes < linear_workspace(rows, in_dim, out_dim, n, far_x)) return T3_WORKSPACE_TOO_SMALL;
         PrefillLinearArgs p = {x, y, static_cast<const uint8_t*>(trellis), nullptr, suh, svh, (uint32_t)rows, (uint32_t)in_dim,
                                (uint32_t)out_dim, (uint32_t)n, mask, x_dtype, workspace, dev_error_ptr(), !cfg.no_overlap};
@@ -740,8 +740,7 @@ int moe_call(const void* x, int x_dtype, size_t rows, const t3_bank* bank, const
     if (int rc = decode_mask(dec, mask)) return rc;
     const t3_config cfg = config();
     if (rows > T3_DECODE_ROWS_MAX && !cfg.prefill) return T3_ENGINE_NOT_IMPLEMENTED;  // src/root.zig:850-852
-    // the prefill chain's launches carry row groups in a grid dimension (65535 at most): 8 rows a group in the last launch,
-    // 64 row-slots a group in the prepare and the middle
+    // the prefill chain's last launch has its rows, eight a group, in a grid dimension (65535 at most)
     if (rows > T3_DECODE_ROWS_MAX && (rows > kPrefillMoeRowsMax || rows * (size_t)topk > kPrefillSlotsMax)) return T3_BAD_EXL3_SHAPE;
     if (rows * (size_t)topk > 0x7FFFFFFFu / (size_t)(bank->hidden > bank->inter ? bank->hidden : bank->inter)) return T3_BAD_EXL3_SHAPE;
     const size_t need = t3_moe_workspace_bytes(rows, topk, bank);

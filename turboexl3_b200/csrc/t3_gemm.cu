@@ -7,7 +7,7 @@
 // proxy fence, and shared memory carries only the rows. The accumulator's columns are rows, so a tile is any multiple of 16
 // rows up to 256 and an expert of 80 rows costs five sixteenths of the MMA time of a 256-row one: nothing is padded to 128.
 //
-// What bounds it: a decoded 16x16 tile costs about 50 issued warp instructions whatever its rows, an MMA of 64 inputs x 128
+// What bounds it: a decoded 16x16 tile costs about 57 issued warp instructions (56.8 at K3, counted) whatever its rows, an MMA of 64 inputs x 128
 // outputs x R rows takes 2 R cycles, so up to about 200 rows a tile the decode's issue slots bound the kernel and past that the
 // tensor cores do. (An MMA that reads its A operand from tensor memory ran at the full rate from 128 columns on: 64 cycles at
 // 128, 128 at 256; with both operands in shared memory a 256-column one took 171.)
@@ -18,7 +18,7 @@
 // A ring stage is 64 weight tiles (64 tensor-memory columns), one of two shapes chosen per tile of rows:
 //   wide   two 128-output blocks x 64 inputs, up to 128 rows: both blocks read one copy of the rows
 //   deep   one block x 128 inputs, up to 256 rows
-// A decode warp takes four tiles along K of a stage: waits, fences and arrivals are paid once a stage.
+// A decode warp takes eight tiles of every other stage: waits, fences and arrivals are paid once for the eight.
 //
 // Epilogue: the 128-point output rotation is a tensor-core product as well, D2 = H128 x z^T with H128 (+-1, f16) resident in
 // tensor memory: accumulators -> f16 z, transposed to shared memory by stmatrix -> MMA over the same columns -> scaled by svh,
@@ -49,8 +49,8 @@ constexpr uint32_t kCodeStages = 4;        // stages of the code ring: even, so 
 constexpr uint32_t kStages = 3;            // operand stages in tensor memory
 static_assert(kCodeStages % 2u == 0u, "see decode_stages");
 // The decode warps work as two groups of eight on alternate stages, a warp on both of a stage's 64 x 128 blocks: eight tiles a
-// visit, so that a visit's waits, arrivals and ring arithmetic are paid half as often as with sixteen warps on every stage
-// (59 -> 54 issued instructions a tile), and sixteen warps to issue from (eight alone left a third of the issue slots empty).
+// visit, so that a visit's waits, arrivals and ring arithmetic are paid half as often as with sixteen warps on every stage (five
+// issued instructions a tile fewer), and sixteen warps to issue from (eight alone left a third of the issue slots empty).
 constexpr uint32_t kGroupWarps = 8;
 constexpr uint32_t kStageTiles = 64;       // weight tiles a stage
 constexpr uint32_t kStageCols = 64;        // tensor-memory columns a stage (32 a 64 x 128 block)

@@ -169,8 +169,10 @@ __device__ __forceinline__ void mma_tile(float (&acc)[RowCap<RM>::kMB][2][4], ui
 // A full stage holds kStageRows tk rows, a warp's share of it kBatch tiles taken two at a time, and with the rate
 // a template constant every shared-memory offset inside a stage is an immediate.
 // HB: tiles whose words and fragments are in registers together (the routed kernels keep two: four spill there).
-// WINDOWS: full-width codewords at the rates whose windows are byte permutations take them so (decode_raw's FULL; the dense kernel:
-// 16384 -> 7168 at K4 38.9 -> 37.0 us; in the routed kernels, out of registers already, the second copy of the loop cost 2 %).
+// WINDOWS: full-width codewords at the rates whose windows are byte permutations take them so (decode_raw's FULL). In the dense kernel
+// at every row capacity: up to 8 rows 16384 -> 7168 at K4 38.9 -> 37.0 us; at capacity 32, where the second copy of the loop adds a few
+// spilled words, 2048 -> 6144 at 32 rows K 2, 4, 8 14.9, 15.2, 18.8 -> 14.3, 14.3, 18.2 and 16384 -> 7168 82.9, 78.5, 111 -> 78.4, 74.8,
+// 107; at 16 mostly (16384 -> 7168 at 9 rows K4 54.0 -> 51.5, 2048 -> 6144 10.2 -> 11.1). In the routed kernels it cost 2 %.
 template <int N, int CB, int RM, int HB = 2, bool WINDOWS = false>
 __device__ __forceinline__ void consume_slab(const uint8_t* ring, uint64_t* full, uint64_t* empty, uint32_t nrows,
                                              uint32_t n_rt, uint32_t mask, Ring rc, const __half* xp, uint32_t xstride,

@@ -67,7 +67,7 @@ struct MoeArgs {
     uint32_t banked;          // decode rows, top-1: inds holds packed ids (bank << 24 | slot); banks 1 and 2 in ext; scores null = 1
     BankTab ext[2];
     void* shared_ready;       // host side only: an event the last launch (the one that reads `shared`) waits for, or null
-    uint32_t row_cap;                  // rows one pass over an expert's weights serves (8, 16 or 32): experts with more members take more passes
+    uint32_t row_cap;                  // rows a CTA's decode of an expert's weights serves (8, 16 or 32): an expert with more members takes more CTAs
     uint32_t split_gu, slice_max_gu;   // K slices of gate|up (cluster = 2 * split_gu), largest slice
     uint32_t split_d, slice_max_d;     // K slices of down
     RingPlan ring_gu, ring_d;
@@ -133,8 +133,8 @@ uint32_t gemv_smem_bytes(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, u
 constexpr uint32_t kGemvSmemLimit = 200u * 1024u;
 uint32_t row_cap_for(uint32_t rows);
 
-// Row limits of the prefill launches, whose row groups are a grid dimension (65535 at most): the dense prepare takes 64
-// rows a group; the routed chain's last launch 8 rows a group, its prepare and middle 64 row-slots a group.
+// Row limits of the prefill calls. The routed chain's last launch has its rows, eight a group, in a grid dimension (65535 at most);
+// the dense and the row-slot limits are what these entry points have always admitted.
 constexpr size_t kPrefillDenseRowsMax = (size_t)65535 * 64;
 constexpr size_t kPrefillMoeRowsMax = (size_t)65535 * 8;
 constexpr size_t kPrefillSlotsMax = (size_t)65535 * 64;
