@@ -21,13 +21,15 @@ uint32_t next_u32() {
 }
 
 // the tile's 256 f16 weights in row-major order as the lane reader produces them
-template <int N, int CB>
+template <int N, int CB, bool FULL = false>
 void tile_by_lanes(const uint32_t* words, uint32_t mask, uint16_t out[256]) {
     for (uint32_t lane = 0; lane < 32; ++lane) {
         t3::LanePlan<N> plan;
         plan.init(lane);
         uint32_t b[4];
-        t3::decode_lane<N, CB>(words, plan, mask, b);
+        uint32_t raw[t3::raw_words(N)];
+        t3::load_lane<N>(words, plan, raw);
+        t3::decode_raw<N, CB, FULL>(raw, plan, mask, b);
         for (uint32_t m = 0; m < 8; ++m) {
             const uint16_t v = (uint16_t)(b[m >> 1] >> ((m & 1) * 16));
             out[t3::tile_row(lane, m) * 16 + t3::tile_col(lane, m)] = v;
@@ -61,6 +63,10 @@ int check_rate(int trials) {
                 if (memcmp(got, want, sizeof got) != 0) ++bad;
                 if (cb == 0) tile_by_lanes_any<0>(words, N, mask, got);
                 else tile_by_lanes_any<1>(words, N, mask, got);
+                if (memcmp(got, want, sizeof got) != 0) ++bad;
+                if (wbits < 16) continue;
+                if (cb == 0) tile_by_lanes<N, 0, true>(words, 0u, got);  // whole windows: the mask is not read
+                else tile_by_lanes<N, 1, true>(words, 0u, got);
                 if (memcmp(got, want, sizeof got) != 0) ++bad;
             }
         }

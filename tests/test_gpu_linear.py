@@ -334,8 +334,8 @@ def test_rows_past_8_with_and_without_the_workspace_give_the_same_bytes(rows):
 @pytest.mark.parametrize("case", [(6144, 2048, 64, t3.MUL1, 512), (2048, 6144, 64, t3.MUL1, 40), (2048, 2048, 36, t3.MCG, 130),
                                   (7168, 1536, 48, t3.MUL1, 400), (1536, 24576, 64, t3.MUL1, 200), (16384, 7168, 32, t3.MUL1, 64)])
 def test_gemm_of_few_rows_cuts_k_into_slices(case):
-    """Calls of 33..256 and of 257..512 rows are few tall CTAs, so K is cut into slices that meet in global memory (the tile's last arriver
-    adds them in slice order). Within the dense bars of the oracle on sampled rows; the same call twice gives the same
+    """Calls of 33..256 and of 257..512 rows are few tall CTAs, so K is cut into slices that meet in global memory (each CTA of
+    the slices' cluster adds them, in slice order, for its share of the rows). Within the dense bars of the oracle on sampled rows; the same call twice gives the same
     bytes; a row's bytes do not depend on the call's row count within an arm (src/hip_tests.zig:870-880 asks it of the first 17
     rows of 40- and 200-row calls)."""
     in_dim, out_dim, n, cb, rows = case
