@@ -12,9 +12,9 @@
 // tensor cores do. (An MMA that reads its A operand from tensor memory ran at the full rate from 128 columns on: 64 cycles at
 // 128, 128 at 256; with both operands in shared memory a 256-column one took 171.)
 //
-// One persistent CTA a multiprocessor, 27 warps by role (the rings run on across tiles, so nothing is set up per tile):
+// One persistent CTA a multiprocessor, 28 warps by role (the rings run on across tiles, so nothing is set up per tile):
 //   warps 0-7    epilogue     warps 8-23  decode     24  codes: TMA into the code ring
-//   25  rows: TMA into the row ring     26  tcgen05.mma
+//   25  rows: TMA into the row ring     26  tcgen05.mma     27  tcgen05.mma of the output rotation
 // A ring stage is 64 weight tiles (64 tensor-memory columns), one of two shapes chosen per tile of rows:
 //   wide   two 128-output blocks x 64 inputs, up to 128 rows: both blocks read one copy of the rows
 //   deep   one block x 128 inputs, up to 256 rows
@@ -43,8 +43,8 @@ namespace t3 {
 namespace {
 
 constexpr uint32_t kEpiWarps = 8, kDecWarps = 16;
-constexpr uint32_t kCodeWarp = kEpiWarps + kDecWarps, kRowWarp = kCodeWarp + 1, kMmaWarp = kCodeWarp + 2;
-constexpr uint32_t kThreads = 32u * (kMmaWarp + 1u);
+constexpr uint32_t kCodeWarp = kEpiWarps + kDecWarps, kRowWarp = kCodeWarp + 1, kMmaWarp = kCodeWarp + 2, kRotWarp = kCodeWarp + 3;
+constexpr uint32_t kThreads = 32u * (kRotWarp + 1u);
 constexpr uint32_t kCodeStages = 4;        // stages of the code ring: even, so that a slot is always the same decode group's
 constexpr uint32_t kStages = 3;            // operand stages in tensor memory
 static_assert(kCodeStages % 2u == 0u, "see decode_stages");
@@ -56,6 +56,11 @@ constexpr uint32_t kStageTiles = 64;       // weight tiles a stage
 constexpr uint32_t kStageCols = 64;        // tensor-memory columns a stage (32 a 64 x 128 block)
 // tensor memory: accumulators in columns 0-255, operand stages in 256-447, H128 (128 x 128 f16) in 448-511
 constexpr uint32_t kTmemCols = 512, kTmemA = 256, kTmemH = 448;
+// Units whose accumulators leave room for one part's rotation beside them in columns 256 - rows .. 255: their accumulators are
+// given back as soon as z is in shared memory, and the next unit's MMAs run under the rotation, the finish and the stores. (A launch
+// has either blocks in pairs or one at a time, so no early unit's accumulators reach another's rotation columns.)
+constexpr uint32_t kEarlyWide = 80, kEarlyDeep = 128;
+static_assert(3u * kEarlyWide <= kTmemA && 2u * kEarlyDeep <= kTmemA, "accumulators and one part's rotation");
 constexpr uint32_t kRowBytes = kGemmTileRows * 128u;   // a row slot: 64 inputs of up to 256 rows
 constexpr uint32_t kKeptBytes = 128u * 128u;           // 64 inputs of a kept weight's 128 outputs, behind the slot's rows
 constexpr uint32_t kZBytes = 2u * 128u * 128u;         // 128 rows x 128 outputs, f16, as two K-major halves; two of them
@@ -71,6 +76,11 @@ struct Sub {
     uint32_t e, first, rows, cols, op, blk, blocks;
     uint32_t k0, k1;  // its range of 64-input steps
     bool wide;
+    bool early;       // the accumulators are free once their sums are in z: the rotation has columns of its own
+    __device__ __forceinline__ uint32_t parts() const { return wide ? blocks : (cols > 128u ? 2u : 1u); }  // of up to 128 columns
+    __device__ __forceinline__ uint32_t part_cols(uint32_t c) const { return wide ? cols : min(128u, cols - 128u * c); }
+    __device__ __forceinline__ uint32_t rot_col(uint32_t c) const { return early ? 256u - cols : part_col(c); }  // its rotation's
+    __device__ __forceinline__ uint32_t part_col(uint32_t c) const { return wide && early ? c * cols : 128u * c; }  // part c's columns
 };
 
 // the CTA's units in order; f(sub) returns false to stop
@@ -94,6 +104,7 @@ __device__ __forceinline__ void for_each_sub(const DecodeGemmArgs& a, F&& f) {
         s.cols = (s.rows + 15u) & ~15u;
         s.wide = a.pair == 2u && s.cols <= 128u;
         s.blocks = s.wide ? nb : 1u;
+        s.early = !sliced && a.svh[0] != nullptr && s.cols <= (a.pair == 2u ? kEarlyWide : kEarlyDeep);
         s.k0 = 0, s.k1 = a.K / 64u;
         if (sliced) s.k0 = 2u * (a.K / 128u * blockIdx.x / a.ksplit), s.k1 = 2u * (a.K / 128u * (blockIdx.x + 1u) / a.ksplit);
         for (uint32_t b = 0; b < nb; b += s.blocks) {
@@ -196,47 +207,83 @@ __device__ __forceinline__ void decode_stages(uint32_t visits, Ring<kCodeStages>
     }
 }
 
-// One 128-column part of a finished accumulator, warp (q, h)'s 16 outputs of it: rotated sums x scale, rounded to f16, then in
-// the output's dtype (PLAIN: rounded once). 16-bit results are transposed into the part's buffer (st_at: where this lane's
-// stmatrix row goes), f32 ones go to y, rows below `live`, at once (y at the part's first row and this lane's output g).
-template <bool PLAIN>
-__device__ __forceinline__ void finish_part(uint32_t taddr, uint32_t cols, float s0, float s1, int dt, uint32_t st_at, float* y,
-                                            size_t N, uint32_t live, uint32_t t) {
+// A warp's 16 outputs of up to 128 accumulator columns, 32 at a time: f(r, v) gets columns r .. r + 31 while the next 32 are on their
+// way (a load's latency for every 32 columns was half of what the epilogue took).
+template <typename F>
+__device__ __forceinline__ void for_columns(uint32_t taddr, uint32_t cols, F&& f) {
+    uint32_t v[2][16];
 #pragma unroll
     for (uint32_t r = 0; r < 128u; r += 64u) {
         if (r >= cols) break;
-        uint32_t v[32];
-        tmem_ld_16x64(taddr + r, v);
-#pragma unroll
-        for (uint32_t p = 0; p < 4u; ++p) {
-            float f[8];
-#pragma unroll
-            for (uint32_t j = 0; j < 8u; ++j) {
-                f[j] = __uint_as_float(v[8u * p + j]);
-                if (!PLAIN) f[j] *= (j & 2u) ? s1 : s0;
-            }
-            if (dt == (int)kF32) {
-#pragma unroll
-                for (uint32_t j = 0; j < 8u; ++j) {
-                    const uint32_t row = r + 16u * p + (j >> 2) * 8u + 2u * t + (j & 1u);
-                    if (row < live) y[row * N + ((j & 2u) ? 8u : 0u)] = round_half(f[j]);
-                }
-            } else if (r + 16u * p < cols) {
-                uint32_t w[4];
-#pragma unroll
-                for (uint32_t j = 0; j < 4u; ++j) {
-                    float2 u = make_float2(f[2u * j], f[2u * j + 1u]);
-                    w[j] = pack_half2(u.x, u.y);
-                    if (dt == (int)kBf16) {
-                        if (!PLAIN) u = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-                        const __nv_bfloat162 o = __floats2bfloat162_rn(u.x, u.y);
-                        w[j] = *reinterpret_cast<const uint32_t*>(&o);
-                    }
-                }
-                stmatrix4_trans(st_at + (r + 16u * p) * 128u, w[0], w[1], w[2], w[3]);
-            }
-        }
+        tmem_ld_16x32(taddr + r, v[0]);
+        tmem_ld_16x32(taddr + r + 32u, v[1]);
+        tmem_ld_wait(v[0]);
+        f(r, v[0]);
+        tmem_ld_wait(v[1]);
+        if (r + 32u < cols) f(r + 32u, v[1]);
     }
+}
+
+// The sums of an accumulator part as f16 z^T, K-major in the part's buffer (st_at: where this lane's stmatrix row goes): the output
+// rotation's B operand
+__device__ __forceinline__ void z_part(uint32_t taddr, uint32_t cols, uint32_t st_at) {
+    for_columns(taddr, cols, [&](uint32_t r, const uint32_t (&v)[16]) {
+#pragma unroll
+        for (uint32_t p = 0; p < 2u; ++p) {
+            auto pk = [&](uint32_t j) { return pack_half2(__uint_as_float(v[8u * p + j]), __uint_as_float(v[8u * p + j + 1u])); };
+            if (r + 16u * p < cols) stmatrix4_trans(st_at + (r + 16u * p) * 128u, pk(0), pk(2), pk(4), pk(6));
+        }
+    });
+}
+
+// (a, b) x s
+__device__ __forceinline__ float2 mul2(uint32_t a, uint32_t b, float s) {
+    float2 r;
+    asm("{\n\t.reg .b64 u, v, w;\n\tmov.b64 u, {%2, %3};\n\tmov.b64 v, {%4, %4};\n\tmul.rn.f32x2 w, u, v;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "r"(a), "r"(b), "f"(s));
+    return r;
+}
+
+// One part of up to 128 columns of a finished accumulator, warp (q, h)'s 16 outputs of it: rotated sums x scale, rounded to f16, then in
+// the output's dtype (PLAIN: rounded once). 16-bit results are transposed into the part's buffer (st_at: where this lane's
+// stmatrix row goes), f32 ones go to y, rows below `live`, at once (y at the part's first row and this lane's output g). A body a
+// dtype: with the three in one the code was long enough to be fetched anew for every tile, 1700 cycles a part against 500.
+template <bool PLAIN, int DT>
+__device__ __forceinline__ void finish_part_as(uint32_t taddr, uint32_t cols, float s0, float s1, uint32_t st_at, float* y, size_t N,
+                                               uint32_t live, uint32_t t) {
+    for_columns(taddr, cols, [&](uint32_t r, const uint32_t (&v)[16]) {
+#pragma unroll
+        for (uint32_t p = 0; p < 2u; ++p) {
+            uint32_t w[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; ++j) {  // rows 8 (j >> 1) + 2t and the next of 16, output g or g + 8 (j odd)
+                const uint32_t a = v[8u * p + 2u * j], b = v[8u * p + 2u * j + 1u];
+                float2 u = PLAIN ? make_float2(__uint_as_float(a), __uint_as_float(b)) : mul2(a, b, (j & 1u) ? s1 : s0);
+                if (DT == (int)kF32) {
+                    const uint32_t row = r + 16u * p + (j >> 1) * 8u + 2u * t;
+                    float* at = y + row * N + ((j & 1u) ? 8u : 0u);
+                    if (row < live) at[0] = round_half(u.x);
+                    if (row + 1u < live) at[N] = round_half(u.y);
+                    continue;
+                }
+                w[j] = pack_half2(u.x, u.y);
+                if (DT == (int)kBf16) {
+                    if (!PLAIN) u = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+                    const __nv_bfloat162 o = __floats2bfloat162_rn(u.x, u.y);
+                    w[j] = *reinterpret_cast<const uint32_t*>(&o);
+                }
+            }
+            if (DT != (int)kF32 && r + 16u * p < cols) stmatrix4_trans(st_at + (r + 16u * p) * 128u, w[0], w[1], w[2], w[3]);
+        }
+    });
+}
+template <bool PLAIN>
+__device__ __forceinline__ void finish_part(uint32_t taddr, uint32_t cols, float s0, float s1, int dt, uint32_t st_at, float* y,
+                                            size_t N, uint32_t live, uint32_t t) {
+    if (dt == (int)kF16) finish_part_as<PLAIN, kF16>(taddr, cols, s0, s1, st_at, y, N, live, t);
+    else if (dt == (int)kBf16) finish_part_as<PLAIN, kBf16>(taddr, cols, s0, s1, st_at, y, N, live, t);
+    else finish_part_as<PLAIN, kF32>(taddr, cols, s0, s1, st_at, y, N, live, t);
 }
 
 // A part's 16-bit rows from its buffer to y, 256 bytes a row (`warp` of the epilogue's eight); a caller's y may be aligned to 8
@@ -256,13 +303,13 @@ __device__ __forceinline__ void store_part(uint32_t buffer, uint16_t* y, size_t 
     }
 }
 
-// The output rotation of a part on the tensor cores (one thread): D2 = H128 x z^T over the part's accumulator columns
-__device__ __forceinline__ void rotate_part(uint32_t tmem, uint32_t z_s, uint32_t c, uint32_t idesc, uint32_t rot_full) {
-    const uint32_t hi = (uint32_t)(umma_desc(0) >> 32), lo = (uint32_t)umma_desc(z_s + c * kZBytes);
+// The output rotation of a part on the tensor cores (one thread): D2 = H128 x z^T into the columns at tmem_d
+__device__ __forceinline__ void rotate_part(uint32_t tmem, uint32_t tmem_d, uint32_t z, uint32_t idesc, uint32_t rot_full) {
+    const uint32_t hi = (uint32_t)(umma_desc(0) >> 32), lo = (uint32_t)umma_desc(z);
 #pragma unroll
     for (uint32_t kk = 0; kk < 8u; ++kk)
-        umma_f16_ts(tmem + 128u * c, tmem + kTmemH + 8u * kk, lo + (((kk >> 2) * 16384u + (kk & 3u) * 32u) >> 4), hi, kk != 0u, idesc);
-    umma_commit(rot_full + 8u * c);
+        umma_f16_ts(tmem_d, tmem + kTmemH + 8u * kk, lo + (((kk >> 2) * 16384u + (kk & 3u) * 32u) >> 4), hi, kk != 0u, idesc);
+    umma_commit(rot_full);
 }
 
 // KEPT: the weight is a kept W_hat (or W_std), [N, K] 16-bit, loaded by TMA beside the rows as a shared-memory operand: the
@@ -277,11 +324,12 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
     // barriers, a full / empty pair a ring slot: codes, operands in tensor memory, rows
     const uint32_t full_c = codes + kCodeStages * stage_bytes, full_a = full_c + 16u * kCodeStages;
     const uint32_t full_b = full_a + 16u * kStages, empty_b = full_b + 8u * 4u;
-    const uint32_t acc_full = empty_b + 8u * 4u, acc_free = acc_full + 8u;
-    // z_full, rot_full: a pair each, one barrier a 128-column part (the epilogue and the MMA warp run both parts ahead)
-    const uint32_t z_full = acc_full + 16u, rot_full = acc_full + 32u;
+    // acc_free: the accumulators may be written again; all_free: the rotation's columns too (the same moment unless Sub::early)
+    const uint32_t acc_full = empty_b + 8u * 4u, acc_free = acc_full + 8u, all_free = acc_full + 16u;
+    // z_full, rot_full: a pair each, one barrier a part of up to 128 columns
+    const uint32_t z_full = acc_full + 24u, rot_full = acc_full + 40u;
     uint8_t* generic = smem_raw + (smem - smem_addr(smem_raw));
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(generic + (acc_full + 48u - smem));
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(generic + (acc_full + 56u - smem));
     volatile uint32_t* dead = tmem_slot + 1;
 
     const uint32_t tid = threadIdx.x, lane = tid & 31u;
@@ -292,7 +340,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         for (uint32_t s = 0; s < kCodeStages; ++s) init(full_c + 16u * s, 1u), init(full_c + 16u * s + 8u, kGroupWarps);
         for (uint32_t s = 0; s < kStages; ++s) init(full_a + 16u * s, kGroupWarps), init(full_a + 16u * s + 8u, 1u);
         for (uint32_t s = 0; s < kSlots; ++s) init(full_b + 8u * s, 1u), init(empty_b + 8u * s, 1u);
-        init(acc_full, 1u), init(acc_free, kEpiWarps);
+        init(acc_full, 1u), init(acc_free, kEpiWarps), init(all_free, kEpiWarps);
         for (uint32_t c = 0; c < 2u; ++c) init(z_full + 8u * c, kEpiWarps), init(rot_full + 8u * c, 1u);
         *dead = 0u;
         mbar_init_fence();
@@ -391,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         });
     } else if (warp == kMmaWarp) {
         // ---- MMA: the whole warp walks the rings, one elected lane issues (see elect_one)
-        uint32_t subs = 0, rots[2] = {0, 0};
+        uint32_t subs = 0;
         Ring<kStages> ring_a;
         Ring<kSlots> ring_b;
         auto wait = [&](uint32_t bar, uint32_t parity, uint32_t bit) {
@@ -401,8 +449,13 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         };
         const uint32_t desc_hi = (uint32_t)(umma_desc(0) >> 32), desc0 = (uint32_t)umma_desc(smem);
         for_each_sub(a, [&](const Sub& s) {
-            if (subs > 0u) wait(acc_free, (subs - 1u) & 1u, kErrMmaWait);
+            if (subs > 0u) {
+                wait(acc_free, (subs - 1u) & 1u, kErrMmaWait);
+                // accumulators wide enough to reach the last unit's rotation (which finished the one before: a phase's parity is enough)
+                if (!s.early) wait(all_free, (subs - 1u) & 1u, kErrMmaWait);
+            }
             ++subs;
+            const uint32_t second = tmem + s.part_col(1);
             const uint32_t idesc = idesc_m128(s.cols) | (KEPT && a.bf16 ? kIdescBf16 : 0u), k64 = s.k1 - s.k0;
             uint32_t acc = 0;
             // four steps of 16 inputs on one row slot against one 64-input operand block (a second block's into its accumulator)
@@ -416,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
                         continue;
                     }
                     umma_f16_ts(tmem, a_col + kk * 8u, lo + kk * 2u, desc_hi, kk ? 1u : acc, idesc);
-                    if (both) umma_f16_ts(tmem + 128u, a_col + 32u + kk * 8u, lo + kk * 2u, desc_hi, kk ? 1u : acc, idesc);
+                    if (both) umma_f16_ts(second, a_col + 32u + kk * 8u, lo + kk * 2u, desc_hi, kk ? 1u : acc, idesc);
                 }
                 umma_commit(empty_b + 8u * ring_b.slot);
             };
@@ -446,15 +499,22 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
                 ring_b.next();
             }
             if (elect_one()) umma_commit(acc_full);
-            if (sliced || a.svh[0] == nullptr) return true;
-            // the output rotation, 128 accumulator columns at a time
-            const uint32_t parts = s.wide ? s.blocks : (s.cols > 128u ? 2u : 1u);
+            return true;
+        });
+    } else if (warp == kRotWarp) {
+        // ---- output rotation, a part at a time, once every epilogue warp's z is in the part's buffer (a warp of its own: the MMA warp
+        // is on the next unit by then)
+        uint32_t turns[2] = {0, 0};
+        if (!sliced && a.svh[0] != nullptr) for_each_sub(a, [&](const Sub& s) {
+            const uint32_t parts = s.parts();
 #pragma unroll
             for (uint32_t c = 0; c < 2u; ++c) {
                 if (c >= parts) break;
-                wait(z_full + 8u * c, rots[c]++ & 1u, kErrMmaWait);
-                const uint32_t rdesc = idesc_m128(s.wide ? s.cols : min(128u, s.cols - 128u * c));
-                if (elect_one()) rotate_part(tmem, z_s, c, rdesc, rot_full);
+                wait_phase<32>(z_full + 8u * c, turns[c]++ & 1u, dead, a.err, kErrMmaWait);
+                tc_fence_after();
+                __syncwarp();
+                const uint32_t to = tmem + s.rot_col(c), idesc = idesc_m128(s.part_cols(c));
+                if (elect_one()) rotate_part(tmem, to, z_s + c * kZBytes, idesc, rot_full + 8u * c);
             }
             return true;
         });
@@ -468,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         const int dt = a.y ? a.y_dt : (int)kF16;
         const bool plain = KEPT && a.svh[0] == nullptr;
         uint16_t* const y16 = a.y ? static_cast<uint16_t*>(a.y) : reinterpret_cast<uint16_t*>(a.z);
-        uint32_t subs = 0, rots[2] = {0, 0};
+        uint32_t subs = 0, rots = 0;  // rots: the next rotation's parity, a bit a part
         auto arrive = [&](uint32_t bar) {
             __syncwarp();
             if (lane == 0) mbar_arrive_addr(bar);
@@ -491,60 +551,64 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
                         if (b < s.blocks) sc[b][j] = kHadScale * __half2float(svh[b * 128u + 8u * j]);
             }
             await(acc_full, subs++ & 1u);
-            const uint32_t parts = s.wide ? s.blocks : (s.cols > 128u ? 2u : 1u);
-            auto part_cols = [&](uint32_t c) { return s.wide ? s.cols : min(128u, s.cols - 128u * c); };
+            const uint32_t parts = s.parts();
             if (sliced) {  // this slice's sums to its place in the slab
                 float* slab = a.part + (((size_t)s.blk * a.ksplit + blockIdx.x) * a.dense_rows + s.first) * 128u + 32u * q + 16u * h + g;
-                for (uint32_t r = 0; r < s.cols; r += 64u) {
-                    uint32_t v[32];
-                    tmem_ld_16x64(my_lanes + r, v);
+#pragma unroll 1
+                for (uint32_t c = 0; c < parts; ++c)
+                    for_columns(my_lanes + 128u * c, s.part_cols(c), [&](uint32_t r, const uint32_t (&v)[16]) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 32u; ++j) {
-                        const uint32_t row = r + (j >> 2) * 8u + 2u * t + (j & 1u);
-                        if (row < s.rows) __stcg(slab + (size_t)row * 128u + ((j & 2u) ? 8u : 0u), __uint_as_float(v[j]));
-                    }
-                }
+                        for (uint32_t j = 0; j < 16u; ++j) {
+                            const uint32_t row = 128u * c + r + (j >> 2) * 8u + 2u * t + (j & 1u);
+                            if (row < s.rows) __stcg(slab + (size_t)row * 128u + ((j & 2u) ? 8u : 0u), __uint_as_float(v[j]));
+                        }
+                    });
                 return true;
             }
-            for (uint32_t c = 0; c < parts && !plain; ++c) {
-                const uint32_t cols = part_cols(c);
-#pragma unroll
-                for (uint32_t r = 0; r < 128u; r += 64u) {
-                    if (r >= cols) break;
-                    uint32_t v[32];
-                    tmem_ld_16x64(my_lanes + 128u * c + r, v);
-#pragma unroll
-                    for (uint32_t p = 0; p < 4u; ++p) {
-                        auto pk = [&](uint32_t j) { return pack_half2(__uint_as_float(v[8u * p + j]), __uint_as_float(v[8u * p + j + 1u])); };
-                        if (r + 16u * p < cols) stmatrix4_trans(st_at + c * kZBytes + (r + 16u * p) * 128u, pk(0), pk(2), pk(4), pk(6));
-                    }
-                }
+            // this warp's z of a part is in its buffer and the columns its rotation goes to are read
+            auto z_done = [&](uint32_t c) {
                 proxy_fence();
                 tc_fence_before();
                 arrive(z_full + 8u * c);
+            };
+            if (!plain) {
+#pragma unroll 1
+                for (uint32_t c = 0; c < parts; ++c) {
+                    z_part(my_lanes + s.part_col(c), s.part_cols(c), st_at + c * kZBytes);
+                    if (c == 0u || !s.early) z_done(c);
+                }
+                if (s.early) {
+                    tc_fence_before();
+                    arrive(acc_free);
+                }
             }
-#pragma unroll
-            for (uint32_t c = 0; c < 2u; ++c) {
-                if (c >= parts) break;
-                if (!plain) await(rot_full + 8u * c, rots[c]++ & 1u);
-                const uint32_t blk = s.blk + (s.wide ? c : 0u), row0 = s.wide ? 0u : 128u * c;
+#pragma unroll 1
+            for (uint32_t c = 0; c < parts; ++c) {
+                if (!plain) {
+                    if (s.early && c == 1u) z_done(c);  // the first part's rotation is read
+                    await(rot_full + 8u * c, (rots >> c) & 1u);
+                    rots ^= 1u << c;
+                }
+                const uint32_t cols = s.part_cols(c), blk = s.blk + (s.wide ? c : 0u), row0 = s.wide ? 0u : 128u * c;
                 const bool second = s.wide && c == 1u;
                 const float s0 = second ? sc[1][0] : sc[0][0], s1 = second ? sc[1][1] : sc[0][1];
                 float* y32 = static_cast<float*>(a.y) + (size_t)(s.first + row0) * a.N + blk * 128u + 32u * q + 16u * h + g;
+                const uint32_t from = my_lanes + s.rot_col(c);
                 if (plain)
-                    finish_part<true>(my_lanes + 128u * c, part_cols(c), s0, s1, dt, st_at + c * kZBytes, y32, a.N, s.rows - row0, t);
+                    finish_part<true>(from, cols, s0, s1, dt, st_at + c * kZBytes, y32, a.N, s.rows - row0, t);
                 else
-                    finish_part<false>(my_lanes + 128u * c, part_cols(c), s0, s1, dt, st_at + c * kZBytes, y32, a.N, s.rows - row0, t);
+                    finish_part<false>(from, cols, s0, s1, dt, st_at + c * kZBytes, y32, a.N, s.rows - row0, t);
             }
-            // the accumulators are read: the next tile may start
+            // everything is read
             tc_fence_before();
-            arrive(acc_free);
+            if (!s.early) arrive(acc_free);
+            arrive(all_free);
             if (dt == (int)kF32) return true;
             meet();
             for (uint32_t c = 0; c < parts; ++c) {
                 const uint32_t row0 = s.wide ? 0u : 128u * c;
                 store_part(z_s + c * kZBytes, y16 + s.op * a.z_op_stride + (size_t)(s.first + row0) * a.N + (s.blk + (s.wide ? c : 0u)) * 128u,
-                           a.N, min(part_cols(c), s.rows - row0), warp, lane);
+                           a.N, min(s.part_cols(c), s.rows - row0), warp, lane);
             }
             meet();  // the buffers are read: the next tile's values may overwrite them
             return true;
@@ -583,7 +647,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         const uint32_t cols = (live + 15u) & ~15u;
         if (live > 0u) {
             if (warp == kMmaWarp) {
-                if (elect_one()) rotate_part(tmem, z_s, 0, idesc_m128(cols), rot_full);
+                if (elect_one()) rotate_part(tmem, tmem, z_s, idesc_m128(cols), rot_full);
             } else if (warp < kEpiWarps) {
                 const uint32_t q = warp & 3u, h = warp >> 2, g = lane >> 2, t = lane & 3u, m = lane >> 3, i8 = lane & 7u;
                 const uint32_t st_at = z_s + (q >> 1) * 16384u + ((m >> 1) * 8u + i8) * 128u + ((((q & 1u) * 4u + h * 2u + (m & 1u)) ^ i8) << 4);
