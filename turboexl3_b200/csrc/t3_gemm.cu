@@ -346,6 +346,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         mbar_init_fence();
     }
     if (warp == kMmaWarp) tmem_alloc(tmem_slot, kTmemCols);
+    if (warp == kRowWarp && lane < 6u) prefetch_map(lane < 4u ? &maps.rows[lane] : &maps.codes[lane == 5u && a.ops > 1u]);
     if (tid == 32u) pdl_trigger();
     tc_fence_before();
     __syncthreads();
@@ -552,17 +553,18 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
             }
             await(acc_full, subs++ & 1u);
             const uint32_t parts = s.parts();
-            if (sliced) {  // this slice's sums to its place in the slab
-                float* slab = a.part + (((size_t)s.blk * a.ksplit + blockIdx.x) * a.dense_rows + s.first) * 128u + 32u * q + 16u * h + g;
+            if (sliced) {
+                // This slice's sums to its place in the slab, a lane an output: a row's 128 are four 128-byte stores. (In the finish's
+                // fragment layout a store went to four rows, 32 bytes each, and 200 rows took 2.7 us.)
+                float* slab = a.part + (((size_t)s.blk * a.ksplit + blockIdx.x) * a.dense_rows + s.first) * 128u + 32u * q + lane;
 #pragma unroll 1
-                for (uint32_t c = 0; c < parts; ++c)
-                    for_columns(my_lanes + 128u * c, s.part_cols(c), [&](uint32_t r, const uint32_t (&v)[16]) {
+                for (uint32_t r = 32u * h; r < s.cols; r += 64u) {
+                    uint32_t v[32];
+                    tmem_ld_32x32(tmem + ((32u * q) << 16) + r, v);
 #pragma unroll
-                        for (uint32_t j = 0; j < 16u; ++j) {
-                            const uint32_t row = 128u * c + r + (j >> 2) * 8u + 2u * t + (j & 1u);
-                            if (row < s.rows) __stcg(slab + (size_t)row * 128u + ((j & 2u) ? 8u : 0u), __uint_as_float(v[j]));
-                        }
-                    });
+                    for (uint32_t j = 0; j < 32u; ++j)
+                        if (r + j < s.rows) __stcg(slab + (size_t)(r + j) * 128u, __uint_as_float(v[j]));
+                }
                 return true;
             }
             // this warp's z of a part is in its buffer and the columns its rotation goes to are read
@@ -618,29 +620,35 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         // The slices of a unit meet: every CTA of the cluster has left its sums in the slab once the cluster's barrier is passed;
         // CTA z then adds the slices, in slice order, of its share of the rows and finishes those.
         tc_fence_before();
-        __threadfence();
         asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
         __syncthreads();
         tc_fence_after();
         Sub s = {};
         for_each_sub(a, [&](const Sub& mine) { s = mine; return true; });
         const uint32_t per = (s.rows + a.ksplit - 1u) / a.ksplit, lo = min(per * blockIdx.x, s.rows), live = min(per, s.rows - lo);
-        const float4* slab = reinterpret_cast<const float4*>(a.part) + ((size_t)s.blk * a.ksplit * a.dense_rows + s.first + lo) * 32u;
-        const size_t next = (size_t)a.dense_rows * 32u;
-        for (uint32_t i = tid; i < live * 32u; i += kThreads) {
-            float4 p[8];
+        const float2* slab = reinterpret_cast<const float2*>(a.part) + ((size_t)s.blk * a.ksplit * a.dense_rows + s.first + lo) * 64u;
+        const size_t next = (size_t)a.dense_rows * 64u;
+        // three pairs of sums a thread and pass: a share of up to 42 rows is one round of loads
+        constexpr uint32_t kAtOnce = 3;
+        for (uint32_t i0 = tid; i0 < live * 64u; i0 += kAtOnce * kThreads) {
+            float2 p[kAtOnce][8];
 #pragma unroll
-            for (uint32_t z = 0; z < 8u; ++z)
-                if (z < a.ksplit) p[z] = __ldcg(slab + z * next + i);
-            float4 sum = p[0];
+            for (uint32_t k = 0; k < kAtOnce; ++k)
 #pragma unroll
-            for (uint32_t z = 1; z < 8u; ++z)
-                if (z < a.ksplit) sum.x += p[z].x, sum.y += p[z].y, sum.z += p[z].z, sum.w += p[z].w;
-            const uint32_t r = i >> 5, o = 4u * (i & 31u);
-            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(z_s + (o >> 6) * 16384u + r * 128u + ((((o & 63u) >> 3) ^ (r & 7u)) << 4) +
-                                                                   (o & 7u) * 2u),
-                         "r"(pack_half2(sum.x, sum.y)), "r"(pack_half2(sum.z, sum.w))
-                         : "memory");
+                for (uint32_t z = 0; z < 8u; ++z)
+                    if (z < a.ksplit && i0 + k * kThreads < live * 64u) p[k][z] = __ldcg(slab + z * next + i0 + k * kThreads);
+#pragma unroll
+            for (uint32_t k = 0; k < kAtOnce; ++k) {
+                const uint32_t i = i0 + k * kThreads, r = i >> 6, o = 2u * (i & 63u);
+                if (i >= live * 64u) break;
+                float2 sum = p[k][0];
+#pragma unroll
+                for (uint32_t z = 1; z < 8u; ++z)
+                    if (z < a.ksplit) sum.x += p[k][z].x, sum.y += p[k][z].y;
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(z_s + (o >> 6) * 16384u + r * 128u + ((((o & 63u) >> 3) ^ (r & 7u)) << 4) + (o & 7u) * 2u),
+                             "r"(pack_half2(sum.x, sum.y))
+                             : "memory");
+            }
         }
         proxy_fence();
         __syncthreads();
