@@ -436,7 +436,9 @@ struct DenseWs {
 // Whether a call's rows are rotated once by a launch of their own instead of inside every CTA: past kFusedRows rows always;
 // up to kFusedRows when a CTA's share of the work would be more than two rotations a warp (many rows on long K slices: each
 // CTA repeats the rotation of its whole slice for every row before its first tensor-core step).
-bool prep_ahead(uint32_t rows, uint32_t slice_max) { return rows > kFusedRows || rows * (slice_max / 128u) > 2u * kConsumerWarps; }
+// On the global exchange always: the launch clears the blocks' arrival counters too (a memset ahead of the GEMV ended its overlap with
+// the stream's previous kernel: 16384 -> 7168 at one row 37.2 us, 34.8 without it).
+bool prep_ahead(const DenseArgs& a) { return a.part || a.rows > kFusedRows || a.rows * (a.slice_max / 128u) > 2u * kConsumerWarps; }
 
 DenseWs dense_ws(uint32_t rows, uint32_t in, uint32_t out, uint32_t global_split, bool ahead) {
     DenseWs w;
@@ -516,7 +518,7 @@ size_t linear_workspace(size_t rows, int in_dim, int out_dim, int n, bool far_x)
     DenseArgs a = {};
     a.in = (uint32_t)in_dim, a.out = (uint32_t)out_dim, a.n = (uint32_t)n, a.rows = (uint32_t)rows;
     if (plan_dense(a, cfg, true) != T3_OK) return 0;
-    return dense_ws(a.rows, a.in, a.out, a.part ? a.split : 0u, far_x || prep_ahead(a.rows, a.slice_max)).total;
+    return dense_ws(a.rows, a.in, a.out, a.part ? a.split : 0u, far_x || prep_ahead(a)).total;
 }
 
 int linear_call(const void* x, int x_dtype, size_t rows, const void* trellis, const void* suh, const void* svh,
@@ -556,12 +558,12 @@ int linear_call(const void* x, int x_dtype, size_t rows, const void* trellis, co
     note_engine(1, (uint64_t)in_dim, (uint64_t)out_dim, (uint64_t)n, 0);
     a.rows = (uint32_t)rows;
     if (int rc = plan_dense(a, cfg, workspace != nullptr)) return rc;
-    bool ahead = far_x || prep_ahead(a.rows, a.slice_max);
+    bool ahead = far_x || prep_ahead(a);
     DenseWs ws = dense_ws(a.rows, a.in, a.out, a.part ? a.split : 0u, ahead);
     bool has_ws = workspace != nullptr && workspace_bytes >= ws.total;
     if (a.part && !has_ws) {  // too small for the global exchange: the cluster kernel, with the rotated rows if those fit
         if (int rc = plan_dense(a, cfg, false)) return rc;
-        ahead = far_x || prep_ahead(a.rows, a.slice_max);
+        ahead = far_x || prep_ahead(a);
         ws = dense_ws(a.rows, a.in, a.out, 0u, ahead);
         has_ws = workspace != nullptr && workspace_bytes >= ws.total;
     }
@@ -570,7 +572,6 @@ int linear_call(const void* x, int x_dtype, size_t rows, const void* trellis, co
     if (a.part) {
         a.part = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + ws.part);
         a.counters = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(workspace) + ws.counters);
-        if (int rc = cuda_status(cudaMemsetAsync(a.counters, 0, (size_t)(a.out / 128u) * 4u, static_cast<cudaStream_t>(stream)))) return rc;
     }
     a.x = x;
     a.y = y;
@@ -619,7 +620,7 @@ int t3_plan_linear(size_t rows, int in_dim, int out_dim, int n, t3_decode dec, t
     char symbol[64];
     std::snprintf(symbol, sizeof symbol, "t3_dense_gemv_%s_n%u_r%u", dec.codebook == T3_MCG ? "mcg" : "mul1", named_rate(a.n), rm);
     int k = 0;
-    const bool ahead = prep_ahead(a.rows, a.slice_max);
+    const bool ahead = prep_ahead(a);
     if (ahead) {  // with the call's workspace: the rows rotated once ahead of the GEMV
         if (max_launches < 2) return -T3_BAD_EXL3_SHAPE;
         fill_launch(&out[k++], "t3_dense_prep", "dense", dim3((a.rows * (a.in / 128u) + 3u) / 4u, 1, 1), 128u, 0u, 1u,

@@ -594,6 +594,8 @@ extern "C" __global__ void __launch_bounds__(128) t3_dense_prep(const DenseArgs 
     const uint32_t task = blockIdx.x * 4u + warp;
     pdl_trigger();  // the GEMV that follows starts its weight stream now
     pdl_wait();     // x may be the previous kernel's output; the prepared rows' last reader has finished
+    if (a.part && blockIdx.x == 0)
+        for (uint32_t b = threadIdx.x; b < a.out / 128u; b += 128u) a.counters[b] = 0u;
     if (task >= a.rows * nb) return;
     const uint32_t row = task / nb, b = task - row * nb;
     prepare_block(a.x, a.x_dt, (size_t)row * a.in + b * 128u, static_cast<const __half*>(a.suh) + b * 128u,
