@@ -50,6 +50,7 @@ uint32_t* g_err_ptr[64] = {};
 unsigned long long* g_trace = nullptr;
 
 constexpr uint32_t kSmemCap = kGemvSmemLimit - kSmemSlack;  // what the carve-up of a GEMV CTA may add up to
+constexpr uint32_t kSmemHalf = 113u * 1024u - kSmemSlack;     // and where two of them fit a multiprocessor (228 KB, 1 KB a CTA reserved)
 constexpr uint32_t kDefaultRing = 64u * 1024u;
 
 uint32_t* dev_error_ptr() {
@@ -96,6 +97,23 @@ uint32_t pick_split(uint32_t nb, uint32_t units, uint32_t fan, uint32_t cap, uin
     return s;
 }
 
+// More than eight K slices, a cluster a 128-output block (`blocks` of them): where all the wider clusters are resident at two CTAs a
+// multiprocessor and the longest slice gets shorter by it. Clusters past about 80 CTAs double up on multiprocessors, and a doubled CTA
+// takes twice as long a 128-input block (1.16 us against 0.58), so what counts is the longest slice, doubled or not. One row, us, eight
+// (four) slices against the count this picks: 4096 -> 2048 7.9 / 7.0 (12), 6144 -> 2048 10.1 / 8.1 (12), 8192 -> 1536 11.5 / 8.2 (16),
+// 6144 -> 3072 10.5 / 9.7 (10), 4096 -> 5120 12.6 / 10.6 (6), 8192 -> 512 7.5 / 5.4 (16). At 17 rows level but for 8192 -> 2048 (24.9 /
+// 16.2) and 4096 -> 1536 (8.4 / 9.1). The limits are the most blocks tried that kept to one round.
+template <typename Fits>  // fits(s): a CTA of s slices holds the prepared rows of the widest call, so that every call takes the same count
+uint32_t widen_split(uint32_t nb, uint32_t blocks, uint32_t s0, Fits&& fits) {
+    static const struct { uint32_t split, blocks; } wider[] = {{6, 40}, {10, 24}, {12, 16}, {14, 12}, {16, 12}};
+    auto cost = [&](uint32_t s) { return ((nb + s - 1u) / s) * (blocks * s <= 80u ? 1u : 2u); };
+    uint32_t best = s0;
+    if (s0 >= 4u)
+        for (const auto& w : wider)
+            if (w.split > s0 && w.split <= nb && blocks <= w.blocks && cost(w.split) < cost(best) && fits(w.split)) best = w.split;
+    return best;
+}
+
 // K slices of a LARGE dense linear (tens of megabytes of codes: milliseconds of integer work, so what counts is that
 // every multiprocessor gets the same share, not the launch's latency): the power of two whose CTAs all
 // fit the device at once — two a multiprocessor, clusters of s — and leave the fullest multiprocessor the fewest
@@ -133,7 +151,14 @@ bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cl
     const uint32_t fixed = gemv_smem(row_cap, xrows, slice_max, cluster, stage_bytes, 0).total;
     if (fixed + stage_bytes > kSmemCap) return false;
     uint32_t budget = g_cfg.ring_bytes ? g_cfg.ring_bytes : kDefaultRing;
-    if (!g_cfg.ring_bytes && budget < 3u * stage_bytes && fixed + 3u * stage_bytes <= 108u * 1024u) budget = 3u * stage_bytes;
+    if (!g_cfg.ring_bytes) {
+        // two CTAs a multiprocessor where three stages (or all there are) leave room for that
+        const uint32_t least = (need < 3u ? need : 3u) * stage_bytes;
+        if (fixed + least <= kSmemHalf) {
+            if (budget < least) budget = least;
+            if (budget > kSmemHalf - fixed) budget = kSmemHalf - fixed;
+        }
+    }
     if (budget > kSmemCap - fixed) budget = kSmemCap - fixed;
     uint32_t stages = budget / stage_bytes;
     stages = stages < 1u ? 1u : stages;
@@ -457,8 +482,13 @@ bool large_linear(uint32_t in, uint32_t out, uint32_t n) { return (uint64_t)in *
 int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     const uint32_t nb = a.in / 128u;
     const bool large = large_linear(a.in, a.out, a.n);
+    auto fits = [&](uint32_t s) {
+        RingPlan ring;
+        return plan_ring(32u, 32u, largest_slice(nb, s), s, a.n, ring);
+    };
     a.split = cfg.dense_split ? (cfg.dense_split < nb ? cfg.dense_split : nb)
-                              : (large ? pick_split_large(nb, a.out / 128u) : pick_split(nb, a.out / 128u, 1u, 8u, one_wave() / 2u));
+                              : (large ? pick_split_large(nb, a.out / 128u)
+                                       : widen_split(nb, a.out / 128u, pick_split(nb, a.out / 128u, 1u, 8u, one_wave() / 2u), fits));
     a.part = nullptr;
     if (large && global_ok && !cfg.dense_split && !cfg.probe) {
         const uint32_t s = pick_split_global(nb, a.out / 128u, a.split);
