@@ -202,12 +202,60 @@ __device__ __forceinline__ void load_16b(const void* p, bool wide, uint32_t (&w)
 }
 __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
 
+// The rotation proper of a block whose scales are signs that w holds already: H128, / sqrt(128), rounded to f16; in place
+__device__ __forceinline__ void scale_out(const float2 (&out)[8][2], uint32_t (&w)[4][4]) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const float2 e = mul2(out[2 * p][t], kHadScale), f = mul2(out[2 * p + 1][t], kHadScale);
+            w[2 * t][p] = pack_half2(e.x, f.x);
+            w[2 * t + 1][p] = pack_half2(e.y, f.y);
+        }
+}
+__device__ __forceinline__ void rotate_signed(uint32_t (&w)[4][4], const HadB& hb) {
+    uint32_t a[8][2];
+    float2 out[8][2];
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            a[2 * p][h] = pack_lo(w[2 * h][p], w[2 * h + 1][p]);
+            a[2 * p + 1][h] = pack_hi(w[2 * h][p], w[2 * h + 1][p]);
+        }
+    h128_mma(a, a, false, hb, out);
+    scale_out(out, w);
+}
+
+// The signs of this lane's 32 scales of a block (at sp as in rotate_block) in one word: word w[s][p]'s two are bits 4 s + p and 16 + 4 s
+// + p. `odd` is set when a scale is not a sign.
+__device__ __forceinline__ uint32_t sign_mask(const __half* sp, bool wide, uint32_t& odd) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        uint32_t sc[4];
+        load_16b(sp + 32 * s, wide, sc);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            odd |= (sc[p] & 0x7FFF7FFFu) ^ 0x3C003C00u;
+            m |= ((sc[p] >> 15) & 0x00010001u) << (4 * s + p);
+        }
+    }
+    return m;
+}
+__device__ __forceinline__ void apply_signs(uint32_t (&w)[4][4], uint32_t m) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) w[s][p] ^= (m << (15 - (4 * s + p))) & 0x80008000u;
+}
+
 // format.prepareInput's rotation of a block: w (f16 pairs, w[s][p] = elements 8 (4 s + q) + 2 p, + 1 of this quad's position) times
 // the scales at sp (f16, this lane's first element; `wide`: 16-byte aligned), H128, / sqrt(128), rounded to f16; in place. Sign
 // scales (the usual suh) are a sign flip of the f16 values, and need no registers past it; with any other a product is taken in
 // f32 and split into an f16 part and the f16 of what is left, so that the sums see the f32 products.
 __device__ __forceinline__ void rotate_block(uint32_t (&w)[4][4], const __half* sp, bool wide, const HadB& hb) {
-    uint32_t a[8][2], odd = 0;
+    uint32_t odd = 0;
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         uint32_t sc[4];
@@ -218,46 +266,32 @@ __device__ __forceinline__ void rotate_block(uint32_t (&w)[4][4], const __half* 
             w[s][p] ^= sc[p] & 0x80008000u;
         }
     }
-    float2 out[8][2];
     if (__any_sync(0xFFFFFFFFu, odd != 0u) == 0) {
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                a[2 * p][h] = pack_lo(w[2 * h][p], w[2 * h + 1][p]);
-                a[2 * p + 1][h] = pack_hi(w[2 * h][p], w[2 * h + 1][p]);
-            }
-        h128_mma(a, a, false, hb, out);
-    } else {
-        uint32_t lo[8][2], rest = 0;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t sc[2][4];
-            load_16b(sp + 64 * h, wide, sc[0]);
-            load_16b(sp + 64 * h + 32, wide, sc[1]);
-#pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                const float2 x0 = unpack_half2(w[2 * h][p]), x1 = unpack_half2(w[2 * h + 1][p]);  // the signs are in already
-                const float2 c0 = unpack_half2(sc[0][p] & 0x7FFF7FFFu), c1 = unpack_half2(sc[1][p] & 0x7FFF7FFFu);
-                const float v[2][2] = {{x0.x * c0.x, x1.x * c1.x}, {x0.y * c0.y, x1.y * c1.y}};
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    a[2 * p + i][h] = pack_half2(v[i][0], v[i][1]);
-                    lo[2 * p + i][h] = pack_half2(v[i][0] - round_half(v[i][0]), v[i][1] - round_half(v[i][1]));
-                    rest |= lo[2 * p + i][h] & 0x7FFF7FFFu;
-                }
-            }
-        }
-        h128_mma(a, lo, __any_sync(0xFFFFFFFFu, rest != 0u) != 0, hb, out);
+        rotate_signed(w, hb);
+        return;
     }
+    uint32_t a[8][2], lo[8][2], rest = 0;
+    float2 out[8][2];
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
+    for (int h = 0; h < 2; ++h) {
+        uint32_t sc[2][4];
+        load_16b(sp + 64 * h, wide, sc[0]);
+        load_16b(sp + 64 * h + 32, wide, sc[1]);
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            const float2 e = mul2(out[2 * p][t], kHadScale), f = mul2(out[2 * p + 1][t], kHadScale);
-            w[2 * t][p] = pack_half2(e.x, f.x);
-            w[2 * t + 1][p] = pack_half2(e.y, f.y);
+        for (int p = 0; p < 4; ++p) {
+            const float2 x0 = unpack_half2(w[2 * h][p]), x1 = unpack_half2(w[2 * h + 1][p]);  // the signs are in already
+            const float2 c0 = unpack_half2(sc[0][p] & 0x7FFF7FFFu), c1 = unpack_half2(sc[1][p] & 0x7FFF7FFFu);
+            const float v[2][2] = {{x0.x * c0.x, x1.x * c1.x}, {x0.y * c0.y, x1.y * c1.y}};
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                a[2 * p + i][h] = pack_half2(v[i][0], v[i][1]);
+                lo[2 * p + i][h] = pack_half2(v[i][0] - round_half(v[i][0]), v[i][1] - round_half(v[i][1]));
+                rest |= lo[2 * p + i][h] & 0x7FFF7FFFu;
+            }
         }
+    }
+    h128_mma(a, lo, __any_sync(0xFFFFFFFFu, rest != 0u) != 0, hb, out);
+    scale_out(out, w);
 }
 
 // eight consecutive elements i .. i + 7 (i a multiple of 8) of an activation array, each rounded to f16
