@@ -1,6 +1,6 @@
 """The prefill GEMM's epilogue and the prepare where their variants meet: row tiles either side of the heights whose accumulators are
-given back early (80 rows in pairs of output blocks, 128 one at a time), an odd last block, and the prepare's walk over runs of positions with sign
-and general scales mixed."""
+given back early (80 rows in pairs of output blocks, 128 one at a time), an odd last block, the prepare's walk over runs of positions
+with sign and general scales mixed, and the one-expert chain that stores its rows without a final sum."""
 import numpy as np
 import pytest
 import torch
@@ -9,7 +9,7 @@ import turboexl3_b200 as t3
 from oracle import binding as ob
 from turboexl3_b200 import synth
 
-from gpu_util import check, dev, host_f32, x_as
+from gpu_util import TORCH_DT, bits16, check, dev, host_f32, x_as
 from test_gpu_moe import check_moe, make_bank
 
 pytestmark = pytest.mark.gpu
@@ -68,4 +68,25 @@ def test_the_prepare_walks_runs_of_positions():
     whole = call(np.arange(rows))
     for r in (np.arange(40), np.arange(rows - 33, rows), np.arange(0, rows, 97)):
         assert torch.equal(whole[r], call(r))
+    assert t3.device_error() == 0
+
+
+@pytest.mark.parametrize("dt,score_dt", [("f16", torch.float32), ("bf16", torch.bfloat16), ("f32", torch.float16)])
+def test_one_expert_prompts_are_weighted_in_the_epilogue(dt, score_dt):
+    """A one-expert bank at one slot a row: the bytes of the same expert in a bank of two, which takes the final sum's launch."""
+    H, I, n = 384, 256, 48
+    arrs = synth.bank(3130, 2, H, I, n)
+    bank = lambda e: t3.Bank(*(t3.Proj(*(dev(arrs[p + f][e]) for f in ("_t", "_suh", "_svh"))) for p in ("gate", "up", "down")))
+    one, two = bank(slice(0, 1)), bank(slice(0, 2))
+    obank = ob.Bank(2, H, I, n, *[arrs[p + f] for p in ("gate", "up", "down") for f in ("_t", "_suh", "_svh")])
+    for rows in (33, 127, 129, 300, 2100):
+        x = x_as(synth.activations(3131 + rows, rows, H), dt)
+        scores = torch.from_numpy(np.random.default_rng(rows).standard_normal((rows, 1)).astype(np.float32)).cuda().to(score_dt)
+        zeros = torch.zeros((1, rows, 1), dtype=torch.int32, device="cuda")
+        y = t3.moe(x.view(1, rows, H), one, zeros, scores.view(1, rows, 1))
+        assert y.dtype == TORCH_DT[dt]
+        assert np.array_equal(bits16(y), bits16(t3.moe(x.view(1, rows, H), two, zeros, scores.view(1, rows, 1)))), rows
+        sample = sorted({0, 31, 32, rows // 2, rows - 1})
+        ref = ob.moe_rows(obank, host_f32(x)[sample], np.zeros((len(sample), 1), np.int32), scores.float().cpu().numpy()[sample])
+        check_moe(host_f32(y).reshape(rows, H)[sample], ref, dt, ("one expert", dt, rows))
     assert t3.device_error() == 0

@@ -303,6 +303,28 @@ __device__ __forceinline__ void store_part(uint32_t buffer, uint16_t* y, size_t 
     }
 }
 
+// The same with each row's f16 values times its score (of the part's first row on), stored as the final sum of one slot a row stores
+// them: 0 + w v in f32, rounded once to y's dtype (y at the part's first value, element `at` of a.y)
+__device__ __forceinline__ void store_scored(uint32_t buffer, const DecodeGemmArgs& a, size_t first, size_t at, uint32_t rows, uint32_t warp, uint32_t lane) {
+    const uint32_t j = lane & 15u;
+#pragma unroll 2
+    for (uint32_t r = 2u * warp + (lane >> 4); r < rows; r += 2u * kEpiWarps) {
+        uint32_t w[4];
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                     : "r"(buffer + (j >> 3) * 16384u + r * 128u + (((j & 7u) ^ (r & 7u)) << 4)));
+        const float score = load_act(a.scores, a.score_dt, first + r);
+#pragma unroll
+        for (uint32_t half = 0; half < 2u; ++half) {
+            const float2 u = unpack_half2(w[2u * half]), v = unpack_half2(w[2u * half + 1u]);
+            float f[4] = {u.x, u.y, v.x, v.y};
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i) f[i] = __fadd_rn(0.0f, __fmul_rn(score, f[i]));
+            store_act4(a.y, a.y_dt, at + r * (size_t)a.N + 8u * j + 4u * half, f);
+        }
+    }
+}
+
 // The output rotation of a part on the tensor cores (one thread): D2 = H128 x z^T into the columns at tmem_d
 __device__ __forceinline__ void rotate_part(uint32_t tmem, uint32_t tmem_d, uint32_t z, uint32_t idesc, uint32_t rot_full) {
     const uint32_t hi = (uint32_t)(umma_desc(0) >> 32), lo = (uint32_t)umma_desc(z);
@@ -526,7 +548,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         const uint32_t m = lane >> 3, i8 = lane & 7u;
         const uint32_t st_at = z_s + (q >> 1) * 16384u + ((m >> 1) * 8u + i8) * 128u + ((((q & 1u) * 4u + h * 2u + (m & 1u)) ^ i8) << 4);
         const uint32_t my_lanes = tmem + ((32u * q + 16u * h) << 16);
-        const int dt = a.y ? a.y_dt : (int)kF16;
+        const int dt = a.y && !a.scores ? a.y_dt : (int)kF16;
         const bool plain = KEPT && a.svh[0] == nullptr;
         uint16_t* const y16 = a.y ? static_cast<uint16_t*>(a.y) : reinterpret_cast<uint16_t*>(a.z);
         uint32_t subs = 0, rots = 0;  // rots: the next rotation's parity, a bit a part
@@ -609,6 +631,11 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
             meet();
             for (uint32_t c = 0; c < parts; ++c) {
                 const uint32_t row0 = s.wide ? 0u : 128u * c;
+                if (a.scores) {
+                    store_scored(z_s + c * kZBytes, a, s.first + row0, (size_t)(s.first + row0) * a.N + (s.blk + (s.wide ? c : 0u)) * 128u,
+                                 min(s.part_cols(c), s.rows - row0), warp, lane);
+                    continue;
+                }
                 store_part(z_s + c * kZBytes, y16 + s.op * a.z_op_stride + (size_t)(s.first + row0) * a.N + (s.blk + (s.wide ? c : 0u)) * 128u,
                            a.N, min(s.part_cols(c), s.rows - row0), warp, lane);
             }

@@ -41,6 +41,8 @@ struct DecodeGemmArgs {
     size_t z_op_stride;
     void* y;
     int y_dt;
+    const void* scores;         // y only, or null: each row's f16 value times its score, as the final sum of one slot a row has it
+    int score_dt;
     // K slices (dense, at least two, eight at most): a cluster of `ksplit` CTAs a unit, slice z running inputs 128 floor(K / 128 *
     // z / ksplit) .. and leaving its f32 accumulators in part [N / 128][ksplit][rows][128]; after the cluster's barrier each CTA
     // adds the slices of its share of the rows in slice order and finishes them. 0 or 1: one CTA runs all of K.
