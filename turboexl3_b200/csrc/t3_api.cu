@@ -691,15 +691,12 @@ int validate_bank(const t3_bank* b, int hidden_of_x) {
 // top-k set.
 int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     const size_t slots = (size_t)a.rows * a.topk;
-    // Members of an expert one CTA's decode of its weights serves. Sized from the geometry's expected members an expert (rows *
-    // topk / experts, with headroom), not from the row count: with many experts a 32-row call still has one or two rows an
-    // expert, and a 32-row pass would pay four times the shared memory and twice the tensor-core steps for nothing. An expert
-    // with more members is served by several CTAs at once, so where those all find a place (few experts: a shared expert's
-    // chain) eight members a CTA is the quickest: 29 rows on one expert of 2048 x 512 took 61 us in one CTA a block, most of it
-    // the 29 prepares and finishes. A row's bytes do not depend on it.
-    const uint32_t expect = (uint32_t)((4u * slots + a.experts - 1u) / a.experts) + 4u;
-    uint32_t rm = row_cap_for(expect < a.rows ? expect : a.rows);
-    if ((uint64_t)(a.experts + slots / 8u) * (a.inter / 128u) * 2u <= one_wave() / 2u) rm = 8u;
+    // Members of an expert one CTA's decode of its weights serves: eight, and sixteen where an expert has more than eight on average (an
+    // expert with more is served by several CTAs at once, and those are quicker than one of a larger capacity, whose every tile costs the
+    // tensor-core steps and the shared memory of all its rows). us at capacity 8 / 16 / 32: 64 experts of 7168 x 2048 at 2 members
+    // an expert 824 / 1179 / 1350, at 4 1104 / 1585 / 1790; 32 of 4096 x 1024 at 6 225 / 253 / 311; 64 of 2048 x 512 at 5 121 / 130 / 145;
+    // 32 of 2048 x 512 at 10 107 / 87 / 93; one expert's 32 rows 32.6 / 32.0 / 47.3. A row's bytes do not depend on it.
+    const uint32_t rm = slots > 8u * (size_t)a.experts && (a.experts + slots / 8u) * (a.inter / 128u) * 2u > one_wave() / 2u ? 16u : 8u;
     a.row_cap = rm;
     a.overlap = !cfg.no_overlap;
     // The K splits depend on hidden and inter only (sized as if a row had eight slots), never on the row count, the top-k

@@ -553,7 +553,8 @@ cudaError_t launch_cluster(KernelFn<Args> fn, const Args& a, dim3 grid, uint32_t
 //   t3_dense_gemv_<codebook>_n<n>_r<rows>      t3_dec_gate_up_<codebook>_n<n>_r<rows>      t3_dec_down_<codebook>_n<n>_r<rows>
 //   t3_dec_merge
 // <codebook> mul1 | mcg (probe2..probe4: the dense kernel's timing probes); <n> the rate's halfwords a tile, 0 = any even
-// rate at run time; <rows> the row capacity of a pass, 8 | 16 | 32.
+// rate at run time; <rows> the row capacity of a pass, 8 | 16 | 32
+// (32: the dense linear only).
 #if T3_CB == 0
 #define T3_CBNAME mul1
 #elif T3_CB == 1
@@ -572,18 +573,19 @@ cudaError_t launch_cluster(KernelFn<Args> fn, const Args& a, dim3 grid, uint32_t
         BODY<NN, RM>(a);                                                                                        \
     }
 #if T3_SERVED
-#define T3_ENTRIES(STEM, BODY, ARGS, NN) T3_ENTRY(STEM, BODY, ARGS, NN, 8) T3_ENTRY(STEM, BODY, ARGS, NN, 16) T3_ENTRY(STEM, BODY, ARGS, NN, 32)
+#define T3_ENTRIES_32(STEM, BODY, ARGS, NN) T3_ENTRY(STEM, BODY, ARGS, NN, 8) T3_ENTRY(STEM, BODY, ARGS, NN, 16) T3_ENTRY(STEM, BODY, ARGS, NN, 32)
+#define T3_ENTRIES_16(STEM, BODY, ARGS, NN) T3_ENTRY(STEM, BODY, ARGS, NN, 8) T3_ENTRY(STEM, BODY, ARGS, NN, 16)
 #else  // the probes exist at the 8-row capacity only
-#define T3_ENTRIES(STEM, BODY, ARGS, NN) T3_ENTRY(STEM, BODY, ARGS, NN, 8)
+#define T3_ENTRIES_32(STEM, BODY, ARGS, NN) T3_ENTRY(STEM, BODY, ARGS, NN, 8)
 #endif
-#define T3_ALL_RATES(STEM, BODY, ARGS)                                                                          \
-    T3_ENTRIES(STEM, BODY, ARGS, 0) T3_ENTRIES(STEM, BODY, ARGS, 16) T3_ENTRIES(STEM, BODY, ARGS, 32)           \
-    T3_ENTRIES(STEM, BODY, ARGS, 48) T3_ENTRIES(STEM, BODY, ARGS, 64) T3_ENTRIES(STEM, BODY, ARGS, 80)          \
-    T3_ENTRIES(STEM, BODY, ARGS, 96) T3_ENTRIES(STEM, BODY, ARGS, 112) T3_ENTRIES(STEM, BODY, ARGS, 128)
-T3_ALL_RATES(t3_dense_gemv, dense_gemv_body, DenseArgs)
+#define T3_ALL_RATES(ENTRIES, STEM, BODY, ARGS)                                                       \
+    ENTRIES(STEM, BODY, ARGS, 0) ENTRIES(STEM, BODY, ARGS, 16) ENTRIES(STEM, BODY, ARGS, 32)          \
+    ENTRIES(STEM, BODY, ARGS, 48) ENTRIES(STEM, BODY, ARGS, 64) ENTRIES(STEM, BODY, ARGS, 80)         \
+    ENTRIES(STEM, BODY, ARGS, 96) ENTRIES(STEM, BODY, ARGS, 112) ENTRIES(STEM, BODY, ARGS, 128)
+T3_ALL_RATES(T3_ENTRIES_32, t3_dense_gemv, dense_gemv_body, DenseArgs)
 #if T3_SERVED
-T3_ALL_RATES(t3_dec_gate_up, moe_gate_up_body, MoeArgs)
-T3_ALL_RATES(t3_dec_down, moe_down_body, MoeArgs)
+T3_ALL_RATES(T3_ENTRIES_16, t3_dec_gate_up, moe_gate_up_body, MoeArgs)
+T3_ALL_RATES(T3_ENTRIES_16, t3_dec_down, moe_down_body, MoeArgs)
 #endif
 #if T3_CB == 0
 extern "C" __global__ void __launch_bounds__(256) t3_dec_merge(const MoeArgs a) { moe_merge_body(a); }
@@ -604,29 +606,30 @@ extern "C" __global__ void __launch_bounds__(128) t3_dense_prep(const DenseArgs 
 #endif
 
 #if T3_SERVED
-#define T3_PICK_RM(STEM, NN, rm) \
+#define T3_PICK_32(STEM, NN, rm) \
     ((rm) == 8 ? T3_NAME(STEM, T3_CBNAME, NN, 8) : ((rm) == 16 ? T3_NAME(STEM, T3_CBNAME, NN, 16) : T3_NAME(STEM, T3_CBNAME, NN, 32)))
+#define T3_PICK_16(STEM, NN, rm) ((rm) == 8 ? T3_NAME(STEM, T3_CBNAME, NN, 8) : T3_NAME(STEM, T3_CBNAME, NN, 16))
 #else
-#define T3_PICK_RM(STEM, NN, rm) T3_NAME(STEM, T3_CBNAME, NN, 8)
+#define T3_PICK_32(STEM, NN, rm) T3_NAME(STEM, T3_CBNAME, NN, 8)
 #endif
 
-#define T3_PICK(STEM, n, rm)                                                       \
-    ((n) == 16    ? T3_PICK_RM(STEM, 16, rm)                                        \
-     : (n) == 32  ? T3_PICK_RM(STEM, 32, rm)                                        \
-     : (n) == 48  ? T3_PICK_RM(STEM, 48, rm)                                        \
-     : (n) == 64  ? T3_PICK_RM(STEM, 64, rm)                                        \
-     : (n) == 80  ? T3_PICK_RM(STEM, 80, rm)                                        \
-     : (n) == 96  ? T3_PICK_RM(STEM, 96, rm)                                        \
-     : (n) == 112 ? T3_PICK_RM(STEM, 112, rm)                                       \
-     : (n) == 128 ? T3_PICK_RM(STEM, 128, rm)                                       \
-                  : T3_PICK_RM(STEM, 0, rm))
+#define T3_PICK(PICK, STEM, n, rm)          \
+    ((n) == 16    ? PICK(STEM, 16, rm)      \
+     : (n) == 32  ? PICK(STEM, 32, rm)      \
+     : (n) == 48  ? PICK(STEM, 48, rm)      \
+     : (n) == 64  ? PICK(STEM, 64, rm)      \
+     : (n) == 80  ? PICK(STEM, 80, rm)      \
+     : (n) == 96  ? PICK(STEM, 96, rm)      \
+     : (n) == 112 ? PICK(STEM, 112, rm)     \
+     : (n) == 128 ? PICK(STEM, 128, rm)     \
+                  : PICK(STEM, 0, rm))
 
 #define T3_CAT2(a, b) a##b
 #define T3_CAT(a, b) T3_CAT2(a, b)
 
 cudaError_t T3_CAT(launch_dense_gemv_cb, T3_CB)(const DenseArgs& a, cudaStream_t stream) {
     const uint32_t rm = row_cap_for(a.rows);
-    KernelFn<DenseArgs> fn = T3_PICK(t3_dense_gemv, a.n, rm);
+    KernelFn<DenseArgs> fn = T3_PICK(T3_PICK_32, t3_dense_gemv, a.n, rm);
     const uint32_t cluster = a.part ? 1u : a.split;
     return launch_cluster(fn, a, dim3(a.split, a.out / 128u, 1), cluster, gemv_smem_bytes(rm, a.rows, a.slice_max, cluster, a.n, a.ring),
                           a.overlap != 0, stream);
@@ -650,14 +653,14 @@ cudaError_t launch_dense_prep(const DenseArgs& a, cudaStream_t stream) {
 #if T3_SERVED
 cudaError_t T3_CAT(launch_moe_gate_up_cb, T3_CB)(const MoeArgs& a, cudaStream_t stream) {
     const uint32_t rm = a.row_cap;
-    KernelFn<MoeArgs> fn = T3_PICK(t3_dec_gate_up, a.n, rm);
+    KernelFn<MoeArgs> fn = T3_PICK(T3_PICK_16, t3_dec_gate_up, a.n, rm);
     return launch_cluster(fn, a, dim3(2u * a.split_gu, a.inter / 128u, a.rows * a.topk), 2u * a.split_gu,
                           gemv_smem_bytes(rm, rm, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu), a.overlap != 0, stream);
 }
 
 cudaError_t T3_CAT(launch_moe_down_cb, T3_CB)(const MoeArgs& a, cudaStream_t stream) {
     const uint32_t rm = a.row_cap;
-    KernelFn<MoeArgs> fn = T3_PICK(t3_dec_down, a.n, rm);
+    KernelFn<MoeArgs> fn = T3_PICK(T3_PICK_16, t3_dec_down, a.n, rm);
     return launch_cluster(fn, a, dim3(a.split_d, a.hidden / 128u, a.rows * a.topk), a.split_d,
                           gemv_smem_bytes(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d), a.overlap != 0, stream);
 }

@@ -67,7 +67,7 @@ struct MoeArgs {
     uint32_t banked;          // decode rows, top-1: inds holds packed ids (bank << 24 | slot); banks 1 and 2 in ext; scores null = 1
     BankTab ext[2];
     void* shared_ready;       // host side only: an event the last launch (the one that reads `shared`) waits for, or null
-    uint32_t row_cap;                  // rows a CTA's decode of an expert's weights serves (8, 16 or 32): an expert with more members takes more CTAs
+    uint32_t row_cap;                  // rows a CTA's decode of an expert's weights serves (8 or 16): an expert with more members takes more CTAs
     uint32_t split_gu, slice_max_gu;   // K slices of gate|up (cluster = 2 * split_gu), largest slice
     uint32_t split_d, slice_max_d;     // K slices of down
     RingPlan ring_gu, ring_d;
