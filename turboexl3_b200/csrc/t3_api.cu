@@ -51,6 +51,10 @@ unsigned long long* g_trace = nullptr;
 
 constexpr uint32_t kSmemCap = kGemvSmemLimit - kSmemSlack;  // what the carve-up of a GEMV CTA may add up to
 constexpr uint32_t kSmemHalf = 113u * 1024u - kSmemSlack;     // and where two of them fit a multiprocessor (228 KB, 1 KB a CTA reserved)
+// What a CTA asks for so that no second one of its kind fits the multiprocessor. The hardware places the clusters of a launch that starts
+// beside its predecessor two CTAs to a multiprocessor while others stay empty, and a doubled CTA takes twice as long, which sets the
+// launch's duration. (A launch of another kind, with less, still fits beside it.)
+constexpr uint32_t kSmemAlone = 115u * 1024u;
 constexpr uint32_t kDefaultRing = 64u * 1024u;
 
 uint32_t* dev_error_ptr() {
@@ -97,21 +101,28 @@ uint32_t pick_split(uint32_t nb, uint32_t units, uint32_t fan, uint32_t cap, uin
     return s;
 }
 
-// More than eight K slices, a cluster a 128-output block (`blocks` of them): where all the wider clusters are resident at two CTAs a
-// multiprocessor and the longest slice gets shorter by it. Clusters past about 80 CTAs double up on multiprocessors, and a doubled CTA
-// takes twice as long a 128-input block (1.16 us against 0.58), so what counts is the longest slice, doubled or not. One row, us, eight
-// (four) slices against the count this picks: 4096 -> 2048 7.9 / 7.0 (12), 6144 -> 2048 10.1 / 8.1 (12), 8192 -> 1536 11.5 / 8.2 (16),
-// 6144 -> 3072 10.5 / 9.7 (10), 4096 -> 5120 12.6 / 10.6 (6), 8192 -> 512 7.5 / 5.4 (16). At 17 rows level but for 8192 -> 2048 (24.9 /
-// 16.2) and 4096 -> 1536 (8.4 / 9.1). The limits are the most blocks tried that kept to one round.
-template <typename Fits>  // fits(s): a CTA of s slices holds the prepared rows of the widest call, so that every call takes the same count
-uint32_t widen_split(uint32_t nb, uint32_t blocks, uint32_t s0, Fits&& fits) {
-    static const struct { uint32_t split, blocks; } wider[] = {{6, 40}, {10, 24}, {12, 16}, {14, 12}, {16, 12}};
-    auto cost = [&](uint32_t s) { return ((nb + s - 1u) / s) * (blocks * s <= 80u ? 1u : 2u); };
-    uint32_t best = s0;
-    if (s0 >= 4u)
-        for (const auto& w : wider)
-            if (w.split > s0 && w.split <= nb && blocks <= w.blocks && cost(w.split) < cost(best) && fits(w.split)) best = w.split;
-    return best;
+// K slices of an ordinary dense linear of nb 128-input and `blocks` 128-output blocks, a cluster of s CTAs a block, and whether its CTAs
+// go one to a multiprocessor (`alone`). The time is the longest slice's: 0.58 us a 128-input block in a CTA that has its multiprocessor to
+// itself and 1.16 in one of two (whatever the rate), and about 0.1 us a CTA of the cluster. So: the count that is cheapest by that, alone
+// where all clusters fit one CTA to a multiprocessor, else two where they fit so; the most clusters of each size that do are
+// cudaOccupancyMaxActiveClusters's, written down because a row's bytes follow from the count and must be the same without a device.
+// One row, us, powers of two up to eight slices against this: 2048 -> 2048 5.3 / 4.7 (six, alone), 6144 -> 2048 10.1 / 7.5 (six), 7168 ->
+// 1536 10.7 / 6.8 (eight), 3072 -> 3072 7.0 / 6.2 (four), 2048 -> 6144 8.0 / 7.4 (two); at 17 rows 8.6 / 7.7, 15.6 / 12.6, 12.6 / 11.7, 10.9 /
+// 10.5, 12.8 / 12.6. Counts past four in the second case are the powers of two: others placed worse.
+// fits(s): a CTA holds the prepared rows of the widest call, so that calls of every row count take the same count.
+template <typename Fits>
+uint32_t pick_split_dense(uint32_t nb, uint32_t blocks, uint32_t& alone, Fits&& fits) {
+    static const uint16_t one[17] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7};
+    static const uint16_t two[17] = {0, 296, 148, 0, 71, 0, 0, 0, 33, 0, 0, 0, 0, 0, 0, 0, 14};
+    uint32_t best = 0, best_cost = ~0u;
+    alone = 0;
+    for (uint32_t s = 1; s <= 16u && s <= nb; ++s) {
+        const uint32_t longest = (nb + s - 1u) / s, single = blocks <= one[s];
+        if (!single && blocks > two[s]) continue;
+        const uint32_t cost = longest * (single ? 58u : 116u) + 10u * s + (single ? 0u : 30u);
+        if (cost < best_cost && (s == 1u || fits(s))) best = s, best_cost = cost, alone = single;
+    }
+    return best ? best : 1u;
 }
 
 // K slices of a LARGE dense linear (tens of megabytes of codes: milliseconds of integer work, so what counts is that
@@ -143,7 +154,7 @@ uint32_t largest_slice(uint32_t nb, uint32_t split) {
 
 // The ring of one GEMV CTA: stages of kStageRows tk rows (two 128-input blocks), as many as the slab needs or the budget
 // holds; three where the default budget holds fewer and two CTAs still fit a multiprocessor.
-bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan& ring) {
+bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan& ring, bool alone = false) {
     const uint32_t row_bytes = 16u * n, nrows = slice_max / 16u;  // nrows is a multiple of 8 (whole 128-blocks)
     const uint32_t stage_rows = kStageRows;
     const uint32_t stage_bytes = stage_rows * row_bytes;
@@ -151,7 +162,7 @@ bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cl
     const uint32_t fixed = gemv_smem(row_cap, xrows, slice_max, cluster, stage_bytes, 0).total;
     if (fixed + stage_bytes > kSmemCap) return false;
     uint32_t budget = g_cfg.ring_bytes ? g_cfg.ring_bytes : kDefaultRing;
-    if (!g_cfg.ring_bytes) {
+    if (!g_cfg.ring_bytes && !alone) {
         // two CTAs a multiprocessor where three stages (or all there are) leave room for that
         const uint32_t least = (need < 3u ? need : 3u) * stage_bytes;
         if (fixed + least <= kSmemHalf) {
@@ -187,8 +198,9 @@ int cuda_status(cudaError_t rc) { return rc == cudaSuccess ? T3_OK : T3_CUDA_ERR
 
 uint32_t row_cap_for(uint32_t rows) { return rows <= 8u ? 8u : (rows <= 16u ? 16u : 32u); }
 
-uint32_t gemv_smem_bytes(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan ring) {
-    return gemv_smem(row_cap, xrows, slice_max, cluster, ring.stage_rows * 16u * n, ring.stages).total + kSmemSlack;
+uint32_t gemv_smem_bytes(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan ring, bool alone) {
+    const uint32_t bytes = gemv_smem(row_cap, xrows, slice_max, cluster, ring.stage_rows * 16u * n, ring.stages).total + kSmemSlack;
+    return alone && bytes < kSmemAlone ? kSmemAlone : bytes;
 }
 
 thread_local const void* g_last_kernel = nullptr;
@@ -482,13 +494,13 @@ bool large_linear(uint32_t in, uint32_t out, uint32_t n) { return (uint64_t)in *
 int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     const uint32_t nb = a.in / 128u;
     const bool large = large_linear(a.in, a.out, a.n);
+    a.alone = 0;
     auto fits = [&](uint32_t s) {
         RingPlan ring;
         return plan_ring(32u, 32u, largest_slice(nb, s), s, a.n, ring);
     };
     a.split = cfg.dense_split ? (cfg.dense_split < nb ? cfg.dense_split : nb)
-                              : (large ? pick_split_large(nb, a.out / 128u)
-                                       : widen_split(nb, a.out / 128u, pick_split(nb, a.out / 128u, 1u, 8u, one_wave() / 2u), fits));
+                              : (large ? pick_split_large(nb, a.out / 128u) : pick_split_dense(nb, a.out / 128u, a.alone, fits));
     a.part = nullptr;
     if (large && global_ok && !cfg.dense_split && !cfg.probe) {
         const uint32_t s = pick_split_global(nb, a.out / 128u, a.split);
@@ -500,13 +512,14 @@ int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     a.overlap = !cfg.no_overlap;
     a.slice_max = largest_slice(nb, a.split);
     // a slice too long for shared memory (its prepared rows) is cut further, up to the widest cluster
-    while (!plan_ring(row_cap_for(a.rows), a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring)) {
+    while (!plan_ring(row_cap_for(a.rows), a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0)) {
         if (a.part) {  // back to the cluster kernel
             a.part = nullptr;
             a.split = pick_split_large(nb, a.out / 128u);
             a.slice_max = largest_slice(nb, a.split);
             continue;
         }
+        a.alone = 0;
         if (a.split * 2u > nb || a.split * 2u > 16u) return T3_ENGINE_NOT_IMPLEMENTED;
         a.split *= 2u;
         a.slice_max = largest_slice(nb, a.split);
@@ -658,11 +671,11 @@ int t3_plan_linear(size_t rows, int in_dim, int out_dim, int n, t3_decode dec, t
     }
     if (ahead)
         fill_launch(&out[k++], symbol, "dense", dim3(a.split, a.out / 128u, 1), 32u * 17u,
-                    gemv_smem_bytes(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring), a.part ? 1u : a.split,
+                    gemv_smem_bytes(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0), a.part ? 1u : a.split,
                     {T3_ROLE_XP, T3_ROLE_Y, T3_ROLE_TRELLIS, T3_ROLE_SVH});
     else
         fill_launch(&out[k++], symbol, "dense", dim3(a.split, a.out / 128u, 1), 32u * 17u,
-                    gemv_smem_bytes(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring), a.part ? 1u : a.split,
+                    gemv_smem_bytes(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0), a.part ? 1u : a.split,
                     {T3_ROLE_X, T3_ROLE_Y, T3_ROLE_TRELLIS, T3_ROLE_SUH, T3_ROLE_SVH});
     if (a.part) out[k - 1].roles[out[k - 1].nroles++] = T3_ROLE_Z;  // the slices' partial sums meet in global memory
     return k;
@@ -732,6 +745,7 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     const uint32_t sms = one_wave() / 2u;
     const uint64_t gu = (uint64_t)2u * a.split_gu * (a.inter / 128u) * slots, down = (uint64_t)a.split_d * (a.hidden / 128u) * slots;
     a.down_early = a.experts > 1u && gu <= sms && (down > sms || gu + down <= sms);
+    a.alone_gu = 0;
     return T3_OK;
 }
 
@@ -840,7 +854,7 @@ int t3_plan_moe(size_t rows, int topk, const t3_bank* bank, t3_decode dec, t3_la
     char symbol[64];
     std::snprintf(symbol, sizeof symbol, "t3_dec_gate_up_%s_n%u_r%u", cb, named_rate(a.n), rm);
     fill_launch(&out[0], symbol, "decode", dim3(2u * a.split_gu, a.inter / 128u, slots), 32u * 17u,
-                gemv_smem_bytes(rm, rm, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu), 2u * a.split_gu,
+                gemv_smem_bytes(rm, rm, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu, a.alone_gu != 0), 2u * a.split_gu,
                 {T3_ROLE_X, T3_ROLE_SLOTS, T3_ROLE_GATE_T, T3_ROLE_UP_T, T3_ROLE_GATE_SUH, T3_ROLE_UP_SUH, T3_ROLE_GATE_SVH,
                  T3_ROLE_UP_SVH, T3_ROLE_DOWN_SUH, T3_ROLE_HD});
     std::snprintf(symbol, sizeof symbol, "t3_dec_down_%s_n%u_r%u", cb, named_rate(a.n), rm);

@@ -631,7 +631,8 @@ cudaError_t T3_CAT(launch_dense_gemv_cb, T3_CB)(const DenseArgs& a, cudaStream_t
     const uint32_t rm = row_cap_for(a.rows);
     KernelFn<DenseArgs> fn = T3_PICK(T3_PICK_32, t3_dense_gemv, a.n, rm);
     const uint32_t cluster = a.part ? 1u : a.split;
-    return launch_cluster(fn, a, dim3(a.split, a.out / 128u, 1), cluster, gemv_smem_bytes(rm, a.rows, a.slice_max, cluster, a.n, a.ring),
+    return launch_cluster(fn, a, dim3(a.split, a.out / 128u, 1), cluster,
+                          gemv_smem_bytes(rm, a.rows, a.slice_max, cluster, a.n, a.ring, a.alone != 0),
                           a.overlap != 0, stream);
 }
 
@@ -655,7 +656,7 @@ cudaError_t T3_CAT(launch_moe_gate_up_cb, T3_CB)(const MoeArgs& a, cudaStream_t 
     const uint32_t rm = a.row_cap;
     KernelFn<MoeArgs> fn = T3_PICK(T3_PICK_16, t3_dec_gate_up, a.n, rm);
     return launch_cluster(fn, a, dim3(2u * a.split_gu, a.inter / 128u, a.rows * a.topk), 2u * a.split_gu,
-                          gemv_smem_bytes(rm, rm, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu), a.overlap != 0, stream);
+                          gemv_smem_bytes(rm, rm, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu, a.alone_gu != 0), a.overlap != 0, stream);
 }
 
 cudaError_t T3_CAT(launch_moe_down_cb, T3_CB)(const MoeArgs& a, cudaStream_t stream) {
