@@ -712,15 +712,19 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     const uint32_t rm = slots > 8u * (size_t)a.experts && (a.experts + slots / 8u) * (a.inter / 128u) * 2u > one_wave() / 2u ? 16u : 8u;
     a.row_cap = rm;
     a.overlap = !cfg.no_overlap;
-    // The K splits depend on hidden and inter only (sized as if a row had eight slots), never on the row count, the top-k
-    // or the bank's size: a row-slot's summation order, hence its bytes, is the same alone and in a batch, and the same in
-    // a one-expert bank (a shared expert, an expert-parallel rank's share) as in the whole bank. A shared expert's chain,
-    // run on a second stream beside the routed chain, then launches the same cluster shapes as the routed one (measured:
-    // a 2-CTA-cluster launch beside 4- or 8-CTA-cluster launches costs a 1-row layer 7 us).
+    // The K splits depend on hidden and inter only (sized as if a row had eight slots), never on the row count or the top-k: a
+    // row-slot's summation order, hence its bytes, is the same alone and in a batch, and the same in every bank of two experts and more
+    // (an expert-parallel rank's share). A one-expert bank (a shared expert's) is cut as the dense linears it is, a few CTAs otherwise
+    // running all of K: its chain of 2048 x 512 at 1, 4 and 29 rows 17.7, 19.8 and 32.4 us -> 10.0, 10.8 and 18.4. The clamped entry keeps
+    // the banks' cut, since a banked call gives its bytes.
     constexpr uint32_t kNominalSlots = 8;
-    a.split_gu = pick_split(a.hidden / 128u, (a.inter / 128u) * kNominalSlots, 2u, 4u, one_wave() / 8u);
+    const uint32_t sms = one_wave() / 2u;
+    const bool dense = a.experts == 1u && !a.banked && a.limit <= 0.0f;
+    a.split_gu = dense ? pick_split(a.hidden / 128u, a.inter / 128u, 2u, 4u, sms)
+                       : pick_split(a.hidden / 128u, (a.inter / 128u) * kNominalSlots, 2u, 4u, one_wave() / 8u);
     a.slice_max_gu = largest_slice(a.hidden / 128u, a.split_gu);
-    a.split_d = pick_split(a.inter / 128u, (a.hidden / 128u) * kNominalSlots, 1u, 8u, one_wave() / 8u);
+    a.split_d = dense ? pick_split(a.inter / 128u, a.hidden / 128u, 1u, 8u, sms)
+                      : pick_split(a.inter / 128u, (a.hidden / 128u) * kNominalSlots, 1u, 8u, one_wave() / 8u);
     a.slice_max_d = largest_slice(a.inter / 128u, a.split_d);
     // sized for the widest row capacity so the split does not move with the rows either
     while (!plan_ring(32u, 32u, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu)) {
@@ -742,10 +746,11 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     // of 4096 x 1024 (64 and 64) 28.9 -> 23.3; against the rule 64 of 2048 x 2048 (128 and 64) 35.6 -> 40.9, 64 of 1024 x 256 (128
     // and 128) 16.1 -> 16.8, and past one wave (two rows and more of the first) 1 % the other way. A one-expert chain, whose
     // neighbour on the stream is another chain, keeps the late start (16 rows of 2048 x 512: 25.3 us against 31.8).
-    const uint32_t sms = one_wave() / 2u;
     const uint64_t gu = (uint64_t)2u * a.split_gu * (a.inter / 128u) * slots, down = (uint64_t)a.split_d * (a.hidden / 128u) * slots;
     a.down_early = a.experts > 1u && gu <= sms && (down > sms || gu + down <= sms);
-    a.alone_gu = 0;
+    // gate|up's CTAs a multiprocessor each where all find one (behind a launch of wider clusters they doubled up: a layer of one row with
+    // its shared expert ahead on the stream 43.9 us, 33.9 so)
+    a.alone_gu = gu <= sms;
     return T3_OK;
 }
 
