@@ -340,3 +340,24 @@ def test_bank_scales_that_are_not_signs():
         ref = ob.moe_rows(obank, x16[sample].astype(np.float32), inds[sample], scores[sample])
         check_moe(host_f32(y).reshape(rows, H)[sample], ref, "f16", ("general scales", rows))
     assert t3.device_error() == 0
+
+
+@pytest.mark.parametrize("dims", [(1920, 128, 48), (2048, 256, 36)])
+def test_down_ctas_that_take_several_blocks(dims):
+    """Calls that touch enough experts for a down CTA to run two output blocks and more (the last one's run cut short): the oracle's
+    rows, and each row's bytes alone, where a CTA runs one block."""
+    H, I, n = dims
+    E, topk, rows = 256, 16, 32
+    bank, obank = make_bank(1500 + n, E, H, I, n)
+    inds, scores = synth.routing(1501, rows, E, topk)
+    inds[:, 0] = 7  # more members than a CTA serves
+    x = dev(synth.activations(1502, rows, H)).view(1, rows, H)
+    di, ds = dev(inds).view(1, rows, topk), dev(scores).view(1, rows, topk)
+    y = t3.moe(x, bank, di, ds)
+    sample = [0, 9, 31]
+    ref = ob.moe_rows(obank, host_f32(x).reshape(rows, H)[sample], inds[sample], scores[sample])
+    check_moe(host_f32(y).reshape(rows, H)[sample], ref, "f16", ("several blocks", dims), terms=1.5)
+    for r in sample:
+        alone = t3.moe(x[:, r:r + 1].contiguous(), bank, di[:, r:r + 1].contiguous(), ds[:, r:r + 1].contiguous())
+        assert np.array_equal(bits16(alone).reshape(H), bits16(y).reshape(rows, H)[r]), r
+    assert t3.device_error() == 0

@@ -154,12 +154,13 @@ uint32_t largest_slice(uint32_t nb, uint32_t split) {
 
 // The ring of one GEMV CTA: stages of kStageRows tk rows (two 128-input blocks), as many as the slab needs or the budget
 // holds; three where the default budget holds fewer and two CTAs still fit a multiprocessor.
-bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan& ring, bool alone = false) {
+bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan& ring, bool alone = false,
+               uint32_t buffers = 1) {
     const uint32_t row_bytes = 16u * n, nrows = slice_max / 16u;  // nrows is a multiple of 8 (whole 128-blocks)
     const uint32_t stage_rows = kStageRows;
     const uint32_t stage_bytes = stage_rows * row_bytes;
-    const uint32_t need = (nrows + stage_rows - 1u) / stage_rows;
-    const uint32_t fixed = gemv_smem(row_cap, xrows, slice_max, cluster, stage_bytes, 0).total;
+    const uint32_t need = buffers * ((nrows + stage_rows - 1u) / stage_rows);
+    const uint32_t fixed = gemv_smem(row_cap, xrows, slice_max, cluster, stage_bytes, 0, buffers).total;
     if (fixed + stage_bytes > kSmemCap) return false;
     uint32_t budget = g_cfg.ring_bytes ? g_cfg.ring_bytes : kDefaultRing;
     if (!g_cfg.ring_bytes && !alone) {
@@ -198,8 +199,9 @@ int cuda_status(cudaError_t rc) { return rc == cudaSuccess ? T3_OK : T3_CUDA_ERR
 
 uint32_t row_cap_for(uint32_t rows) { return rows <= 8u ? 8u : (rows <= 16u ? 16u : 32u); }
 
-uint32_t gemv_smem_bytes(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan ring, bool alone) {
-    const uint32_t bytes = gemv_smem(row_cap, xrows, slice_max, cluster, ring.stage_rows * 16u * n, ring.stages).total + kSmemSlack;
+uint32_t gemv_smem_bytes(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan ring, bool alone,
+                         uint32_t buffers) {
+    const uint32_t bytes = gemv_smem(row_cap, xrows, slice_max, cluster, ring.stage_rows * 16u * n, ring.stages, buffers).total + kSmemSlack;
     return alone && bytes < kSmemAlone ? kSmemAlone : bytes;
 }
 
@@ -737,7 +739,14 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
         a.split_d *= 2u;
         a.slice_max_d = largest_slice(a.inter / 128u, a.split_d);
     }
-    if (!plan_ring(rm, rm, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu) || !plan_ring(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d))
+    // Output blocks of down a CTA takes in turn, where it runs all of K: as many, in powers of two, as leave the experts that the call
+    // touches (under uniform routing) ten CTAs a multiprocessor. 29 rows of 512 experts of 2048 x 512 266 us with one, 253 with two (what
+    // this gives), 255 with four; 32 rows of 128 of 4096 x 1024 436, 426, 440; with five CTAs a multiprocessor 64 of 7168 x 2048 lost 3 %.
+    const double touched = a.experts * (1.0 - std::exp(-(double)slots / a.experts));
+    a.per_d = 1u;
+    while (a.split_d == 1u && a.per_d < 8u && a.per_d * 2u <= a.hidden / 128u && touched * (a.hidden / 128u) / (2u * a.per_d) >= 10.0 * sms) a.per_d *= 2u;
+    if (!plan_ring(rm, rm, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu) ||
+        !plan_ring(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d, false, a.per_d > 1u ? 2u : 1u))
         return T3_ENGINE_NOT_IMPLEMENTED;
     // When gate|up lets the down launch start: at once (its CTAs then fetch their first codes beside gate|up's) or when its own codes
     // are all on the way. At once where gate|up leaves multiprocessors idle, unless down's CTAs would then double up on those while
@@ -865,12 +874,12 @@ int t3_plan_moe(size_t rows, int topk, const t3_bank* bank, t3_decode dec, t3_la
     std::snprintf(symbol, sizeof symbol, "t3_dec_down_%s_n%u_r%u", cb, named_rate(a.n), rm);
     if (topk == 1) {
         fill_launch(&out[1], symbol, "decode", dim3(a.split_d, a.hidden / 128u, slots), 32u * 17u,
-                    gemv_smem_bytes(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d), a.split_d,
+                    gemv_smem_bytes(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d, false, a.per_d > 1u ? 2u : 1u), a.split_d,
                     {T3_ROLE_HD, T3_ROLE_SLOTS, T3_ROLE_DOWN_T, T3_ROLE_DOWN_SVH, T3_ROLE_SCORES, T3_ROLE_Y});
         return 2;
     }
     fill_launch(&out[1], symbol, "decode", dim3(a.split_d, a.hidden / 128u, slots), 32u * 17u,
-                gemv_smem_bytes(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d), a.split_d,
+                gemv_smem_bytes(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d, false, a.per_d > 1u ? 2u : 1u), a.split_d,
                 {T3_ROLE_HD, T3_ROLE_SLOTS, T3_ROLE_DOWN_T, T3_ROLE_DOWN_SVH, T3_ROLE_ZD});
     fill_launch(&out[2], "t3_dec_merge", "decode", dim3((a.hidden + 255u) / 256u, a.rows, 1), 256u, 0u, 1u,
                 {T3_ROLE_ZD, T3_ROLE_SCORES, T3_ROLE_Y});

@@ -386,8 +386,37 @@ __device__ __forceinline__ void moe_gate_up_body(const MoeArgs& a) {
     }
 }
 
+// One finished row of the down projection, v of slot `slot`'s block hb, by one warp: the value the merge weights by the slot's score
+__device__ __forceinline__ void store_down(const MoeArgs& a, const float (&v)[4], uint32_t slot, uint32_t hb, uint32_t lane) {
+    const uint32_t H = a.hidden;
+    if (a.topk == 1u) {
+        // One slot a row: the merge has nothing to gather, so the weighted value (and the shared-expert add)
+        // is stored here and the merge launch is skipped. The arithmetic is the merge kernel's, 0 + w v included.
+        const float w = a.scores ? load_act(a.scores, a.score_dt, slot) : 1.0f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const size_t o = (size_t)slot * H + hb * 128u + lane + 32u * q;
+            float acc = __fadd_rn(0.0f, __fmul_rn(w, v[q]));
+            if (a.shared) {
+                store_act(a.y, a.y_dt, o, acc);
+                acc = __fadd_rn(load_act(a.y, a.y_dt, o), load_act(a.shared, a.y_dt, o));
+            }
+            store_act(a.y, a.y_dt, o, acc);
+        }
+        return;
+    }
+    __half* vo = static_cast<__half*>(a.v) + (size_t)slot * H + hb * 128u;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) vo[lane + 32u * q] = __float2half_rn(v[q]);
+}
+
 // grid (SD, hidden/128, row-slots), cluster (SD, 1, 1): the down projection of every member of the slot's expert from the
-// prepared rows hd, finished per row-slot into v (f16): the value the merge weights by the slot's score.
+// prepared rows hd, finished per row-slot into v (f16).
+//
+// Where one CTA runs all of K (SD 1), a CTA takes `a.per_d` output blocks in turn and the others of the grid's column leave at once: a
+// block of 512 inputs is a quarter of a microsecond's decode a warp, and finding the members, setting up and fetching the prepared rows
+// were a third of the instructions. The copy warp runs on into the next block's codes while the one before is finished, by a warp a row that moves
+// on from block to block.
 template <int N, int RM>
 __device__ __forceinline__ void moe_down_body(const MoeArgs& a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -395,9 +424,11 @@ __device__ __forceinline__ void moe_down_body(const MoeArgs& a) {
     __shared__ uint32_t s_masks[kMaxSlots / 32u];
     __shared__ uint16_t s_members[RM];
     cg::cluster_group cluster = cg::this_cluster();
-    const uint32_t rank = cluster.block_rank(), csize = a.split_d, hb = blockIdx.y, j = blockIdx.z;
+    const uint32_t csize = a.split_d, hb0 = blockIdx.y, j = blockIdx.z, rank = csize == 1u ? 0u : cluster.block_rank();
+    const bool own = csize == 1u;
+    if (own && hb0 % a.per_d != 0u) return;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t H = a.hidden, I = a.inter;
+    const uint32_t H = a.hidden, I = a.inter, blocks = own ? min(a.per_d, H / 128u - hb0) : 1u;
     // the routing was complete before the gate|up launch started, so it can be read ahead of pdl_wait
     const Members mem = find_members<RM>(a, j, s_members, s_masks);
     if (mem.skip) return;
@@ -408,20 +439,25 @@ __device__ __forceinline__ void moe_down_body(const MoeArgs& a) {
     const uint32_t nblk = b1 - b0, nrows = nblk * 8u;
     const uint32_t tile_bytes = 2u * a.n, row_bytes = 16u * a.n, out_tiles = H / 16u;
     const Ring rc{a.ring_d.stage_rows, a.ring_d.stages};
-    const CtaSmem c = carve(smem, gemv_smem(RM, RM, a.slice_max_d, csize, rc.stage_rows * row_bytes, rc.stages));
+    const GemvSmem L = gemv_smem(RM, RM, a.slice_max_d, csize, rc.stage_rows * row_bytes, rc.stages, a.per_d > 1u ? 2u : 1u);
+    const CtaSmem c = carve(smem, L);
     const uint32_t xstride = a.slice_max_d + kXpPad;
     init_barriers(c, rc.stages);
     __syncthreads();
 
     const size_t expert_bytes = (size_t)(I / 16u) * out_tiles * tile_bytes;
-    const uint8_t* wsrc = T3_BANK_FIELD(a, id, down_t) + e * expert_bytes + ((size_t)(b0 * 8u) * out_tiles + hb * 8u) * tile_bytes;
-    if (warp == 0) prefetch_l2(static_cast<const __half*>(T3_BANK_FIELD(a, id, down_svh)) + (size_t)e * H + hb * 128u, 256u, lane);
+    const uint8_t* wsrc = T3_BANK_FIELD(a, id, down_t) + e * expert_bytes + ((size_t)(b0 * 8u) * out_tiles + hb0 * 8u) * tile_bytes;
+    const __half* svh = static_cast<const __half*>(T3_BANK_FIELD(a, id, down_svh)) + (size_t)e * H + hb0 * 128u;
+    if (warp == 0) prefetch_l2(svh, blocks * 256u, lane);
     const uint32_t owned = rows_owned(RM, csize);
     RingPos pos;
     const uint32_t count = mem.count;
     if (warp == kConsumerWarps) {
-        produce_slab(c.ring, c.full, c.empty, wsrc, (size_t)out_tiles * tile_bytes, nrows, row_bytes, rc, pos, lane, a.err);
-        pdl_trigger();
+        for (uint32_t k = 0; k < blocks; ++k) {
+            produce_slab(c.ring, c.full, c.empty, wsrc + (size_t)k * 8u * tile_bytes, (size_t)out_tiles * tile_bytes, nrows, row_bytes, rc, pos, lane,
+                         a.err);
+            if (k == 0) pdl_trigger();
+        }
     } else {
         pdl_trigger();
         pdl_wait();  // hd is the gate|up launch's output
@@ -436,8 +472,33 @@ __device__ __forceinline__ void moe_down_body(const MoeArgs& a) {
             }
         }
         named_sync(1, kConsumerThreads);
-        gemv_and_push<N, RM>(cluster, c, nrows, a.n, a.mask, rc, xstride, count, pos, count, rank, csize, warp, lane, a.err);
+        const uint32_t tcol = warp & (kTileWarps - 1u), kg = warp / kTileWarps, tile = (L.recv - L.local) / 4u / (a.per_d > 1u ? 2u : 1u);
+#pragma unroll 1
+        for (uint32_t k = 0; k < blocks; ++k) {
+            float acc[RowCap<RM>::kMB][2][4] = {};
+            consume_slab<N, CB, RM>(c.ring, c.full, c.empty, nrows, a.n, a.mask, rc, c.xp, xstride, count, pos, tcol, kg, lane, acc, a.err);
+            // tiles by parity: a warp that is a block ahead writes the other one, and the barriers keep it from being two ahead
+            float *local = c.local + (k & 1u) * tile, *sums = c.recv + (k & 1u) * tile;
+            if (kg == 1) store_local<RM>(local, acc, tcol, lane);
+            named_sync(1, kConsumerThreads);
+            if (!own) {
+                if (kg == 0) push_partial<RM>(cluster, c.recv, local, acc, count, rank, csize, tcol, lane);
+                break;
+            }
+            if (kg == 0) keep_partial<RM>(sums, local, acc, count, tcol, lane);
+            named_sync(1, kConsumerThreads);
+            const uint32_t m = (warp + 16u - (5u * k & 15u)) & 15u;
+            if (m < count) {
+                float v[4], sv[4];
+                load_scales(svh + k * 128u, lane, sv);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = sums[m * kPartialStride + lane + 32u * q];
+                finish_block(v, sv, lane);
+                store_down(a, v, s_members[m], hb0 + k, lane);
+            }
+        }
     }
+    if (own) return;
     cluster_arrive();
     if (rank >= count) return;
     cluster_wait();
@@ -445,29 +506,10 @@ __device__ __forceinline__ void moe_down_body(const MoeArgs& a) {
         for (uint32_t i = warp; i * csize + rank < count; i += kConsumerWarps) {
             const uint32_t m = i * csize + rank;
             float v[4], sv[4];
-            load_scales(static_cast<const __half*>(T3_BANK_FIELD(a, id, down_svh)) + (size_t)e * H + hb * 128u, lane, sv);
+            load_scales(svh, lane, sv);
             gather_owned(c.recv, owned, i, 0, 1, csize, lane, v);
             finish_block(v, sv, lane);
-            const uint32_t slot = s_members[m];
-            if (a.topk == 1u) {
-                // One slot a row: the merge has nothing to gather, so the weighted value (and the shared-expert add)
-                // is stored here and the merge launch is skipped. The arithmetic is the merge kernel's, 0 + w v included.
-                const float w = a.scores ? load_act(a.scores, a.score_dt, slot) : 1.0f;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const size_t o = (size_t)slot * H + hb * 128u + lane + 32u * q;
-                    float acc = __fadd_rn(0.0f, __fmul_rn(w, v[q]));
-                    if (a.shared) {
-                        store_act(a.y, a.y_dt, o, acc);
-                        acc = __fadd_rn(load_act(a.y, a.y_dt, o), load_act(a.shared, a.y_dt, o));
-                    }
-                    store_act(a.y, a.y_dt, o, acc);
-                }
-                continue;
-            }
-            __half* vo = static_cast<__half*>(a.v) + (size_t)slot * H + hb * 128u;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) vo[lane + 32u * q] = __float2half_rn(v[q]);
+            store_down(a, v, s_members[m], hb0, lane);
         }
     }
 }
@@ -663,7 +705,7 @@ cudaError_t T3_CAT(launch_moe_down_cb, T3_CB)(const MoeArgs& a, cudaStream_t str
     const uint32_t rm = a.row_cap;
     KernelFn<MoeArgs> fn = T3_PICK(T3_PICK_16, t3_dec_down, a.n, rm);
     return launch_cluster(fn, a, dim3(a.split_d, a.hidden / 128u, a.rows * a.topk), a.split_d,
-                          gemv_smem_bytes(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d), a.overlap != 0, stream);
+                          gemv_smem_bytes(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d, false, a.per_d > 1u ? 2u : 1u), a.overlap != 0, stream);
 }
 
 #endif  // T3_SERVED

@@ -57,15 +57,16 @@ struct GemvSmem {
 __host__ __device__ inline uint32_t rows_owned(uint32_t rm, uint32_t cluster) { return (rm + cluster - 1u) / cluster; }
 // xrows: prepared rows held (the routed kernels hold a pass's row capacity; the dense linear only its live rows: the
 // tensor-core steps read a row past the last live one from the last live one, and nobody looks at what that gives)
+// buffers: partial-sum tiles, two where a CTA runs several output blocks (the next one's sums come in while one is finished)
 __host__ __device__ inline GemvSmem gemv_smem(uint32_t rm, uint32_t xrows, uint32_t slice_k, uint32_t cluster, uint32_t stage_bytes,
-                                              uint32_t stages) {
+                                              uint32_t stages, uint32_t buffers = 1) {
     GemvSmem s;
     s.bars = 0;
     s.xp = 2u * kMaxStages * 8u + 128u;  // the ring's full and empty barriers, then one for prepared rows copied in
     const uint32_t xp_bytes = xrows * (slice_k + kXpPad) * 2u;
     s.local = s.xp + ((xp_bytes + 127u) & ~127u);
-    s.recv = s.local + ((rm * kPartialStride * 4u + 127u) & ~127u);
-    s.ring = s.recv + ((cluster * rows_owned(rm, cluster) * kPartialStride * 4u + 127u) & ~127u);
+    s.recv = s.local + buffers * ((rm * kPartialStride * 4u + 127u) & ~127u);
+    s.ring = s.recv + buffers * ((cluster * rows_owned(rm, cluster) * kPartialStride * 4u + 127u) & ~127u);
     s.total = s.ring + stage_bytes * stages;
     return s;
 }
@@ -296,6 +297,21 @@ __device__ __forceinline__ void push_partial(cg::cluster_group& cluster, float* 
                 const uint32_t col = tcol * 16u + fragment_col<RM>(lane, e);
                 float* dst = cluster.map_shared_rank(recv, m % csize) + (rank * owned + m / csize) * kPartialStride;
                 dst[col] = acc[mb][nt][e] + local[m * kPartialStride + col];
+            }
+}
+
+// The same where no other CTA shares the rows: each live row's sums into this CTA's own tile
+template <int RM>
+__device__ __forceinline__ void keep_partial(float* sums, const float* local, const float (&acc)[RowCap<RM>::kMB][2][4], uint32_t count,
+                                             uint32_t tcol, uint32_t lane) {
+#pragma unroll
+    for (int mb = 0; mb < RowCap<RM>::kMB; ++mb)
+#pragma unroll
+        for (int nt = 0; nt < Frags<RM>::kNt; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const uint32_t m = fragment_row<RM>(lane, mb, nt, e), at = m * kPartialStride + tcol * 16u + fragment_col<RM>(lane, e);
+                if (m < count) sums[at] = acc[mb][nt][e] + local[at];
             }
 }
 

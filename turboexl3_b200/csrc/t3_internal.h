@@ -71,6 +71,7 @@ struct MoeArgs {
     uint32_t row_cap;                  // rows a CTA's decode of an expert's weights serves (8 or 16): an expert with more members takes more CTAs
     uint32_t split_gu, slice_max_gu;   // K slices of gate|up (cluster = 2 * split_gu), largest slice
     uint32_t split_d, slice_max_d;     // K slices of down
+    uint32_t per_d;                    // output blocks of down a CTA takes (1 unless split_d is)
     uint32_t alone_gu;                 // gate|up's CTAs take more than half a multiprocessor's shared memory each (see kSmemAlone)
     RingPlan ring_gu, ring_d;
     uint32_t down_early;               // gate|up lets the down launch start as soon as it has the routing (see plan_moe_decode)
@@ -130,7 +131,8 @@ cudaError_t launch_moe_down(const MoeArgs& a, int codebook, cudaStream_t stream)
 cudaError_t launch_moe_merge(const MoeArgs& a, cudaStream_t stream);
 
 // shared-memory bytes the GEMV CTAs of a plan need (for admission before launch)
-uint32_t gemv_smem_bytes(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan ring, bool alone = false);
+uint32_t gemv_smem_bytes(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan ring, bool alone = false,
+                         uint32_t buffers = 1);
 // the most dynamic shared memory a GEMV CTA may be launched with
 constexpr uint32_t kGemvSmemLimit = 200u * 1024u;
 uint32_t row_cap_for(uint32_t rows);
