@@ -200,7 +200,7 @@ __device__ __forceinline__ void load_16b(const void* p, bool wide, uint32_t (&w)
         w[0] = u.x, w[1] = u.y, w[2] = v.x, w[3] = v.y;
     }
 }
-__device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
+__host__ __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
 
 // The rotation proper of a block whose scales are signs that w holds already: H128, / sqrt(128), rounded to f16; in place
 __device__ __forceinline__ void scale_out(const float2 (&out)[8][2], uint32_t (&w)[4][4]) {

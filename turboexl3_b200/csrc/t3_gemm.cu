@@ -303,7 +303,34 @@ __device__ __forceinline__ void store_part(uint32_t buffer, uint16_t* y, size_t 
     }
 }
 
-// The same with each row's f16 values times its score (of the part's first row on), stored as the final sum of one slot a row stores
+// A part's rows by TMA, boxes of at least eight rows (a box starts where the 128-byte swizzle does), and what is left of it by the warp
+// (x: the part's first output, y: its first row in maps.out, at: that value's place in memory). Lane 0 keeps the copies as a bulk group.
+__device__ __forceinline__ void send_part(const GemmMaps& maps, uint32_t buffer, int x, int y, uint16_t* at, size_t N, uint32_t rows, uint32_t lane) {
+    const uint32_t whole = rows & ~7u;
+    if (lane == 0) {
+        uint32_t r = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < 5u; ++i) {
+            const uint32_t h = 128u >> i;
+            if (whole - r < h) continue;
+            tma_store_2d(&maps.out[i], x, y + (int)r, buffer + r * 128u);
+            tma_store_2d(&maps.out[i], x + 64, y + (int)r, buffer + 16384u + r * 128u);
+            r += h;
+        }
+        bulk_commit();
+    }
+    for (uint32_t i = lane; i < (rows - whole) * 16u; i += 32u) {
+        const uint32_t r = whole + (i >> 4), j = i & 15u;
+        uint4 w;
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w)
+                     : "r"(buffer + (j >> 3) * 16384u + r * 128u + (((j & 7u) ^ (r & 7u)) << 4)));
+        *reinterpret_cast<uint4*>(at + r * N + 8u * j) = w;
+    }
+    __syncwarp();
+}
+
+// store_part with each row's f16 values times its score (of the part's first row on), stored as the final sum of one slot a row stores
 // them: 0 + w v in f32, rounded once to y's dtype (y at the part's first value, element `at` of a.y)
 __device__ __forceinline__ void store_scored(uint32_t buffer, const DecodeGemmArgs& a, size_t first, size_t at, uint32_t rows, uint32_t warp, uint32_t lane) {
     const uint32_t j = lane & 15u;
@@ -350,8 +377,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
     const uint32_t acc_full = empty_b + 8u * 4u, acc_free = acc_full + 8u, all_free = acc_full + 16u;
     // z_full, rot_full: a pair each, one barrier a part of up to 128 columns
     const uint32_t z_full = acc_full + 24u, rot_full = acc_full + 40u;
+    // and with outputs by TMA: a part's values are in its buffer, its buffer is read
+    const uint32_t fin_full = acc_full + 56u, z_free = acc_full + 72u;
     uint8_t* generic = smem_raw + (smem - smem_addr(smem_raw));
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(generic + (acc_full + 56u - smem));
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(generic + (acc_full + 88u - smem));
     volatile uint32_t* dead = tmem_slot + 1;
 
     const uint32_t tid = threadIdx.x, lane = tid & 31u;
@@ -363,7 +392,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         for (uint32_t s = 0; s < kStages; ++s) init(full_a + 16u * s, kGroupWarps), init(full_a + 16u * s + 8u, 1u);
         for (uint32_t s = 0; s < kSlots; ++s) init(full_b + 8u * s, 1u), init(empty_b + 8u * s, 1u);
         init(acc_full, 1u), init(acc_free, kEpiWarps), init(all_free, kEpiWarps);
-        for (uint32_t c = 0; c < 2u; ++c) init(z_full + 8u * c, kEpiWarps), init(rot_full + 8u * c, 1u);
+        for (uint32_t c = 0; c < 2u; ++c) init(z_full + 8u * c, kEpiWarps), init(rot_full + 8u * c, 1u), init(fin_full + 8u * c, kEpiWarps), init(z_free + 8u * c, 1u);
         *dead = 0u;
         mbar_init_fence();
     }
@@ -526,8 +555,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         });
     } else if (warp == kRotWarp) {
         // ---- output rotation, a part at a time, once every epilogue warp's z is in the part's buffer (a warp of its own: the MMA warp
-        // is on the next unit by then)
+        // is on the next unit by then); then the finished parts' way out, where that is by TMA: the epilogue warps, which have a sixth of
+        // the issue slots beside the decode, are on to the next unit meanwhile
         uint32_t turns[2] = {0, 0};
+        uint16_t* const y16 = a.y ? static_cast<uint16_t*>(a.y) : reinterpret_cast<uint16_t*>(a.z);
         if (!sliced && a.svh[0] != nullptr) for_each_sub(a, [&](const Sub& s) {
             const uint32_t parts = s.parts();
 #pragma unroll
@@ -539,6 +570,22 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
                 const uint32_t to = tmem + s.rot_col(c), idesc = idesc_m128(s.part_cols(c));
                 if (elect_one()) rotate_part(tmem, to, z_s + c * kZBytes, idesc, rot_full + 8u * c);
             }
+            if (!a.bulk_out) return true;
+#pragma unroll
+            for (uint32_t c = 0; c < 2u; ++c) {
+                if (c >= parts) break;
+                wait_phase<32>(fin_full + 8u * c, (turns[c] - 1u) & 1u, dead, a.err, kErrMmaWait);
+                __syncwarp();
+                const uint32_t row = s.first + (s.wide ? 0u : 128u * c), x = (s.blk + (s.wide ? c : 0u)) * 128u;
+                send_part(maps, z_s + c * kZBytes, (int)x, (int)(s.op * a.op_rows + row), y16 + s.op * a.z_op_stride + (size_t)row * a.N + x, a.N,
+                          min(s.part_cols(c), s.rows - (s.wide ? 0u : 128u * c)), lane);
+            }
+            if (lane == 0) {
+                if (parts == 2u) bulk_wait_read<1>(), mbar_arrive_addr(z_free);
+                bulk_wait_read<0>();
+                mbar_arrive_addr(z_free + 8u * (parts - 1u));
+            }
+            __syncwarp();
             return true;
         });
     } else {
@@ -552,6 +599,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         const bool plain = KEPT && a.svh[0] == nullptr;
         uint16_t* const y16 = a.y ? static_cast<uint16_t*>(a.y) : reinterpret_cast<uint16_t*>(a.z);
         uint32_t subs = 0, rots = 0;  // rots: the next rotation's parity, a bit a part
+        const bool bulk = a.bulk_out != 0u && !plain;
         auto arrive = [&](uint32_t bar) {
             __syncwarp();
             if (lane == 0) mbar_arrive_addr(bar);
@@ -598,6 +646,10 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
             if (!plain) {
 #pragma unroll 1
                 for (uint32_t c = 0; c < parts; ++c) {
+                    if (bulk) {  // the buffer's last part has left
+                        wait_phase<32>(z_free + 8u * c, ((rots >> c) & 1u) ^ 1u, dead, a.err, kErrMmaWait);
+                        __syncwarp();
+                    }
                     z_part(my_lanes + s.part_col(c), s.part_cols(c), st_at + c * kZBytes);
                     if (c == 0u || !s.early) z_done(c);
                 }
@@ -622,12 +674,16 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
                     finish_part<true>(from, cols, s0, s1, dt, st_at + c * kZBytes, y32, a.N, s.rows - row0, t);
                 else
                     finish_part<false>(from, cols, s0, s1, dt, st_at + c * kZBytes, y32, a.N, s.rows - row0, t);
+                if (bulk) {
+                    proxy_fence();
+                    arrive(fin_full + 8u * c);
+                }
             }
             // everything is read
             tc_fence_before();
             if (!s.early) arrive(acc_free);
             arrive(all_free);
-            if (dt == (int)kF32) return true;
+            if (dt == (int)kF32 || bulk) return true;
             meet();
             for (uint32_t c = 0; c < parts; ++c) {
                 const uint32_t row0 = s.wide ? 0u : 128u * c;

@@ -15,6 +15,7 @@ constexpr uint32_t kGemmTileRows = 256;
 // The operands as TMA sees them
 struct GemmMaps {
     CUtensorMap rows[4];   // the prepared rows, f16 [rows, K]: boxes of 64 inputs x 256, 128, 64 and 32 rows (tiled_rows)
+    CUtensorMap out[5];    // with DecodeGemmArgs::bulk_out: the 16-bit outputs [rows, N], boxes of 64 outputs x 128, 64, 32, 16 and 8 rows
     CUtensorMap codes[2];  // a weight's (or bank's) codes as 64-bit words [expert, K / 16, N n / 64]: boxes of 4 tile rows x 8 tiles
 };
 
@@ -41,6 +42,7 @@ struct DecodeGemmArgs {
     size_t z_op_stride;
     void* y;
     int y_dt;
+    uint32_t bulk_out;          // 16-bit results leave by TMA (maps.out); y or z then starts on 16 bytes
     const void* scores;         // y only, or null: each row's f16 value times its score, as the final sum of one slot a row has it
     int score_dt;
     // K slices (dense, at least two, eight at most): a cluster of `ksplit` CTAs a unit, slice z running inputs 128 floor(K / 128 *

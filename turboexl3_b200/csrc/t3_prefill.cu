@@ -425,6 +425,13 @@ bool make_row_maps(GemmMaps* maps, const void* rows_base, uint64_t rows, uint32_
     return true;
 }
 
+// the outputs' maps (see GemmMaps::out), 16-bit [rows, N]
+bool make_out_maps(GemmMaps* maps, const void* base, uint64_t rows, uint32_t N) {
+    for (int i = 0; i < 5; ++i)
+        if (!make_a_map(&maps->out[i], base, rows, N, 128u >> i)) return false;
+    return true;
+}
+
 // the decode GEMM's maps: the prepared rows [rows, K] and the codes of one weight (experts 1) or bank, for up to two ops
 bool make_gemm_maps(GemmMaps* maps, const void* rows_base, uint64_t rows, uint32_t K, const void* op0, const void* op1, uint32_t N,
                     uint32_t n, uint32_t experts) {
@@ -549,6 +556,8 @@ cudaError_t launch_prefill_linear(const PrefillLinearArgs& p, int codebook, cuda
     d.ksplit = ksplit;
     d.part = reinterpret_cast<float*>(ws + up256((size_t)p.rows * p.in * 2u));  // a sliced call's slab, behind the prepared rows
     d.kept = p.resident != nullptr;
+    d.bulk_out = ksplit == 1u && p.x_dt != (int)kF32 && aligned16(p.y);
+    if (d.bulk_out && !make_out_maps(&maps, p.y, p.rows, p.out)) return cudaErrorNotSupported;
     d.err = p.err;
     // Overlapped, the GEMM's set-up and first codes run beside the prepare, which counts in a short call; in a long one the GEMM's
     // CTAs take the prepare's slots. Overlapped against not, 2048 -> 6144: 21.4 / 23.2 us at 520 rows, 51.5 / 52.8 at 2048, 71.1 / 71.3
@@ -714,6 +723,8 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
             GemmMaps maps;
             if (!make_gemm_maps(&maps, rows, rows_total, g.K, down ? t.down_t : t.gate_t, down ? nullptr : t.up_t, g.N, g.n, t.experts))
                 return cudaErrorNotSupported;
+            g.bulk_out = g.scores == nullptr;
+            if (g.bulk_out && !make_out_maps(&maps, g.z, (uint64_t)g.ops * S, g.N)) return cudaErrorNotSupported;
             const cudaError_t e = launch_decode_gemm(maps, g, (uint32_t)(units < (1u << 20) ? units : 1u << 20), codebook, stream);
             if (e != cudaSuccess) return e;
             *launches += 1;
