@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
     } else if (warp == kRowWarp) {
         // ---- row ring: 64 inputs of the tile's rows a slot. The rows are the previous kernel's output; the other roles' inputs
         // are not, so the codes stream in and the first stages decode while that kernel finishes.
-        pdl_wait();
+        if (!a.beside) pdl_wait();
         Ring<kSlots> ring;
         for_each_sub(a, [&](const Sub& s) {
             const int row0 = (int)(s.op * a.op_rows + s.first);
@@ -489,6 +489,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
             }
             return true;
         });
+        if (a.beside) pdl_wait();
     } else if (warp == kMmaWarp) {
         // ---- MMA: the whole warp walks the rings, one elected lane issues (see elect_one)
         uint32_t subs = 0;

@@ -56,6 +56,8 @@ struct DecodeGemmArgs {
     int overlap;                // launch with the programmatic-dependent-launch attribute: the rows (and nothing else that is read
                                 // here but weights and, routed, the tiles) are the stream's previous kernel's output, and that
                                 // kernel lets this one start only after its own wait
+    uint32_t beside;            // with overlap: the rows were complete before the stream's previous kernel (a GEMM of another bank on the
+                                // same rows) started, so they are not waited for; this kernel still ends after that one
 };
 
 // max_units: an upper bound of the launch's units of work (the kernel is persistent; a smaller grid serves a small call)

@@ -725,6 +725,9 @@ cudaError_t launch_prefill_moe(const MoeArgs& a, const MixedBanks* mixed, void* 
                 return cudaErrorNotSupported;
             g.bulk_out = g.scores == nullptr;
             if (g.bulk_out && !make_out_maps(&maps, g.z, (uint64_t)g.ops * S, g.N)) return cudaErrorNotSupported;
+            // A bank's CTAs start as the one's before it run out of units (the first bank's start after the rows are complete): three banks
+            // of 170 experts are five rounds each with the last half empty, 4096 rows of 512 experts at 2, 3 and 4 bits 728 -> 703 us
+            if (b > 0u) g.overlap = a.overlap, g.beside = a.overlap != 0;
             const cudaError_t e = launch_decode_gemm(maps, g, (uint32_t)(units < (1u << 20) ? units : 1u << 20), codebook, stream);
             if (e != cudaSuccess) return e;
             *launches += 1;
