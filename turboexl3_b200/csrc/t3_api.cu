@@ -473,11 +473,13 @@ struct DenseWs {
     size_t xp, part, counters, total;
 };
 // Whether a call's rows are rotated once by a launch of their own instead of inside every CTA: past kFusedRows rows always;
-// up to kFusedRows when a CTA's share of the work would be more than two rotations a warp (many rows on long K slices: each
-// CTA repeats the rotation of its whole slice for every row before its first tensor-core step).
+// up to kFusedRows when a CTA's share of the work would be more than five rotations a warp (many rows on long K slices: each
+// CTA repeats the rotation of its whole slice for every row before its first tensor-core step). Ahead / in the CTA, us: 8192 -> 2048 at 4
+// rows (2.8 rotations a warp) 12.7 / 11.2, 6144 -> 2048 at 8 (4) 10.4 / 9.8, 8192 -> 2048 at 8 (5.5) 12.8 / 12.6, 4096 -> 8192 at 8 (8)
+// 15.8 / 16.9.
 // On the global exchange always: the launch clears the blocks' arrival counters too (a memset ahead of the GEMV ended its overlap with
 // the stream's previous kernel: 16384 -> 7168 at one row 37.2 us, 34.8 without it).
-bool prep_ahead(const DenseArgs& a) { return a.part || a.rows > kFusedRows || a.rows * (a.slice_max / 128u) > 2u * kConsumerWarps; }
+bool prep_ahead(const DenseArgs& a) { return a.part || a.rows > kFusedRows || a.rows * (a.slice_max / 128u) > 5u * kConsumerWarps; }
 
 DenseWs dense_ws(uint32_t rows, uint32_t in, uint32_t out, uint32_t global_split, bool ahead) {
     DenseWs w;
