@@ -88,12 +88,10 @@ uint32_t one_wave() {
     return v;
 }
 
-// K slices for `units` independent (output block, job) pairs over nb 128-blocks of K: the smallest power of two, at most
-// `cap`, that brings the grid (units x slices x `fan` CTAs a slice) to `target` CTAs, never past one wave. A dense linear
-// aims at one CTA a multiprocessor (a second slot stays free for the next launch to start under this one); a routed call
-// aims at an eighth of a wave for a nominal row's slots, because its grid grows with the rows and longer CTAs amortise
-// their fixed part (measured on config 3: split 1 instead of 2 is as fast at 1 and 4 rows and 10 % faster at 16 and 32).
-// (Other counts work too, slices may differ by a block, but measured slower than the nearest power of two below them.)
+// K slices of a routed projection for `units` independent (output block, job) pairs over nb 128-blocks of K: the smallest power of two,
+// at most `cap`, that brings the grid (units x slices x `fan` CTAs a slice) to `target` CTAs, never past one wave. A bank's call aims
+// at an eighth of a wave for a nominal row's slots, because its grid grows with the rows and longer CTAs amortise
+// their fixed part (512 experts of 2048 x 512: one slice is as fast as two at 1 and 4 rows and 10 % faster at 16 and 32).
 uint32_t pick_split(uint32_t nb, uint32_t units, uint32_t fan, uint32_t cap, uint32_t target) {
     uint32_t s = 1;
     while (s * 2u <= nb && s * 2u <= cap && (uint64_t)units * fan * s < target && (uint64_t)units * fan * s * 2u <= one_wave())

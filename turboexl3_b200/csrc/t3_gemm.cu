@@ -7,23 +7,25 @@
 // proxy fence, and shared memory carries only the rows. The accumulator's columns are rows, so a tile is any multiple of 16
 // rows up to 256 and an expert of 80 rows costs five sixteenths of the MMA time of a 256-row one: nothing is padded to 128.
 //
-// What bounds it: a decoded 16x16 tile costs about 57 issued warp instructions (56.8 at K3, counted) whatever its rows, an MMA of 64 inputs x 128
-// outputs x R rows takes 2 R cycles, so up to about 200 rows a tile the decode's issue slots bound the kernel and past that the
-// tensor cores do. (An MMA that reads its A operand from tensor memory ran at the full rate from 128 columns on: 64 cycles at
+// What bounds it: a decoded 16x16 tile costs about 55 issued warp instructions at K3 and 44 at K4 whatever its rows, an MMA of 64 inputs x
+// 128 outputs x R rows takes 2 R cycles, so up to about 200 rows a tile the decode's issue slots bound the kernel and past that the
+// tensor cores do. Calls of thousands of rows run at the board's power limit (980 W, 1.4 to 1.8 GHz), where what a pass costs is its
+// energy: with the decode skipped 2048 -> 6144 at 4096 rows took 88 us of 117, with the rows' copies skipped 103. (An MMA that reads its A operand from tensor memory ran at the full rate from 128 columns on: 64 cycles at
 // 128, 128 at 256; with both operands in shared memory a 256-column one took 171.)
 //
 // One persistent CTA a multiprocessor, 28 warps by role (the rings run on across tiles, so nothing is set up per tile):
 //   warps 0-7    epilogue     warps 8-23  decode     24  codes: TMA into the code ring
-//   25  rows: TMA into the row ring     26  tcgen05.mma     27  tcgen05.mma of the output rotation
+//   25  rows: TMA into the row ring     26  tcgen05.mma     27  the output rotation's tcgen05.mma, finished tiles out by TMA
 // A ring stage is 64 weight tiles (64 tensor-memory columns), one of two shapes chosen per tile of rows:
 //   wide   two 128-output blocks x 64 inputs, up to 128 rows: both blocks read one copy of the rows
 //   deep   one block x 128 inputs, up to 256 rows
 // A decode warp takes eight tiles of every other stage: waits, fences and arrivals are paid once for the eight.
 //
 // Epilogue: the 128-point output rotation is a tensor-core product as well, D2 = H128 x z^T with H128 (+-1, f16) resident in
-// tensor memory: accumulators -> f16 z, transposed to shared memory by stmatrix -> MMA over the same columns -> scaled by svh,
-// rounded, transposed again and stored in 256-byte runs. (On the warps' mma.sync with butterflies a row cost four times the
-// instructions, and issue slots are what the decode needs.)
+// tensor memory: accumulators -> f16 z, transposed to shared memory by stmatrix -> MMA over the same columns, or free ones (Sub::early) ->
+// scaled by svh, rounded, transposed again and sent out by TMA or stored in 256-byte runs. (On the warps' mma.sync with butterflies a row
+// cost four times the instructions, and issue slots are what the decode needs.) From a 256-row tile's last MMA to the next tile's first took
+// 5900 cycles of 23300 and takes 4400 of 20400; of a routed pair of 80-row tiles (512 inputs) 6500 of 13400, now 3000 to 4000 of 10400.
 //
 // Every wait is bounded: one that runs out sets a bit of the device error word and a flag that ends every other role's waits,
 // and the CTA walks to its exit, freeing its tensor memory on the way.
