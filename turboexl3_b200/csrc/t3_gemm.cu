@@ -363,6 +363,31 @@ __device__ __forceinline__ void rotate_part(uint32_t tmem, uint32_t tmem_d, uint
     umma_commit(rot_full);
 }
 
+__device__ __forceinline__ void add_to(float2& a, float2 b) { a.x += b.x, a.y += b.y; }
+__device__ __forceinline__ void add_to(float4& a, float4 b) { a.x += b.x, a.y += b.y, a.z += b.z, a.w += b.w; }
+// Sums over `slices` (at most MOST) of `count` values `next` apart, in slice order; f(at, sums) gets those of values `at` ..
+template <uint32_t MOST, typename V, typename F>
+__device__ __forceinline__ void sum_slices(const float* slab, size_t next, uint32_t slices, uint32_t count, uint32_t tid, F&& f) {
+    constexpr uint32_t kAtOnce = 3, kWide = sizeof(V) / 4u;
+    for (uint32_t i0 = tid * kWide; i0 < count; i0 += kAtOnce * kThreads * kWide) {
+        V p[kAtOnce][MOST];
+#pragma unroll
+        for (uint32_t k = 0; k < kAtOnce; ++k)
+#pragma unroll
+            for (uint32_t z = 0; z < MOST; ++z)
+                if (z < slices && i0 + k * kThreads * kWide < count) p[k][z] = __ldcg(reinterpret_cast<const V*>(slab + z * next + i0 + k * kThreads * kWide));
+#pragma unroll
+        for (uint32_t k = 0; k < kAtOnce; ++k) {
+            if (i0 + k * kThreads * kWide >= count) break;
+            V sum = p[k][0];
+#pragma unroll
+            for (uint32_t z = 1; z < MOST; ++z)
+                if (z < slices) add_to(sum, p[k][z]);
+            f(i0 + k * kThreads * kWide, sum);
+        }
+    }
+}
+
 // KEPT: the weight is a kept W_hat (or W_std), [N, K] 16-bit, loaded by TMA beside the rows as a shared-memory operand: the
 // same products in the same order, nothing decoded.
 template <int NN, int CB, bool KEPT = false>
@@ -712,30 +737,21 @@ __global__ void __launch_bounds__(kThreads, 1) decode_gemm_kernel(const __grid_c
         Sub s = {};
         for_each_sub(a, [&](const Sub& mine) { s = mine; return true; });
         const uint32_t per = (s.rows + a.ksplit - 1u) / a.ksplit, lo = min(per * blockIdx.x, s.rows), live = min(per, s.rows - lo);
-        const float2* slab = reinterpret_cast<const float2*>(a.part) + ((size_t)s.blk * a.ksplit * a.dense_rows + s.first + lo) * 64u;
-        const size_t next = (size_t)a.dense_rows * 64u;
-        // three pairs of sums a thread and pass: a share of up to 42 rows is one round of loads
-        constexpr uint32_t kAtOnce = 3;
-        for (uint32_t i0 = tid; i0 < live * 64u; i0 += kAtOnce * kThreads) {
-            float2 p[kAtOnce][8];
-#pragma unroll
-            for (uint32_t k = 0; k < kAtOnce; ++k)
-#pragma unroll
-                for (uint32_t z = 0; z < 8u; ++z)
-                    if (z < a.ksplit && i0 + k * kThreads < live * 64u) p[k][z] = __ldcg(slab + z * next + i0 + k * kThreads);
-#pragma unroll
-            for (uint32_t k = 0; k < kAtOnce; ++k) {
-                const uint32_t i = i0 + k * kThreads, r = i >> 6, o = 2u * (i & 63u);
-                if (i >= live * 64u) break;
-                float2 sum = p[k][0];
-#pragma unroll
-                for (uint32_t z = 1; z < 8u; ++z)
-                    if (z < a.ksplit) sum.x += p[k][z].x, sum.y += p[k][z].y;
-                asm volatile("st.shared.b32 [%0], %1;" ::"r"(z_s + (o >> 6) * 16384u + r * 128u + ((((o & 63u) >> 3) ^ (r & 7u)) << 4) + (o & 7u) * 2u),
-                             "r"(pack_half2(sum.x, sum.y))
-                             : "memory");
-            }
-        }
+        const float* slab = a.part + ((size_t)s.blk * a.ksplit * a.dense_rows + s.first + lo) * 128u;
+        const size_t next = (size_t)a.dense_rows * 128u;
+        auto put = [&](uint32_t at, uint32_t w) {  // two rounded sums, values `at` and at + 1 of the share
+            const uint32_t r = at >> 7, o = at & 127u;
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(z_s + (o >> 6) * 16384u + r * 128u + ((((o & 63u) >> 3) ^ (r & 7u)) << 4) + (o & 7u) * 2u), "r"(w)
+                         : "memory");
+        };
+        // three loads a slice and thread at once: of two values of up to eight slices, or of four of up to four
+        if (a.ksplit > 4u)
+            sum_slices<8, float2>(slab, next, a.ksplit, live * 128u, tid, [&](uint32_t at, float2 v) { put(at, pack_half2(v.x, v.y)); });
+        else
+            sum_slices<4, float4>(slab, next, a.ksplit, live * 128u, tid, [&](uint32_t at, float4 v) {
+                put(at, pack_half2(v.x, v.y));
+                put(at + 2u, pack_half2(v.z, v.w));
+            });
         proxy_fence();
         __syncthreads();
         const uint32_t cols = (live + 15u) & ~15u;
