@@ -354,3 +354,14 @@ def test_gemm_of_few_rows_cuts_k_into_slices(case):
     assert np.array_equal(bits16(y[:few]), bits16(head))
     assert t3.device_error() == 0
 
+
+
+@pytest.mark.parametrize("in_dim,out_dim,n", [(2560, 9728, 64), (12288, 4608, 48), (13824, 5120, 32)])
+def test_a_wide_linears_row_alone_equals_the_row_in_a_batch(in_dim, out_dim, n):
+    """Shapes whose best cut for one row a CTA may not hold 32 rows of: the cut, hence a row's bytes, is one all the same."""
+    dec = t3.Decode(t3.MUL1)
+    trellis, suh, svh = (dev(a) for a in synth.linear(31, in_dim, out_dim, n))
+    x = torch.randn((32, in_dim), generator=torch.Generator().manual_seed(5)).half().cuda()
+    want = t3.linear(x, trellis, suh, svh, dec)
+    for rows in (1, 3, 8, 9, 17):
+        assert torch.equal(t3.linear(x[:rows], trellis, suh, svh, dec), want[:rows]), rows

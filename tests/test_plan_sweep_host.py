@@ -58,6 +58,53 @@ def test_dense_plans_are_launchable(codebook):
         assert lib().t3_linear_workspace_bytes(1, i, o, 64) == 0  # one row of a trunk-sized linear runs without a workspace
 
 
+def _large(i, o, n):
+    return i * o * n >= 24 * 1024 * 1024 * 128  # linears of 24 MB of codes and up: a rule of their own
+
+
+ONE_A_SM = [0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7]     # clusters of each size resident at once, a CTA a multiprocessor
+TWO_A_SM = {1: 296, 2: 148, 3: 88, 4: 71, 5: 50, 6: 45, 7: 37, 8: 33, 16: 14}  # and two, with those of three and five taken shorter
+
+
+def _slice_cost(i, o, n, s):
+    """Three times the time of a row plus that of 32 rows (10 ns) of `s` K slices, by the times a 128-input block takes; None where a CTA
+    cannot hold the prepared rows of 32 rows (200 KB, two CTAs a multiprocessor up to 113 KB; 128 bytes are kept for alignment)."""
+    nb, blocks, up = i // 128, o // 128, lambda v: (v + 127) // 128 * 128
+    longest = -(-nb // s)
+    stages = (longest + 1) // 2
+    rows, tile = up(32 * (longest * 128 + 16) * 2), 32 * 136 * 4
+    size = lambda least: 640 + max(rows, tile) + up(s * -(-32 // s) * 136 * 4) + 256 * n * min(stages, least)
+    if size(1) > SMEM_LIMIT - 128:
+        return None
+    single = blocks <= ONE_A_SM[s]
+
+    def rounds(at_once, block, last, fixed):
+        full, rest = divmod(blocks, at_once)
+        return full * (longest * block + fixed) + (longest * (last if rest <= ONE_A_SM[s] else block) + fixed if rest else 0)
+
+    row = rounds(ONE_A_SM[s], 58, 58, 300 + 10 * s) if single else rounds(TWO_A_SM[s], 116, 58, 300 + 10 * s)
+    if single or size(3) > 113 * 1024 - 128:
+        many = rounds(ONE_A_SM[s], 80, 80, 640 + 10 * s)
+    else:
+        many = rounds(TWO_A_SM[s], 260, 80, 640 + 10 * s)
+    return 3 * row + (many * 7 // 5 if size(2) > SMEM_LIMIT - 128 else many)
+
+
+def test_a_shape_has_one_slice_count_and_it_is_no_dearer_than_a_power_of_two():
+    """A row's bytes follow from how K is cut, so a dense linear under 24 MB of codes is cut the same way at every row count; and the
+    cut is never one that a power of two up to eight beats by the rule's own times (12288 -> 4608 once ran one row uncut: 64 us for 24)."""
+    outs = list(range(512, 16385, 512)) + [640, 896, 1408, 9728, 19456, 24576]
+    for i, o, n in itertools.product(list(range(512, 16385, 512)) + [640, 1920, 13952], outs, (16, 32, 48, 64, 80, 96, 128)):
+        if _large(i, o, n):
+            continue
+        counts = {t3.plan_linear(rows, i, o, n)[-1]["grid"][0] for rows in (1, 4, 8, 9, 16, 17, 32)}
+        assert len(counts) == 1, (i, o, n, counts)
+        own = _slice_cost(i, o, n, counts.pop())
+        for s in (1, 2, 4, 8):
+            if s <= i // 128 and (other := _slice_cost(i, o, n, s)) is not None:
+                assert own is not None and own <= other, (i, o, n, s)
+
+
 def test_routed_plans_are_launchable():
     geoms = [(8, 128, 128), (10, 512, 2048), (64, 2048, 512), (128, 2048, 768), (256, 7168, 2048), (32, 4096, 1536), (16, 1024, 4096)]
     for (experts, hidden, inter), n, rows, topk in itertools.product(geoms, [16, 48, 64, 128, 36], [1, 3, 8, 16, 32], [1, 2, 8, 10]):

@@ -56,6 +56,7 @@ constexpr uint32_t kSmemHalf = 113u * 1024u - kSmemSlack;     // and where two o
 // launch's duration. (A launch of another kind, with less, still fits beside it.)
 constexpr uint32_t kSmemAlone = 115u * 1024u;
 constexpr uint32_t kDefaultRing = 64u * 1024u;
+constexpr uint32_t kTile32 = 32u * kPartialStride * 4u;  // the partial-sum tile of row capacity 32
 
 uint32_t* dev_error_ptr() {
     int dev = 0;
@@ -97,30 +98,6 @@ uint32_t pick_split(uint32_t nb, uint32_t units, uint32_t fan, uint32_t cap, uin
     while (s * 2u <= nb && s * 2u <= cap && (uint64_t)units * fan * s < target && (uint64_t)units * fan * s * 2u <= one_wave())
         s *= 2u;
     return s;
-}
-
-// K slices of an ordinary dense linear of nb 128-input and `blocks` 128-output blocks, a cluster of s CTAs a block, and whether its CTAs
-// go one to a multiprocessor (`alone`). The time is the longest slice's: 0.58 us a 128-input block in a CTA that has its multiprocessor to
-// itself and 1.16 in one of two (whatever the rate), and about 0.1 us a CTA of the cluster. So: the count that is cheapest by that, alone
-// where all clusters fit one CTA to a multiprocessor, else two where they fit so; the most clusters of each size that do are
-// cudaOccupancyMaxActiveClusters's, written down because a row's bytes follow from the count and must be the same without a device.
-// One row, us, powers of two up to eight slices against this: 2048 -> 2048 5.3 / 4.7 (six, alone), 6144 -> 2048 10.1 / 7.5 (six), 7168 ->
-// 1536 10.7 / 6.8 (eight), 3072 -> 3072 7.0 / 6.2 (four), 2048 -> 6144 8.0 / 7.4 (two); at 17 rows 8.6 / 7.7, 15.6 / 12.6, 12.6 / 11.7, 10.9 /
-// 10.5, 12.8 / 12.6. Counts past four in the second case are the powers of two: others placed worse.
-// fits(s): a CTA holds the prepared rows of the widest call, so that calls of every row count take the same count.
-template <typename Fits>
-uint32_t pick_split_dense(uint32_t nb, uint32_t blocks, uint32_t& alone, Fits&& fits) {
-    static const uint16_t one[17] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7};
-    static const uint16_t two[17] = {0, 296, 148, 0, 71, 0, 0, 0, 33, 0, 0, 0, 0, 0, 0, 0, 14};
-    uint32_t best = 0, best_cost = ~0u;
-    alone = 0;
-    for (uint32_t s = 1; s <= 16u && s <= nb; ++s) {
-        const uint32_t longest = (nb + s - 1u) / s, single = blocks <= one[s];
-        if (!single && blocks > two[s]) continue;
-        const uint32_t cost = longest * (single ? 58u : 116u) + 10u * s + (single ? 0u : 30u);
-        if (cost < best_cost && (s == 1u || fits(s))) best = s, best_cost = cost, alone = single;
-    }
-    return best ? best : 1u;
 }
 
 // K slices of a LARGE dense linear (tens of megabytes of codes: milliseconds of integer work, so what counts is that
@@ -169,7 +146,10 @@ bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cl
             if (budget > kSmemHalf - fixed) budget = kSmemHalf - fixed;
         }
     }
-    if (budget > kSmemCap - fixed) budget = kSmemCap - fixed;
+    // (at row capacity 32 what the tile over the rows saves goes to a second stage, not to a third: 16384 -> 7168 at 32 rows 75.3 us with two,
+    // 77.7 with three)
+    const uint32_t most = kSmemCap - fixed, spared = local_over_rows(row_cap) ? kTile32 : 0u;
+    if (budget + spared > most) budget = 2u * stage_bytes + spared > most ? (2u * stage_bytes > most ? most : 2u * stage_bytes) : most - spared;
     uint32_t stages = budget / stage_bytes;
     stages = stages < 1u ? 1u : stages;
     stages = stages > need ? need : stages;
@@ -177,6 +157,11 @@ bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cl
     ring.stage_rows = stage_rows;
     ring.stages = stages;
     return true;
+}
+
+// Whether a CTA holds the prepared rows of `rows` rows of a slice, at row capacity `row_cap`, beside a partial-sum tile of its own and a stage
+bool holds_rows(uint32_t row_cap, uint32_t rows, uint32_t slice_max, uint32_t cluster, uint32_t n) {
+    return gemv_smem(row_cap, rows, slice_max, cluster, kStageRows * 16u * n, 1u).total + (local_over_rows(row_cap) ? kTile32 : 0u) <= kSmemCap;
 }
 
 bool dtype_ok(int dt) { return dt == T3_F32 || dt == T3_F16 || dt == T3_BF16; }
@@ -490,6 +475,48 @@ DenseWs dense_ws(uint32_t rows, uint32_t in, uint32_t out, uint32_t global_split
 
 bool large_linear(uint32_t in, uint32_t out, uint32_t n) { return (uint64_t)in * out * n >= (uint64_t)24u * 1024u * 1024u * 128u; }
 
+// K slices of an ordinary dense linear of nb 128-input and `blocks` 128-output blocks, a cluster of s CTAs a block, and whether its CTAs go
+// one to a multiprocessor (`alone`): one count a shape and rate, so that a row's bytes are the same alone and in a batch. Only counts whose
+// CTAs hold the prepared rows of 32 rows are asked, and the cheapest by its longest slice's time is taken, three times a row's and once that of
+// 32 rows. One row: 0.58 us a 128-input block in a CTA that has its multiprocessor to itself, 1.16 in one of two (whatever the rate), and 3 a
+// round; 32 rows: 0.8, 2.6 and 6.4, and two fifths more where the ring has one stage. Placement: alone where all clusters fit one CTA to a
+// multiprocessor (16 blocks a slice, alone / as they come: 12.8 / 20.3 us, up to the last cluster that fits); else in rounds of as many as fit
+// two to a multiprocessor, a last round that fits singly at the single rate; at 32 rows two fit only where their shared memory does. The
+// most clusters of each size are cudaOccupancyMaxActiveClusters's, less what clusters of three and five leave when they start beside others
+// (92 and 56 output blocks in them ran two rounds: 7.9 -> 9.3 and 13.1 -> 16.5 us), written down because the count must be the same
+// without a device; two to a multiprocessor past eight slices is known for sixteen.
+// us at 1 / 8 / 17 / 32 rows, powers of two up to eight -> this: 12288 -> 4608 K3 27.8 / 32.9 / 42.2 / 53.4 -> (six) 23.6 / 25.7 / 41.7 /
+// 42.8; 13824 -> 5120 K2 34.3 / 35.8 / 56.5 / 58.0 -> (six) 24.6 / 27.3 / 44.7 / 43.1; 10240 -> 4608 K4 22.9 / 28.6 / 35.7 / 43.8 -> (six) 19.6 /
+// 21.6 / 33.9 / 36.4; 2560 -> 9728 K4 15.3 / 18.7 / 22.5 / 29.1 -> (three) 12.3 / 15.0 / 19.1 / 24.6; one row of 2048 -> 2048 5.3 -> (six,
+// alone) 4.7, 6144 -> 2048 10.1 -> (six) 7.5, 7168 -> 1536 10.7 -> (eight) 6.8. The other way where no count that suits one row holds 32, which
+// is at K1 and K2: 6144 -> 14336 K2 31.0 / 32.6 / 53.3 / 68.3 -> (three) 33.9 / 41.6 / 54.1 / 61.1, 11264 -> 8704 K1 30.8 / 34.5 / 79 / 84 -> (five)
+// 40.2 / 48.2 / 61 / 66.
+uint32_t pick_split_dense(uint32_t nb, uint32_t blocks, uint32_t n, uint32_t& alone) {
+    static const uint16_t one[17] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7};
+    static const uint16_t two[17] = {0, 296, 148, 88, 71, 50, 45, 37, 33, 0, 0, 0, 0, 0, 0, 0, 14};
+    uint32_t best = 0, best_cost = ~0u;
+    alone = 0;
+    for (uint32_t s = 1; s <= 16u && s <= nb; ++s) {
+        const bool single = blocks <= one[s];
+        if (!single && !two[s]) continue;
+        const uint32_t longest = (nb + s - 1u) / s, at_once = single ? one[s] : two[s];
+        auto rounds = [&](uint32_t fit, uint32_t block, uint32_t block_single, uint32_t fixed) {  // in 10 ns
+            const uint32_t full = blocks / fit, rest = blocks - full * fit;
+            return full * (longest * block + fixed) + (rest ? longest * (rest <= one[s] ? block_single : block) + fixed : 0u);
+        };
+        const uint32_t row = rounds(at_once, single ? 58u : 116u, 58u, 300u + 10u * s);
+        if (3u * row >= best_cost) continue;
+        const uint32_t stage = kStageRows * 16u * n, stages = (longest * kBlockRows + kStageRows - 1u) / kStageRows;
+        const uint32_t held = gemv_smem(32u, 32u, longest * 128u, s, 0, 0).total;
+        if (held + stage > kSmemCap) continue;
+        const bool pair = !single && held + (stages < 3u ? stages : 3u) * stage <= kSmemHalf;
+        uint32_t rows = pair ? rounds(at_once, 260u, 80u, 640u + 10u * s) : rounds(one[s], 80u, 80u, 640u + 10u * s);
+        if (stages > 1u && held + 2u * stage > kSmemCap) rows = rows * 7u / 5u;
+        if (3u * row + rows < best_cost) best = s, best_cost = 3u * row + rows, alone = single;
+    }
+    return best;  // 0: no count holds 32 rows
+}
+
 // The launch shape of a dense linear at decode rows: the K split (cluster size) and the code ring. a.rows, in, out, n set.
 // global_ok: the call has its workspace, so a large linear may take the global exchange (a.part is set non-null as a mark;
 // the caller points it into the workspace).
@@ -497,12 +524,9 @@ int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     const uint32_t nb = a.in / 128u;
     const bool large = large_linear(a.in, a.out, a.n);
     a.alone = 0;
-    auto fits = [&](uint32_t s) {
-        RingPlan ring;
-        return plan_ring(32u, 32u, largest_slice(nb, s), s, a.n, ring);
-    };
     a.split = cfg.dense_split ? (cfg.dense_split < nb ? cfg.dense_split : nb)
-                              : (large ? pick_split_large(nb, a.out / 128u) : pick_split_dense(nb, a.out / 128u, a.alone, fits));
+                              : (large ? pick_split_large(nb, a.out / 128u) : pick_split_dense(nb, a.out / 128u, a.n, a.alone));
+    if (a.split == 0u) a.split = nb < 16u ? nb : 16u;
     a.part = nullptr;
     if (large && global_ok && !cfg.dense_split && !cfg.probe) {
         const uint32_t s = pick_split_global(nb, a.out / 128u, a.split);
@@ -513,8 +537,11 @@ int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     }
     a.overlap = !cfg.no_overlap;
     a.slice_max = largest_slice(nb, a.split);
-    // a slice too long for shared memory (its prepared rows) is cut further, up to the widest cluster
-    while (!plan_ring(row_cap_for(a.rows), a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0)) {
+    // A slice too long for shared memory (its prepared rows) is cut further, up to the widest cluster. A large linear's keeps room for a
+    // tile of its own: with what is left where it does not, one ring stage (8704 -> 13312 K6 at 17 rows in two slices 108 us, in four 81).
+    const uint32_t rm = row_cap_for(a.rows);
+    while ((large && !holds_rows(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n)) ||
+           !plan_ring(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0)) {
         if (a.part) {  // back to the cluster kernel
             a.part = nullptr;
             a.split = pick_split_large(nb, a.out / 128u);
@@ -729,12 +756,12 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
                       : pick_split(a.inter / 128u, (a.hidden / 128u) * kNominalSlots, 1u, 8u, one_wave() / 8u);
     a.slice_max_d = largest_slice(a.inter / 128u, a.split_d);
     // sized for the widest row capacity so the split does not move with the rows either
-    while (!plan_ring(32u, 32u, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu)) {
+    while (!holds_rows(32u, 32u, a.slice_max_gu, 2u * a.split_gu, a.n)) {
         if (a.split_gu * 2u > a.hidden / 128u || a.split_gu * 2u > 8u) return T3_ENGINE_NOT_IMPLEMENTED;
         a.split_gu *= 2u;
         a.slice_max_gu = largest_slice(a.hidden / 128u, a.split_gu);
     }
-    while (!plan_ring(32u, 32u, a.slice_max_d, a.split_d, a.n, a.ring_d)) {
+    while (!holds_rows(32u, 32u, a.slice_max_d, a.split_d, a.n)) {
         if (a.split_d * 2u > a.inter / 128u || a.split_d * 2u > 16u) return T3_ENGINE_NOT_IMPLEMENTED;
         a.split_d *= 2u;
         a.slice_max_d = largest_slice(a.inter / 128u, a.split_d);

@@ -71,6 +71,7 @@ __device__ __forceinline__ void gemv_and_push(cg::cluster_group& cluster, const 
     const uint32_t tcol = warp & (kTileWarps - 1u), kg = warp / kTileWarps;
     float acc[RowCap<RM>::kMB][2][4] = {};
     consume_slab<N, CB, RM, HB, WINDOWS>(c.ring, c.full, c.empty, nrows, n, mask, rc, c.xp, xstride, xrows, pos, tcol, kg, lane, acc, err);
+    if (local_over_rows(RM)) named_sync(1, kConsumerThreads);  // every warp has read the prepared rows
     if (kg == 1) store_local<RM>(c.local, acc, tcol, lane);
     named_sync(1, kConsumerThreads);
     if (kg == 0) push_partial<RM>(cluster, c.recv, c.local, acc, count, rank, csize, tcol, lane);
@@ -158,6 +159,7 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
             const uint32_t tcol = warp & (kTileWarps - 1u), kg = warp / kTileWarps;
             float acc[RowCap<RM>::kMB][2][4] = {};
             consume_slab<N, CB, RM, kDenseBatch, true>(c.ring, c.full, c.empty, nrows, a.n, a.mask, rc, c.xp, xstride, a.rows, pos, tcol, kg, lane, acc, a.err);
+            if (local_over_rows(RM)) named_sync(1, kConsumerThreads);
             if (kg == 1) store_local<RM>(c.local, acc, tcol, lane);
             named_sync(1, kConsumerThreads);
             if (kg == 0) {
