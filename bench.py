@@ -696,6 +696,7 @@ def run_ours(args) -> None:
     if rank == 0 and not args.quick:
         # the 21 linears with nothing ordering them
         try:
+            t3.configure(no_overlap=True, dense_split=args.dense_split)  # what t3_config says of many branches at once
             bgraphs = [graph_of(lambda c=c: step_branches(c)) for c in range(COPIES)]
             for s in range(3):
                 bgraphs[s % COPIES].replay()
@@ -707,9 +708,11 @@ def run_ours(args) -> None:
 
             us = time_us(replay_next, 30)
             extra["concurrent"] = {"value": round(STEP_BYTES / us / 1e3, 1), "unit": UNIT, "us_per_step": round(us, 1),
-                                   "what": "the step's 21 independent linears as parallel branches of one CUDA graph"}
+                                   "what": "the step's 21 independent linears as parallel branches of one CUDA graph (no_overlap)"}
         except Exception as exc:
             extra["concurrent"] = {"error": type(exc).__name__}
+        finally:
+            t3.configure(dense_split=args.dense_split)
         # per-linear device time: a graph of one launch per weight copy
         def per_linear():
             cases = {}

@@ -94,7 +94,10 @@ typedef struct {
     uint32_t ring_bytes;     /* shared-memory bytes a GEMV CTA's code ring may take; 0 = default */
     uint32_t dense_split;    /* K slices of a dense GEMV cluster (1..16); 0 = choose from the shape */
     int no_overlap;          /* 1: launches wait for the stream's previous kernel to finish before they start (no
-                                programmatic dependent launch); for measurements */
+                                programmatic dependent launch), and decode-row CTAs leave room for another launch's on their
+                                multiprocessor. For a program that keeps the device busy from four streams or graph branches and more (21
+                                linears side by side 1120 GB/s of code bytes, 845 without), and for measurements; one stream's
+                                launches are a seventh slower so. A row's bytes are the same either way */
     int probe;               /* timing probes only, never a served kernel (decode.Geometry.probe, src/core/decode.zig:34-35):
                                 t3_linear calls of up to 8 rows launch the dense GEMV with 1 the codebook hash skipped, 2 the
                                 window extraction skipped too, 3 nothing but the code stream (a stage is released as soon

@@ -105,6 +105,22 @@ def test_a_shape_has_one_slice_count_and_it_is_no_dearer_than_a_power_of_two():
                 assert own is not None and own <= other, (i, o, n, s)
 
 
+def test_launches_that_do_not_overlap_leave_room_for_another_streams():
+    """A decode-row launch that starts beside its predecessor keeps its multiprocessors to itself (more than half their shared memory, by
+    one CTA); with no_overlap two CTAs fit one again (228 KB, 1 KB a CTA reserved), in the same cut of K."""
+    shapes = [(2048, 2048), (2048, 6144), (6144, 2048), (3072, 3072), (7168, 1536)]
+    plans = lambda: [t3.plan_linear(1, i, o, n)[-1] for i, o in shapes for n in (16, 64, 128)] + [t3.plan_moe(1, 10, 512, 2048, 512, 48)[0]]
+    half = 228 * 1024 // 2 - 1024
+    apart = plans()
+    try:
+        t3.configure(no_overlap=True)
+        beside = plans()
+    finally:
+        t3.configure()
+    assert all(p["shared"] > half for p in apart) and all(p["shared"] <= half for p in beside)
+    assert [p["grid"] for p in apart] == [p["grid"] for p in beside]
+
+
 def test_routed_plans_are_launchable():
     geoms = [(8, 128, 128), (10, 512, 2048), (64, 2048, 512), (128, 2048, 768), (256, 7168, 2048), (32, 4096, 1536), (16, 1024, 4096)]
     for (experts, hidden, inter), n, rows, topk in itertools.product(geoms, [16, 48, 64, 128, 36], [1, 3, 8, 16, 32], [1, 2, 8, 10]):

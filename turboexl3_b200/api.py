@@ -199,7 +199,8 @@ def _trellis_ok(t: torch.Tensor) -> bool:
 
 def configure(prefill: bool = True, ring_bytes: int = 0, dense_split: int = 0, no_overlap: bool = False, probe: int = 0) -> None:
     """core.config.configure (src/core/config.zig:175): process-wide, before the first call. probe 1..3 swaps the dense
-    decode-row kernel for a timing probe (see t3_config in include/t3.h): measurements only."""
+    decode-row kernel for a timing probe (see t3_config in include/t3.h): measurements only. no_overlap: for decode-row calls that
+    keep four streams or graph branches busy at once; one stream is quicker without."""
     cfg = _Config(int(prefill), ring_bytes, dense_split, int(no_overlap), int(probe))
     _check(lib().t3_configure(C.byref(cfg)))
 

@@ -53,7 +53,10 @@ constexpr uint32_t kSmemCap = kGemvSmemLimit - kSmemSlack;  // what the carve-up
 constexpr uint32_t kSmemHalf = 113u * 1024u - kSmemSlack;     // and where two of them fit a multiprocessor (228 KB, 1 KB a CTA reserved)
 // What a CTA asks for so that no second one of its kind fits the multiprocessor. The hardware places the clusters of a launch that starts
 // beside its predecessor two CTAs to a multiprocessor while others stay empty, and a doubled CTA takes twice as long, which sets the
-// launch's duration. (A launch of another kind, with less, still fits beside it.)
+// launch's duration. (A launch of another kind, with less, still fits beside it.) Where launches do not start so (no_overlap) nothing of
+// the kind is asked for: other streams' launches may share the multiprocessors. The 21 linears of 2048 x 2048, 2048 x 6144 and 6144 x 2048 at
+// seven rates, one row, on 1 / 2 / 4 / 21 streams: 157 / 130 / 131 / 126 us overlapped and alone, 181 / 132 / 97 / 95 with no_overlap (and 236 / 126 /
+// 96 / 96 overlapped and not alone; 180 / 117 / 112 / 111 with the fewer slices a launch of before).
 constexpr uint32_t kSmemAlone = 115u * 1024u;
 constexpr uint32_t kDefaultRing = 64u * 1024u;
 constexpr uint32_t kTile32 = 32u * kPartialStride * 4u;  // the partial-sum tile of row capacity 32
@@ -527,6 +530,7 @@ int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     a.split = cfg.dense_split ? (cfg.dense_split < nb ? cfg.dense_split : nb)
                               : (large ? pick_split_large(nb, a.out / 128u) : pick_split_dense(nb, a.out / 128u, a.n, a.alone));
     if (a.split == 0u) a.split = nb < 16u ? nb : 16u;
+    if (cfg.no_overlap) a.alone = 0;  // see kSmemAlone
     a.part = nullptr;
     if (large && global_ok && !cfg.dense_split && !cfg.probe) {
         const uint32_t s = pick_split_global(nb, a.out / 128u, a.split);
@@ -786,7 +790,7 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     a.down_early = a.experts > 1u && gu <= sms && (down > sms || gu + down <= sms);
     // gate|up's CTAs a multiprocessor each where all find one (behind a launch of wider clusters they doubled up: a layer of one row with
     // its shared expert ahead on the stream 43.9 us, 33.9 so)
-    a.alone_gu = gu <= sms;
+    a.alone_gu = gu <= sms && a.overlap;
     return T3_OK;
 }
 
