@@ -205,10 +205,15 @@ uint32_t pair_ctas(size_t positions, uint32_t nblk) {
 // 256 threads. Dense and one-expert calls (where null): positions are the call's rows. Routed: position p reads row
 // where[p].x with the scales of its expert (where[p].y); the second op (up) reuses the row with its own suh.
 //
-// A quad keeps one 128-block and walks `chunk` consecutive positions: sorted positions share their expert in runs, so the block's
+// RUNS: a quad keeps one 128-block and walks `chunk` consecutive positions: sorted positions share their expert in runs, so the block's
 // scales are read once a run and kept as two words of signs. What bounds the kernel is L1: a 16-byte access of eight quads touches
 // eight lines, and of 24 accesses for a pair of ops eight were scales and four the row read twice. 40960 slots of 2048 x 2: 95 us (87 %
-// of L1's rate), 81 with the signs kept, 72 with the row kept in registers too (three CTAs a multiprocessor; with four it spilled).
+// of L1's rate), 81 with the signs kept, 72 with the row kept in registers too (three CTAs a multiprocessor; with four it spilled). Scales
+// that are not signs are read again for every position, which takes what it took without the runs: 114 us either way.
+// Else (one op, calls of a round or two of warps) a quad takes one (position, block) and nothing stands between its loads of the row and of
+// the scales. Linears, us, in the other form / this: 2048 -> 6144 at 520 rows 20.5 / 20.2, 3072 -> 3072 at 300 21.6 / 21.4, 6144 -> 2048 at
+// 400 22.9 / 22.4. (With registers for four CTAs a multiprocessor 20.5, 20.8 and 22.9, but 2048 -> 6144 at 128 17.4 -> 17.8. Two ops, which
+// would read the row twice, lose: 64 experts of 4096 x 1024 at 300 rows 233.0 / 234.2.)
 struct PrepArgs {
     const void* x;
     int x_dt;
@@ -220,21 +225,27 @@ struct PrepArgs {
     uint32_t topk;
     __half* xp;  // [ops][positions][K]
 };
+template <bool RUNS>
 __global__ void __launch_bounds__(256, 3) prep_rows_kernel(const __grid_constant__ PrepArgs a) {
     const uint32_t lane = threadIdx.x & 31u, q = lane & 3u, nblk = a.K >> 7;
-    const uint32_t units = (a.positions + a.chunk - 1u) / a.chunk * nblk;  // (the callers keep positions x width under 2^31)
+    const uint32_t chunk = RUNS ? a.chunk : 1u, units = (a.positions + chunk - 1u) / chunk * nblk;  // (the callers keep positions x width under 2^31)
     pdl_wait();
     pdl_trigger();  // after the wait: the GEMM that follows reads the tiles ahead of its own
     const bool wide_x = aligned16(a.x);
     const HadB hb = had_b(lane);
+    auto put = [&](const uint32_t (&w)[4][4], uint32_t op, uint32_t p, uint32_t col) {
+        uint4* o = reinterpret_cast<uint4*>(a.xp + ((size_t)op * a.positions + p) * a.K + col);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) o[4 * s] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+    };
     for (uint32_t u0 = (blockIdx.x * 8u + (threadIdx.x >> 5)) * 8u; u0 < units; u0 += gridDim.x * kPairsPerCta) {
         const uint32_t u = min(u0 + (lane >> 2), units - 1u), c = u / nblk, col = (u - c * nblk) * 128u + 8u * q;
         const bool mine = u0 + (lane >> 2) < units;
         uint32_t held = 0, signs[2] = {0u, 0u};  // the expert whose signs are held
         bool fresh = a.chunk > 1u, plain = fresh;  // (with one position a quad there is nothing to keep)
 #pragma unroll 1
-        for (uint32_t i = 0; i < a.chunk; ++i) {
-            const uint32_t at = c * a.chunk + i, p = min(at, a.positions - 1u);
+        for (uint32_t i = 0; i < chunk; ++i) {
+            const uint32_t at = c * chunk + i, p = min(at, a.positions - 1u);
             uint32_t row, id = 0;
             if (a.where) {
                 const uint2 w = a.where[p];
@@ -244,6 +255,15 @@ __global__ void __launch_bounds__(256, 3) prep_rows_kernel(const __grid_constant
             }
             const size_t scale_at = (size_t)a.ids.expert(id) * a.K + col;
             const uint32_t bank = a.ids.bank(id);
+            if (!RUNS) {
+                const __half* sp = a.suh[0][bank] + scale_at;
+                uint32_t w[4][4];
+#pragma unroll
+                for (int s = 0; s < 4; ++s) load_half8(a.x, a.x_dt, wide_x, (size_t)row * a.K + col + 32u * s, w[s]);
+                rotate_block(w, sp, aligned16(sp), hb);
+                if (mine) put(w, 0u, p, col);
+                continue;
+            }
             if (a.chunk > 1u && __any_sync(0xFFFFFFFFu, fresh || id != held)) {
                 uint32_t odd = 0;
                 for (uint32_t op = 0; op < a.ops; ++op) {
@@ -272,11 +292,7 @@ __global__ void __launch_bounds__(256, 3) prep_rows_kernel(const __grid_constant
                     const __half* sp = (op ? a.suh[1][bank] : a.suh[0][bank]) + scale_at;
                     rotate_block(w, sp, aligned16(sp), hb);
                 }
-                if (mine && at < a.positions) {
-                    uint4* o = reinterpret_cast<uint4*>(a.xp + ((size_t)op * a.positions + p) * a.K + col);
-#pragma unroll
-                    for (int s = 0; s < 4; ++s) o[4 * s] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
-                }
+                if (mine && at < a.positions) put(w, op, p, col);
             }
         }
     }
@@ -285,7 +301,7 @@ __global__ void __launch_bounds__(256, 3) prep_rows_kernel(const __grid_constant
 cudaError_t launch_prep(PrepArgs& pa, bool overlap, cudaStream_t stream) {
     const size_t pairs = (size_t)pa.positions * (pa.K / 128u), chunk = pairs / ((size_t)one_wave_ctas() * 32u * 8u * 2u);
     pa.chunk = (uint32_t)(chunk < 1u ? 1u : chunk > 8u ? 8u : chunk);
-    return launch_overlapped(prep_rows_kernel, dim3(pair_ctas((pa.positions + pa.chunk - 1u) / pa.chunk, pa.K / 128u)), 256, 0, stream, overlap, 1, pa);
+    return launch_overlapped(pa.chunk > 1u || pa.ops > 1u ? prep_rows_kernel<true> : prep_rows_kernel<false>, dim3(pair_ctas((pa.positions + pa.chunk - 1u) / pa.chunk, pa.K / 128u)), 256, 0, stream, overlap, 1, pa);
 }
 
 __device__ __forceinline__ float swiglu_f32(float g, float u, float limit, int clamp_at) {
