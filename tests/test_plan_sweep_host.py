@@ -4,8 +4,11 @@ needs to be a valid one (cluster, shared memory, grid) checked from the plan alo
 The reference plans its launches from the shape as well (src/hip/plan.zig, src/core/partition.zig:1-80); the splits here
 are this library's own, so the properties are the ones any split must have.
 """
+import ctypes
 import itertools
+import os
 import re
+import subprocess
 
 import pytest
 
@@ -103,6 +106,20 @@ def test_a_shape_has_one_slice_count_and_it_is_no_dearer_than_a_power_of_two():
         for s in (1, 2, 4, 8):
             if s <= i // 128 and (other := _slice_cost(i, o, n, s)) is not None:
                 assert own is not None and own <= other, (i, o, n, s)
+
+
+def test_a_smaller_device_holds_its_share_of_the_clusters(tmp_path):
+    """The clusters resident at once are written down for 148 multiprocessors: on a device (or a share of one) with fewer, a launch that
+    counts on a multiprocessor a CTA has no more clusters than their share."""
+    so = str(tmp_path / "split.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", os.path.join(os.path.dirname(__file__), "host_emul", "split_emul.cpp"), "-o", so],
+                   check=True)
+    split = ctypes.CDLL(so).split_emul
+    for sms, nb, blocks in itertools.product((148, 132, 74, 18), (4, 16, 48, 128), range(1, 200)):
+        s, alone = split(sms, nb, blocks) % 100, split(sms, nb, blocks) >= 100
+        assert 1 <= s <= min(nb, 16)
+        assert not alone or blocks <= ONE_A_SM[s] * sms // 148, (sms, nb, blocks, s)
+    assert split(148, 16, 16) == 106 and split(74, 16, 16) != 106  # 2048 -> 2048: sixteen clusters of six take 96 multiprocessors
 
 
 def test_launches_that_do_not_overlap_leave_room_for_another_streams():
