@@ -361,3 +361,28 @@ def test_down_ctas_that_take_several_blocks(dims):
         alone = t3.moe(x[:, r:r + 1].contiguous(), bank, di[:, r:r + 1].contiguous(), ds[:, r:r + 1].contiguous())
         assert np.array_equal(bits16(alone).reshape(H), bits16(y).reshape(rows, H)[r]), r
     assert t3.device_error() == 0
+
+
+def test_an_expert_alone_in_its_bank_is_cut_as_a_linear():
+    """Decode rows: banks of two experts and more cut K one way, so an expert's bytes are the same in each of them; a one-expert bank is
+    cut as the dense linears it is, with bytes of its own within the order of the f32 sums, except under a clamp, where it keeps the
+    banks' cut. Either way a row's bytes are the same alone and in a batch."""
+    H, I, n = 2048, 512, 48
+    arrs = synth.bank(3140, 3, H, I, n)
+    bank = lambda e: t3.Bank(*(t3.Proj(*(dev(arrs[p + f][:e]) for f in ("_t", "_suh", "_svh"))) for p in ("gate", "up", "down")))
+    obank = ob.Bank(3, H, I, n, *[arrs[p + f] for p in ("gate", "up", "down") for f in ("_t", "_suh", "_svh")])
+    dec, (one, two, three) = t3.Decode.mul1, (bank(e) for e in (1, 2, 3))
+    x16 = synth.activations(3141, 32, H)
+    x = dev(x16)
+    full = {}
+    for rows in (32, 17, 8, 1):
+        xr, ids, ones = x[:rows].view(1, rows, H), torch.zeros((1, rows, 1), dtype=torch.int32, device="cuda"), torch.ones((1, rows, 1), device="cuda")
+        y = {k: bits16(t3.moe(xr, b, ids, ones, dec)).reshape(rows, H) for k, b in (("one", one), ("two", two), ("three", three))}
+        y["clamped"] = bits16(t3.moe_swiglu(xr, one, ids, ones, dec, 100)).reshape(rows, H)  # a clamp nothing reaches
+        assert np.array_equal(y["two"], y["three"]) and np.array_equal(y["two"], y["clamped"]), rows
+        ref = ob.moe_rows(obank, x16[:rows].astype(np.float32), np.zeros((rows, 1), np.int32), np.ones((rows, 1), np.float32))
+        for k in ("one", "two"):
+            full.setdefault(k, y[k])
+            assert np.array_equal(full[k][:rows], y[k]), (k, rows)
+            check_moe(y[k].view(np.float16).astype(np.float32), ref, "f16", ("one expert's bank", k, rows))
+    assert t3.device_error() == 0

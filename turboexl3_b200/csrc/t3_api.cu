@@ -701,15 +701,19 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     // expert with more is served by several CTAs at once, and those are quicker than one of a larger capacity, whose every tile costs the
     // tensor-core steps and the shared memory of all its rows). us at capacity 8 / 16 / 32: 64 experts of 7168 x 2048 at 2 members
     // an expert 824 / 1179 / 1350, at 4 1104 / 1585 / 1790; 32 of 4096 x 1024 at 6 225 / 253 / 311; 64 of 2048 x 512 at 5 121 / 130 / 145;
-    // 32 of 2048 x 512 at 10 107 / 87 / 93; one expert's 32 rows 32.6 / 32.0 / 47.3. A row's bytes do not depend on it.
+    // 32 of 2048 x 512 at 10 107 / 87 / 93; one expert's 32 rows 32.6 / 32.0 / 47.3. Skewed routing does not turn it: 32 rows of top-8
+    // with one expert in none, 12, 16 and all of the rows, capacity 8 / 16, 64 experts of 2048 x 512 107 / 125, 108 / 124, 109 / 124, 115 /
+    // 125; 128 of 2048 x 768 205 / 246 .. 202 / 239; 64 of 4096 x 1024 335 / 423 .. 343 / 424; 64 of 7168 x 2048 1081 / 1544 .. 1121 / 1539.
+    // A row's bytes do not depend on it.
     const uint32_t rm = slots > 8u * (size_t)a.experts && (a.experts + slots / 8u) * (a.inter / 128u) * 2u > one_wave() / 2u ? 16u : 8u;
     a.row_cap = rm;
     a.overlap = !cfg.no_overlap;
     // The K splits depend on hidden and inter only (sized as if a row had eight slots), never on the row count or the top-k: a
     // row-slot's summation order, hence its bytes, is the same alone and in a batch, and the same in every bank of two experts and more
     // (an expert-parallel rank's share). A one-expert bank (a shared expert's) is cut as the dense linears it is, a few CTAs otherwise
-    // running all of K: its chain of 2048 x 512 at 1, 4 and 29 rows 17.7, 19.8 and 32.4 us -> 10.0, 10.8 and 18.4. The clamped entry keeps
-    // the banks' cut, since a banked call gives its bytes.
+    // running all of K: its chain of 2048 x 512 at 1, 4 and 29 rows 17.7, 19.8 and 32.4 us -> 10.0, 10.8 and 18.4. So an expert alone in its
+    // bank (an expert-parallel rank's only one, a rate's only one in a mixed layer) gives bytes of its own, within the f32 order of the sums. A
+    // call with a clamp keeps the banks' cut, since a banked call gives its bytes.
     constexpr uint32_t kNominalSlots = 8;
     const uint32_t sms = one_wave() / 2u;
     const bool dense = a.experts == 1u && !a.banked && a.limit <= 0.0f;

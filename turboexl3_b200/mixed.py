@@ -5,7 +5,8 @@ bank's geometry carries a single rate: src/core/decode.zig Geometry.rate), so a 
 different bit widths is held as one sub-bank per rate. This module routes such a layer: every row-slot goes to the sub-bank
 that holds its expert (the finished down projection `v`, f16, exactly what the single-bank chain feeds its merge), and the
 score-weighted sum runs once over all slots in slot order — so the result is the one a single bank of those experts would
-give, whatever the bucketing. Past 32 rows the whole layer is one native call (`api.moe_mixed`); decode rows, more than eight
+give, whatever the bucketing (an expert that is its rate's only one has, at decode rows, the sums of a bank of one, which is cut
+like a dense linear: the same within their f32 order). Past 32 rows the whole layer is one native call (`api.moe_mixed`); decode rows, more than eight
 rates, banks that are empty or differ in their inner width, and injected stand-ins run each sub-bank's slots at top-1 with
 score 1 and merge with `t3.moe_merge`.
 """

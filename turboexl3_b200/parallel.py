@@ -7,7 +7,8 @@ The reference runs on a single device and has no counterpart to this file. The p
   received (top-1, score 1: the finished down projection `v`, f16), the `v` rows travel back (all-to-all "combine"), and
   the home rank does the score-weighted sum in slot order (`t3.moe_merge`). The weighted sum happens at home in the same
   order whatever G is, so the result does not depend on the number of ranks beyond the kernels' own path choice
-  (decode-row chain up to 32 received rows, prefill chain past that).
+  (decode-row chain up to 32 received rows, prefill chain past that; a rank that owns one expert cuts its decode rows like a
+  dense linear's).
 * Dense trunk linears, column-sharded at 128-column granularity: the output rotation and svh are per 128-output block and
   the input rotation depends on x only, so a rank computes complete output columns with no partial sums; shards are
   gathered with an all-gather.
