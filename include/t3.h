@@ -121,10 +121,12 @@ int t3_dequant(const void* trellis, int in_dim, int out_dim, int n, t3_decode de
  * decoders, out[cw] = f16 bits (device pointer to 65,536 uint16). */
 int t3_codebook_table(t3_decode dec, void* out, void* stream);
 
-/* root.linear (src/root.zig:309-351): y [rows, out] in x's dtype for x [rows, in]. `workspace` may be null when
- * t3_linear_workspace_bytes returns 0 for the call (up to 8 rows). For 9 to 32 rows the workspace (rows x in f16, 256-byte
- * aligned) is OPTIONAL: with it the rows are rotated once by a launch of their own ahead of the GEMV, without it every CTA
- * rotates its own copy; the same bytes either way. Past 32 rows it is required (256-byte aligned): the prepared rows, and
+/* root.linear (src/root.zig:309-351): y [rows, out] in x's dtype for x [rows, in]. Up to 32 rows the workspace
+ * (256-byte aligned) is OPTIONAL, and t3_linear_workspace_bytes is 0 for most calls of up to 8 rows on linears under 24 MB of codes.
+ * With it, past 8 rows and where a CTA's slice is long, the rows are rotated once by a launch of their own (rows x in f16), else every
+ * CTA rotates its own copy: the same bytes either way. On linears of 24 MB and more it also holds the K slices' partial sums and
+ * arrival counters, at every row count; without it, or with one smaller than the call asks for, such a linear takes the slower cluster
+ * kernel, whose K may be cut otherwise (the sums' f32 order differs). Past 32 rows it is required (256-byte aligned): the prepared rows, and
  * for calls of up to 512 rows on a linear with few 128-column blocks the partial sums of the K slices such a call is cut
  * into (the slices meet there; the slice counts of the two arms, 33..256 and 257..512 rows, follow in and out alone, so a
  * row's bytes do not depend on the row count within an arm, nor past 512 rows). */

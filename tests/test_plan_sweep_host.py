@@ -147,7 +147,7 @@ def test_routed_plans_are_launchable():
         slots = rows * topk
         assert len(chain) == (2 if topk == 1 else 3), (experts, hidden, inter, n, rows, topk)
         gu, down = chain[0], chain[1]
-        assert re.fullmatch(r"t3_dec_gate_up_mul1_n\d+_r(8|16|32)", gu["symbol"]) and re.fullmatch(r"t3_dec_down_mul1_n\d+_r(8|16|32)", down["symbol"])
+        assert re.fullmatch(r"t3_dec_gate_up_mul1_n\d+_r(8|16)", gu["symbol"]) and re.fullmatch(r"t3_dec_down_mul1_n\d+_r(8|16)", down["symbol"])
         for l, blocks, k_blocks in ((gu, inter // 128, hidden // 128), (down, hidden // 128, inter // 128)):
             gx, gy, gz = l["grid"]
             assert (gy, gz) == (blocks, slots) and l["group"] == "decode" and l["block"] == 544

@@ -547,9 +547,9 @@ size_t linear_workspace(size_t rows, int in_dim, int out_dim, int n, bool far_x)
     if (in_dim <= 0 || out_dim <= 0 || rows < 1) return 0;
     if (rows > T3_DECODE_ROWS_MAX) return prefill_linear_workspace(rows, (uint32_t)in_dim, (uint32_t)out_dim);
     if (in_dim % 128 != 0 || out_dim % 128 != 0 || !rate_ok(n)) return 0;
-    // Decode rows. Up to 8 rows of an ordinary linear: nothing (the kernel keeps everything on chip). 9 to 32 rows: the rows
-    // rotated once ahead of the GEMV. Linears of 24 MB of codes and up: the K slices' partial sums, when a slice count that
-    // fills the multiprocessors evenly exists for the shape. All optional: a call without it takes the cluster kernel.
+    // Decode rows. Up to 8 rows of an ordinary linear: nothing, unless its K slices are long (see prep_ahead). 9 to 32 rows: the rows
+    // rotated once ahead of the GEMV. Linears of 24 MB of codes and up, where a slice count that fills the multiprocessors evenly
+    // exists for the shape: the rotated rows and the K slices' partial sums. All optional: a call without it takes the cluster kernel.
     const t3_config cfg = config();
     DenseArgs a = {};
     a.in = (uint32_t)in_dim, a.out = (uint32_t)out_dim, a.n = (uint32_t)n, a.rows = (uint32_t)rows;

@@ -7,11 +7,11 @@
 // proxy fence, and shared memory carries only the rows. The accumulator's columns are rows, so a tile is any multiple of 16
 // rows up to 256 and an expert of 80 rows costs five sixteenths of the MMA time of a 256-row one: nothing is padded to 128.
 //
-// What bounds it: a decoded 16x16 tile costs about 55 issued warp instructions at K3 and 44 at K4 whatever its rows, an MMA of 64 inputs x
-// 128 outputs x R rows takes 2 R cycles, so up to about 200 rows a tile the decode's issue slots bound the kernel and past that the
-// tensor cores do. Calls of thousands of rows run at the board's power limit (980 W, 1.4 to 1.8 GHz), where what a pass costs is its
-// energy: with the decode skipped 2048 -> 6144 at 4096 rows took 88 us of 117, with the rows' copies skipped 103. (An MMA that reads its A operand from tensor memory ran at the full rate from 128 columns on: 64 cycles at
-// 128, 128 at 256; with both operands in shared memory a 256-column one took 171.)
+// What bounds it: a decoded 16x16 tile costs about 55 issued warp instructions, epilogue and waits included (55.3 of a routed gate|up at K3, 55.2
+// of 2048 -> 6144 at K4; 67 of a routed down, whose units are 512 inputs), an MMA of 64 inputs x 128 outputs x R rows takes 2 R cycles,
+// so up to about 200 rows a tile the decode's issue slots bound the kernel and past that the tensor cores do. Calls of thousands of rows run at the board's power limit (980 W, 1.4 to 1.8 GHz), where what a pass costs is its
+// energy: with the decode skipped 2048 -> 6144 at 4096 rows took 88 us of 117, with the rows' copies skipped 103. (An MMA that
+// reads its A operand from tensor memory ran at the full rate from 128 columns on: 64 cycles at 128, 128 at 256; with both operands in shared memory a 256-column one took 171.)
 //
 // One persistent CTA a multiprocessor, 28 warps by role (the rings run on across tiles, so nothing is set up per tile):
 //   warps 0-7    epilogue     warps 8-23  decode     24  codes: TMA into the code ring
