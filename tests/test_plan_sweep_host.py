@@ -76,7 +76,7 @@ def _slice_cost(i, o, n, s):
     longest = -(-nb // s)
     stages = (longest + 1) // 2
     rows, tile = up(32 * (longest * 128 + 16) * 2), 32 * 136 * 4
-    size = lambda least: 640 + max(rows, tile) + up(s * -(-32 // s) * 136 * 4) + 256 * n * min(stages, least)
+    size = lambda least: 640 + rows + (0 if longest >= 4 else tile) + up(s * -(-32 // s) * 136 * 4) + 256 * n * min(stages, least)
     if size(1) > SMEM_LIMIT - 128:
         return None
     single = blocks <= ONE_A_SM[s]

@@ -60,7 +60,7 @@ constexpr uint32_t kSmemHalf = 113u * 1024u - kSmemSlack;     // and where two o
 // 96 / 96 overlapped and not alone; 180 / 117 / 112 / 111 with the fewer slices a launch of before).
 constexpr uint32_t kSmemAlone = 115u * 1024u;
 constexpr uint32_t kDefaultRing = 64u * 1024u;
-constexpr uint32_t kTile32 = 32u * kPartialStride * 4u;  // the partial-sum tile of row capacity 32
+constexpr uint32_t kOverBlocks = 4;  // of a slice, whose rows (17 and more) are at least a partial-sum tile's size
 
 uint32_t* dev_error_ptr() {
     int dev = 0;
@@ -134,12 +134,12 @@ uint32_t largest_slice(uint32_t nb, uint32_t split) {
 // The ring of one GEMV CTA: stages of kStageRows tk rows (two 128-input blocks), as many as the slab needs or the budget
 // holds; three where the default budget holds fewer and two CTAs still fit a multiprocessor.
 bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan& ring, bool alone = false,
-               uint32_t buffers = 1) {
+               uint32_t buffers = 1, bool over = false) {
     const uint32_t row_bytes = 16u * n, nrows = slice_max / 16u;  // nrows is a multiple of 8 (whole 128-blocks)
     const uint32_t stage_rows = kStageRows;
     const uint32_t stage_bytes = stage_rows * row_bytes;
     const uint32_t need = buffers * ((nrows + stage_rows - 1u) / stage_rows);
-    const uint32_t fixed = gemv_smem(row_cap, xrows, slice_max, cluster, stage_bytes, 0, buffers).total;
+    const uint32_t fixed = gemv_smem(row_cap, xrows, slice_max, cluster, stage_bytes, 0, buffers, over).total;
     if (fixed + stage_bytes > kSmemCap) return false;
     uint32_t budget = g_cfg.ring_bytes ? g_cfg.ring_bytes : kDefaultRing;
     if (!g_cfg.ring_bytes && !alone) {
@@ -150,10 +150,8 @@ bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cl
             if (budget > kSmemHalf - fixed) budget = kSmemHalf - fixed;
         }
     }
-    // (at row capacity 32 what the tile over the rows saves goes to a second stage, not to a third: 16384 -> 7168 at 32 rows 75.3 us with two,
-    // 77.7 with three)
-    const uint32_t most = kSmemCap - fixed, spared = local_over_rows(row_cap) ? kTile32 : 0u;
-    if (budget + spared > most) budget = 2u * stage_bytes + spared > most ? (2u * stage_bytes > most ? most : 2u * stage_bytes) : most - spared;
+    if (budget > kSmemCap - fixed) budget = kSmemCap - fixed;
+    if (over && budget > 2u * stage_bytes) budget = 2u * stage_bytes;  // (a third stage: 16384 -> 7168 at 32 rows 75.3 -> 77.7 us)
     uint32_t stages = budget / stage_bytes;
     stages = stages < 1u ? 1u : stages;
     stages = stages > need ? need : stages;
@@ -161,11 +159,6 @@ bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cl
     ring.stage_rows = stage_rows;
     ring.stages = stages;
     return true;
-}
-
-// Whether a CTA holds the prepared rows of `rows` rows of a slice, at row capacity `row_cap`, beside a partial-sum tile of its own and a stage
-bool holds_rows(uint32_t row_cap, uint32_t rows, uint32_t slice_max, uint32_t cluster, uint32_t n) {
-    return gemv_smem(row_cap, rows, slice_max, cluster, kStageRows * 16u * n, 1u).total + (local_over_rows(row_cap) ? kTile32 : 0u) <= kSmemCap;
 }
 
 bool dtype_ok(int dt) { return dt == T3_F32 || dt == T3_F16 || dt == T3_BF16; }
@@ -187,8 +180,8 @@ int cuda_status(cudaError_t rc) { return rc == cudaSuccess ? T3_OK : T3_CUDA_ERR
 uint32_t row_cap_for(uint32_t rows) { return rows <= 8u ? 8u : (rows <= 16u ? 16u : 32u); }
 
 uint32_t gemv_smem_bytes(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan ring, bool alone,
-                         uint32_t buffers) {
-    const uint32_t bytes = gemv_smem(row_cap, xrows, slice_max, cluster, ring.stage_rows * 16u * n, ring.stages, buffers).total + kSmemSlack;
+                         uint32_t buffers, bool over) {
+    const uint32_t bytes = gemv_smem(row_cap, xrows, slice_max, cluster, ring.stage_rows * 16u * n, ring.stages, buffers, over).total + kSmemSlack;
     return alone && bytes < kSmemAlone ? kSmemAlone : bytes;
 }
 
@@ -486,7 +479,7 @@ int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     const uint32_t nb = a.in / 128u;
     const bool large = large_linear(a.in, a.out, a.n);
     a.alone = 0;
-    auto held = [](uint32_t s, uint32_t longest) { return gemv_smem(32u, 32u, longest * 128u, s, 0, 0).total; };
+    auto held = [](uint32_t s, uint32_t longest) { return gemv_smem(32u, 32u, longest * 128u, s, 0, 0, 1u, longest >= kOverBlocks).total; };
     a.split = cfg.dense_split ? (cfg.dense_split < nb ? cfg.dense_split : nb)
                               : (large ? pick_split_large(nb, a.out / 128u) : pick_split_dense(one_wave() / 2u, nb, a.out / 128u, kStageRows * 16u * a.n, kSmemCap, kSmemHalf, a.alone, held));
     if (a.split == 0u) a.split = nb < 16u ? nb : 16u;
@@ -501,11 +494,19 @@ int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     }
     a.overlap = !cfg.no_overlap;
     a.slice_max = largest_slice(nb, a.split);
-    // A slice too long for shared memory (its prepared rows) is cut further, up to the widest cluster. A large linear's keeps room for a
-    // tile of its own: with what is left where it does not, one ring stage (8704 -> 13312 K6 at 17 rows in two slices 108 us, in four 81).
+    // A slice too long for shared memory (its prepared rows) is cut further, up to the widest cluster. Past 16 rows the partial-sum tile goes
+    // over the rows where the ring would have less than two stages otherwise, or where two CTAs fit a multiprocessor only so; not a large
+    // linear's, which is cut further (8704 -> 13312 K6 at 17 rows in two slices of one stage 108 us, in four 81).
     const uint32_t rm = row_cap_for(a.rows);
-    while ((large && !holds_rows(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n)) ||
-           !plan_ring(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0)) {
+    auto planned = [&] {
+        const uint32_t cluster = a.part ? 1u : a.split, need = (a.slice_max / 16u + kStageRows - 1u) / kStageRows;
+        auto bytes = [&](uint32_t stages, bool over) {
+            return gemv_smem(rm, a.rows, a.slice_max, cluster, kStageRows * 16u * a.n, need < stages ? need : stages, 1u, over).total;
+        };
+        a.tile_over = rm == 32u && !large && a.slice_max >= kOverBlocks * 128u && (bytes(2u, false) > kSmemCap || (!a.alone && bytes(3u, false) > kSmemHalf && bytes(3u, true) <= kSmemHalf));
+        return plan_ring(rm, a.rows, a.slice_max, cluster, a.n, a.ring, a.alone != 0, 1u, a.tile_over != 0);
+    };
+    while (!planned()) {
         if (a.part) {  // back to the cluster kernel
             a.part = nullptr;
             a.split = pick_split_large(nb, a.out / 128u);
@@ -664,11 +665,11 @@ int t3_plan_linear(size_t rows, int in_dim, int out_dim, int n, t3_decode dec, t
     }
     if (ahead)
         fill_launch(&out[k++], symbol, "dense", dim3(a.split, a.out / 128u, 1), 32u * 17u,
-                    gemv_smem_bytes(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0), a.part ? 1u : a.split,
+                    gemv_smem_bytes(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0, 1u, a.tile_over != 0), a.part ? 1u : a.split,
                     {T3_ROLE_XP, T3_ROLE_Y, T3_ROLE_TRELLIS, T3_ROLE_SVH});
     else
         fill_launch(&out[k++], symbol, "dense", dim3(a.split, a.out / 128u, 1), 32u * 17u,
-                    gemv_smem_bytes(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0), a.part ? 1u : a.split,
+                    gemv_smem_bytes(rm, a.rows, a.slice_max, a.part ? 1u : a.split, a.n, a.ring, a.alone != 0, 1u, a.tile_over != 0), a.part ? 1u : a.split,
                     {T3_ROLE_X, T3_ROLE_Y, T3_ROLE_TRELLIS, T3_ROLE_SUH, T3_ROLE_SVH});
     if (a.part) out[k - 1].roles[out[k - 1].nroles++] = T3_ROLE_Z;  // the slices' partial sums meet in global memory
     return k;
@@ -724,12 +725,12 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
                       : pick_split(a.inter / 128u, (a.hidden / 128u) * kNominalSlots, 1u, 8u, one_wave() / 8u);
     a.slice_max_d = largest_slice(a.inter / 128u, a.split_d);
     // sized for the widest row capacity so the split does not move with the rows either
-    while (!holds_rows(32u, 32u, a.slice_max_gu, 2u * a.split_gu, a.n)) {
+    while (!plan_ring(32u, 32u, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu)) {
         if (a.split_gu * 2u > a.hidden / 128u || a.split_gu * 2u > 8u) return T3_ENGINE_NOT_IMPLEMENTED;
         a.split_gu *= 2u;
         a.slice_max_gu = largest_slice(a.hidden / 128u, a.split_gu);
     }
-    while (!holds_rows(32u, 32u, a.slice_max_d, a.split_d, a.n)) {
+    while (!plan_ring(32u, 32u, a.slice_max_d, a.split_d, a.n, a.ring_d)) {
         if (a.split_d * 2u > a.inter / 128u || a.split_d * 2u > 16u) return T3_ENGINE_NOT_IMPLEMENTED;
         a.split_d *= 2u;
         a.slice_max_d = largest_slice(a.inter / 128u, a.split_d);

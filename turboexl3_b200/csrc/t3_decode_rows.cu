@@ -67,11 +67,11 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 template <int N, int RM, int HB = 2, bool WINDOWS = false>
 __device__ __forceinline__ void gemv_and_push(cg::cluster_group& cluster, const CtaSmem& c, uint32_t nrows, uint32_t n,
                                               uint32_t mask, Ring rc, uint32_t xstride, uint32_t xrows, RingPos& pos, uint32_t count,
-                                              uint32_t rank, uint32_t csize, uint32_t warp, uint32_t lane, uint32_t* err) {
+                                              uint32_t rank, uint32_t csize, uint32_t warp, uint32_t lane, uint32_t* err, bool over = false) {
     const uint32_t tcol = warp & (kTileWarps - 1u), kg = warp / kTileWarps;
     float acc[RowCap<RM>::kMB][2][4] = {};
     consume_slab<N, CB, RM, HB, WINDOWS>(c.ring, c.full, c.empty, nrows, n, mask, rc, c.xp, xstride, xrows, pos, tcol, kg, lane, acc, err);
-    if (local_over_rows(RM)) named_sync(1, kConsumerThreads);  // every warp has read the prepared rows
+    if (over) named_sync(1, kConsumerThreads);  // every warp has read the prepared rows
     if (kg == 1) store_local<RM>(c.local, acc, tcol, lane);
     named_sync(1, kConsumerThreads);
     if (kg == 0) push_partial<RM>(cluster, c.recv, c.local, acc, count, rank, csize, tcol, lane);
@@ -97,7 +97,7 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
     const uint32_t nblk = b1 - b0, nrows = nblk * 8u;
     const uint32_t tile_bytes = 2u * a.n, row_bytes = 16u * a.n, out_tiles = a.out / 16u;
     const Ring rc{a.ring.stage_rows, a.ring.stages};
-    const CtaSmem c = carve(smem, gemv_smem(RM, a.rows, a.slice_max, csize, rc.stage_rows * row_bytes, rc.stages));
+    const CtaSmem c = carve(smem, gemv_smem(RM, a.rows, a.slice_max, csize, rc.stage_rows * row_bytes, rc.stages, 1u, RM == 32 && a.tile_over != 0u));
     const uint32_t xstride = a.slice_max + kXpPad;
 
     const bool traced = a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
@@ -132,7 +132,10 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
         }
     } else {
         pdl_trigger();
-        load_scales(static_cast<const __half*>(a.svh) + blk * 128u, lane, sv);  // weights-side: ahead of the wait
+        // weights-side: ahead of the wait (at row capacity 32 into L2 only: registers held through the loop spill)
+        const __half* const svh = static_cast<const __half*>(a.svh) + blk * 128u;
+        if (RM < 32) load_scales(svh, lane, sv);
+        else if (warp == 1) prefetch_l2(svh, 256u, lane);
         if (a.xp_g == nullptr) {
             if (warp == 0) prefetch_l2(static_cast<const __half*>(a.suh) + b0 * 128u, nblk * 256u, lane);
             pdl_wait();  // x may be the previous kernel's output
@@ -153,13 +156,14 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
             a.trace[3] = clock64();
         }
         if (!global) {
-            gemv_and_push<N, RM, kDenseBatch, true>(cluster, c, nrows, a.n, a.mask, rc, xstride, a.rows, pos, a.rows, rank, csize, warp, lane, a.err);
+            gemv_and_push<N, RM, kDenseBatch, true>(cluster, c, nrows, a.n, a.mask, rc, xstride, a.rows, pos, a.rows, rank, csize, warp, lane, a.err,
+                                                 RM == 32 && a.tile_over != 0u);
         } else {
             // the slice's sums to global memory; the block's last arriver adds the slices in slice order and finishes
             const uint32_t tcol = warp & (kTileWarps - 1u), kg = warp / kTileWarps;
             float acc[RowCap<RM>::kMB][2][4] = {};
             consume_slab<N, CB, RM, kDenseBatch, true>(c.ring, c.full, c.empty, nrows, a.n, a.mask, rc, c.xp, xstride, a.rows, pos, tcol, kg, lane, acc, a.err);
-            if (local_over_rows(RM)) named_sync(1, kConsumerThreads);
+            if (RM == 32 && a.tile_over != 0u) named_sync(1, kConsumerThreads);
             if (kg == 1) store_local<RM>(c.local, acc, tcol, lane);
             named_sync(1, kConsumerThreads);
             if (kg == 0) {
@@ -181,6 +185,7 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
             if (tid == 0) s_last = atomicAdd(&a.counters[blk], 1u) == a.split - 1u;
             named_sync(1, kConsumerThreads);
             if (!s_last) return;
+            if (RM == 32) load_scales(static_cast<const __half*>(a.svh) + blk * 128u, lane, sv);
             __threadfence();
             for (uint32_t row = warp; row < a.rows; row += kConsumerWarps) {
                 float v[4];
@@ -198,6 +203,7 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
             }
             return;
         }
+        if (RM == 32) load_scales(static_cast<const __half*>(a.svh) + blk * 128u, lane, sv);
         if (traced && tid == 0) a.trace[4] = clock64();
     }
     if (global) return;  // the copy warp: its copies have landed (the consumers waited for each)
@@ -676,7 +682,7 @@ cudaError_t T3_CAT(launch_dense_gemv_cb, T3_CB)(const DenseArgs& a, cudaStream_t
     KernelFn<DenseArgs> fn = T3_PICK(T3_PICK_32, t3_dense_gemv, a.n, rm);
     const uint32_t cluster = a.part ? 1u : a.split;
     return launch_cluster(fn, a, dim3(a.split, a.out / 128u, 1), cluster,
-                          gemv_smem_bytes(rm, a.rows, a.slice_max, cluster, a.n, a.ring, a.alone != 0),
+                          gemv_smem_bytes(rm, a.rows, a.slice_max, cluster, a.n, a.ring, a.alone != 0, 1u, a.tile_over != 0),
                           a.overlap != 0, stream);
 }
 

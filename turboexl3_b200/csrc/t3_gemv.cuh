@@ -58,18 +58,17 @@ __host__ __device__ inline uint32_t rows_owned(uint32_t rm, uint32_t cluster) { 
 // xrows: prepared rows held (the routed kernels hold a pass's row capacity; the dense linear only its live rows: the
 // tensor-core steps read a row past the last live one from the last live one, and nobody looks at what that gives)
 // buffers: partial-sum tiles, two where a CTA runs several output blocks (the next one's sums come in while one is finished)
-// At row capacity 32 the K groups' tile lies over the prepared rows, which have been read by then (store_local's callers see to it): 17 KB
-// for slices that would not fit otherwise or leave one ring stage (12288 -> 6144 K2 at 32 rows in five slices 45 us; in eight, the fewest
-// that fitted, 68), at a barrier a launch: 2048 -> 6144 at 32 rows 14.8 -> 14.9.
-__host__ __device__ constexpr bool local_over_rows(uint32_t rm) { return rm == 32u; }
+// over: the K groups' tile lies over the prepared rows, which have been read by then (store_local's callers see to it, at a barrier: 2048 ->
+// 6144 at 17 rows 13.3 -> 13.6 us). At row capacity 32, for slices that would not fit otherwise or leave one ring stage: 12288 -> 6144 K2 at
+// 32 rows in five slices 45 us; in eight, the fewest that fitted, 68.
 __host__ __device__ inline GemvSmem gemv_smem(uint32_t rm, uint32_t xrows, uint32_t slice_k, uint32_t cluster, uint32_t stage_bytes,
-                                              uint32_t stages, uint32_t buffers = 1) {
+                                              uint32_t stages, uint32_t buffers = 1, bool over = false) {
     GemvSmem s;
     s.bars = 0;
     s.xp = 2u * kMaxStages * 8u + 128u;  // the ring's full and empty barriers, then one for prepared rows copied in
     const uint32_t xp_bytes = xrows * (slice_k + kXpPad) * 2u;
     const uint32_t xp_end = s.xp + ((xp_bytes + 127u) & ~127u);
-    s.local = local_over_rows(rm) ? s.xp : xp_end;
+    s.local = over ? s.xp : xp_end;
     s.recv = s.local + buffers * ((rm * kPartialStride * 4u + 127u) & ~127u);
     s.recv = s.recv > xp_end ? s.recv : xp_end;
     s.ring = s.recv + buffers * ((cluster * rows_owned(rm, cluster) * kPartialStride * 4u + 127u) & ~127u);

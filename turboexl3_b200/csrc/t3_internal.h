@@ -37,6 +37,7 @@ struct DenseArgs {
     int overlap;              // launch with the programmatic-dependent-launch attribute
     uint32_t* err;
     unsigned long long* trace;  // optional: SM cycle counts at the phases of CTA (0, 0) (see t3_set_trace)
+    uint32_t tile_over;       // row capacity 32: the K groups' partial-sum tile lies over the prepared rows (see gemv_smem)
 };
 
 // One more bank of a banked call (an expert streamer's slot banks: the same geometry and rate, its own slot count)
@@ -132,7 +133,7 @@ cudaError_t launch_moe_merge(const MoeArgs& a, cudaStream_t stream);
 
 // shared-memory bytes the GEMV CTAs of a plan need (for admission before launch)
 uint32_t gemv_smem_bytes(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan ring, bool alone = false,
-                         uint32_t buffers = 1);
+                         uint32_t buffers = 1, bool over = false);
 // the most dynamic shared memory a GEMV CTA may be launched with
 constexpr uint32_t kGemvSmemLimit = 200u * 1024u;
 uint32_t row_cap_for(uint32_t rows);

@@ -36,6 +36,7 @@ uint32_t pick_split_dense(uint32_t sms, uint32_t nb, uint32_t blocks, uint32_t s
         if (one == 0u || (!single && two == 0u)) continue;
         const uint32_t longest = (nb + s - 1u) / s, at_once = single ? one : two;
         auto rounds = [&](uint32_t fit, uint32_t block, uint32_t block_single, uint32_t fixed) {  // in 10 ns
+            if (blocks <= fit) return longest * block + fixed;
             const uint32_t full = blocks / fit, rest = blocks - full * fit;
             return full * (longest * block + fixed) + (rest ? longest * (rest <= one ? block_single : block) + fixed : 0u);
         };
