@@ -138,6 +138,19 @@ def test_launches_that_do_not_overlap_leave_room_for_another_streams():
     assert [p["grid"] for p in apart] == [p["grid"] for p in beside]
 
 
+def test_a_gate_up_launch_keeps_its_multiprocessors_only_where_all_its_clusters_fit_so():
+    """CTAs that ask for more than half a multiprocessor's shared memory are one to a multiprocessor: no launch asks for that whose clusters
+    do not all fit the device so (the ones left over would wait for a whole second round)."""
+    asked = 0
+    for rows, inter in itertools.product(range(1, 33), (128, 256, 384, 512, 1024)):
+        for topk in (1, 2, 6, 8, 10, 16):
+            gu = t3.plan_moe(rows, topk, 64, 2048, inter, 16)[0]  # (a ring small enough to leave room for a second CTA)
+            if gu["shared"] > 113 * 1024:
+                asked += 1
+                assert rows * topk * (inter // 128) <= ONE_A_SM[gu["cluster"]], (rows, inter, topk, gu)
+    assert asked > 0
+
+
 def test_routed_plans_are_launchable():
     geoms = [(8, 128, 128), (10, 512, 2048), (64, 2048, 512), (128, 2048, 768), (256, 7168, 2048), (32, 4096, 1536), (16, 1024, 4096)]
     for (experts, hidden, inter), n, rows, topk in itertools.product(geoms, [16, 48, 64, 128, 36], [1, 3, 8, 16, 32], [1, 2, 8, 10]):

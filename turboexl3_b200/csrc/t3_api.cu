@@ -753,9 +753,10 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     // neighbour on the stream is another chain, keeps the late start (16 rows of 2048 x 512: 25.3 us against 31.8).
     const uint64_t gu = (uint64_t)2u * a.split_gu * (a.inter / 128u) * slots, down = (uint64_t)a.split_d * (a.hidden / 128u) * slots;
     a.down_early = a.experts > 1u && gu <= sms && (down > sms || gu + down <= sms);
-    // gate|up's CTAs a multiprocessor each where all find one (behind a launch of wider clusters they doubled up: a layer of one row with
-    // its shared expert ahead on the stream 43.9 us, 33.9 so)
-    a.alone_gu = gu <= sms && a.overlap;
+    // gate|up's CTAs a multiprocessor each where all its clusters find room so (behind a launch of wider clusters they doubled up: a layer of
+    // one row with its shared expert ahead on the stream 43.9 us, 33.9 so; clusters past that wait for a second round: two rows of top-8 in
+    // 64 experts of 2048 x 128, sixteen clusters of eight, 17.6 us alone and 15.2 not, fifteen 13.6 alone)
+    a.alone_gu = slots * (a.inter / 128u) <= clusters_alone(sms, 2u * a.split_gu) && a.overlap;
     return T3_OK;
 }
 

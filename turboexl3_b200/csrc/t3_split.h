@@ -5,6 +5,13 @@
 
 namespace t3 {
 
+// The most clusters of `size` CTAs that `sms` multiprocessors hold at once with a multiprocessor a CTA:
+// cudaOccupancyMaxActiveClusters's for 148 (other devices take their share), written down because plans must be the same without a device.
+inline uint32_t clusters_alone(uint32_t sms, uint32_t size) {
+    static const uint16_t kOne[17] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7};
+    return kOne[size] * sms / 148u;
+}
+
 // K slices of an ordinary dense linear of nb 128-input and `blocks` 128-output blocks, a cluster of s CTAs a block, and whether its CTAs go
 // one to a multiprocessor (`alone`): one count a shape and rate, so that a row's bytes are the same alone and in a batch. Only counts whose
 // CTAs hold the prepared rows of 32 rows are asked, and the cheapest by its longest slice's time is taken, three times a row's and once that of
@@ -26,12 +33,11 @@ namespace t3 {
 // multiprocessor; held(s, longest): the bytes a CTA of s slices holds beside its ring at 32 rows. 0: no count holds 32 rows.
 template <typename Held>
 uint32_t pick_split_dense(uint32_t sms, uint32_t nb, uint32_t blocks, uint32_t stage, uint32_t cap, uint32_t half, uint32_t& alone, Held&& held) {
-    static const uint16_t kOne[17] = {0, 148, 74, 45, 33, 26, 22, 15, 15, 15, 11, 7, 7, 7, 7, 7, 7};
     static const uint16_t kTwo[17] = {0, 296, 148, 88, 71, 50, 45, 37, 33, 0, 0, 0, 0, 0, 0, 0, 14};
     uint32_t best = 0, best_cost = ~0u;
     alone = 0;
     for (uint32_t s = 1; s <= 16u && s <= nb; ++s) {
-        const uint32_t one = kOne[s] * sms / 148u, two = kTwo[s] * sms / 148u;
+        const uint32_t one = clusters_alone(sms, s), two = kTwo[s] * sms / 148u;
         const bool single = blocks <= one;
         if (one == 0u || (!single && two == 0u)) continue;
         const uint32_t longest = (nb + s - 1u) / s, at_once = single ? one : two;
