@@ -342,10 +342,10 @@ def test_bank_scales_that_are_not_signs():
     assert t3.device_error() == 0
 
 
-@pytest.mark.parametrize("dims", [(1920, 128, 48), (2048, 256, 36)])
+@pytest.mark.parametrize("dims", [(1920, 128, 48), (2048, 256, 36), (3840, 128, 48), (7040, 128, 32)])
 def test_down_ctas_that_take_several_blocks(dims):
-    """Calls that touch enough experts for a down CTA to run two output blocks and more (the last one's run cut short): the oracle's
-    rows, and each row's bytes alone, where a CTA runs one block."""
+    """Calls that touch enough experts for a down CTA to run two, two, four and eight output blocks (the last CTA's run is short but in the
+    second; from the third block on a partial-sum tile is used again): the oracle's rows, and each row's bytes alone, where a CTA runs one block."""
     H, I, n = dims
     E, topk, rows = 256, 16, 32
     bank, obank = make_bank(1500 + n, E, H, I, n)

@@ -209,8 +209,9 @@ __device__ __forceinline__ void decode_stages(uint32_t visits, Ring<kCodeStages>
     }
 }
 
-// A warp's 16 outputs of up to 128 accumulator columns, 32 at a time: f(r, v) gets columns r .. r + 31 while the next 32 are on their
-// way (a load's latency for every 32 columns was half of what the epilogue took).
+// A warp's 16 outputs of up to 128 accumulator columns: f(r, v) gets columns r .. r + 31. Two loads are on their way at once and one
+// wait is for both (tcgen05.wait::ld knows no single load; a load's latency for every 32 columns was half of what the epilogue took); the second
+// wait only keeps its registers' use behind it.
 template <typename F>
 __device__ __forceinline__ void for_columns(uint32_t taddr, uint32_t cols, F&& f) {
     uint32_t v[2][16];
