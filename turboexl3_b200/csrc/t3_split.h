@@ -36,7 +36,9 @@ uint32_t pick_split_dense(uint32_t sms, uint32_t nb, uint32_t blocks, uint32_t s
     static const uint16_t kTwo[17] = {0, 296, 148, 88, 71, 50, 45, 37, 33, 0, 0, 0, 0, 0, 0, 0, 14};
     uint32_t best = 0, best_cost = ~0u;
     alone = 0;
-    for (uint32_t s = 1; s <= 16u && s <= nb; ++s) {
+#pragma GCC unroll 16  // with s known the divisions are products: 27 to 54 ns, 63 to 84 without
+    for (uint32_t s = 16u; s > 0u; --s) {  // from the short slices down: the long ones fall to the first test
+        if (s > nb) continue;
         const uint32_t one = clusters_alone(sms, s), two = kTwo[s] * sms / 148u;
         const bool single = blocks <= one;
         if (one == 0u || (!single && two == 0u)) continue;
@@ -47,13 +49,13 @@ uint32_t pick_split_dense(uint32_t sms, uint32_t nb, uint32_t blocks, uint32_t s
             return full * (longest * block + fixed) + (rest ? longest * (rest <= one ? block_single : block) + fixed : 0u);
         };
         const uint32_t row = rounds(at_once, single ? 58u : 116u, 58u, 300u + 10u * s);
-        if (3u * row >= best_cost) continue;
+        if (3u * row + longest * 80u + 640u + 10u * s > best_cost) continue;
         const uint32_t stages = (longest + 1u) / 2u, bytes = held(s, longest);
         if (bytes + stage > cap) continue;
         const bool pair = !single && bytes + (stages < 3u ? stages : 3u) * stage <= half;
         uint32_t rows = pair ? rounds(at_once, 260u, 80u, 640u + 10u * s) : rounds(one, 80u, 80u, 640u + 10u * s);
         if (stages > 1u && bytes + 2u * stage > cap) rows = rows * 7u / 5u;
-        if (3u * row + rows < best_cost) best = s, best_cost = 3u * row + rows, alone = single;
+        if (3u * row + rows <= best_cost) best = s, best_cost = 3u * row + rows, alone = single;
     }
     return best;
 }
