@@ -478,12 +478,12 @@ bool large_linear(uint32_t in, uint32_t out, uint32_t n) { return (uint64_t)in *
 int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     const uint32_t nb = a.in / 128u;
     const bool large = large_linear(a.in, a.out, a.n);
-    a.alone = 0;
+    uint32_t alone = 0;
     auto held = [](uint32_t s, uint32_t longest) { return gemv_smem(32u, 32u, longest * 128u, s, 0, 0, 1u, longest >= kOverBlocks).total; };
     a.split = cfg.dense_split ? (cfg.dense_split < nb ? cfg.dense_split : nb)
-                              : (large ? pick_split_large(nb, a.out / 128u) : pick_split_dense(one_wave() / 2u, nb, a.out / 128u, kStageRows * 16u * a.n, kSmemCap, kSmemHalf, a.alone, held));
+                              : (large ? pick_split_large(nb, a.out / 128u) : pick_split_dense(one_wave() / 2u, nb, a.out / 128u, kStageRows * 16u * a.n, kSmemCap, kSmemHalf, alone, held));
     if (a.split == 0u) a.split = nb < 16u ? nb : 16u;
-    if (cfg.no_overlap) a.alone = 0;  // see kSmemAlone
+    a.alone = alone != 0u && !cfg.no_overlap;  // see kSmemAlone
     a.part = nullptr;
     if (large && global_ok && !cfg.dense_split && !cfg.probe) {
         const uint32_t s = pick_split_global(nb, a.out / 128u, a.split);

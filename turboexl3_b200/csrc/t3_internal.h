@@ -32,13 +32,15 @@ struct DenseArgs {
     uint32_t* counters;       // with part: [out/128] arrivals a block, zero before the launch; the last arriver finishes the block
     uint32_t split;           // K slices (the cluster size unless `part` is set)
     uint32_t slice_max;       // inputs of the largest K slice
-    uint32_t alone;           // a CTA takes more than half a multiprocessor's shared memory (see kSmemAlone)
+    uint16_t alone;           // a CTA takes more than half a multiprocessor's shared memory (see kSmemAlone)
+    uint16_t tile_over;       // row capacity 32: the K groups' partial-sum tile lies over the prepared rows (see gemv_smem)
     RingPlan ring;
     int overlap;              // launch with the programmatic-dependent-launch attribute
     uint32_t* err;
     unsigned long long* trace;  // optional: SM cycle counts at the phases of CTA (0, 0) (see t3_set_trace)
-    uint32_t tile_over;       // row capacity 32: the K groups' partial-sum tile lies over the prepared rows (see gemv_smem)
 };
+// (136 bytes of arguments, us a launch: 2048 -> 6144 K3 at one row 7.66 -> 7.72, 9216 -> 2688 10.52 -> 10.61)
+static_assert(sizeof(DenseArgs) <= 128, "two lines of the constant cache");
 
 // One more bank of a banked call (an expert streamer's slot banks: the same geometry and rate, its own slot count)
 struct BankTab {
