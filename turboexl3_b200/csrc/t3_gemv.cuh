@@ -70,7 +70,7 @@ __host__ __device__ inline GemvSmem gemv_smem(uint32_t rm, uint32_t xrows, uint3
     const uint32_t xp_end = s.xp + ((xp_bytes + 127u) & ~127u);
     s.local = over ? s.xp : xp_end;
     s.recv = s.local + buffers * ((rm * kPartialStride * 4u + 127u) & ~127u);
-    s.recv = s.recv > xp_end ? s.recv : xp_end;
+    if (over && s.recv < xp_end) s.recv = xp_end;
     s.ring = s.recv + buffers * ((cluster * rows_owned(rm, cluster) * kPartialStride * 4u + 127u) & ~127u);
     s.total = s.ring + stage_bytes * stages;
     return s;
