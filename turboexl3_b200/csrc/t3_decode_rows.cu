@@ -64,14 +64,14 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 
 // The consumer side of one pass once xp is ready: GEMV over the slab, the two K groups joined, the partial pushed to the
 // rows' owners. `count` live rows.
-template <int N, int RM, int HB = 2, bool WINDOWS = false>
+template <int N, int RM, int HB = 2, bool WINDOWS = false, bool OVER = false>
 __device__ __forceinline__ void gemv_and_push(cg::cluster_group& cluster, const CtaSmem& c, uint32_t nrows, uint32_t n,
                                               uint32_t mask, Ring rc, uint32_t xstride, uint32_t xrows, RingPos& pos, uint32_t count,
-                                              uint32_t rank, uint32_t csize, uint32_t warp, uint32_t lane, uint32_t* err, bool over = false) {
+                                              uint32_t rank, uint32_t csize, uint32_t warp, uint32_t lane, uint32_t* err) {
     const uint32_t tcol = warp & (kTileWarps - 1u), kg = warp / kTileWarps;
     float acc[RowCap<RM>::kMB][2][4] = {};
     consume_slab<N, CB, RM, HB, WINDOWS>(c.ring, c.full, c.empty, nrows, n, mask, rc, c.xp, xstride, xrows, pos, tcol, kg, lane, acc, err);
-    if (over) named_sync(1, kConsumerThreads);  // every warp has read the prepared rows
+    if (OVER) named_sync(1, kConsumerThreads);  // every warp has read the prepared rows
     if (kg == 1) store_local<RM>(c.local, acc, tcol, lane);
     named_sync(1, kConsumerThreads);
     if (kg == 0) push_partial<RM>(cluster, c.recv, c.local, acc, count, rank, csize, tcol, lane);
@@ -80,7 +80,11 @@ __device__ __forceinline__ void gemv_and_push(cg::cluster_group& cluster, const 
 // ---------------------------------------------------------------------------------------------- dense linear
 
 // grid (split, out / 128), cluster (split, 1, 1) — or no cluster when the partial sums meet in global memory (a.part)
-template <int N, int RM>
+//
+// OVER (row capacity 32): the K groups' partial-sum tile lies over the prepared rows (DenseArgs::tile_over). A kernel of its own: as a flag of the
+// launch it cost every launch of 17 to 32 rows up to 4 % by the registers it took (896 -> 9856 K5 at 24 rows 14.0 -> 14.7 us, 6272 -> 15616 K5 at 32
+// 72.3 -> 75.3), with a barrier no one needs.
+template <int N, int RM, bool OVER = false>
 __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* smem = aligned_smem(smem_raw);
@@ -97,7 +101,7 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
     const uint32_t nblk = b1 - b0, nrows = nblk * 8u;
     const uint32_t tile_bytes = 2u * a.n, row_bytes = 16u * a.n, out_tiles = a.out / 16u;
     const Ring rc{a.ring.stage_rows, a.ring.stages};
-    const CtaSmem c = carve(smem, gemv_smem(RM, a.rows, a.slice_max, csize, rc.stage_rows * row_bytes, rc.stages, 1u, RM == 32 && a.tile_over != 0u));
+    const CtaSmem c = carve(smem, gemv_smem(RM, a.rows, a.slice_max, csize, rc.stage_rows * row_bytes, rc.stages, 1u, OVER));
     const uint32_t xstride = a.slice_max + kXpPad;
 
     const bool traced = a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
@@ -132,10 +136,7 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
         }
     } else {
         pdl_trigger();
-        // weights-side: ahead of the wait (at row capacity 32 into L2 only: registers held through the loop spill)
-        const __half* const svh = static_cast<const __half*>(a.svh) + blk * 128u;
-        if (RM < 32) load_scales(svh, lane, sv);
-        else if (warp == 1) prefetch_l2(svh, 256u, lane);
+        load_scales(static_cast<const __half*>(a.svh) + blk * 128u, lane, sv);  // weights-side: ahead of the wait
         if (a.xp_g == nullptr) {
             if (warp == 0) prefetch_l2(static_cast<const __half*>(a.suh) + b0 * 128u, nblk * 256u, lane);
             pdl_wait();  // x may be the previous kernel's output
@@ -156,14 +157,13 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
             a.trace[3] = clock64();
         }
         if (!global) {
-            gemv_and_push<N, RM, kDenseBatch, true>(cluster, c, nrows, a.n, a.mask, rc, xstride, a.rows, pos, a.rows, rank, csize, warp, lane, a.err,
-                                                 RM == 32 && a.tile_over != 0u);
+            gemv_and_push<N, RM, kDenseBatch, true, OVER>(cluster, c, nrows, a.n, a.mask, rc, xstride, a.rows, pos, a.rows, rank, csize, warp, lane, a.err);
         } else {
             // the slice's sums to global memory; the block's last arriver adds the slices in slice order and finishes
             const uint32_t tcol = warp & (kTileWarps - 1u), kg = warp / kTileWarps;
             float acc[RowCap<RM>::kMB][2][4] = {};
             consume_slab<N, CB, RM, kDenseBatch, true>(c.ring, c.full, c.empty, nrows, a.n, a.mask, rc, c.xp, xstride, a.rows, pos, tcol, kg, lane, acc, a.err);
-            if (RM == 32 && a.tile_over != 0u) named_sync(1, kConsumerThreads);
+            if (OVER) named_sync(1, kConsumerThreads);
             if (kg == 1) store_local<RM>(c.local, acc, tcol, lane);
             named_sync(1, kConsumerThreads);
             if (kg == 0) {
@@ -185,7 +185,6 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
             if (tid == 0) s_last = atomicAdd(&a.counters[blk], 1u) == a.split - 1u;
             named_sync(1, kConsumerThreads);
             if (!s_last) return;
-            if (RM == 32) load_scales(static_cast<const __half*>(a.svh) + blk * 128u, lane, sv);
             __threadfence();
             for (uint32_t row = warp; row < a.rows; row += kConsumerWarps) {
                 float v[4];
@@ -203,7 +202,6 @@ __device__ __forceinline__ void dense_gemv_body(const DenseArgs& a) {
             }
             return;
         }
-        if (RM == 32) load_scales(static_cast<const __half*>(a.svh) + blk * 128u, lane, sv);
         if (traced && tid == 0) a.trace[4] = clock64();
     }
     if (global) return;  // the copy warp: its copies have landed (the consumers waited for each)
@@ -604,7 +602,7 @@ cudaError_t launch_cluster(KernelFn<Args> fn, const Args& a, dim3 grid, uint32_t
 //   t3_dec_merge
 // <codebook> mul1 | mcg (probe2..probe4: the dense kernel's timing probes); <n> the rate's halfwords a tile, 0 = any even
 // rate at run time; <rows> the row capacity of a pass, 8 | 16 | 32
-// (32: the dense linear only).
+// (32: the dense linear only, which has a second kernel of it, 32_over: see dense_gemv_body).
 #if T3_CB == 0
 #define T3_CBNAME mul1
 #elif T3_CB == 1
@@ -623,7 +621,12 @@ cudaError_t launch_cluster(KernelFn<Args> fn, const Args& a, dim3 grid, uint32_t
         BODY<NN, RM>(a);                                                                                        \
     }
 #if T3_SERVED
-#define T3_ENTRIES_32(STEM, BODY, ARGS, NN) T3_ENTRY(STEM, BODY, ARGS, NN, 8) T3_ENTRY(STEM, BODY, ARGS, NN, 16) T3_ENTRY(STEM, BODY, ARGS, NN, 32)
+#define T3_ENTRY_OVER(STEM, BODY, ARGS, NN)                                                                          \
+    extern "C" __global__ void __launch_bounds__(kGemvThreads, 2) T3_NAME(STEM, T3_CBNAME, NN, 32_over)(const ARGS a) { \
+        BODY<NN, 32, true>(a);                                                                                       \
+    }
+#define T3_ENTRIES_32(STEM, BODY, ARGS, NN)                                                                                          \
+    T3_ENTRY(STEM, BODY, ARGS, NN, 8) T3_ENTRY(STEM, BODY, ARGS, NN, 16) T3_ENTRY(STEM, BODY, ARGS, NN, 32) T3_ENTRY_OVER(STEM, BODY, ARGS, NN)
 #define T3_ENTRIES_16(STEM, BODY, ARGS, NN) T3_ENTRY(STEM, BODY, ARGS, NN, 8) T3_ENTRY(STEM, BODY, ARGS, NN, 16)
 #else  // the probes exist at the 8-row capacity only
 #define T3_ENTRIES_32(STEM, BODY, ARGS, NN) T3_ENTRY(STEM, BODY, ARGS, NN, 8)
@@ -656,8 +659,11 @@ extern "C" __global__ void __launch_bounds__(128) t3_dense_prep(const DenseArgs 
 #endif
 
 #if T3_SERVED
-#define T3_PICK_32(STEM, NN, rm) \
-    ((rm) == 8 ? T3_NAME(STEM, T3_CBNAME, NN, 8) : ((rm) == 16 ? T3_NAME(STEM, T3_CBNAME, NN, 16) : T3_NAME(STEM, T3_CBNAME, NN, 32)))
+#define T3_PICK_32(STEM, NN, rm)                       \
+    ((rm) == 8    ? T3_NAME(STEM, T3_CBNAME, NN, 8)    \
+     : (rm) == 16 ? T3_NAME(STEM, T3_CBNAME, NN, 16)   \
+     : (rm) == 32 ? T3_NAME(STEM, T3_CBNAME, NN, 32)   \
+                  : T3_NAME(STEM, T3_CBNAME, NN, 32_over))
 #define T3_PICK_16(STEM, NN, rm) ((rm) == 8 ? T3_NAME(STEM, T3_CBNAME, NN, 8) : T3_NAME(STEM, T3_CBNAME, NN, 16))
 #else
 #define T3_PICK_32(STEM, NN, rm) T3_NAME(STEM, T3_CBNAME, NN, 8)
@@ -679,7 +685,7 @@ extern "C" __global__ void __launch_bounds__(128) t3_dense_prep(const DenseArgs 
 
 cudaError_t T3_CAT(launch_dense_gemv_cb, T3_CB)(const DenseArgs& a, cudaStream_t stream) {
     const uint32_t rm = row_cap_for(a.rows);
-    KernelFn<DenseArgs> fn = T3_PICK(T3_PICK_32, t3_dense_gemv, a.n, rm);
+    KernelFn<DenseArgs> fn = T3_PICK(T3_PICK_32, t3_dense_gemv, a.n, rm + a.tile_over);  // 33: 32_over
     const uint32_t cluster = a.part ? 1u : a.split;
     return launch_cluster(fn, a, dim3(a.split, a.out / 128u, 1), cluster,
                           gemv_smem_bytes(rm, a.rows, a.slice_max, cluster, a.n, a.ring, a.alone != 0, 1u, a.tile_over != 0),
