@@ -272,8 +272,9 @@ int t3_linear_unrot(const void* x, int x_dtype, size_t rows, const void* w_std_t
  * pattern t3_<group>_<kernel>_<profile>...:
  *   t3_dense_gemv_<mul1|mcg>_n<n>_r<8|16|32>   t3_dense_prep   t3_dec_gate_up_<..>_n<n>_r<..>   t3_dec_down_<..>_n<n>_r<..>
  *   t3_dec_merge
- * (capacity 32: the dense kernels, and a second one of it, r32_over; n = halfwords a tile for the rates with kernels of their
- * own, 0 for the run-time-rate kernels). t3_plan_linear and
+ * (capacity 32: the dense kernels; n = halfwords a tile for the rates with kernels of their own, 0 for the run-time-rate
+ * kernels). Launches whose partial-sum tile lies over the prepared rows (long K slices, 17 rows and more) run the twin <symbol>_over, which
+ * t3_plan_linear and t3_last_kernel_symbol report as <symbol>: the capacity's. t3_plan_linear and
  * t3_plan_moe give, without launching, the launches t3_linear / t3_moe would record for a decode-row call under the
  * current configuration: each kernel takes ONE argument block (DenseArgs / MoeArgs of csrc/t3_internal.h) whose buffers are
  * listed by role, numbered as plan.Role is. They return the number of launches written, or minus a t3_status. Prefill

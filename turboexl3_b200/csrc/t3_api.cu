@@ -655,7 +655,7 @@ int t3_plan_linear(size_t rows, int in_dim, int out_dim, int n, t3_decode dec, t
     if (int rc = plan_dense(a, cfg, true)) return -rc;
     const uint32_t rm = row_cap_for(a.rows);
     char symbol[64];
-    std::snprintf(symbol, sizeof symbol, "t3_dense_gemv_%s_n%u_r%u%s", dec.codebook == T3_MCG ? "mcg" : "mul1", named_rate(a.n), rm, a.tile_over ? "_over" : "");
+    std::snprintf(symbol, sizeof symbol, "t3_dense_gemv_%s_n%u_r%u", dec.codebook == T3_MCG ? "mcg" : "mul1", named_rate(a.n), rm);
     int k = 0;
     const bool ahead = prep_ahead(a);
     if (ahead) {  // with the call's workspace: the rows rotated once ahead of the GEMV

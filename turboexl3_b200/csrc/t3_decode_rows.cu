@@ -602,7 +602,7 @@ cudaError_t launch_cluster(KernelFn<Args> fn, const Args& a, dim3 grid, uint32_t
 //   t3_dec_merge
 // <codebook> mul1 | mcg (probe2..probe4: the dense kernel's timing probes); <n> the rate's halfwords a tile, 0 = any even
 // rate at run time; <rows> the row capacity of a pass, 8 | 16 | 32
-// (32: the dense linear only, which has a second kernel of it, 32_over: see dense_gemv_body).
+// (32: the dense linear only, which has a twin, 32_over, that plans and t3_last_kernel_symbol report under the same name: see dense_gemv_body).
 #if T3_CB == 0
 #define T3_CBNAME mul1
 #elif T3_CB == 1
@@ -687,9 +687,11 @@ cudaError_t T3_CAT(launch_dense_gemv_cb, T3_CB)(const DenseArgs& a, cudaStream_t
     const uint32_t rm = row_cap_for(a.rows);
     KernelFn<DenseArgs> fn = T3_PICK(T3_PICK_32, t3_dense_gemv, a.n, rm + a.tile_over);  // 33: 32_over
     const uint32_t cluster = a.part ? 1u : a.split;
-    return launch_cluster(fn, a, dim3(a.split, a.out / 128u, 1), cluster,
-                          gemv_smem_bytes(rm, a.rows, a.slice_max, cluster, a.n, a.ring, a.alone != 0, 1u, a.tile_over != 0),
-                          a.overlap != 0, stream);
+    const cudaError_t rc = launch_cluster(fn, a, dim3(a.split, a.out / 128u, 1), cluster,
+                                          gemv_smem_bytes(rm, a.rows, a.slice_max, cluster, a.n, a.ring, a.alone != 0, 1u, a.tile_over != 0),
+                                          a.overlap != 0, stream);
+    if (a.tile_over) note_symbol(reinterpret_cast<const void*>(T3_PICK(T3_PICK_32, t3_dense_gemv, a.n, rm)));
+    return rc;
 }
 
 #if T3_CB == 0
