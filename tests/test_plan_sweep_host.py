@@ -138,6 +138,22 @@ def test_launches_that_do_not_overlap_leave_room_for_another_streams():
     assert [p["grid"] for p in apart] == [p["grid"] for p in beside]
 
 
+def test_a_large_linear_keeps_its_multiprocessors_where_all_its_clusters_fit_so():
+    """Linears of 24 MB of codes and up: CTAs that all find a multiprocessor each are not placed two to one beside empty ones (5760 -> 17920 K4 at
+    one row once took 45.7 us for 30.7, by a ring that let two of them fit)."""
+    asked = 0
+    for i, o, n in itertools.product(range(2048, 16385, 640), range(2048, 24577, 640), (32, 48, 64, 80, 96, 128)):
+        if not _large(i, o, n) or i * o > 16384 * 7168:
+            continue
+        for rows in (1, 8, 16):
+            p = t3.plan_linear(rows, i, o, n)[-1]
+            fits = p["grid"][1] <= ONE_A_SM[p["cluster"]] if p["cluster"] > 1 else p["grid"][0] * p["grid"][1] <= 148
+            if fits:
+                asked += 1
+                assert p["shared"] > 113 * 1024, (rows, i, o, n, p)
+    assert asked > 1000
+
+
 def test_a_gate_up_launch_keeps_its_multiprocessors_only_where_all_its_clusters_fit_so():
     """CTAs that ask for more than half a multiprocessor's shared memory are one to a multiprocessor: no launch asks for that whose clusters
     do not all fit the device so (the ones left over would wait for a whole second round)."""

@@ -133,7 +133,7 @@ uint32_t largest_slice(uint32_t nb, uint32_t split) {
 
 // The ring of one GEMV CTA: stages of kStageRows tk rows (two 128-input blocks), as many as the slab needs or the budget
 // holds; three where the default budget holds fewer and two CTAs still fit a multiprocessor.
-bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan& ring, bool alone = false,
+bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cluster, uint32_t n, RingPlan& ring, uint32_t alone = 0,
                uint32_t buffers = 1, bool over = false) {
     const uint32_t row_bytes = 16u * n, nrows = slice_max / 16u;  // nrows is a multiple of 8 (whole 128-blocks)
     const uint32_t stage_rows = kStageRows;
@@ -142,12 +142,13 @@ bool plan_ring(uint32_t row_cap, uint32_t xrows, uint32_t slice_max, uint32_t cl
     const uint32_t fixed = gemv_smem(row_cap, xrows, slice_max, cluster, stage_bytes, 0, buffers, over).total;
     if (fixed + stage_bytes > kSmemCap) return false;
     uint32_t budget = g_cfg.ring_bytes ? g_cfg.ring_bytes : kDefaultRing;
-    if (!g_cfg.ring_bytes && !alone) {
-        // two CTAs a multiprocessor where three stages (or all there are) leave room for that
+    if (!g_cfg.ring_bytes) {
+        // three stages (or all there are), where two CTAs a multiprocessor leave room for that if it holds two; in a CTA that has its
+        // multiprocessor to itself for a large linear (9088 -> 5632 K8 at one row 22.3 -> 20.8 us; 1664 -> 6912 K8 at 32 rows 12.0 -> 12.4)
         const uint32_t least = (need < 3u ? need : 3u) * stage_bytes;
-        if (fixed + least <= kSmemHalf) {
+        if (alone == 2u || (alone == 0u && fixed + least <= kSmemHalf)) {
             if (budget < least) budget = least;
-            if (budget > kSmemHalf - fixed) budget = kSmemHalf - fixed;
+            if (alone == 0u && budget > kSmemHalf - fixed) budget = kSmemHalf - fixed;
         }
     }
     if (budget > kSmemCap - fixed) budget = kSmemCap - fixed;
@@ -494,6 +495,14 @@ int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
     }
     a.overlap = !cfg.no_overlap;
     a.slice_max = largest_slice(nb, a.split);
+    // A large linear's CTAs go one to a multiprocessor too where they all fit so (one row, us, two CTAs a multiprocessor / one: 3456 -> 15616 K4
+    // 31.4 / 19.2, 16384 -> 6272 K5, three slices, 60.6 / 35.1, 9984 -> 8576 K3, clusters of two, 47.3 / 29.2, 2688 -> 15232 K8 25.0 / 16.4)
+    auto place_large = [&] {
+        if (!large || !a.overlap || cfg.dense_split) return;
+        const uint32_t sms = one_wave() / 2u, blocks = a.out / 128u;
+        a.alone = (a.part ? a.split * blocks <= sms : blocks <= clusters_alone(sms, a.split)) ? 2u : 0u;
+    };
+    place_large();
     // A slice too long for shared memory (its prepared rows) is cut further, up to the widest cluster. Past 16 rows the partial-sum tile goes
     // over the rows where the ring would have less than two stages otherwise, or where two CTAs fit a multiprocessor only so; not a large
     // linear's, which is cut further (8704 -> 13312 K6 at 17 rows in two slices of one stage 108 us, in four 81).
@@ -504,13 +513,14 @@ int plan_dense(DenseArgs& a, const t3_config& cfg, bool global_ok) {
             return gemv_smem(rm, a.rows, a.slice_max, cluster, kStageRows * 16u * a.n, need < stages ? need : stages, 1u, over).total;
         };
         a.tile_over = rm == 32u && !large && a.slice_max >= kOverBlocks * 128u && (bytes(2u, false) > kSmemCap || (!a.alone && bytes(3u, false) > kSmemHalf && bytes(3u, true) <= kSmemHalf));
-        return plan_ring(rm, a.rows, a.slice_max, cluster, a.n, a.ring, a.alone != 0, 1u, a.tile_over != 0);
+        return plan_ring(rm, a.rows, a.slice_max, cluster, a.n, a.ring, a.alone, 1u, a.tile_over != 0);
     };
     while (!planned()) {
         if (a.part) {  // back to the cluster kernel
             a.part = nullptr;
             a.split = pick_split_large(nb, a.out / 128u);
             a.slice_max = largest_slice(nb, a.split);
+            place_large();
             continue;
         }
         a.alone = 0;
@@ -742,7 +752,7 @@ int plan_moe_decode(MoeArgs& a, const t3_config& cfg) {
     a.per_d = 1u;
     while (a.split_d == 1u && a.per_d < 8u && a.per_d * 2u <= a.hidden / 128u && touched * (a.hidden / 128u) / (2u * a.per_d) >= 10.0 * sms) a.per_d *= 2u;
     if (!plan_ring(rm, rm, a.slice_max_gu, 2u * a.split_gu, a.n, a.ring_gu) ||
-        !plan_ring(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d, false, a.per_d > 1u ? 2u : 1u))
+        !plan_ring(rm, rm, a.slice_max_d, a.split_d, a.n, a.ring_d, 0u, a.per_d > 1u ? 2u : 1u))
         return T3_ENGINE_NOT_IMPLEMENTED;
     // When gate|up lets the down launch start: at once (its CTAs then fetch their first codes beside gate|up's) or when its own codes
     // are all on the way. At once where gate|up leaves multiprocessors idle, unless down's CTAs would then double up on those while

@@ -32,7 +32,7 @@ struct DenseArgs {
     uint32_t* counters;       // with part: [out/128] arrivals a block, zero before the launch; the last arriver finishes the block
     uint32_t split;           // K slices (the cluster size unless `part` is set)
     uint32_t slice_max;       // inputs of the largest K slice
-    uint16_t alone;           // a CTA takes more than half a multiprocessor's shared memory (see kSmemAlone)
+    uint16_t alone;           // a CTA takes more than half a multiprocessor's shared memory (see kSmemAlone); 2: a large linear's
     uint16_t tile_over;       // row capacity 32: the K groups' partial-sum tile lies over the prepared rows (see gemv_smem)
     RingPlan ring;
     int overlap;              // launch with the programmatic-dependent-launch attribute
