@@ -457,10 +457,16 @@ struct DenseWs {
 // up to kFusedRows when a CTA's share of the work would be more than five rotations a warp (many rows on long K slices: each
 // CTA repeats the rotation of its whole slice for every row before its first tensor-core step). Ahead / in the CTA, us: 8192 -> 2048 at 4
 // rows (2.8 rotations a warp) 12.7 / 11.2, 6144 -> 2048 at 8 (4) 10.4 / 9.8, 8192 -> 2048 at 8 (5.5) 12.8 / 12.6, 4096 -> 8192 at 8 (8)
-// 15.8 / 16.9.
+// 15.8 / 16.9. Where CTAs share a multiprocessor, in one round, and rotate five rows and more, two a warp is the end: 640 -> 23040 K5 at 7 rows
+// (2.2) 11.7 / 12.1, 1280 -> 22272 K5 at 8 (5) 18.9 / 20.5, 2560 -> 11776 K4 at 8 (5) 17.0 / 18.6, in all 59 shapes of the kind measured; at
+// three and four rows, and in several rounds, as many are slower ahead (10368 -> 8576 K2 at 3 41.5 / 38.8), and clusters of eight and more find worse
+// places behind another launch (6016 -> 4224 K8 at 8, 33 of them, 18.0 / 14.7).
 // On the global exchange always: the launch clears the blocks' arrival counters too (a memset ahead of the GEMV ended its overlap with
 // the stream's previous kernel: 16384 -> 7168 at one row 37.2 us, 34.8 without it).
-bool prep_ahead(const DenseArgs& a) { return a.part || a.rows > kFusedRows || a.rows * (a.slice_max / 128u) > 5u * kConsumerWarps; }
+bool prep_ahead(const DenseArgs& a) {
+    const bool shared = !a.alone && a.overlap && a.rows >= 5u && a.split < 8u && a.split * (a.out / 128u) <= one_wave();
+    return a.part || a.rows > kFusedRows || a.rows * (a.slice_max / 128u) > (shared ? 2u : 5u) * kConsumerWarps;
+}
 
 DenseWs dense_ws(uint32_t rows, uint32_t in, uint32_t out, uint32_t global_split, bool ahead) {
     DenseWs w;
